@@ -851,7 +851,7 @@ def main():
         traffic = NCU_DRAM_BYTES_PER_CELL_STAGE[(args.config, path_used)] * T * K_rk
     chain = {"fused": "K x [k_node(boundary-cell vertices) -> k_grad(boundary cells) -> k_bc || k_tile, k_flux_bc]",
              "fused-node-kernel": "K x [k_node, k_grad(boundary cells) -> k_bc || k_tile, k_flux_bc]",
-             "phases": "K x [k_node, k_grad, k_bc || k_eflux, k_flux, k_flux_bc]"}[path_used]
+             "phases": "K x [k_node, k_grad, k_bc || k_cell, k_flux_bc]"}[path_used]
     roofline = {
         "bound": "hbm", "achieved": achieved, "peak": pk.get("hbm_gbs"), "unit": "GB/s",
         "frac": achieved / pk["hbm_gbs"], "traffic": traffic,
@@ -876,7 +876,7 @@ def main():
                 "steps": e2e_steps},
         "gpu_launches": gpu_launches,
         "stage_kernels": path_used,
-        "block_sizes": tuned if tuned is not None else "library defaults (node 128, grad 64, eflux 64 FP64 / 128 mixed, flux 64)",
+        "block_sizes": tuned if tuned is not None else "library defaults (node 128, grad 64)",
         "setup": setup,
         "roofline": roofline,
         "clocks": clk.summary(),

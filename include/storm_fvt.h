@@ -336,28 +336,29 @@ STORM_FVT_API int storm_fvt_last_timing(const StormFvtHandle* hd, double* step_m
                           double* flux_kernel_ms, int64_t* flux_kernel_launches);
 
 /* Per-kernel device time (ms) and launch counts of the last storm_fvt_step call in
- * kernel timing mode, indexed 0 node (vertex depth), 1 grad (gradients/limiter),
- * 2 bc (open boundaries), 3 flux (per-cell gather of the face fluxes + sources + RK
- * update), 4 fric (friction and reduction partials), 5 final (iteration scalars),
- * 6 eflux (interior-edge fluxes), 7 tile (the fused stage kernel).  On the fused path
- * 1 and 3 time the boundary cells' gradient and update kernels only. */
+ * kernel timing mode, indexed 0 node (vertex depth), 1 grad (gradients/limiter and the
+ * face states), 2 bc (open boundaries), 3 flux (edge fluxes, sources, RK update and, in
+ * an FP64 iteration's last stage, the friction step), 4 fric (friction and reduction
+ * partials where they have a kernel of their own), 5 final (iteration scalars), 6 unused,
+ * 7 tile (the fused stage kernel).  On the fused path 1 and 3 time the boundary cells'
+ * gradient and update kernels only. */
 STORM_FVT_API int storm_fvt_kernel_times(const StormFvtHandle* hd, double* ms, int64_t* launches);
 
 /* Project autotuner: first times `iters` whole iterations of each stage path
  * (storm_fvt_set_stage_path) and keeps the fastest, then times `iters` iterations per
- * candidate block size of the node, gradient, edge-flux and cell kernels on this
- * handle's meshes (per-kernel CUDA events) and keeps the fastest of each;
- * re-captures the iteration graph and restores the state it started from.  `chosen`
- * (may be NULL) receives the four sizes; storm_fvt_stage_path reports the path. */
+ * candidate block size of the node and gradient kernels on this handle's meshes
+ * (per-kernel CUDA events) and keeps the fastest of each; re-captures the iteration
+ * graph and restores the state it started from.  `chosen` (may be NULL) receives four
+ * sizes: node, gradient, and twice the cell slots of a block of the cell kernel;
+ * storm_fvt_stage_path reports the path. */
 STORM_FVT_API int storm_fvt_autotune(StormFvtHandle* hd, int32_t iters, int32_t* chosen);
 
 /* Stage kernels of the captured iteration.  No counterpart in the reference (it
  * selects how this library schedules the same arithmetic; FP64 results are bitwise
  * the same either way, mixed-precision ones agree to within that path's own error,
  * its FP32 kernels being compiled with FMA contraction):
- *   STORM_STAGE_PHASES  k_node, k_grad, k_eflux, k_flux per stage (gradients and edge
- *                       fluxes pass through device memory between the kernels);
- *                       the default;
+ *   STORM_STAGE_PHASES  k_node, k_grad, k_cell per stage (face states pass through device
+ *                       memory between the last two); the default;
  *   STORM_STAGE_FUSED   one fused kernel per stage over Morton tiles of 256 cells
  *                       (vertex depths, gradients, edge fluxes and the RK update of a
  *                       tile in shared memory);

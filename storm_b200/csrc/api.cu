@@ -9,6 +9,7 @@
 
 #include <algorithm>
 #include <climits>
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <new>
@@ -47,8 +48,8 @@ struct StormFvtHandle {
   std::vector<uint8_t> have_scen_state;
   int device = 0;
   cudaStream_t stream = nullptr;
-  cudaStream_t side = nullptr;       // boundary kernel, overlapped with k_flux
-  cudaEvent_t fork_ev[4] = {}, join_ev[4] = {}, eflux_ev[4] = {};
+  cudaStream_t side = nullptr;       // boundary kernel, overlapped with the cells' kernels
+  cudaEvent_t fork_ev[4] = {}, join_ev[4] = {}, eflux_ev[4] = {}, gen_ev[4] = {};
   void* arena = nullptr;
   void* arena32 = nullptr;  // FP32 geometry copies (mixed precision only)
   Dev d{};
@@ -73,7 +74,9 @@ struct StormFvtHandle {
   // block sizes of the stage kernels (storm_fvt_autotune picks them)
   // block sizes of the node, gradient, edge-flux and cell kernels: the autotuner's
   // choice on the 2M meander (FP64; the mixed path takes 128 for the edge fluxes)
-  int bs_node = 128, bs_grad = 64, bs_eflux = 64, bs_flux = 64;
+  int bs_node = 128, bs_grad = 64;
+  size_t cell_smem = 0;  // k_cell's dynamic shared memory
+  int n_sm = 148;
   // output pass (storm_fvt_output_vertices): device buffers, allocated at first use
   void* out_buf = nullptr;
   size_t out_bytes = 0;
@@ -96,7 +99,7 @@ struct StormFvtHandle {
   void* xchg_buf = nullptr;
   int32_t *send_slots = nullptr, *recv_slots = nullptr;
   int n_send = 0, n_recv = 0;
-  double *u_a2 = nullptr, *v_a2 = nullptr;
+  Rec* q2 = nullptr;  // the fused path's second state buffer
 };
 
 namespace {
@@ -164,8 +167,9 @@ int enqueue_step(StormFvtHandle* h, bool timing, size_t* fev_used, int only = -1
   const Dev& d = h->d;
   const int T = d.T, K = d.K;
   const int gT = (T + h->bs_grad - 1) / h->bs_grad;
-  const int gF = (T + h->bs_flux - 1) / h->bs_flux;
-  const int gE = (d.ne + h->bs_eflux - 1) / h->bs_eflux;
+  const int gG = (d.ngen + 31) / 32;  // cells off the common stencil: one warp to a block, spread over the SMs
+  const int gC = T / kRed;  // k_cell: one block per reduction block of cell slots
+  const int bC = gC <= h->n_sm ? 512 : 256;
   // in timing mode every launch is bracketed by an event pair tagged with its class
   auto mark = [&](int cls) -> int {
     if (!timing) return 0;
@@ -185,10 +189,14 @@ int enqueue_step(StormFvtHandle* h, bool timing, size_t* fev_used, int only = -1
   // residual smoothing and linked partitions
   const bool fused = h->tiles_ok && h->want_tiles && !linked && d.ncv == 0 && !rs;
   h->use_tiles = fused;
-  const double *u_in = d.u_a, *v_in = d.v_a;
-  double *u_out = d.u_a, *v_out = d.v_a;
-  auto launch = [&](int which, int grid, int block, size_t smem, cudaStream_t st, int s, const double* hs,
-                    uint8_t* dry, uint8_t* dry_next) {
+  const Rec* q = d.q;
+  Rec* qo = d.q;
+  // whole FP64 iterations on the phase path: the last stage's cell kernels do the friction
+  // step too (parts of a mesh and smoothed residuals have it in a kernel of its own, and
+  // so has the mixed path, whose cell kernels are compiled with FMA contraction)
+  const bool fric_fused = !fused && only < 0 && !linked && d.nhalo == 0 && !rs && !h->mixed;
+  int mode = CELL_UPDATE;
+  auto launch = [&](int which, int grid, int block, size_t smem, cudaStream_t st, int s) {
     StageLaunch L;
     L.which = which;
     L.grid = dim3(grid);
@@ -196,35 +204,26 @@ int enqueue_step(StormFvtHandle* h, bool timing, size_t* fev_used, int only = -1
     L.smem = smem;
     L.stream = st;
     L.s = s;
-    L.hs = hs;
-    L.dry = dry;
-    L.dry_next = dry_next;
+    L.mode = mode;
     L.rku_prev = d.rku + (size_t)(s - 1) * T;
     L.rkv_prev = d.rkv + (size_t)(s - 1) * T;
-    L.u_in = u_in;
-    L.v_in = v_in;
-    L.u_out = u_out;
-    L.v_out = v_out;
+    L.q = q;
+    L.qo = qo;
     L.tiles = &h->td;
     launch_stage(L, d, h->gd, h->gf, h->mixed);
   };
   if (only < 0 && linked && !d.steady && d.dt_op != 0) launch_link_dt(d, h->stream);
   for (int s = 1; s <= K; s++) {
-    const double* hs = d.rkh + (size_t)(s - 1) * T;
-    uint8_t* dry = (s & 1) ? d.dry_a : d.dry_b;
-    uint8_t* dry_next = (s & 1) ? d.dry_b : d.dry_a;
     const int gB = (d.nbc_cells + kFluxThreads - 1) / kFluxThreads;
-    if (fused) {  // stage s reads one velocity buffer and writes the other
-      u_in = (s & 1) ? d.u_a : h->u_a2;
-      v_in = (s & 1) ? d.v_a : h->v_a2;
-      u_out = (s & 1) ? h->u_a2 : d.u_a;
-      v_out = (s & 1) ? h->v_a2 : d.v_a;
+    if (fused) {  // stage s reads one state buffer and writes the other
+      q = (s & 1) ? d.q : h->q2;
+      qo = (s & 1) ? h->q2 : d.q;
     }
     if (only >= 0 && s != only) continue;
     const bool tile_nodes = fused && h->td.nodes;
     if (!tile_nodes) {
       if (mark(KT_NODE)) return STORM_ERR_CUDA;
-      launch_node(d, hs, dry, nullptr, 0, h->bs_node, h->stream);
+      launch_node(d, q, nullptr, 0, !fused, s == K, h->bs_node, h->stream);
       if (done()) return STORM_ERR_CUDA;
     }
     if (fused) {
@@ -235,73 +234,85 @@ int enqueue_step(StormFvtHandle* h, bool timing, size_t* fev_used, int only = -1
         // cells once both are done
         CK(cudaEventRecord(h->fork_ev[s], h->stream));
         CK(cudaStreamWaitEvent(h->side, h->fork_ev[s], 0));
-        if (tile_nodes) launch_node(d, hs, dry, h->bc_nodes, h->n_bc_nodes, 128, h->side);
-        launch(STAGE_GRAD_BC, gB, kFluxThreads, 0, h->side, s, hs, dry, dry_next);
-        if (d.nbdr > 0) launch(STAGE_BC, d.nbdr, 128, h->bc_smem, h->side, s, hs, dry, dry_next);
+        if (tile_nodes) launch_node(d, q, h->bc_nodes, h->n_bc_nodes, false, true, 128, h->side);
+        launch(STAGE_GRAD_BC, gB, kFluxThreads, 0, h->side, s);
+        if (d.nbdr > 0) launch(STAGE_BC, d.nbdr, 128, h->bc_smem, h->side, s);
         CK(cudaEventRecord(h->join_ev[s], h->side));
-        launch(STAGE_TILE, nt, kTileThreadsHost, h->tile_smem, h->stream, s, hs, dry, dry_next);
+        launch(STAGE_TILE, nt, kTileThreadsHost, h->tile_smem, h->stream, s);
         CK(cudaStreamWaitEvent(h->stream, h->join_ev[s], 0));
-        launch(STAGE_FLUX_BC, gB, kFluxThreads, 0, h->stream, s, hs, dry, dry_next);
+        launch(STAGE_FLUX_BC_TILE, gB, kFluxThreads, 0, h->stream, s);
       } else {
         if (gB > 0) {
           if (tile_nodes) {
             if (mark(KT_NODE)) return STORM_ERR_CUDA;
-            launch_node(d, hs, dry, h->bc_nodes, h->n_bc_nodes, 128, h->stream);
+            launch_node(d, q, h->bc_nodes, h->n_bc_nodes, false, true, 128, h->stream);
             if (done()) return STORM_ERR_CUDA;
           }
           if (mark(KT_GRAD)) return STORM_ERR_CUDA;
-          launch(STAGE_GRAD_BC, gB, kFluxThreads, 0, h->stream, s, hs, dry, dry_next);
+          launch(STAGE_GRAD_BC, gB, kFluxThreads, 0, h->stream, s);
           if (done()) return STORM_ERR_CUDA;
           if (d.nbdr > 0) {
             if (mark(KT_BC)) return STORM_ERR_CUDA;
-            launch(STAGE_BC, d.nbdr, 128, h->bc_smem, h->stream, s, hs, dry, dry_next);
+            launch(STAGE_BC, d.nbdr, 128, h->bc_smem, h->stream, s);
             if (done()) return STORM_ERR_CUDA;
           }
         }
         if (mark(KT_TILE)) return STORM_ERR_CUDA;
-        launch(STAGE_TILE, nt, kTileThreadsHost, h->tile_smem, h->stream, s, hs, dry, dry_next);
+        launch(STAGE_TILE, nt, kTileThreadsHost, h->tile_smem, h->stream, s);
         if (done()) return STORM_ERR_CUDA;
         if (gB > 0) {
           if (mark(KT_FLUX)) return STORM_ERR_CUDA;
-          launch(STAGE_FLUX_BC, gB, kFluxThreads, 0, h->stream, s, hs, dry, dry_next);
+          launch(STAGE_FLUX_BC_TILE, gB, kFluxThreads, 0, h->stream, s);
           if (done()) return STORM_ERR_CUDA;
         }
       }
       continue;
     }
-    if (mark(KT_GRAD)) return STORM_ERR_CUDA;
-    launch(STAGE_GRAD, gT, h->bs_grad, 0, h->stream, s, hs, dry, dry_next);
-    if (d.ncv > 0) launch(STAGE_CULVERT, (d.ncv + 127) / 128, 128, 0, h->stream, s, hs, dry, dry_next);
-    if (done()) return STORM_ERR_CUDA;
-    const int sF = rs ? STAGE_PHI : STAGE_FLUX, sFB = rs ? STAGE_PHI_BC : STAGE_FLUX_BC;
-    if (d.nbdr > 0 && !timing) {
-      // k_bc on the side stream overlaps k_eflux; the cells with an open-boundary face
-      // (k_flux_bc: their own values, the edge fluxes and k_bc's contributions) are
-      // then finished on the side stream beside k_flux of all the other cells
-      CK(cudaEventRecord(h->fork_ev[s], h->stream));
-      CK(cudaStreamWaitEvent(h->side, h->fork_ev[s], 0));
-      launch(STAGE_BC, d.nbdr, 128, h->bc_smem, h->side, s, hs, dry, dry_next);
-      if (gE > 0) launch(STAGE_EFLUX, gE, h->bs_eflux, 0, h->stream, s, hs, dry, dry_next);
-      CK(cudaEventRecord(h->eflux_ev[s], h->stream));
-      CK(cudaStreamWaitEvent(h->side, h->eflux_ev[s], 0));
-      if (gB > 0) launch(sFB, gB, kFluxThreads, 0, h->side, s, hs, dry, dry_next);
-      CK(cudaEventRecord(h->join_ev[s], h->side));
-      launch(sF, gF, h->bs_flux, 0, h->stream, s, hs, dry, dry_next);
-      CK(cudaStreamWaitEvent(h->stream, h->join_ev[s], 0));
+    mode = rs ? CELL_PHI : fric_fused && s == K ? CELL_FRIC : CELL_UPDATE;
+    if (!timing) {
+      // the cells along the mesh boundary, the open-boundary kernel that needs only
+      // those, and then the update of the cells with an open-boundary face (their own
+      // values, the edge fluxes and k_bc's contributions) run on the side stream beside
+      // the kernels of all the other cells
+      if (gG > 0) {
+        CK(cudaEventRecord(h->fork_ev[s], h->stream));
+        CK(cudaStreamWaitEvent(h->side, h->fork_ev[s], 0));
+        launch(STAGE_GRAD_GEN, gG, 32, 0, h->side, s);
+        CK(cudaEventRecord(h->gen_ev[s], h->side));
+      }
+      launch(STAGE_GRAD, gT, h->bs_grad, 0, h->stream, s);
+      if (gG > 0) {
+        CK(cudaStreamWaitEvent(h->stream, h->gen_ev[s], 0));
+      } else if (d.nbdr > 0) {  // k_bc's cells are among k_grad's
+        CK(cudaEventRecord(h->fork_ev[s], h->stream));
+        CK(cudaStreamWaitEvent(h->side, h->fork_ev[s], 0));
+      }
+      const bool forked = gG > 0 || d.nbdr > 0;
+      if (d.ncv > 0) launch(STAGE_CULVERT, (d.ncv + 127) / 128, 128, 0, h->stream, s);
+      if (d.nbdr > 0) launch(STAGE_BC, d.nbdr, 128, h->bc_smem, h->side, s);
+      if (gB > 0) {
+        // the neighbours' face records (k_grad), the culverts
+        CK(cudaEventRecord(h->eflux_ev[s], h->stream));
+        CK(cudaStreamWaitEvent(h->side, h->eflux_ev[s], 0));
+        launch(STAGE_FLUX_BC, gB, kFluxThreads, 0, h->side, s);
+      }
+      if (forked) CK(cudaEventRecord(h->join_ev[s], h->side));
+      launch(STAGE_CELL, gC, bC, h->cell_smem, h->stream, s);
+      if (forked) CK(cudaStreamWaitEvent(h->stream, h->join_ev[s], 0));
     } else {
+      if (mark(KT_GRAD)) return STORM_ERR_CUDA;
+      if (gG > 0) launch(STAGE_GRAD_GEN, gG, 32, 0, h->stream, s);
+      launch(STAGE_GRAD, gT, h->bs_grad, 0, h->stream, s);
+      if (d.ncv > 0) launch(STAGE_CULVERT, (d.ncv + 127) / 128, 128, 0, h->stream, s);
+      if (done()) return STORM_ERR_CUDA;
       if (d.nbdr > 0) {
         if (mark(KT_BC)) return STORM_ERR_CUDA;
-        launch(STAGE_BC, d.nbdr, 128, h->bc_smem, h->stream, s, hs, dry, dry_next);
-        if (done()) return STORM_ERR_CUDA;
-      }
-      if (gE > 0) {
-        if (mark(KT_EFLUX)) return STORM_ERR_CUDA;
-        launch(STAGE_EFLUX, gE, h->bs_eflux, 0, h->stream, s, hs, dry, dry_next);
+        launch(STAGE_BC, d.nbdr, 128, h->bc_smem, h->stream, s);
         if (done()) return STORM_ERR_CUDA;
       }
       if (mark(KT_FLUX)) return STORM_ERR_CUDA;
-      launch(sF, gF, h->bs_flux, 0, h->stream, s, hs, dry, dry_next);
-      if (gB > 0) launch(sFB, gB, kFluxThreads, 0, h->stream, s, hs, dry, dry_next);
+      launch(STAGE_CELL, gC, bC, h->cell_smem, h->stream, s);
+      if (gB > 0) launch(STAGE_FLUX_BC, gB, kFluxThreads, 0, h->stream, s);
       if (done()) return STORM_ERR_CUDA;
     }
     if (rs) {  // solverFVT.f90:238-256, then the update of every cell
@@ -310,21 +321,23 @@ int enqueue_step(StormFvtHandle* h, bool timing, size_t* fev_used, int only = -1
       for (int k = 0; k < h->opt.rsavg_passes; k++)
         for (size_t c = 0; c + 1 < Lm.rs_off.size(); c++)
           launch_rsavg(d, Lm.rs_off[c], Lm.rs_off[c + 1] - Lm.rs_off[c], h->stream);
-      launch(STAGE_UPDATE, (T + 127) / 128, 128, 0, h->stream, s, hs, dry, dry_next);
+      launch(STAGE_UPDATE, (T + 127) / 128, 128, 0, h->stream, s);
       if (done()) return STORM_ERR_CUDA;
     }
     // halo cells of linked partitions take their owners' new level and flags
-    if (linked && d.nhalo > 0 && s < K) launch_halo(d, s, dry_next, nullptr, h->stream);
+    if (linked && d.nhalo > 0 && s < K) launch_halo(d, s, nullptr, h->stream);
   }
   if (only > 0) {
     CK(cudaGetLastError());
     return 0;
   }
   if (linked && d.steady) launch_link_fric(d, h->stream);
-  if (mark(KT_FRIC)) return STORM_ERR_CUDA;
-  launch_fric(d, u_out, v_out, h->stream);
-  if (done()) return STORM_ERR_CUDA;
-  if (linked && d.nhalo > 0) launch_halo(d, 0, d.dry_a, d.dry_out, h->stream);
+  if (!fric_fused) {
+    if (mark(KT_FRIC)) return STORM_ERR_CUDA;
+    launch_fric(d, qo, h->stream);
+    if (done()) return STORM_ERR_CUDA;
+  }
+  if (linked && d.nhalo > 0) launch_halo(d, 0, d.dry_out, h->stream);
   if (mark(KT_FINAL)) return STORM_ERR_CUDA;
   k_final<<<d.nscen, kFinalThreadsHost, 0, h->stream>>>(d);
   if (done()) return STORM_ERR_CUDA;
@@ -364,6 +377,7 @@ void release(StormFvtHandle* h) {
     if (h->fork_ev[i]) cudaEventDestroy(h->fork_ev[i]);
     if (h->join_ev[i]) cudaEventDestroy(h->join_ev[i]);
     if (h->eflux_ev[i]) cudaEventDestroy(h->eflux_ev[i]);
+    if (h->gen_ev[i]) cudaEventDestroy(h->gen_ev[i]);
   }
   if (h->side) cudaStreamDestroy(h->side);
   if (h->stream) cudaStreamDestroy(h->stream);
@@ -489,7 +503,15 @@ int upload(StormFvtHandle* h) {
   size_t o_cvry = cpy(L.cv_ry, ncv), o_cvz = cpy(L.cv_zinv, ncv), o_cvh = cpy(L.cv_head, ncvt);
   size_t o_cvq = cpy(L.cv_q, ncvt), o_cvcc = cpy(L.cvc_cell, ncvc), o_cvco = cpy(L.cvc_code, ncvc);
   size_t o_cvsrc = A.take(sizeof(double) * ncv);
-  size_t o_nst = cpy(L.nst, T), o_ford = cpy(L.forder, T), o_hvm = cpy(L.hvmask, T), o_fk = cpy(L.fkind, T3);
+  // k_grad's common path; first order reads no stencil, so every cell is on it
+  auto common = [&](size_t c) {
+    return h->opt.opt_limiter == 0 || (L.plain[c] && !(L.forder[c] & kOrderHasBc));
+  };
+  std::vector<uint8_t> nst = L.nst, last(T, 0);
+  for (const ScenarioInfo& I : h->info) last[I.last_cell] = 1;
+  for (size_t c = 0; c < (size_t)T; c++)
+    nst[c] |= (uint8_t)((common(c) ? kNstPlain : 0) | (last[c] ? kNstLast : 0) | ((L.forder[c] & kOrderHasBc) ? kNstBc : 0));
+  size_t o_nst = cpy(nst, T), o_ford = cpy(L.forder, T), o_hvm = cpy(L.hvmask, T), o_fk = cpy(L.fkind, T3);
   // face kinds and references in summation order (static; see Dev::fko)
   std::vector<uint16_t> fko(T, 0);
   std::vector<int32_t> frefo(T3, 0);
@@ -499,6 +521,83 @@ int upload(StormFvtHandle* h) {
       fko[c] |= (uint16_t)((L.fkind[(size_t)j * T + c] & 7) << (3 * t));
       frefo[(size_t)t * T + c] = L.fref[(size_t)j * T + c];
     }
+  // stage-boundary slot of a node, -2 for the other ends of wall edges (whose depth the
+  // wall fluxes read), -1 for the rest
+  std::vector<int16_t> node_code = L.node_hbc;
+  for (int32_t w = 0; w < L.nwall; w++)
+    for (int32_t n : {L.wall_p1[w], L.wall_p2[w]})
+      if (node_code[n] == -1) node_code[n] = -2;
+  // face records (see Dev::fs): interior edges' two sides, and walls where they slip
+  std::vector<int32_t> fpos(T3, -1);
+  for (size_t q = 0; q < T3; q++) {
+    const int kind = L.fkind[q] & 7;
+    if (kind == FACE_LEFT || kind == FACE_RIGHT) fpos[q] = 2 * L.fref[q] + (kind == FACE_RIGHT);
+    else if (kind == FACE_WALL && h->opt.btype == 1) fpos[q] = 2 * L.ne + L.fref[q];
+  }
+  const size_t nrec = 2 * (size_t)L.ne + (h->opt.btype == 1 ? (size_t)L.nwall : 0);
+  // k_cell's work lists (edges are sorted by their smaller slot), and per cell its faces'
+  // places in them
+  const int32_t nct = T / kRed;
+  std::vector<CellTile> ct(nct, CellTile{});
+  std::vector<std::vector<int32_t>> back(nct);
+  for (int32_t e = 0; e < L.ne; e++) {
+    const int32_t a = std::min(L.eL[e], L.eR[e]) / kRed, b = std::max(L.eL[e], L.eR[e]) / kRed;
+    if (ct[a].nr == 0) ct[a].er0 = e;
+    ct[a].nr++;
+    if (b != a) back[b].push_back(e);
+  }
+  std::vector<int32_t> cbe;
+  int32_t cne_max = 1, cnw_max = 1;
+  for (int32_t t = 0; t < nct; t++) {
+    ct[t].boff = (int32_t)cbe.size();
+    ct[t].nb = (int32_t)back[t].size();
+    cbe.insert(cbe.end(), back[t].begin(), back[t].end());
+    cne_max = std::max(cne_max, ct[t].nr + ct[t].nb);
+  }
+  std::vector<WallRec> walls;
+  std::vector<int32_t> wall_at(std::max(L.nwall, 1), 0);
+  for (size_t c = 0; c < (size_t)T; c++)
+    for (int j = 0; j < 3; j++) {
+      const size_t q = (size_t)j * T + c;
+      if ((L.fkind[q] & 7) != FACE_WALL) continue;
+      const int32_t w = L.fref[q];
+      CellTile& k = ct[c / kRed];
+      if (k.nw == 0) k.w0 = (int32_t)walls.size();
+      wall_at[w] = k.nw++;
+      cnw_max = std::max(cnw_max, k.nw);
+      walls.push_back({L.fnx[q], L.fny[q], L.flen[q], L.wall_p1[w], L.wall_p2[w], (int32_t)c, 2 * L.ne + w});
+    }
+  std::vector<uint32_t> fdesc(T, 0);
+  std::vector<uint16_t> lfe(T3, 0);
+  std::vector<float> rad(T, 0.0f);
+  for (size_t c = 0; c < (size_t)T; c++) {
+    fdesc[c] = L.forder[c] | ((uint32_t)fko[c] << 8) | (L.cell_sid[c] >= 0 ? kDescReal : 0);
+    const CellTile& k = ct[c / kRed];
+    double r = 0.0;
+    for (int t = 0; t < 3; t++) {
+      const size_t q = (size_t)((L.forder[c] >> (2 * t)) & 3) * T + c;
+      const int kind = L.fkind[q] & 7;
+      const int32_t e = L.fref[q];
+      if (kind == FACE_LEFT || kind == FACE_RIGHT) {
+        if (e >= k.er0 && e < k.er0 + k.nr) {
+          lfe[(size_t)t * T + c] = (uint16_t)(e - k.er0);
+        } else {
+          const auto b0 = cbe.begin() + k.boff, b1 = b0 + k.nb;  // increasing
+          lfe[(size_t)t * T + c] = (uint16_t)(k.nr + (std::lower_bound(b0, b1, e) - b0));
+        }
+      } else if (kind == FACE_WALL) {
+        lfe[(size_t)t * T + c] = (uint16_t)wall_at[e];
+      }
+      const int32_t v = L.vert[(size_t)t * T + c];
+      r = std::max({r, std::fabs(L.node_x[v] - L.xc[c]), std::fabs(L.node_y[v] - L.yc[c])});
+    }
+    rad[c] = std::nextafter((float)r, INFINITY);
+  }
+  size_t o_ct = cpy(ct, nct), o_cbe = cpy(cbe, std::max<size_t>(cbe.size(), 1));
+  size_t o_walls = cpy(walls, std::max<size_t>(walls.size(), 1)), o_fdesc = cpy(fdesc, T), o_lfe = cpy(lfe, T3);
+  size_t o_rad = cpy(rad, T), o_ccol = A.take(9 * kCellCols * sizeof(CellCol)), o_bcp = A.take(8 * 5 * std::max<size_t>(L.bc_cells.size(), 1));
+  const size_t gblk_bytes = (((size_t)T + 31) / 32) * (h->mixed ? sizeof(GradBlock<float>) : sizeof(GradBlock<double>));
+  size_t o_fpos = cpy(fpos, T3), o_fs = A.take(sizeof(Rec) * std::max<size_t>(nrec, 1)), o_gblk = A.take(gblk_bytes);
   size_t o_fko = cpy(fko, T), o_frefo = cpy(frefo, T3);
   size_t o_vert = cpy(L.vert, T3), o_t3 = cpy(L.t2t3, T3), o_fref = cpy(L.fref, T3), o_sid = cpy(L.st_id, TK);
   size_t o_rcx = cpy(L.rc_x, T3), o_rcy = cpy(L.rc_y, T3), o_fnx = cpy(L.fnx, T3), o_fny = cpy(L.fny, T3);
@@ -506,7 +605,7 @@ int upload(StormFvtHandle* h) {
   size_t o_sw = cpy(L.st_w, TK), o_sdx = cpy(L.st_dx, TK), o_sdy = cpy(L.st_dy, TK);
   size_t o_wp1 = cpy(L.wall_p1, nwall), o_wp2 = cpy(L.wall_p2, nwall);
   size_t o_zv = cpy(L.zvtx, N), o_nx = cpy(L.node_x, N), o_ny = cpy(L.node_y, N), o_n2w = cpy(L.n2t_w, nnz);
-  size_t o_n2o = cpy(L.n2t_off, (size_t)N + 1), o_n2c = cpy(L.n2t_cell, nnz), o_nh = cpy(L.node_hbc, N);
+  size_t o_n2o = cpy(L.n2t_off, (size_t)N + 1), o_n2c = cpy(L.n2t_cell, nnz), o_nh = cpy(node_code, N);
   size_t o_bk = cpy(L.bdr_kind, nbdr), o_bs = cpy(L.bdr_slot, nbdr), o_bo = cpy(L.bdr_off, nbdr);
   size_t o_bcn = cpy(L.bdr_cnt, nbdr), o_bcc = cpy(L.bce_cell, nbce), o_bcs = cpy(L.bce_slot, nbce);
   size_t o_bnx = cpy(L.bce_nx, nbce), o_bny = cpy(L.bce_ny, nbce), o_btx = cpy(L.bce_tx, nbce);
@@ -514,6 +613,10 @@ int upload(StormFvtHandle* h) {
   size_t o_tst = cpy(L.ts_t, nts), o_tsv = cpy(L.ts_v, nts);
   size_t o_csid = cpy(L.cell_sid, T), o_nsid = cpy(L.node_sid, N);
   size_t o_esid = cpy(L.edge_sid, std::max(L.ne, 1)), o_bsid = cpy(L.bdr_sid, nbdr);
+  std::vector<int32_t> gen;
+  for (int32_t c = 0; c < T; c++)
+    if (L.cell_sid[c] >= 0 && !common(c)) gen.push_back(c);
+  size_t o_gen = cpy(gen, std::max<size_t>(gen.size(), 1));
   size_t o_bcl = cpy(L.bc_cells, std::max<size_t>(L.bc_cells.size(), 1));
   const bool rsavg = h->opt.rsavg_passes > 0;
   size_t o_rsc = cpy(L.rs_cells, std::max<size_t>(L.rs_cells.size(), 1));
@@ -537,12 +640,12 @@ int upload(StormFvtHandle* h) {
   // state
   const size_t TL = (size_t)(K + 1) * T;
   size_t o_rkh = A.take(8 * TL), o_rku = A.take(8 * TL), o_rkv = A.take(8 * TL);
-  size_t o_ua = A.take(8 * (size_t)T), o_va = A.take(8 * (size_t)T), o_vz = A.take((size_t)T);
-  size_t o_ub = h->mixed ? A.take(8 * (size_t)T) : 0, o_vb = h->mixed ? A.take(8 * (size_t)T) : 0;
-  size_t o_ua2 = A.take(8 * (size_t)T), o_va2 = A.take(8 * (size_t)T);
+  size_t o_q = A.take(sizeof(Rec) * (size_t)T), o_q2 = A.take(sizeof(Rec) * (size_t)T);
+  size_t o_io = A.take(8 * 2 * (size_t)T), o_cm = A.take(T), o_fdry = A.take(T);
+  size_t o_ub = A.take(8 * (size_t)T), o_vb = A.take(8 * (size_t)T);
   size_t o_g[6];
   for (int i = 0; i < 6; i++) o_g[i] = A.take(8 * (size_t)T);
-  size_t o_dra = A.take(T), o_drb = A.take(T), o_hv = A.take(8 * (size_t)N), o_vw = A.take(N);
+  size_t o_hv = A.take(8 * (size_t)N), o_vw = A.take(N);
   size_t o_dro = A.take(T);
   size_t o_pm = A.take(8 * (size_t)T), o_bcc3 = A.take(8 * 3 * nbce), o_rec = A.take(8 * 3 * nbce);
   size_t o_part = A.take(8 * 8 * (size_t)nblk), o_sc = A.take(sizeof(Scalars) * (size_t)h->nscen);
@@ -607,15 +710,19 @@ int upload(StormFvtHandle* h) {
   d.nscen = h->nscen;
   d.t_real = h->nscen == 1 ? h->info[0].cell_cnt : T;
   d.lsq_derived = L.lsq_derived ? 1 : 0;
+  d.node_quick = 1;
+  for (double w : L.n2t_w)
+    if (!(w > 0.0 && w < 1.0e300)) d.node_quick = 0;
   d.rkh = at<double>(B, o_rkh); d.rku = at<double>(B, o_rku); d.rkv = at<double>(B, o_rkv);
-  d.u_a = at<double>(B, o_ua); d.v_a = at<double>(B, o_va); d.vzero = at<uint8_t>(B, o_vz);
-  d.u_b = h->mixed ? at<double>(B, o_ub) : nullptr;
-  d.v_b = h->mixed ? at<double>(B, o_vb) : nullptr;
-  h->u_a2 = at<double>(B, o_ua2); h->v_a2 = at<double>(B, o_va2);
+  d.q = at<Rec>(B, o_q); d.io = at<double>(B, o_io); d.cmark = at<uint8_t>(B, o_cm);
+  d.fdry = at<uint8_t>(B, o_fdry);
+  d.u_b = at<double>(B, o_ub); d.v_b = at<double>(B, o_vb);
+  d.fs = at<Rec>(B, o_fs); d.fpos = at<int32_t>(B, o_fpos); d.gblk = at<unsigned char>(B, o_gblk);
+  h->q2 = at<Rec>(B, o_q2);
   d.vox = at<double>(B, o_vox); d.voy = at<double>(B, o_voy);
   d.delh_x = at<double>(B, o_g[0]); d.delh_y = at<double>(B, o_g[1]); d.delu_x = at<double>(B, o_g[2]);
   d.delu_y = at<double>(B, o_g[3]); d.delv_x = at<double>(B, o_g[4]); d.delv_y = at<double>(B, o_g[5]);
-  d.dry_a = at<uint8_t>(B, o_dra); d.dry_b = at<uint8_t>(B, o_drb); d.hvtx = at<double>(B, o_hv);
+  d.hvtx = at<double>(B, o_hv);
   d.dry_out = at<uint8_t>(B, o_dro);
   d.rs_cells = at<int32_t>(B, o_rsc); d.phi = at<double>(B, o_phi); d.phi0 = at<double>(B, o_phi0);
   d.rs_fac1 = 1.0 / (1.0 + o.rsavg_eps * 3.0);  // solverFVT.f90:59-60
@@ -623,7 +730,16 @@ int upload(StormFvtHandle* h) {
   d.vwet = at<uint8_t>(B, o_vw); d.phimax = at<double>(B, o_pm); d.bc_c = at<double>(B, o_bcc3);
   d.bc_rec = at<double>(B, o_rec); d.part = at<double>(B, o_part); d.nblk_red = nblk;
   d.sc = at<Scalars>(B, o_sc);
+  d.ct = at<CellTile>(B, o_ct); d.cbe = at<int32_t>(B, o_cbe); d.walls = at<WallRec>(B, o_walls);
+  d.cne_max = cne_max; d.cnw_max = cnw_max;
+  d.fdesc = at<uint32_t>(B, o_fdesc); d.lfe = at<uint16_t>(B, o_lfe); d.rad = at<float>(B, o_rad);
+  d.bcpart = at<double>(B, o_bcp); d.ccol = at<CellCol>(B, o_ccol);
+  CK(cudaDeviceGetAttribute(&h->n_sm, cudaDevAttrMultiProcessorCount, h->device));
+  h->cell_smem = cell_smem_bytes(d, h->mixed);
+  if (h->cell_smem > 48 * 1024) set_cell_smem_limit((int)h->cell_smem);
   d.nbc_cells = (int32_t)L.bc_cells.size();
+  d.ngen = (int32_t)gen.size();
+  d.gen_cells = at<int32_t>(B, o_gen);
   d.ne = L.ne;
   d.eL = at<int32_t>(B, o_eL); d.eR = at<int32_t>(B, o_eR); d.eslot = at<uint8_t>(B, o_es);
   d.enx = at<double>(B, o_enx); d.eny = at<double>(B, o_eny); d.elen = at<double>(B, o_el);
@@ -683,6 +799,20 @@ int upload(StormFvtHandle* h) {
     }
   }
   d.bc_cells = at<int32_t>(B, o_bcl);
+  {
+    std::vector<CellCol> cols(9 * kCellCols);
+    for (int s = 1; s <= K; s++)
+      for (int m = 0; m < 3; m++)
+        cell_columns(d, h->gd, h->gf, h->mixed, s, m, &cols[((s - 1) * 3 + m) * kCellCols]);
+    CK(cudaMemcpy(d.ccol, cols.data(), cols.size() * sizeof(CellCol), cudaMemcpyHostToDevice));
+    StageLaunch P{};
+    P.which = STAGE_PACK;
+    P.grid = dim3((T + 255) / 256);
+    P.block = dim3(256);
+    P.stream = h->stream;
+    launch_stage(P, d, h->gd, h->gf, h->mixed);
+    CK(cudaGetLastError());
+  }
   // per-scenario scalars: boundary values, series offsets, ranges
   std::vector<Scalars> s0(h->nscen);
   int32_t ts_base = 0;
@@ -711,6 +841,10 @@ int upload(StormFvtHandle* h) {
     x.last_cell = I.last_cell;
     x.blk_off = I.blk_off;
     x.blk_cnt = I.blk_cnt;
+    const auto bc0 = std::lower_bound(L.bc_cells.begin(), L.bc_cells.end(), I.cell_off);
+    const auto bc1 = std::lower_bound(bc0, L.bc_cells.end(), I.cell_off + I.cell_cnt);
+    x.bc_off = (int32_t)(bc0 - L.bc_cells.begin());
+    x.bc_cnt = (int32_t)(bc1 - bc0);
   }
   CK(cudaMemcpy(d.sc, s0.data(), sizeof(Scalars) * s0.size(), cudaMemcpyHostToDevice));
   int rct = upload_tiles(h);
@@ -814,7 +948,6 @@ int storm_fvt_create_batch(const StormFvtMesh* const* meshes, int32_t n, const S
   h->opt = *opt;
   h->device = opt->device;
   h->mixed = opt->precision == STORM_PREC_MIXED;
-  if (h->mixed) h->bs_eflux = 128;
   h->nscen = n;
   try {
     h->parts.resize(n);
@@ -852,6 +985,7 @@ int storm_fvt_create_batch(const StormFvtMesh* const* meshes, int32_t n, const S
     e = cudaEventCreateWithFlags(&h->fork_ev[i], cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->join_ev[i], cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->eflux_ev[i], cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->gen_ev[i], cudaEventDisableTiming);
   }
   if (e == cudaSuccess) e = cudaEventCreate(&h->ev0);
   if (e == cudaSuccess) e = cudaEventCreate(&h->ev1);
@@ -899,8 +1033,8 @@ int storm_fvt_set_scenario_state(StormFvtHandle* h, int32_t sid, const double* h
   });
   const Dev& d = h->d;
   CK(cudaMemcpyAsync(d.rkh + I.cell_off, buf, 8 * (size_t)Ts, cudaMemcpyHostToDevice, h->stream));
-  CK(cudaMemcpyAsync(d.u_a + I.cell_off, buf + Ts, 8 * (size_t)Ts, cudaMemcpyHostToDevice, h->stream));
-  CK(cudaMemcpyAsync(d.v_a + I.cell_off, buf + 2 * (size_t)Ts, 8 * (size_t)Ts, cudaMemcpyHostToDevice,
+  CK(cudaMemcpyAsync(d.rku + I.cell_off, buf + Ts, 8 * (size_t)Ts, cudaMemcpyHostToDevice, h->stream));
+  CK(cudaMemcpyAsync(d.rkv + I.cell_off, buf + 2 * (size_t)Ts, 8 * (size_t)Ts, cudaMemcpyHostToDevice,
                      h->stream));
   k_init<<<I.blk_cnt, kRed, 0, h->stream>>>(d, I.cell_off);
   k_init_final<<<1, kRed, 0, h->stream>>>(d, sid);
@@ -1053,8 +1187,11 @@ int storm_fvt_get_scenario_state(StormFvtHandle* h, int32_t sid, double* hh, dou
   const Dev& d = h->d;
   const int co = I.cell_off, no = I.node_off;
   int rc;
-  if ((rc = round({{d.rkh + co, hh, Ts, &P.cell_old}, {d.u_a + co, u, Ts, &P.cell_old},
-                   {d.v_a + co, v, Ts, &P.cell_old}})))
+  if (u || v) {
+    launch_split(d, co, Ts, 0, h->stream);
+    CK(cudaGetLastError());
+  }
+  if ((rc = round({{d.rkh + co, hh, Ts, &P.cell_old}, {d.io, u, Ts, &P.cell_old}, {d.io + Ts, v, Ts, &P.cell_old}})))
     return rc;
   if ((rc = round({{d.rkh + co, rkh, Ts, &P.cell_old}, {d.rku + co, rku, Ts, &P.cell_old},
                    {d.rkv + co, rkv, Ts, &P.cell_old}})))
@@ -1212,7 +1349,9 @@ int storm_fvt_get_drycell(StormFvtHandle* h, int32_t* dry) {
   const HostLayout& P = h->parts[0];
   const int Ts = P.T;
   std::vector<uint8_t> b(Ts);
-  CK(cudaMemcpyAsync(b.data(), h->d.dry_a, Ts, cudaMemcpyDeviceToHost, h->stream));
+  launch_split(h->d, 0, Ts, 1, h->stream);
+  CK(cudaGetLastError());
+  CK(cudaMemcpyAsync(b.data(), h->d.io, Ts, cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
   for (int c = 0; c < Ts; c++) dry[P.cell_old[c]] = b[c] ? 1 : 0;
   return STORM_OK;
@@ -1252,14 +1391,13 @@ int storm_fvt_autotune(StormFvtHandle* h, int32_t iters, int32_t* chosen) {
   // snapshot of the mutable state (restored afterwards: tuning does not advance the run)
   const Dev& d = h->d;
   const size_t T = (size_t)d.T, L = (size_t)(d.K + 1) * T;
-  const size_t bytes = 8 * (3 * L + 2 * T) + 2 * T + sizeof(Scalars) * (size_t)h->nscen;
+  const size_t bytes = 8 * 3 * L + sizeof(Rec) * T + sizeof(Scalars) * (size_t)h->nscen;
   char* snap = nullptr;
   CK(cudaMalloc(&snap, bytes));
   struct Piece {
     void* p;
     size_t n;
-  } pieces[] = {{d.rkh, 8 * L}, {d.rku, 8 * L}, {d.rkv, 8 * L}, {d.u_a, 8 * T}, {d.v_a, 8 * T},
-                {d.dry_a, T}, {d.dry_b, T}, {d.sc, sizeof(Scalars) * (size_t)h->nscen}};
+  } pieces[] = {{d.rkh, 8 * L}, {d.rku, 8 * L}, {d.rkv, 8 * L}, {d.q, sizeof(Rec) * T}, {d.sc, sizeof(Scalars) * (size_t)h->nscen}};
   size_t off = 0;
   for (auto& pc : pieces) {
     CK(cudaMemcpyAsync(snap + off, pc.p, pc.n, cudaMemcpyDeviceToDevice, h->stream));
@@ -1304,9 +1442,7 @@ int storm_fvt_autotune(StormFvtHandle* h, int32_t iters, int32_t* chosen) {
     int cls;
     int cand[3];
   } knobs[] = {{&h->bs_node, KT_NODE, {64, 128, 256}},
-               {&h->bs_grad, KT_GRAD, {64, 128, 256}},
-               {&h->bs_eflux, KT_EFLUX, {32, 64, 128}},
-               {&h->bs_flux, KT_FLUX, {32, 64, 128}}};
+               {&h->bs_grad, KT_GRAD, {64, 128, 256}}};
   const bool was_timing = h->timing;
   h->timing = true;
   for (auto& kb : knobs) {
@@ -1336,8 +1472,7 @@ int storm_fvt_autotune(StormFvtHandle* h, int32_t iters, int32_t* chosen) {
   if (chosen) {
     chosen[0] = h->bs_node;
     chosen[1] = h->bs_grad;
-    chosen[2] = h->bs_eflux;
-    chosen[3] = h->bs_flux;
+    chosen[2] = chosen[3] = kRed;  // k_cell: edge fluxes and cell update, one shape
   }
   // re-capture the iteration graph with the chosen shapes
   if (h->exec) cudaGraphExecDestroy(h->exec);
@@ -1493,18 +1628,9 @@ int storm_fvt_iter_finish(StormFvtHandle* h, const double* sums, StormFvtStepSta
   return 0;
 }
 
-// velocity buffers and dry flags of the state after stage `level` (after_fric = 0) or
-// after the friction step (level 0)
-static void part_buffers(StormFvtHandle* h, int level, int after_fric, double** u, double** v, uint8_t** dry) {
-  const Dev& d = h->d;
-  if (after_fric || !h->use_tiles) {
-    *u = d.u_a;
-    *v = d.v_a;
-  } else {
-    *u = (level & 1) ? h->u_a2 : d.u_a;
-    *v = (level & 1) ? h->v_a2 : d.v_a;
-  }
-  *dry = after_fric ? d.dry_a : ((level & 1) ? d.dry_b : d.dry_a);
+// state buffer after stage `level` (after_fric = 0) or after the friction step (level 0)
+static Rec* part_state(StormFvtHandle* h, int level, int after_fric) {
+  return (after_fric || !h->use_tiles || !(level & 1)) ? h->d.q : h->q2;
 }
 
 int storm_fvt_pack_halo(StormFvtHandle* h, int32_t level, int32_t after_fric, double* dev_out) {
@@ -1514,10 +1640,7 @@ int storm_fvt_pack_halo(StormFvtHandle* h, int32_t level, int32_t after_fric, do
   if (level < 0 || level > h->d.K || (after_fric && level != 0))
     return set_error(STORM_ERR_ARG, "storm_fvt_pack_halo: level out of range (0 after the friction step)");
   if (h->n_send > 0 && !dev_out) return set_error(STORM_ERR_ARG, "storm_fvt_pack_halo: null buffer");
-  double *u, *v;
-  uint8_t* dry;
-  part_buffers(h, level, after_fric, &u, &v, &dry);
-  launch_pack(h->d, level, h->n_send, h->send_slots, u, v, dev_out, h->stream);
+  launch_pack(h->d, level, h->n_send, h->send_slots, part_state(h, level, after_fric), dev_out, h->stream);
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(h->stream));
   return 0;
@@ -1530,10 +1653,7 @@ int storm_fvt_unpack_halo(StormFvtHandle* h, int32_t level, int32_t after_fric, 
   if (level < 0 || level > h->d.K || (after_fric && level != 0))
     return set_error(STORM_ERR_ARG, "storm_fvt_unpack_halo: level out of range (0 after the friction step)");
   if (h->n_recv > 0 && !dev_in) return set_error(STORM_ERR_ARG, "storm_fvt_unpack_halo: null buffer");
-  double *u, *v;
-  uint8_t* dry;
-  part_buffers(h, level, after_fric, &u, &v, &dry);
-  launch_unpack(h->d, level, h->n_recv, h->recv_slots, dev_in, u, v, dry, h->stream);
+  launch_unpack(h->d, level, h->n_recv, h->recv_slots, dev_in, part_state(h, level, after_fric), h->stream);
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(h->stream));
   return 0;

@@ -15,6 +15,33 @@ namespace storm {
 
 constexpr int kMaxBdrDev = 16;
 
+// 32 bytes moved by one 256-bit load or store.  A cell's stage-input state: depth, bed
+// elevation, velocities (find_dry_cells follows from them).  One side of an edge: the
+// face state h, u, v reconstructed from a cell's gradients (invisc_fluxes.f90:53-81, h
+// clipped at zero), with the cell's bed elevation (Roe, HLL) or celerity (Rusanov) in z;
+// a dry cell's face record has h = -1.
+struct alignas(32) Rec {
+  double h, z, u, v;
+};
+
+// k_cell's work list: for every block of 256 cell slots the interior edges whose smaller
+// slot is in it (a contiguous range), those whose larger one is (listed), and its walls.
+struct CellTile {
+  int32_t er0, nr, boff, nb, w0, nw, pad0, pad1;
+};
+// One of the columns k_cell copies to shared memory: a block takes `bytes` from
+// base + block * bytes to offset `dst`.
+struct CellCol {
+  const unsigned char* base;
+  uint32_t bytes, dst;
+};
+constexpr int kCellCols = 32;  // a column for each lane of a warp
+struct WallRec {  // a wall edge with a flux, sorted by cell
+  double nx, ny, len;  // normal out of the cell
+  int32_t p1, p2;      // ends, in walledg1 order
+  int32_t cell, rec;   // rec: its face record (slip walls)
+};
+
 // Per-scenario scalars that live on the device (one struct per scenario of the
 // handle, written by the kernels), followed by the scenario's static description.
 struct Scalars {
@@ -35,6 +62,7 @@ struct Scalars {
   int32_t n_in, n_out;
   int32_t last_cell;            // merged id of element n_elems (steady friction dt)
   int32_t blk_off, blk_cnt;     // reduction blocks of the scenario's cell range
+  int32_t bc_off, bc_cnt;       // its cells with an open-boundary face in Dev::bc_cells
   int32_t pad2;
   int32_t out_type[kMaxBdrDev];
   int32_t ts_off[2 * kMaxBdrDev], ts_cnt[2 * kMaxBdrDev];  // inflows, then outflows
@@ -80,7 +108,24 @@ struct Dev {
   const int32_t *eL, *eR;
   const uint8_t* eslot;
   const double *enx, *eny, *elen, *ez0;
-  double* efx;              // [3][ne] flux * length of the last k_eflux
+  // face records of a stage: the two sides of interior edge e at 2e (e(1)) and 2e+1
+  // (e(2)), then one per wall on slip-wall runs; written by k_grad, read by k_cell
+  Rec* fs;
+  uint8_t* fdry;            // [T] the cell's records hold the dry mark already
+  const int32_t* fpos;      // [3][T] record of each face of a cell (-1: none)
+  const CellTile* ct;       // [T/256]
+  CellCol* ccol;            // [3 stages][3 modes][kCellCols], bytes 0: none
+  const int32_t* cbe;       // listed edges (CellTile::boff, nb)
+  const WallRec* walls;     // [nwall] (CellTile::w0, nw)
+  int32_t cne_max, cnw_max; // most edges and walls of a tile
+  // per cell: forder | fko << 8 | kDescReal; the tile's edge or wall of its faces in
+  // summation order ([3][T]); largest |vertex - centroid| component, rounded up
+  const uint32_t* fdesc;
+  const uint16_t* lfe;
+  const float* rad;
+  // k_grad's per-cell constants, 32 cells to a block (GradBlock<R>)
+  unsigned char* gblk;
+  double* efx;              // [3][ne] fused path: flux * length of the edges k_flux_bc reads
   uint8_t* eok;             // [ne] the edge produced a flux (not skipped)
   // nodes
   const double *zvtx, *node_x, *node_y, *n2t_w;
@@ -91,18 +136,24 @@ struct Dev {
   const double *bce_nx, *bce_ny, *bce_tx, *bce_ty, *bce_len, *bce_zmid;
   const double *ts_t, *ts_v;
   // state
-  double *rkh, *rku, *rkv;  // [K+1][T]
-  double *u_a, *v_a;        // stage-input velocities (find_dry_cells, LSQ)
-  // the velocities this stage's fluxes use (after hgradfix2 / to_vertices zeroing):
-  // FP64 path, a flag per cell (1: zero, else the stage-input u, v); mixed path, the
-  // values themselves (read by the lighter FP32 edge kernel while still in L2)
-  uint8_t* vzero;
+  // RK levels [K+1][T].  rkh holds levels 0 and K-1 only (stage s reads level s-1 from
+  // its input record, and level 0 or the record is all its combination takes of h)
+  double *rkh, *rku, *rkv;
+  Rec* q;                   // stage-input state of every cell (phase path: updated in place)
+  double* io;               // [2][T] scratch of the state read-back
+  // the velocities this stage's fluxes use (after hgradfix2 / to_vertices zeroing) and
+  // the velocity gradients del*: of the cells with an open-boundary face only, for k_bc
+  // (the other faces' states are in fs); the depth gradient delh: of every cell
   double *u_b, *v_b;
   double *delh_x, *delh_y, *delu_x, *delu_y, *delv_x, *delv_y;
-  uint8_t *dry_a, *dry_b;   // stage dry flags (ping-pong)
   uint8_t* dry_out;         // find_dry_cells before the friction step (the output pass)
   double* hvtx;             // vertex depth after enforce_bcs (wall fluxes, output)
-  uint8_t* vwet;            // hvtx > h_dry before enforce_bcs (to_vertices.f90:44-55)
+  // to_vertices.f90:44-55, a vertex with hvtx <= h_dry before enforce_bcs: on the fused
+  // path a flag per node; on the phase path a mark on each of its wet cells, set by
+  // k_node and taken by k_grad (few: the cells along a wet/dry front)
+  uint8_t* vwet;
+  uint8_t* cmark;
+  int32_t node_quick;       // the IDW weights are all positive (see k_node)
   double* phimax;           // MAX(|phi|) of the last stage (stop criterion)
   // residual smoothing: phi and its copy [3][T], cells by colour of the t2t stencil
   double *phi, *phi0;
@@ -111,7 +162,11 @@ struct Dev {
   int32_t bc_cache;         // k_bc keeps the inflow fixed point's invariants in shared memory
   double* bc_c;             // [3][nbce] boundary contributions to phi
   double* bc_rec;           // [3][nbce] reconstructed boundary-edge h, u, v
+  double* bcpart;           // [5][nbc_cells] reduction terms of the cells with an open-boundary face
   double* part;             // [5][nblk] reduction partials, field-major (blocks never span scenarios)
+  // cells whose stencil is not their three face neighbours (HostLayout::plain)
+  int32_t ngen;
+  const int32_t* gen_cells;
   int32_t nbc_cells;        // cells with an open-boundary face (finished after k_bc)
   const int32_t* bc_cells;
   int32_t nblk_red;
@@ -127,6 +182,18 @@ struct Geo {
   const R *vox, *voy;  // [3][T] vertex minus centroid (bed_slope_STD), in R
   R *delh_x, *delh_y, *delu_x, *delu_y, *delv_x, *delv_y;
   R* efx;  // [3][ne]
+};
+
+// Constants of 32 consecutive cells that k_grad reads, each field's 32 values together:
+// one base address and fixed offsets serve a warp's loads, and they come from one
+// contiguous piece of memory.
+template <class R>
+struct GradBlock {
+  R w[3][32], dx[3][32], dy[3][32], rx[3][32], ry[3][32], dzx[32], dzy[32];
+  double zmax[32];
+  int32_t id[3][32];    // face neighbours (t2t3)
+  int32_t fpos[3][32];  // Dev::fpos
+  int32_t nst[32];      // stencil count and flags (Dev::nst)
 };
 
 // Device view of the tile plan of the fused stage kernel (TilePlan in storm_internal.h).
@@ -148,49 +215,57 @@ struct TileDev {
 };
 
 // One launch of a templated stage kernel (see launch_stage in fvt_kernels.cu).
-enum StageKernel { STAGE_GRAD, STAGE_BC, STAGE_EFLUX, STAGE_FLUX, STAGE_FLUX_BC, STAGE_PHI, STAGE_PHI_BC,
-                   STAGE_UPDATE, STAGE_CULVERT, STAGE_GRAD_BC, STAGE_TILE };
+enum StageKernel { STAGE_GRAD, STAGE_BC, STAGE_CELL, STAGE_FLUX_BC, STAGE_FLUX_BC_TILE,
+                   STAGE_UPDATE, STAGE_CULVERT, STAGE_GRAD_BC, STAGE_TILE, STAGE_PACK, STAGE_GRAD_GEN };
+// What a cell kernel does with phi: the RK update; phi itself for the residual smoothing;
+// the update and, in the last stage, the friction step and the iteration's reductions.
+enum CellMode { CELL_UPDATE = 0, CELL_PHI = 1, CELL_FRIC = 2 };
 struct StageLaunch {
   int which;
   dim3 grid, block;
   size_t smem;
   cudaStream_t stream;
   int s;
-  const double* hs;
-  const uint8_t* dry;
-  uint8_t* dry_next;
+  int mode;  // CellMode (STAGE_CELL, STAGE_FLUX_BC)
   double *rku_prev, *rkv_prev;
-  // stage-input velocities and where the stage writes its new ones (the same arrays
-  // for the phase kernels; ping-pong buffers for the fused tile kernel)
-  const double *u_in, *v_in;
-  double *u_out, *v_out;
+  // stage-input state and where the stage writes its new one (the same array for the
+  // phase kernels; ping-pong buffers for the fused tile kernel)
+  const Rec* q;
+  Rec* qo;
   const TileDev* tiles;  // STAGE_TILE only
 };
 size_t tile_smem_bytes(const TileDev& t, bool mixed);
 int tile_blocks_per_sm(bool mixed, size_t smem);  // resident CTAs of k_tile per SM
 void set_tile_smem_limit(int bytes);
+size_t cell_smem_bytes(const Dev& d, bool mixed);  // k_cell's dynamic shared memory
+void set_cell_smem_limit(int bytes);
+// the columns of stage s in a mode
+void cell_columns(const Dev& d, const Geo<double>& Gd, const Geo<float>& Gf, bool mixed, int s, int mode, CellCol* out);
 void launch_stage(const StageLaunch& L, const Dev& d, const Geo<double>& Gd, const Geo<float>& Gf, bool mixed);
 void set_bc_smem_limit(int bytes);
 // Linked partitions: halo exchange of one level (+ up to two flag arrays), the shared
 // friction dt before k_fric, the shared dt / stop test after k_final.
-void launch_halo(const Dev& d, int level, uint8_t* f1, uint8_t* f2, cudaStream_t st);
+void launch_halo(const Dev& d, int level, uint8_t* f1, cudaStream_t st);
 void launch_link_fric(const Dev& d, cudaStream_t st);
 void launch_link(const Dev& d, cudaStream_t st);
 void launch_link_dt(const Dev& d, cudaStream_t st);
 // Friction, hvalve and the iteration partials (halo cells left out when linked).
-void launch_fric(const Dev& d, const double* u_src, const double* v_src, cudaStream_t st);
+void launch_fric(const Dev& d, const Rec* src, cudaStream_t st);
 void launch_rsavg(const Dev& d, int off, int cnt, cudaStream_t st);
 // One part of a mesh per process: set dt (which 0) or the friction dt (1), pack /
 // unpack [6][n] halo values of the listed slots, finish the iteration with the sums
 // of all parts {sumtop, sumbot, tmass, max |phi|}.
 void launch_part_scalar(const Dev& d, int which, double v, cudaStream_t st);
-void launch_pack(const Dev& d, int level, int n, const int32_t* slots, const double* u, const double* v,
-                 double* out, cudaStream_t st);
-void launch_unpack(const Dev& d, int level, int n, const int32_t* slots, const double* in, double* u, double* v,
-                   uint8_t* dry, cudaStream_t st);
+void launch_pack(const Dev& d, int level, int n, const int32_t* slots, const Rec* q, double* out, cudaStream_t st);
+void launch_unpack(const Dev& d, int level, int n, const int32_t* slots, const double* in, Rec* q, cudaStream_t st);
+// State read-back of the cells [c0, c0+n): velocities into d.io ([2][n]), or the dry
+// flags of the next iteration's first stage (bytes)
+void launch_split(const Dev& d, int c0, int n, int dry, cudaStream_t st);
 void launch_part_finish(const Dev& d, const double* sums, cudaStream_t st);
-// k_node over every node (list == nullptr) or the n listed nodes
-void launch_node(const Dev& d, const double* hs, const uint8_t* dry, const int32_t* list, int n, int block,
+// k_node over every node (list == nullptr) or the n listed nodes.  mark: the phase
+// path's form (cell marks; depths of every node only if full, else only where a stage
+// reads them), otherwise a wet flag and a depth per node
+void launch_node(const Dev& d, const Rec* q, const int32_t* list, int n, bool mark, bool full, int block,
                  cudaStream_t st);
 
 // The output pass (to_vertices, ctr2vtx of cd, error_est(2)) after an iteration.

@@ -5,28 +5,33 @@
 //                       nodes (to_vertices.f90:26-41, enforce_bcs.f90:37-56)
 //   k_grad   per cell : find_dry_cells state, lsq_grad_array x3, limiterBJ x3, delh -= delz
 //                       (cell_grads.f90), hgradfix2.f90:48-98, zeroing of cells with a
-//                       vertex depth <= h_dry (to_vertices.f90:44-55)
+//                       vertex depth <= h_dry (to_vertices.f90:44-55), and the states at
+//                       the three faces; the cells along the mesh boundary in a launch of
+//                       their own
 //   k_bc     per open boundary (one CTA): inflowQbyH / inflowH / outflowbyH /
 //                       crit_outflow / free_flow, including the inflow fixed point
-//   k_eflux  per interior edge: the Roe/HLL/Rusanov flux (with the I1 wet/dry wall test)
-//                       evaluated once, in the reference's orientation, times the length
-//   k_flux   per cell : the cell's face contributions (edge fluxes from k_eflux, the
-//                       wenslp3/weslp2 walls, boundary contributions) added in the order
-//                       invisc_fluxes.f90 scatters them, bed_slope_STD + adjustZb, the
-//                       SSP-RK combination, vclip, h >= 0 and wet/dry hysteresis
-//                       (k_flux_bc: the cells with an open-boundary face, after k_bc)
+//   k_cell   per block of 256 cells: the Roe/HLL/Rusanov flux (with the I1 wet/dry wall
+//                       test) of their edges in the reference's orientation, times the
+//                       length, the wenslp3/weslp2 walls; then each cell's contributions
+//                       added in the order invisc_fluxes.f90 scatters them,
+//                       bed_slope_STD + adjustZb, the SSP-RK combination, vclip, h >= 0
+//                       and wet/dry hysteresis (k_flux_bc: the cells with an open-boundary
+//                       face, after k_bc)
 // and one iteration ends with
-//   k_fric  per cell : find_dry_cells, fric_terms_impl, the numerical valve, the
+//   friction per cell : find_dry_cells, fric_terms_impl, the numerical valve, the
 //                      RK level copy, block partials of sumtop/sumbot/tmass/max|phi|/dt
+//                      (in the last stage's k_cell, or in k_fric)
 //   k_final one CTA per scenario: deterministic reduction of the partials, stop test,
 //                      clocks, get_time_bcs.
 // No float atomics: every sum is a fixed-order tree or a serial loop, so the results
 // are reproducible run to run.
+#include <cstddef>
 #include <cstdint>
 #include <mutex>
 
 #include "fvt_device.cuh"
 #include "storm_internal.h"
+#include "umma.cuh"
 
 namespace storm {
 
@@ -66,6 +71,48 @@ __device__ __forceinline__ double qdiv(double a, double b) {
 // magnitude), whose error is far below the FP32 rounding the path already accepts.
 __device__ __forceinline__ float qdiv(float a, float b) { return __fdividef(a, b); }
 
+// Quotients by one denominator, without the division's slow path inline.  FP64: a
+// Newton-Raphson reciprocal y of b from the hardware's seed (one cubic and one quadratic
+// step), then for each numerator a*y and two residual corrections q += (a - b q) y with
+// fused multiply-adds; the first brings q within one ulp of a/b, the second then rounds
+// it correctly (Markstein's theorem: P. W. Markstein, "Computation of elementary
+// functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34, 1990), so the
+// result is the bits of a / b.  The theorem needs a correctly rounded y (the last
+// Newton step gives it unless b's significand is all ones) and operands whose quotient
+// and residual neither overflow nor become subnormal; for others, `bad` is set and the
+// caller takes the division itself.  A zero numerator's quotient is a*y exactly.
+template <class R>
+struct Den;
+template <>
+struct Den<double> {
+  double b, y;
+  __device__ __forceinline__ static bool ordinary(double x) {
+    return (unsigned)((__double2hiint(x) & 0x7fffffff) - 0x23d00000) < 0x38500000u;  // 2^-450 .. 2^451
+  }
+  __device__ __forceinline__ Den(double b_, bool* bad) : b(b_) {
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    const double e = __fma_rn(-b, y, 1.0);
+    y = __fma_rn(y, __fma_rn(e, e, e), y);
+    y = __fma_rn(y, __fma_rn(-b, y, 1.0), y);
+    const bool ones = (__double2hiint(b) & 0xfffff) == 0xfffff && __double2loint(b) == -1;
+    *bad = *bad || !ordinary(b) || ones;
+  }
+  __device__ __forceinline__ double quot(double a, bool* bad) const {
+    const double q0 = a * y;
+    double q = __fma_rn(__fma_rn(-b, q0, a), y, q0);
+    q = __fma_rn(__fma_rn(-b, q, a), y, q);
+    const bool zero = a == kZero;
+    *bad = *bad || !(zero || ordinary(a));
+    return zero ? q0 : q;
+  }
+};
+template <>
+struct Den<float> {
+  float b;
+  __device__ __forceinline__ Den(float b_, bool*) : b(b_) {}
+  __device__ __forceinline__ float quot(float a, bool*) const { return qdiv(a, b); }
+};
+
 // sqrt with a zero argument answered directly (sqrt(+-0) = +-0 under IEEE), for the
 // same reason as qdiv: still water and dry sides make zero arguments common.
 __device__ __forceinline__ double qsqrt(double x) {
@@ -95,6 +142,33 @@ __device__ __forceinline__ bool dry_flag(double h, double u, double v, double h_
   *umag = um;
   if (!dry && (h < h_wet) && equals(um, kZero)) dry = true;
   return dry;
+}
+
+// Records, as two 128-bit loads or stores.
+__device__ __forceinline__ Rec ld_rec(const Rec* p) {
+  const double2 a = *reinterpret_cast<const double2*>(p), b = *(reinterpret_cast<const double2*>(p) + 1);
+  return Rec{a.x, a.y, b.x, b.y};
+}
+// The same, never merged with an earlier load: read again from L1 instead of held.
+__device__ __forceinline__ Rec ld_rec_again(const Rec* p) {
+  Rec r;
+  asm volatile("ld.global.v2.f64 {%0, %1}, [%2];" : "=d"(r.h), "=d"(r.z) : "l"(p));
+  asm volatile("ld.global.v2.f64 {%0, %1}, [%2+16];" : "=d"(r.u), "=d"(r.v) : "l"(p));
+  return r;
+}
+__device__ __forceinline__ void st_rec(Rec* p, const Rec& r) {
+  *reinterpret_cast<double2*>(p) = make_double2(r.h, r.z);
+  *(reinterpret_cast<double2*>(p) + 1) = make_double2(r.u, r.v);
+}
+
+// find_dry_cells.f90:25-42 of a cell's record
+__device__ __forceinline__ bool rec_dry(const Dev& d, const Rec& r) {
+  if (r.h < d.h_dry) return true;
+  if (!(r.h < d.h_wet)) return false;
+  // equals(sqrt(s), 0): true for a zero, and (its comparison being negated) for an
+  // infinite or NaN speed
+  const double s = r.u * r.u + r.v * r.v;
+  return !(s > kZero && s <= kVlarge);
 }
 
 // Whether cell slot c (node n, edge e) belongs to a scenario that is still running.
@@ -187,6 +261,66 @@ __device__ __forceinline__ void flux_roe(R nx, R ny, R hleft, R uleft, R vleft, 
   for (int i = 0; i < 3; i++) flux[i] = R(kHalf) * (fr[i] * nx + gr[i] * ny + fl[i] * nx + gl[i] * ny - aq[i]);
 }
 
+// flux_roe in FP64 with its five quotients by two shared denominators, and without the
+// steps that change no bit of the flux: products with the eigenvector matrix's zero and
+// ones, and the sums' leading zeros (they would only turn a -0 into +0, and the sign of
+// a zero is lost in the cell's sum).  `bad` is set where an operand needs flux_roe's own
+// divisions (see Den).
+__device__ __forceinline__ void flux_roe_fast(double nx, double ny, double hleft, double uleft, double vleft,
+                                              double hright, double uright, double vright, double* flux, bool* bad) {
+  const double delta = 0.10;
+  const double hul = hleft * uleft, hvl = hleft * vleft, hur = hright * uright, hvr = hright * vright;
+  const double pl = kHalf * kG * hleft * hleft, pr = kHalf * kG * hright * hright;
+  const double fl1 = hul * uleft + pl, fl2 = hul * vleft, gl2 = hvl * vleft + pl;
+  const double fr1 = hur * uright + pr, fr2 = hur * vright, gr2 = hvr * vright + pr;
+  hleft = fmax2(hleft, SMALL_F);
+  const double hls = sqrt(hleft);
+  hright = fmax2(hright, SMALL_F);
+  const double hrs = sqrt(hright);
+  const Den<double> den(hrs + hls, bad);
+  const double uavg = den.quot(uright * hrs + uleft * hls, bad);
+  const double vavg = den.quot(vright * hrs + vleft * hls, bad);
+  const double cavg = sqrt(kHalf * kG * (hleft + hright));
+  const double q0 = hright - hleft, q1 = hright * uright - hleft * uleft, q2 = hright * vright - hleft * vleft;
+  const double cx = cavg * nx, cy = cavg * ny, un = uavg * nx + vavg * ny;
+  const Den<double> dc(cavg, bad);
+  const double a = dc.quot(kHalf * un, bad), bx = dc.quot(kHalf * nx, bad), by = dc.quot(kHalf * ny, bad);
+  const double l00 = -(uavg * ny - vavg * nx);
+  const double l10 = a + kHalf, l20 = -a + kHalf;
+  const double e0 = fmax2(fabs(un), delta), e1 = fmax2(fabs(un - cavg), delta), e2 = fmax2(fabs(un + cavg), delta);
+  // rows of (rev . eig), the first being (0, e1, e2)
+  const double t10 = ny * e0, t11 = (uavg - cx) * e1, t12 = (uavg + cx) * e2;
+  const double t20 = -nx * e0, t21 = (vavg - cy) * e1, t22 = (vavg + cy) * e2;
+  // times lev = {{l00, ny, -nx}, {l10, -bx, -by}, {l20, bx, by}}, times q
+  const double a0 = ((e1 * l10 + e2 * l20) * q0 + (e1 * -bx + e2 * bx) * q1) + (e1 * -by + e2 * by) * q2;
+  const double a1 = (((t10 * l00 + t11 * l10) + t12 * l20) * q0 + ((t10 * ny + t11 * -bx) + t12 * bx) * q1) +
+                    ((t10 * -nx + t11 * -by) + t12 * by) * q2;
+  const double a2 = (((t20 * l00 + t21 * l10) + t22 * l20) * q0 + ((t20 * ny + t21 * -bx) + t22 * bx) * q1) +
+                    ((t20 * -nx + t21 * -by) + t22 * by) * q2;
+  flux[0] = kHalf * (hur * nx + hvr * ny + hul * nx + hvl * ny - a0);
+  flux[1] = kHalf * (fr1 * nx + fr2 * ny + fl1 * nx + fl2 * ny - a1);
+  flux[2] = kHalf * (fr2 * nx + gr2 * ny + fl2 * nx + gl2 * ny - a2);
+}
+__device__ __noinline__ void flux_roe_careful(double nx, double ny, double hleft, double uleft, double vleft,
+                                              double hright, double uright, double vright, double* flux) {
+  flux_roe<double>(nx, ny, hleft, uleft, vleft, hright, uright, vright, flux);
+}
+__device__ __forceinline__ void flux_roe_edge(double nx, double ny, double hleft, double uleft, double vleft,
+                                              double hright, double uright, double vright, double* flux) {
+  bool bad = false;
+  flux_roe_fast(nx, ny, hleft, uleft, vleft, hright, uright, vright, flux, &bad);
+  if (bad) flux_roe_careful(nx, ny, hleft, uleft, vleft, hright, uright, vright, flux);
+}
+__device__ __forceinline__ void flux_roe_edge(float nx, float ny, float hleft, float uleft, float vleft, float hright,
+                                              float uright, float vright, float* flux) {
+  flux_roe<float>(nx, ny, hleft, uleft, vleft, hright, uright, vright, flux);
+}
+
+// a x + b y.  The mixed path's is contracted in this one way whatever surrounds it, so
+// that moving the flux functions between kernels does not move its roundings.
+__device__ __forceinline__ double dot2(double a, double x, double b, double y) { return a * x + b * y; }
+__device__ __forceinline__ float dot2(float a, float x, float b, float y) { return __fmaf_rn(b, y, __fmul_rn(a, x)); }
+
 // flux_HLL.f90:41-110 with its two defects fixed (flux(3) assigned; the whole HLL
 // numerator divided by sright - sleft).  The debug stop at :88-91 sets *bad.
 template <class R>
@@ -194,20 +328,20 @@ __device__ __forceinline__ void flux_hll(R nx, R ny, R hleft, R uleft, R vleft, 
                                          R h0, R* flux, bool* bad) {
   R cleft = qsqrt(R(kG) * hleft);
   R cright = qsqrt(R(kG) * hright);
-  R ustar = R(kHalf) * ((uleft + uright) * nx + (vleft + vright) * ny) + cleft - cright;
-  R cstar = R(kHalf) * (cleft + cright) + ((uleft - uright) * nx + (vleft - vright) * ny) / R(4.0);
+  R ustar = R(kHalf) * dot2(uleft + uright, nx, vleft + vright, ny) + cleft - cright;
+  R cstar = R(kHalf) * (cleft + cright) + dot2(uleft - uright, nx, vleft - vright, ny) / R(4.0);
   R sleft, sright, aux1, aux2;
-  if (hleft < h0) sleft = uright * nx + vright * ny - R(2.0) * cright;
-  else if (hright < h0) sleft = uleft * nx + vleft * ny - cleft;
+  if (hleft < h0) sleft = dot2(uright, nx, vright, ny) - R(2.0) * cright;
+  else if (hright < h0) sleft = dot2(uleft, nx, vleft, ny) - cleft;
   else {
-    aux1 = uleft * nx + vleft * ny - cleft;
+    aux1 = dot2(uleft, nx, vleft, ny) - cleft;
     aux2 = ustar - cstar;
     sleft = fmin2(aux1, aux2);
   }
-  if (hleft < h0) sright = uright * nx + vright * ny + cright;
-  else if (hright < h0) sright = uleft * nx + vleft * ny + R(2.0) * cleft;
+  if (hleft < h0) sright = dot2(uright, nx, vright, ny) + cright;
+  else if (hright < h0) sright = dot2(uleft, nx, vleft, ny) + R(2.0) * cleft;
   else {
-    aux1 = uright * nx + vright * ny - cright;
+    aux1 = dot2(uright, nx, vright, ny) - cright;
     aux2 = ustar + cstar;
     sright = fmax2(aux1, aux2);
   }
@@ -256,8 +390,8 @@ __device__ __forceinline__ void flux_rusanov(R nx, R ny, R hleft, R uleft, R vle
   gr[0] = hright * vright;
   gr[1] = hright * uright * vright;
   gr[2] = hright * vright * vright + R(kHalf) * R(kG) * hright * hright;
-  R ul = uleft * nx + vleft * ny;
-  R ur = uright * nx + vright * ny;
+  R ul = dot2(uleft, nx, vleft, ny);
+  R ur = dot2(uright, nx, vright, ny);
   R splus = fmax2(fabs(ul) + cl, fabs(ur) + cr);
   q[0] = hright - hleft;
   q[1] = hright * uright - hleft * uleft;
@@ -415,12 +549,12 @@ __global__ void __launch_bounds__(kRedThreads) k_init(Dev d, int c0) {
   const int c = c0 + blockIdx.x * blockDim.x + threadIdx.x;
   double dtc = kVlarge;
   if (c < d.T && d.cell_sid[c] >= 0) {
-    double h = d.rkh[c], u = d.u_a[c], v = d.v_a[c];
+    double h = d.rkh[c], u = d.rku[c], v = d.rkv[c];  // level 0 holds h, u, v as uploaded
     d.rku[c] = h * u;
     d.rkv[c] = h * v;
+    st_rec(d.q + c, Rec{h, d.z[c], u, v});
     double um;
     bool dry = dry_flag(h, u, v, d.h_dry, d.h_wet, &um);
-    d.dry_a[c] = dry;
     double wc = dry ? kZero : sqrt(kG * h);
     double dl = um + wc + SMALL_F;
     dtc = d.cfl * d.area[c] / (dl * d.perim[c]);
@@ -465,6 +599,17 @@ __global__ void __launch_bounds__(kRedThreads) k_init_final(Dev d, int sid) {
 // Vertex water surface and depth of one stage (to_vertices.f90:26-41: ctr2vtxWSE type
 // 3, cap at the highest wet neighbour, positivity_vtx; enforce_bcs.f90:37-56 for the
 // stage nodes).  cell(q, &dry, &h, &z) gives the q-th incident cell (n2t order).
+__device__ __forceinline__ void node_finish(const Dev& d, int n, double zv0, int counter, double id, double a,
+                                            double zetaref, double* hv_out, bool* wet_out) {
+  double zv = counter > 0 ? a / id : zv0;
+  zv = fmin2(zv, zetaref);
+  double hv = zv - zv0;
+  if (hv < kZero) hv = kZero;
+  *wet_out = hv > d.h_dry;
+  const int b = d.node_hbc[n];
+  if (b >= 0) hv = fmax2(kZero, d.sc[d.node_sid[n]].hbc[b] - zv0);  // stage node (-2: a wall end)
+  *hv_out = hv;
+}
 template <class CellF>
 __device__ __forceinline__ void node_depth(const Dev& d, int n, int b0, int b1, CellF cell, double* hv_out,
                                            bool* wet_out) {
@@ -483,21 +628,23 @@ __device__ __forceinline__ void node_depth(const Dev& d, int n, int b0, int b1, 
     a = a + w * zeta;
     zetaref = fmax2(zeta, zetaref);
   }
-  double zv = counter > 0 ? a / id : zv0;
-  zv = fmin2(zv, zetaref);
-  double hv = zv - zv0;
-  if (hv < kZero) hv = kZero;
-  *wet_out = hv > d.h_dry;
-  const int b = d.node_hbc[n];
-  if (b >= 0) hv = fmax2(kZero, d.sc[d.node_sid[n]].hbc[b] - zv0);
-  *hv_out = hv;
+  node_finish(d, n, zv0, counter, id, a, zetaref, hv_out, wet_out);
 }
 
 #ifndef STORM_FVT_F32_TU
 // Every node, or the listed nodes (the vertices of the cells with an open-boundary
 // face, ahead of their gradients on the side stream of the fused path).
-__global__ void __launch_bounds__(256) k_node(Dev d, const double* __restrict__ hs, const uint8_t* __restrict__ dry,
-                                              const int32_t* __restrict__ list, int nlist) {
+//
+// kMark (the phase path): the stage needs of most nodes only whether their depth
+// exceeds h_dry, and that only where it does not.  The IDW mean of positive weights
+// lies between the smallest and the largest wet stage around the node, so where both
+// are on one side of bed + h_dry (by far more than the mean's rounding) neither the
+// weights nor the mean are needed.  The depth itself is computed where a stage reads
+// it (wall ends, stage nodes: node_hbc != -1) and for every node in the last stage.
+constexpr int kNodeBatch = 8;
+template <bool kMark>
+__global__ void __launch_bounds__(256) k_node(Dev d, const Rec* __restrict__ rec, const int32_t* __restrict__ list,
+                                              int nlist, int full) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   int n;
   if (list) {
@@ -508,17 +655,81 @@ __global__ void __launch_bounds__(256) k_node(Dev d, const double* __restrict__ 
     n = i;
   }
   if (!item_live(d, d.node_sid, n)) return;
+  const int b0 = d.n2t_off[n], b1 = d.n2t_off[n + 1];
+  if (kMark && !full && d.node_quick && d.node_hbc[n] == -1) {
+    const double zv0 = d.zvtx[n];
+    double lo = kVlarge, hi = -kVlarge, sum = kZero;
+    int counter = 0;
+    for (int q0 = b0; q0 < b1; q0 += kNodeBatch) {  // a batch's indices, then its cells
+      int k[kNodeBatch];
+#pragma unroll
+      for (int j = 0; j < kNodeBatch; j++) k[j] = q0 + j < b1 ? d.n2t_cell[q0 + j] : -1;
+      double2 hz[kNodeBatch];
+#pragma unroll
+      for (int j = 0; j < kNodeBatch; j++)
+        hz[j] = k[j] >= 0 ? *reinterpret_cast<const double2*>(rec + k[j]) : make_double2(-kOne, kZero);
+#pragma unroll
+      for (int j = 0; j < kNodeBatch; j++) {
+        if (hz[j].x < d.h_dry) continue;
+        if (hz[j].x < d.h_wet && rec_dry(d, rec[k[j]])) continue;
+        const double zeta = hz[j].x + hz[j].y;
+        lo = fmin2(lo, zeta);
+        hi = fmax2(hi, zeta);
+        sum = sum + zeta;
+        counter++;
+      }
+    }
+    if (counter == 0) return;  // no wet cell to mark
+    const double eps = 1.0e-12 * (fmax2(fabs(lo), fabs(hi)) + fabs(zv0));
+    const bool finite = sum - sum == kZero;
+    if (finite && lo - zv0 > d.h_dry + eps) return;  // wet
+    if (finite && hi - zv0 < d.h_dry - eps) {        // not wet
+      for (int q = b0; q < b1; q++) {
+        const int k = d.n2t_cell[q];
+        if (!rec_dry(d, ld_rec(rec + k))) d.cmark[k] = 1;
+      }
+      return;
+    }
+  }
+  // node_depth, the loads of a batch of incident cells issued together
+  const double zv0 = d.zvtx[n];
+  double id = kZero, a = kZero, zetaref = zv0;
+  int counter = 0;
+  for (int q0 = b0; q0 < b1; q0 += kNodeBatch) {
+    int k[kNodeBatch];
+    double w[kNodeBatch];
+#pragma unroll
+    for (int j = 0; j < kNodeBatch; j++) {
+      k[j] = q0 + j < b1 ? d.n2t_cell[q0 + j] : -1;
+      w[j] = q0 + j < b1 ? d.n2t_w[q0 + j] : kZero;
+    }
+    double2 hz[kNodeBatch];
+#pragma unroll
+    for (int j = 0; j < kNodeBatch; j++)
+      hz[j] = k[j] >= 0 ? *reinterpret_cast<const double2*>(rec + k[j]) : make_double2(-kOne, kZero);
+#pragma unroll
+    for (int j = 0; j < kNodeBatch; j++) {
+      if (hz[j].x < d.h_dry) continue;
+      if (hz[j].x < d.h_wet && rec_dry(d, rec[k[j]])) continue;
+      const double zeta = hz[j].x + hz[j].y;
+      counter++;
+      id = id + w[j];
+      a = a + w[j] * zeta;
+      zetaref = fmax2(zeta, zetaref);
+    }
+  }
   double hv;
   bool wet;
-  node_depth(d, n, d.n2t_off[n], d.n2t_off[n + 1],
-             [&](int q, bool* dk, double* hk, double* zk) {
-               const int k = d.n2t_cell[q];
-               *dk = dry[k] != 0;
-               *hk = hs[k];
-               *zk = d.z[k];
-             },
-             &hv, &wet);
-  d.vwet[n] = wet;
+  node_finish(d, n, zv0, counter, id, a, zetaref, &hv, &wet);
+  if (kMark) {
+    if (!wet)
+      for (int q = b0; q < b1; q++) {
+        const int k = d.n2t_cell[q];
+        if (!rec_dry(d, ld_rec(rec + k))) d.cmark[k] = 1;
+      }
+  } else {
+    d.vwet[n] = wet;
+  }
   d.hvtx[n] = hv;
 }
 #endif  // !STORM_FVT_F32_TU
@@ -567,16 +778,13 @@ __device__ __forceinline__ float limited_r(double q0, double qn, float g_x, floa
 // Neighbour values of the gradient and flux arithmetic: read from global memory by
 // slot (the phase kernels) or from a tile's shared-memory copy by local id (k_tile).
 struct NbGlobal {
-  const double* __restrict__ hs;
-  const double* __restrict__ z;
-  const double* __restrict__ u;
-  const double* __restrict__ v;
-  const uint8_t* __restrict__ dry;
-  __device__ __forceinline__ double H(int i) const { return hs[i]; }
-  __device__ __forceinline__ double Z(int i) const { return z[i]; }
-  __device__ __forceinline__ double U(int i) const { return u[i]; }
-  __device__ __forceinline__ double V(int i) const { return v[i]; }
-  __device__ __forceinline__ bool D(int i) const { return dry[i] != 0; }
+  const Dev& d;
+  const Rec* __restrict__ q;
+  __device__ __forceinline__ double H(int i) const { return q[i].h; }
+  __device__ __forceinline__ double Z(int i) const { return q[i].z; }
+  __device__ __forceinline__ double U(int i) const { return q[i].u; }
+  __device__ __forceinline__ double V(int i) const { return q[i].v; }
+  __device__ __forceinline__ bool D(int i) const { return rec_dry(d, q[i]); }
 };
 struct NbShared {
   const double *h, *z, *u, *v;
@@ -603,16 +811,6 @@ struct GradOut {
   bool vz;   // ub, vb are the zeros hgradfix2 / to_vertices set (else the cell's u, v)
 };
 
-// The velocity the flux kernels use for cell x this stage (k_grad's ub, vb): FP64,
-// the zero hgradfix2 / to_vertices set or the stage-input value, from a flag; mixed,
-// the stored value (stored is the velocity array k_grad wrote, d.u_b or d.v_b).
-template <class R>
-__device__ __forceinline__ double post_fix(const Dev& d, const double* __restrict__ vel,
-                                           const double* __restrict__ stored, int x) {
-  if (sizeof(R) == 8) return d.vzero[x] ? kZero : vel[x];
-  return stored[x];
-}
-
 template <class R, class NB, class ST, class VW>
 __device__ __forceinline__ GradOut<R> cell_gradients(const Dev& d, const Geo<R>& G, const NB& nb, int c, int self,
                                                      const int (&t3)[3], ST st, VW vwet, R* rcx, R* rcy) {
@@ -627,7 +825,7 @@ __device__ __forceinline__ GradOut<R> cell_gradients(const Dev& d, const Geo<R>&
     // the layout found them bit-equal to lsq_a/b/c for every cell)
     constexpr bool kF64 = sizeof(R) == 8;
     double sa = 0.0, sb = 0.0, sc = 0.0;
-    const int n = d.nst[c];
+    const int n = d.nst[c] & kNstCount;
     int k0 = 0;
     if (n >= 3) {  // interior cells: the three face neighbours, all gathers issued together
       int jj[3];
@@ -763,25 +961,398 @@ __device__ __forceinline__ GradOut<R> cell_gradients(const Dev& d, const Geo<R>&
   return o;
 }
 
-// Gradients of every cell (list == nullptr) or of the listed cells (the cells with an
-// open-boundary face, ahead of the boundary kernel), stored for the phase kernels.
-template <class R, bool kList>
-__global__ void __launch_bounds__(256, 5) k_grad(Dev d, Geo<R> G, const double* __restrict__ hs,
-                                              const uint8_t* __restrict__ dry, double* __restrict__ rku_prev,
-                                              double* __restrict__ rkv_prev, const double* __restrict__ u_in,
-                                              const double* __restrict__ v_in) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  int c;
-  if (kList) {
-    if (i >= d.nbc_cells) return;
-    c = d.bc_cells[i];
-  } else {
-    if (i >= d.T) return;
-    c = i;
+// The limiter of one field over its three faces (min of limited_r), a face at a time.
+// FP64: the ratios num/delq are compared by cross products, which order them beyond
+// doubt when the products differ by more than their rounding (rounding is monotonic, so
+// the smallest exact ratio has the smallest rounded one), and only the smallest is
+// divided.  Products too close to tell, subnormal or not finite set `bad`.
+template <class R>
+struct Limit3;
+template <>
+struct Limit3<double> {
+  double n = kOne, d = kOne;  // the smallest ratio so far
+  bool any = false;
+  __device__ __forceinline__ void face(double q0, double qn, double gx, double gy, double rx, double ry, bool* bad) {
+    const double delq = (q0 + gx * rx + gy * ry) - q0;
+    const double num = ((delq < 0 ? qn < q0 : qn > q0) ? qn : q0) - q0;
+    const double an = fabs(num), ad = fabs(delq);
+    // the ratio counts as one if equals(delq, zero), which holds up to 2^-1023 and for
+    // infinities and NaN, or if it exceeds one
+    constexpr double kTiny = 1.1125369292536007e-308;
+    const bool cnt = ad > kTiny && ad <= kVlarge && !(an > ad);
+    const double p = fabs(num * d), q = fabs(n * delq);
+    constexpr double kBelow = 1.0 - 1.0e-15;
+    const bool less = p < q * kBelow, more = q < p * kBelow;
+    const bool cmp = any && cnt && n != kZero;
+    *bad = *bad || (cmp && !((less && q > 1.0e-290) || (more && p > 1.0e-290))) || (cnt && !(an <= ad));
+    const bool take = any ? cmp && less : cnt;
+    n = take ? num : n;
+    d = take ? delq : d;
+    any = any || cnt;
   }
+  __device__ __forceinline__ double value(bool* bad) const {
+    const double r = Den<double>(d, bad).quot(n, bad);  // 1/1 if no ratio counts
+    return any ? r : kOne;
+  }
+};
+template <>
+struct Limit3<float> {
+  float r = 0.f;
+  bool any = false;
+  __device__ __forceinline__ void face(double q0, double qn, float gx, float gy, float rx, float ry, bool*) {
+    const float x = limited_r(q0, qn, gx, gy, rx, ry);
+    r = any ? fmin2(r, x) : x;
+    any = true;
+  }
+  __device__ __forceinline__ float value(bool*) const { return r; }
+};
+
+// Stores of one cell's gradients and face records (phase path).
+template <class R>
+__device__ __forceinline__ void store_grad(const Dev& d, const Geo<R>& G, const GradBlock<R>& B, int ln, int c,
+                                           const GradOut<R>& g, const Rec& own, bool dry_c, bool bc,
+                                           double* __restrict__ rku_prev, double* __restrict__ rkv_prev, double x) {
+  if (g.fix) {
+    rku_prev[c] = kZero;
+    rkv_prev[c] = kZero;
+  }
+  G.delh_x[c] = g.hx; G.delh_y[c] = g.hy;
+  if (bc) {
+    G.delu_x[c] = g.ux; G.delu_y[c] = g.uy;
+    G.delv_x[c] = g.vx; G.delv_y[c] = g.vy;
+    d.u_b[c] = g.ub;
+    d.v_b[c] = g.vb;
+  }
+  if (dry_c) return;
+  Rec r;
+  r.z = x;
+#pragma unroll
+  for (int m = 0; m < 3; m++) {
+    const int p = B.fpos[m][ln];
+    const R rx = B.rx[m][ln], ry = B.ry[m][ln];
+    r.h = recon(own.h, g.hx, rx, g.hy, ry);
+    if (r.h < kZero) r.h = kZero;
+    r.u = recon(g.ub, g.ux, rx, g.uy, ry);
+    r.v = recon(g.vb, g.vx, rx, g.vy, ry);
+    if (p >= 0) st_rec(d.fs + p, r);
+  }
+}
+
+// A cell's dry mark in the face records (see k_grad); whether its gradients are needed.
+template <class R>
+__device__ __forceinline__ bool grad_begin(const Dev& d, const GradBlock<R>& B, int ln, int c, int s, const Rec& own,
+                                           bool dry_c, bool was_dry, bool bc) {
+  if (dry_c) {
+    // a dry cell's face states are a mark, written when the cell falls dry; its depth
+    // gradient is read by the output step alone (after the last stage), the rest by
+    // k_bc alone
+    if (!was_dry) {
+#pragma unroll
+      for (int m = 0; m < 3; m++) {
+        const int p = B.fpos[m][ln];
+        if (p >= 0) st_rec(d.fs + p, Rec{-kOne, d.flux == STORM_FLUX_RUSANOV ? kZero : own.z, kZero, kZero});
+      }
+      d.fdry[c] = 1;
+    }
+    return s == d.K || bc;
+  }
+  if (was_dry) d.fdry[c] = 0;
+  return true;
+}
+
+// A cell with an operand k_grad's own arithmetic leaves out (see Den, Limit3), by
+// cell_gradients.
+template <class R>
+__device__ __noinline__ void grad_careful(const Dev& d, const Geo<R>& G, const Rec* __restrict__ q, int c,
+                                          bool mark, double* __restrict__ rku_prev, double* __restrict__ rkv_prev) {
+  const int T = d.T, ln = c & 31;
+  const GradBlock<R>& B = reinterpret_cast<const GradBlock<R>*>(d.gblk)[c >> 5];
+  const Rec own = ld_rec(q + c);
+  const bool dry_c = rec_dry(d, own);
+  int t3[3];
+  for (int j = 0; j < 3; j++) t3[j] = B.id[j][ln];
+  const GradOut<R> g = cell_gradients<R>(d, G, NbGlobal{d, q}, c, c, t3, [&](int k) { return d.st_id[k * T + c]; },
+                                         [&](int) { return !mark; }, (R*)nullptr, (R*)nullptr);
+  const double x = d.flux == STORM_FLUX_RUSANOV ? (dry_c ? kZero : sqrt(kG * own.h)) : own.z;
+  store_grad<R>(d, G, B, ln, c, g, own, dry_c, (B.nst[ln] & kNstBc) != 0, rku_prev, rkv_prev, x);
+}
+
+// The constants of GradBlock from the per-cell columns (once per handle).
+template <class R>
+__global__ void __launch_bounds__(256) k_pack_geo(Dev d, Geo<R> G) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= d.T) return;
+  const int T = d.T, ln = c & 31;
+  GradBlock<R>& B = reinterpret_cast<GradBlock<R>*>(d.gblk)[c >> 5];
+  for (int k = 0; k < 3; k++) {
+    const int q = k * T + c;
+    const bool st = k < d.kst;  // meshes whose largest stencil is smaller have no such row
+    B.w[k][ln] = st ? G.st_w[q] : R(0);
+    B.dx[k][ln] = st ? G.st_dx[q] : R(0);
+    B.dy[k][ln] = st ? G.st_dy[q] : R(0);
+    B.rx[k][ln] = G.rc_x[q];
+    B.ry[k][ln] = G.rc_y[q];
+    B.id[k][ln] = d.t2t3[q];
+    B.fpos[k][ln] = d.fpos[q];
+  }
+  B.dzx[ln] = G.delz_x[c];
+  B.dzy[ln] = G.delz_y[c];
+  B.zmax[ln] = d.zmax[c];
+  B.nst[ln] = d.nst[c];
+}
+
+// The LSQ sums of a cell over its stencil (lsq_grad_array.f90:60-73); FP64 also the
+// sums lsq_a, b, c are made of.
+template <class R>
+struct LsqSums {
+  double sa = 0.0, sb = 0.0, sc = 0.0;
+  R zx = R(0), zy = R(0), ux = R(0), uy = R(0), vx = R(0), vy = R(0);
+  __device__ __forceinline__ void add(const Rec& n, const Rec& own, R w, R dx, R dy) {
+    const double zeta_c = own.h + own.z;
+    const R pz = (R)((n.h + n.z) - zeta_c), pu = (R)(n.u - own.u), pv = (R)(n.v - own.v);
+    zx = zx + w * pz * dx;
+    zy = zy + w * pz * dy;
+    ux = ux + w * pu * dx;
+    uy = uy + w * pu * dy;
+    vx = vx + w * pv * dx;
+    vy = vy + w * pv * dy;
+    if (sizeof(R) == 8) {
+      sa = sa + (double)w * (double)dx * (double)dx;
+      sb = sb + (double)w * (double)dx * (double)dy;
+      sc = sc + (double)w * (double)dy * (double)dy;
+    }
+  }
+};
+
+// ... over a listed stencil of n cells, four at a time: their indices and weights, then
+// the cells.
+template <class R>
+__device__ __forceinline__ LsqSums<R> lsq_sums_listed(const Dev& d, const Geo<R>& G, const Rec* __restrict__ q, const Rec& own,
+                                                       int c, int n) {
+  LsqSums<R> S;
+  for (int k0 = 0; k0 < n; k0 += 4) {
+    int j[4];
+    R w[4], dx[4], dy[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const int r = (k0 + k < n ? k0 + k : k0) * d.T + c;
+      j[k] = d.st_id[r];
+      w[k] = G.st_w[r];
+      dx[k] = G.st_dx[r];
+      dy[k] = G.st_dy[r];
+    }
+    const Rec m[4] = {ld_rec(q + j[0]), ld_rec(q + j[1]), ld_rec(q + j[2]), ld_rec(q + j[3])};
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+      if (k0 + k < n) S.add(m[k], own, w[k], dx[k], dy[k]);
+  }
+  return S;
+}
+
+// Steady runs: the local time step of a cell from its stage input (solverFVT.f90:259-270).
+__device__ __forceinline__ double local_dt(const Dev& d, const Rec& own, bool dry_c, double area, double perim) {
+  const double um = (own.h < d.h_dry) ? kZero : qsqrt(own.u * own.u + own.v * own.v);
+  const double wc = dry_c ? kZero : sqrt(kG * own.h);
+  double delt = um + wc;
+  if (delt < SMALL_F) delt = 1.044;
+  return d.cfl * area / (delt * perim);
+}
+
+// Gradients of every cell and the face states made from them (phase path): the sums and
+// the limiter of cell_gradients in the same order, the same bits, without the terms
+// nothing reads (a gradient that hgradfix2 replaces, a dry cell's velocities).  The cells
+// whose stencil is their three face neighbours in slot order (HostLayout::plain) take
+// their constants from one bulk copy per warp.
+// The other cells (along the mesh boundary, with longer stencils) have blocks of their
+// own, the first of the grid: a warp that held one of them would take several times as
+// long as its neighbours.
+//
+// What bounds it is latency: about 1,100 instructions a warp, a third of them FP64, on
+// data two dependent loads away.  80 registers and 24 warps an SM without spills beat 40
+// warps that spill (the spills were more L2 traffic than the mesh).  Two-million-cell
+// meander, per stage: 156 us with the constants read column by column, the boundary
+// cells among the others and 48 registers; 116 us as it stands (98 us before the
+// boundary cells' launch, which the graph runs beside it).
+// Two passes over the neighbours, the second reading them again from L1: the registers
+// of one pass do not have to live through the other, so nothing is spilled.
+#define PHASE_BARRIER() asm volatile("" ::: "memory")
+template <class R, bool kGen>
+__global__ void __launch_bounds__(256, 3) k_grad(const __grid_constant__ Dev d, const __grid_constant__ Geo<R> G,
+                                                  int s, const Rec* __restrict__ q, double* __restrict__ rku_prev,
+                                                  double* __restrict__ rkv_prev) {
+  extern __shared__ __align__(128) unsigned char grad_smem[];
+  __shared__ uint64_t bars[8];
+  const int ln = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  GradBlock<R>& B = reinterpret_cast<GradBlock<R>*>(grad_smem)[wp];
+  int c, nst, id0, id1, id2;
+  if (kGen) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= d.ngen) return;
+    c = d.gen_cells[i];
+    const GradBlock<R>& S = reinterpret_cast<const GradBlock<R>*>(d.gblk)[c >> 5];
+    const int l = c & 31;
+    nst = S.nst[l];
+    id0 = S.id[0][l];
+    id1 = S.id[1][l];
+    id2 = S.id[2][l];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {  // the columns the later steps read (this thread's own)
+      B.rx[k][ln] = S.rx[k][l];
+      B.ry[k][ln] = S.ry[k][l];
+      B.fpos[k][ln] = S.fpos[k][l];
+    }
+    B.dzx[ln] = S.dzx[l];
+    B.dzy[ln] = S.dzy[l];
+    B.zmax[ln] = S.zmax[l];
+  } else {
+    c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c - ln >= d.T) return;  // whole warps: the cell slots come in blocks of 256
+    // the warp's block of constants, one bulk copy beside the state loads below
+    const GradBlock<R>* src = reinterpret_cast<const GradBlock<R>*>(d.gblk) + (c >> 5);
+    if (ln == 0) {
+      umma::mbar_init(&bars[wp], 1);
+      umma::fence_async_smem();
+      // first order reads no stencil weights: the copy starts behind them
+      const uint32_t skip = d.lim == 0 ? (uint32_t)offsetof(GradBlock<R>, rx) : 0, n = sizeof(GradBlock<R>) - skip;
+      umma::mbar_expect(&bars[wp], n);
+      umma::bulk_load(reinterpret_cast<unsigned char*>(&B) + skip, reinterpret_cast<const unsigned char*>(src) + skip, n,
+                      &bars[wp]);
+    }
+    id0 = src->id[0][ln];
+    id1 = src->id[1][ln];
+    id2 = src->id[2][ln];
+    nst = src->nst[ln];
+  }
+  id0 = id0 < 0 ? c : id0;  // a face without a neighbour takes the cell's own values
+  id1 = id1 < 0 ? c : id1;
+  id2 = id2 < 0 ? c : id2;
+  const Rec own = ld_rec_again(q + c);
+  const bool was_dry = d.fdry[c] != 0, mark = d.cmark[c] != 0;
+  const bool live = cell_live(d, c);
+  const bool bc = (nst & kNstBc) != 0;
+  if (!kGen) {
+    __syncwarp();
+    if (!umma::mbar_wait(&bars[wp], 0)) {  // cannot happen: a copy within this GPU
+      if (live) atomicOr(&d.sc[cell_scenario(d, c)].status, 4);
+      umma::mbar_wait(&bars[wp], 0);
+      return;
+    }
+    if (!(nst & kNstPlain)) return;
+  }
+  if (!live) return;
+  const bool dry_c = rec_dry(d, own);
+  // steady runs: the friction step's dt is the last element's local one of the last
+  // stage, set here because the last stage's cell kernel also does the friction step
+  if (sizeof(R) == 8 && (nst & kNstLast) && s == d.K && d.steady)
+    d.sc[cell_scenario(d, c)].delt_fric = local_dt(d, own, dry_c, d.area[c], d.perim[c]);
+  if (!grad_begin<R>(d, B, ln, c, s, own, dry_c, was_dry, bc)) return;
+  if (mark) d.cmark[c] = 0;
+  constexpr bool kF64 = sizeof(R) == 8;
+  const bool vel = !dry_c || bc;
+  const double x = d.flux == STORM_FLUX_RUSANOV ? (dry_c ? kZero : sqrt(kG * own.h)) : own.z;
+  const double zeta_c = own.h + own.z;
+  bool bad = false;
+  GradOut<R> o;
+  o.ub = own.u;
+  o.vb = own.v;
+  o.hx = o.hy = o.ux = o.uy = o.vx = o.vy = R(0);
+  o.fix = false;
+  if (!dry_c) {
+    if (zeta_c < B.zmax[ln]) {  // hgradfix2.f90:48-98
+      const Rec n0 = ld_rec_again(q + id0), n1 = ld_rec_again(q + id1), n2 = ld_rec_again(q + id2);
+      const bool free = (rec_dry(d, n0) && n0.z < zeta_c) || (rec_dry(d, n1) && n1.z < zeta_c) ||
+                        (rec_dry(d, n2) && n2.z < zeta_c);
+      o.fix = !free;
+    }
+    if (o.fix || mark) {  // to_vertices.f90:44-55
+      o.ub = kZero;
+      o.vb = kZero;
+    }
+  }
+  if (o.fix) {
+    o.hx = -B.dzx[ln];
+    o.hy = -B.dzy[ln];
+  } else {
+    if (d.lim == 1 || d.lim == 2) {
+      R ai, bi, ci, det;
+      {
+        LsqSums<R> S;
+        if (!kGen) {
+          const Rec n[3] = {ld_rec(q + id0), ld_rec(q + id1), ld_rec(q + id2)};
+#pragma unroll
+          for (int k = 0; k < 3; k++) S.add(n[k], own, B.w[k][ln], B.dx[k][ln], B.dy[k][ln]);
+        } else {
+          S = lsq_sums_listed<R>(d, G, q, own, c, nst & kNstCount);
+        }
+        if (kF64 && d.lsq_derived) {
+          ai = (R)S.sa;
+          bi = (R)S.sb;
+          ci = (R)S.sc;
+          det = (R)(S.sa * S.sc - S.sb * S.sb);
+        } else {
+          ai = G.lsq_a[c];
+          bi = G.lsq_b[c];
+          ci = G.lsq_c[c];
+          det = G.lsq_det[c];
+        }
+        const Den<R> den(det, &bad);
+        o.hx = den.quot(ci * S.zx - bi * S.zy, &bad);
+        o.hy = den.quot(ai * S.zy - S.zx * bi, &bad);
+        if (vel) {
+          o.ux = den.quot(ci * S.ux - bi * S.uy, &bad);
+          o.uy = den.quot(ai * S.uy - S.ux * bi, &bad);
+          o.vx = den.quot(ci * S.vx - bi * S.vy, &bad);
+          o.vy = den.quot(ai * S.vy - S.vx * bi, &bad);
+        }
+      }
+      if (d.lim == 2) {  // limiterBJ.f90:42-81, beta = one
+        PHASE_BARRIER();
+        Limit3<R> lz, lu, lv;
+        const Rec nn[3] = {ld_rec_again(q + id0), ld_rec_again(q + id1), ld_rec_again(q + id2)};
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+          const Rec& n = nn[j];
+          const R rx = B.rx[j][ln], ry = B.ry[j][ln];
+          lz.face(zeta_c, n.h + n.z, o.hx, o.hy, rx, ry, &bad);
+          if (vel) {
+            lu.face(own.u, n.u, o.ux, o.uy, rx, ry, &bad);
+            lv.face(own.v, n.v, o.vx, o.vy, rx, ry, &bad);
+          }
+        }
+        const R mz = lz.value(&bad);
+        o.hx = mz * o.hx;
+        o.hy = mz * o.hy;
+        if (vel) {
+          const R mu = lu.value(&bad), mv = lv.value(&bad);
+          o.ux = mu * o.ux;
+          o.uy = mu * o.uy;
+          o.vx = mv * o.vx;
+          o.vy = mv * o.vy;
+        }
+      }
+    }
+    o.hx = o.hx - B.dzx[ln];
+    o.hy = o.hy - B.dzy[ln];
+  }
+  PHASE_BARRIER();
+  if (bad) {
+    grad_careful<R>(d, G, q, c, mark, rku_prev, rkv_prev);
+    return;
+  }
+  store_grad<R>(d, G, B, ln, c, o, own, dry_c, bc, rku_prev, rkv_prev, x);
+}
+
+// Gradients of the cells with an open-boundary face (fused path: for k_bc on the side
+// stream, beside the tiles that compute every cell's).
+template <class R>
+__global__ void __launch_bounds__(128) k_grad_bc(Dev d, Geo<R> G, const Rec* __restrict__ q,
+                                                 double* __restrict__ rku_prev, double* __restrict__ rkv_prev) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= d.nbc_cells) return;
+  const int c = d.bc_cells[i];
   if (!cell_live(d, c)) return;
   const int T = d.T;
-  const NbGlobal nb{hs, d.z, u_in, v_in, dry};
+  const NbGlobal nb{d, q};
   int t3[3];
 #pragma unroll
   for (int j = 0; j < 3; j++) t3[j] = d.t2t3[j * T + c];
@@ -795,11 +1366,15 @@ __global__ void __launch_bounds__(256, 5) k_grad(Dev d, Geo<R> G, const double* 
   G.delh_x[c] = g.hx; G.delh_y[c] = g.hy;
   G.delu_x[c] = g.ux; G.delu_y[c] = g.uy;
   G.delv_x[c] = g.vx; G.delv_y[c] = g.vy;
-  if (sizeof(R) == 8) {
-    d.vzero[c] = g.vz;
-  } else {
-    d.u_b[c] = g.ub;
-    d.v_b[c] = g.vb;
+  d.u_b[c] = g.ub;
+  d.v_b[c] = g.vb;
+  for (int m = 0; m < 3; m++) {  // slip walls: the record k_flux_bc reads
+    const int p = d.fpos[m * T + c];
+    if (p < 2 * d.ne) continue;
+    const R rx = G.rc_x[m * T + c], ry = G.rc_y[m * T + c];
+    Rec r{recon(q[c].h, g.hx, rx, g.hy, ry), kZero, recon(g.ub, g.ux, rx, g.uy, ry), recon(g.vb, g.vx, rx, g.vy, ry)};
+    if (r.h < kZero) r.h = kZero;
+    st_rec(d.fs + p, r);
   }
 }
 
@@ -811,9 +1386,7 @@ __global__ void __launch_bounds__(256, 5) k_grad(Dev d, Geo<R> G, const double* 
 constexpr int kBcThreads = 128;
 
 template <class R>
-__global__ void __launch_bounds__(kBcThreads) k_bc(Dev d, Geo<R> G, const double* __restrict__ hs,
-                                                   const uint8_t* __restrict__ dry, const double* __restrict__ u_in,
-                                                   const double* __restrict__ v_in) {
+__global__ void __launch_bounds__(kBcThreads) k_bc(Dev d, Geo<R> G, const Rec* __restrict__ rec) {
   const int b = blockIdx.x;
   Scalars* const sc = &d.sc[d.bdr_sid[b]];
   if (sc->converged) return;
@@ -831,9 +1404,9 @@ __global__ void __launch_bounds__(kBcThreads) k_bc(Dev d, Geo<R> G, const double
   for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
     const int i = d.bce_cell[off + e], m = d.bce_slot[off + e];
     const int q = m * T + i;
-    d.bc_rec[off + e] = recon(hs[i], G.delh_x[i], G.rc_x[q], G.delh_y[i], G.rc_y[q]);
-    d.bc_rec[NB + off + e] = recon(post_fix<R>(d, u_in, d.u_b, i), G.delu_x[i], G.rc_x[q], G.delu_y[i], G.rc_y[q]);
-    d.bc_rec[2 * NB + off + e] = recon(post_fix<R>(d, v_in, d.v_b, i), G.delv_x[i], G.rc_x[q], G.delv_y[i], G.rc_y[q]);
+    d.bc_rec[off + e] = recon(rec[i].h, G.delh_x[i], G.rc_x[q], G.delh_y[i], G.rc_y[q]);
+    d.bc_rec[NB + off + e] = recon(d.u_b[i], G.delu_x[i], G.rc_x[q], G.delu_y[i], G.rc_y[q]);
+    d.bc_rec[2 * NB + off + e] = recon(d.v_b[i], G.delv_x[i], G.rc_x[q], G.delv_y[i], G.rc_y[q]);
   }
   __syncthreads();
   auto put = [&](int e, double c1, double c2, double c3) {
@@ -862,7 +1435,7 @@ __global__ void __launch_bounds__(kBcThreads) k_bc(Dev d, Geo<R> G, const double
     uint8_t* v0 = okc + cnt;               // [cnt] wet-only mask
     for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
       const int i = d.bce_cell[off + e];
-      const bool dr = dry[i];
+      const bool dr = rec_dry(d, rec[i]);
       v0[e] = !(wet_only && dr);
       const double hleft = dr ? kZero : fmax2(d.bc_rec[off + e], kZero);
       tA[e] = hleft * d.bce_len[off + e];
@@ -982,7 +1555,7 @@ __global__ void __launch_bounds__(kBcThreads) k_bc(Dev d, Geo<R> G, const double
     }
     for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
       const int i = d.bce_cell[off + e];
-      const bool dr = dry[i];
+      const bool dr = rec_dry(d, rec[i]);
       ok[e] = !(wet_only && dr);
       double hleft = dr ? kZero : fmax2(d.bc_rec[off + e], kZero);
       tA[e] = hleft * d.bce_len[off + e];
@@ -1004,7 +1577,7 @@ __global__ void __launch_bounds__(kBcThreads) k_bc(Dev d, Geo<R> G, const double
       const double atotal = s_atotal;
       for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
         const int i = d.bce_cell[off + e];
-        bool valid = !(wet_only && dry[i]);
+        bool valid = !(wet_only && rec_dry(d, rec[i]));
         double hleft = null_area ? sc->bch_max : d.bc_rec[off + e], uedg, vedg;
         if (hleft < h_dry) {
           hleft = fmax2(hleft, kZero);
@@ -1050,7 +1623,7 @@ __global__ void __launch_bounds__(kBcThreads) k_bc(Dev d, Geo<R> G, const double
     const double atotal = newatotal;  // :130
     for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
       const int i = d.bce_cell[off + e];
-      bool valid = !(wet_only && dry[i]);
+      bool valid = !(wet_only && rec_dry(d, rec[i]));
       double hleft = null_area ? sc->bch_max : d.bc_rec[off + e], uedg, vedg;
       if (hleft < h_dry) {
         hleft = fmax2(hleft, kZero);
@@ -1093,7 +1666,7 @@ __global__ void __launch_bounds__(kBcThreads) k_bc(Dev d, Geo<R> G, const double
   // The remaining routines have no cross-edge coupling.
   for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
     const int i = d.bce_cell[off + e];
-    const bool dr = dry[i];
+    const bool dr = rec_dry(d, rec[i]);
     const double nx = d.bce_nx[off + e], ny = d.bce_ny[off + e];
     const double tx = d.bce_tx[off + e], ty = d.bce_ty[off + e];
     const double len = d.bce_len[off + e], zmid = d.bce_zmid[off + e];
@@ -1104,7 +1677,7 @@ __global__ void __launch_bounds__(kBcThreads) k_bc(Dev d, Geo<R> G, const double
     if (kind == BC_HIN) {  // inflowH.f90:28-93
       double uedg, vedg;
       hleft = fmax2(hleft, kZero);
-      if (hs[i] < h_dry) { uedg = kZero; vedg = kZero; }
+      if (rec[i].h < h_dry) { uedg = kZero; vedg = kZero; }
       else { uedg = ur0; vedg = vr0; }
       const double hright = fmax2(kZero, sc->qin[slot] - zmid);
       double uleft = uedg * nx + vedg * ny;
@@ -1180,7 +1753,7 @@ __global__ void __launch_bounds__(kBcThreads) k_bc(Dev d, Geo<R> G, const double
       hleft = fmax2(hleft, kZero);
       if (hleft < h_dry) valid = false;
       else {
-        if (hs[i] < h_dry) { uedg = kZero; vedg = kZero; }
+        if (rec[i].h < h_dry) { uedg = kZero; vedg = kZero; }
         else { uedg = ur0; vedg = vr0; }
         const double uleft = uedg, vleft = vedg;
         double hright = hleft, uright = uleft, vright = vleft;
@@ -1213,28 +1786,14 @@ struct EdgeState {
   double h, u, v;
 };
 
-template <class R>
-__device__ __forceinline__ EdgeState edge_state(const Dev& d, const Geo<R>& G, const double* __restrict__ hs,
-                                                const double* __restrict__ u_in, const double* __restrict__ v_in,
-                                                int x, int m) {
-  const int q = m * d.T + x;
-  const R rx = G.rc_x[q], ry = G.rc_y[q];
-  EdgeState s;
-  s.h = recon(hs[x], G.delh_x[x], rx, G.delh_y[x], ry);
-  if (s.h < kZero) s.h = kZero;
-  s.u = recon(post_fix<R>(d, u_in, d.u_b, x), G.delu_x[x], rx, G.delu_y[x], ry);
-  s.v = recon(post_fix<R>(d, v_in, d.v_b, x), G.delv_x[x], rx, G.delv_y[x], ry);
-  return s;
-}
-
 // invisc_fluxes.f90:39-147 for an interior edge from its two face states: left =
-// e(1), right = e(2), dl/dr their dry flags, zl/zr their bed elevations and hl/hr
-// their cell depths (Rusanov's cell celerities); returns false when the edge is
+// e(1), right = e(2), dl/dr their dry flags, zl/zr their bed elevations and cl/cr
+// their cells' celerities (Rusanov; zero when dry); returns false when the edge is
 // skipped.  The wet/dry tests and the I1 stage comparison run on the FP64 face
 // states; the flux function in R.
 template <class R>
 __device__ __forceinline__ bool edge_flux(const Dev& d, bool dl, bool dr, const EdgeState& sl, const EdgeState& sr,
-                                          double zl, double zr, double hl, double hr, R nx, R ny, double z0e, R* f,
+                                          double zl, double zr, double cl, double cr, R nx, R ny, double z0e, R* f,
                                           bool* bad) {
   if (dl && dr) return false;
   double hleft = kZero, uleft = kZero, vleft = kZero, hright = kZero, uright = kZero, vright = kZero;
@@ -1262,139 +1821,160 @@ __device__ __forceinline__ bool edge_flux(const Dev& d, bool dl, bool dr, const 
   } else if (d.flux == STORM_FLUX_HLL) {
     flux_hll<R>(nx, ny, (R)hleft, (R)uleft, (R)vleft, (R)hright, (R)uright, (R)vright, (R)d.h_dry, f, bad);
   } else if (d.flux == STORM_FLUX_RUSANOV) {
-    const R cl = dl ? R(kZero) : (R)sqrt(kG * hl);  // wavec (solverFVT.f90:180-181)
-    const R cr = dr ? R(kZero) : (R)sqrt(kG * hr);
-    flux_rusanov<R>(nx, ny, (R)hleft, (R)uleft, (R)vleft, cl, (R)hright, (R)uright, (R)vright, cr, f);
+    flux_rusanov<R>(nx, ny, (R)hleft, (R)uleft, (R)vleft, (R)cl, (R)hright, (R)uright, (R)vright, (R)cr, f);
   } else {
-    flux_roe<R>(nx, ny, (R)hleft, (R)uleft, (R)vleft, (R)hright, (R)uright, (R)vright, f);
+    flux_roe_edge(nx, ny, (R)hleft, (R)uleft, (R)vleft, (R)hright, (R)uright, (R)vright, f);
   }
   return true;
 }
 
-// The same for the edge between L=e(1) (slot ml) and R=e(2) (slot mr), with the face
-// states reconstructed from the stored gradients.
+// The flux of interior edge e (invisc_fluxes.f90:39-147) in the reference's orientation
+// (left = edges(k)%e(1)) from its two face records; false when the edge is skipped.
 template <class R>
-__device__ __forceinline__ bool interior_flux(const Dev& d, const Geo<R>& G, const double* __restrict__ hs,
-                                              const uint8_t* __restrict__ dry, const double* __restrict__ u_in,
-                                              const double* __restrict__ v_in, int L, int ml, int Rc, int mr, R nx,
-                                              R ny, double z0e, R* f, bool* bad) {
-  const bool dl = dry[L], dr = dry[Rc];
-  if (dl && dr) return false;
-  EdgeState sl{kZero, kZero, kZero}, sr{kZero, kZero, kZero};
-  if (!dl) sl = edge_state(d, G, hs, u_in, v_in, L, ml);
-  if (!dr) sr = edge_state(d, G, hs, u_in, v_in, Rc, mr);
-  return edge_flux<R>(d, dl, dr, sl, sr, d.z[L], d.z[Rc], hs[L], hs[Rc], nx, ny, z0e, f, bad);
-}
-
-// Interior-edge fluxes of one stage (invisc_fluxes.f90:39-147), one thread per edge:
-// the flux of edge k is evaluated once, in the reference's orientation (left =
-// edges(k)%e(1)), and stored as f*length, the amount the reference subtracts from
-// phi(e(1),:) and adds to phi(e(2),:).
-template <class R>
-__global__ void __launch_bounds__(128, 8) k_eflux(Dev d, Geo<R> G, const double* __restrict__ hs,
-                                               const uint8_t* __restrict__ dry, const double* __restrict__ u_in,
-                                               const double* __restrict__ v_in) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= d.ne) return;
-  if (!item_live(d, d.edge_sid, e)) return;
-  const int L = d.eL[e], Rc = d.eR[e];
-  const uint8_t sl = d.eslot[e];
-  R f[3];
-  bool bad = false;
-  const bool ok = interior_flux<R>(d, G, hs, dry, u_in, v_in, L, sl & 3, Rc, (sl >> 2) & 3, G.enx[e], G.eny[e],
-                                   (dry[L] || dry[Rc]) ? d.ez0[e] : kZero, f, &bad);
-  d.eok[e] = ok;
-  if (ok) {
-    const R len = G.elen[e];
-    G.efx[e] = f[0] * len;
-    G.efx[d.ne + e] = f[1] * len;
-    G.efx[2 * d.ne + e] = f[2] * len;
+__device__ __forceinline__ bool interior_flux(const Dev& d, const Geo<R>& G, int e, R* f, bool* bad) {
+  const Rec a = ld_rec(d.fs + 2 * (size_t)e), b = ld_rec(d.fs + 2 * (size_t)e + 1);
+  const R nx = G.enx[e], ny = G.eny[e];
+  const bool dl = a.h == -kOne, dr = b.h == -kOne, rus = d.flux == STORM_FLUX_RUSANOV;
+  double zl = a.z, zr = b.z, z0 = kZero;
+  if (dl || dr) {
+    z0 = d.ez0[e];
+    if (rus) {
+      zl = d.z[d.eL[e]];
+      zr = d.z[d.eR[e]];
+    }
   }
-  if (bad) atomicOr(&d.sc[d.edge_sid[e]].status, 2);
+  return edge_flux<R>(d, dl, dr, EdgeState{a.h, a.u, a.v}, EdgeState{b.h, b.u, b.v}, zl, zr, a.z, b.z, nx, ny, z0, f,
+                      bad);
 }
 
 // bed_slope_STD.f90:23-70 with adjustZb.f90:41-70: the amounts g*h*gradzb*area that
-// are subtracted from phi(i,2:3), from the cell's depth gradient (dhx, dhy).  The
-// vertex offsets from the centroid (node - centroid, the reference's own differences)
-// are precomputed per cell; the adjust test (a negative reconstructed vertex depth)
-// and the adjusted gradient run in double on both paths.
-__device__ __forceinline__ void bed_source(const Dev& d, const Geo<double>& G, int c, double h_c, double dhx,
-                                           double dhy, double* s2, double* s3) {
-  const int T = d.T;
-  double hp[3];
-  bool adjust = false;
-#pragma unroll
-  for (int i = 0; i < 3; i++) {
-    const int q = i * T + c;
-    hp[i] = h_c + dhx * d.vox[q] + dhy * d.voy[q];
-    if (hp[i] < kZero) adjust = true;
-  }
-  double gx, gy;
-  if (adjust) {
-    double zp[3], x[3], y[3];
-#pragma unroll
-    for (int i = 0; i < 3; i++) {
-      const int vid = d.vert[i * T + c];
-      hp[i] = fmin2(kZero, hp[i]);
-      zp[i] = d.zvtx[vid] + hp[i];
-      x[i] = d.node_x[vid];
-      y[i] = d.node_y[vid];
-    }
-    const double b1 = y[1] - y[2], c1 = x[2] - x[1];
-    const double b2 = y[2] - y[0], c2 = x[0] - x[2];
-    const double b3 = y[0] - y[1], c3 = x[1] - x[0];
-    const double a = kHalf / d.area[c];
-    gx = a * (b1 * zp[0] + b2 * zp[1] + b3 * zp[2]);
-    gy = a * (c1 * zp[0] + c2 * zp[1] + c3 * zp[2]);
-  } else {
-    gx = G.delz_x[c];
-    gy = G.delz_y[c];
-  }
-  *s2 = kG * h_c * gx * d.area[c];
-  *s3 = kG * h_c * gy * d.area[c];
+// are subtracted from phi(i,2:3), from the cell's depth gradient (dhx, dhy) and its bed
+// gradient (zx, zy).  The vertex offsets from the centroid (node - centroid, the
+// reference's own differences) are precomputed per cell; the adjust test (a negative
+// reconstructed vertex depth) and the adjusted gradient run in double on both paths.
+// rad bounds the offsets' components: where the depth exceeds what the gradient can take
+// off within it (by more than any rounding) no vertex depth is negative, and the offsets
+// are not read.
+__device__ __forceinline__ bool bed_plain(double h_c, double dhx, double dhy, float rad) {
+  return h_c > (fabs(dhx) + fabs(dhy)) * (double)rad * 1.00001;
 }
-__device__ __forceinline__ void bed_source(const Dev& d, const Geo<float>& G, int c, double h_c, float dhx,
-                                           float dhy, double* s2, double* s3) {
+// adjustZb's gradient from the vertex depths hp; false: none is negative
+__device__ __forceinline__ bool bed_adjusted(const Dev& d, int c, const double (&hp)[3], double area, double* gx,
+                                             double* gy) {
+  if (!(hp[0] < kZero) && !(hp[1] < kZero) && !(hp[2] < kZero)) return false;
   const int T = d.T;
-  double hp[3];
-  bool adjust = false;
+  double zp[3], x[3], y[3];
 #pragma unroll
   for (int i = 0; i < 3; i++) {
-    const int q = i * T + c;
-    hp[i] = h_c + (double)(dhx * G.vox[q] + dhy * G.voy[q]);
-    if (hp[i] < kZero) adjust = true;
+    const int vid = d.vert[i * T + c];
+    zp[i] = d.zvtx[vid] + fmin2(kZero, hp[i]);
+    x[i] = d.node_x[vid];
+    y[i] = d.node_y[vid];
   }
-  if (adjust) {
-    double zp[3], x[3], y[3];
+  const double b1 = y[1] - y[2], c1 = x[2] - x[1];
+  const double b2 = y[2] - y[0], c2 = x[0] - x[2];
+  const double b3 = y[0] - y[1], c3 = x[1] - x[0];
+  const double a = kHalf / area;
+  *gx = a * (b1 * zp[0] + b2 * zp[1] + b3 * zp[2]);
+  *gy = a * (c1 * zp[0] + c2 * zp[1] + c3 * zp[2]);
+  return true;
+}
+__device__ __forceinline__ void bed_source(const Dev& d, int c, double h_c, double dhx, double dhy, double zx,
+                                           double zy, double area, float rad, const Geo<double>&, double* s2,
+                                           double* s3) {
+  double gx = zx, gy = zy;
+  if (!bed_plain(h_c, dhx, dhy, rad)) {
+    double hp[3];
 #pragma unroll
     for (int i = 0; i < 3; i++) {
-      const int vid = d.vert[i * T + c];
-      zp[i] = d.zvtx[vid] + fmin2(kZero, hp[i]);
-      x[i] = d.node_x[vid];
-      y[i] = d.node_y[vid];
+      const int q = i * d.T + c;
+      hp[i] = h_c + dhx * d.vox[q] + dhy * d.voy[q];
     }
-    const double a = kHalf / d.area[c];
-    const double gx = a * ((y[1] - y[2]) * zp[0] + (y[2] - y[0]) * zp[1] + (y[0] - y[1]) * zp[2]);
-    const double gy = a * ((x[2] - x[1]) * zp[0] + (x[0] - x[2]) * zp[1] + (x[1] - x[0]) * zp[2]);
-    *s2 = kG * h_c * gx * d.area[c];
-    *s3 = kG * h_c * gy * d.area[c];
-  } else {
-    const float ga = 9.81f * (float)h_c * (float)d.area[c];
-    *s2 = (double)(ga * G.delz_x[c]);
-    *s3 = (double)(ga * G.delz_y[c]);
+    bed_adjusted(d, c, hp, area, &gx, &gy);
   }
+  *s2 = kG * h_c * gx * area;
+  *s3 = kG * h_c * gy * area;
+}
+__device__ __forceinline__ void bed_source(const Dev& d, int c, double h_c, float dhx, float dhy, float zx, float zy,
+                                           double area, float rad, const Geo<float>& G, double* s2, double* s3) {
+  if (!bed_plain(h_c, (double)dhx, (double)dhy, rad)) {
+    double hp[3], gx, gy;
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+      const int q = i * d.T + c;
+      hp[i] = h_c + (double)(dhx * G.vox[q] + dhy * G.voy[q]);
+    }
+    if (bed_adjusted(d, c, hp, area, &gx, &gy)) {
+      *s2 = kG * h_c * gx * area;
+      *s3 = kG * h_c * gy * area;
+      return;
+    }
+  }
+  const float ga = 9.81f * (float)h_c * (float)area;
+  *s2 = (double)(ga * zx);
+  *s3 = (double)(ga * zy);
+}
+
+// Wall terms: f2 len and f3 len are subtracted from phi(i,2:3); zero where the routine
+// skips the edge.
+// wenslp3_fluxes.f90:34-67, from the vertex depths at the edge's ends
+__device__ __forceinline__ void wall_noslip(const Dev& d, double h1, double h2, double nx, double ny, double* f2,
+                                            double* f3) {
+  double hedge = qsqrt((h1 * h1 + h1 * h2 + h2 * h2) * kOneThird);
+  if (hedge < kZero) hedge = kZero;
+  const bool skip = hedge < d.h_dry;
+  *f2 = skip ? kZero : kHalf * kG * hedge * hedge * nx;
+  *f3 = skip ? kZero : kHalf * kG * hedge * hedge * ny;
+}
+// weslp2_fluxes.f90:34-76, from the cell's own reconstructed state at the edge
+__device__ __forceinline__ void wall_slip(const Dev& d, const EdgeState& o, double nx, double ny, double* f2,
+                                          double* f3) {
+  *f2 = *f3 = kZero;
+  const double hleft = o.h;
+  if (hleft < d.h_dry) return;
+  const double tx = -ny, ty = nx;  // edges%tang flipped with the normal
+  double uright = o.u * tx + o.v * ty;
+  uright = uright + 2.0 * sqrt(kG * hleft);
+  const double hright = uright * uright / 4.0 / kG;
+  const double g2 = kHalf * kG * hright * hright * nx;
+  const double g3 = kHalf * kG * hright * hright * ny;
+  const double dh = kZero;
+  *f2 = g2 + dh * nx;
+  *f3 = g3 + dh * ny;
+}
+__device__ __forceinline__ void wall_flux(const Dev& d, const WallRec& w, double* f2, double* f3) {
+  *f2 = *f3 = kZero;
+  if (rec_dry(d, d.q[w.cell])) return;
+  if (d.btype == 0) {
+    wall_noslip(d, d.hvtx[w.p1], d.hvtx[w.p2], w.nx, w.ny, f2, f3);
+  } else {
+    const Rec r = ld_rec(d.fs + w.rec);
+    wall_slip(d, EdgeState{r.h, r.u, r.v}, w.nx, w.ny, f2, f3);
+  }
+}
+// culvert sources and sinks (solverFVT.f90:227-233) of cell c added to p1
+__device__ __forceinline__ double culvert_terms(const Dev& d, int c, double p1) {
+  int lo = 0, hi = d.ncvc;  // first term of cell c
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (d.cvc_cell[mid] < c) lo = mid + 1;
+    else hi = mid;
+  }
+  for (int k = lo; k < d.ncvc && d.cvc_cell[k] == c; k++) {
+    const int code = d.cvc_code[k];
+    if (code & 1) p1 = p1 + d.cvsrc[code >> 1];
+    else p1 = p1 - d.cvsrc[code >> 1];
+  }
+  return p1;
 }
 
 // Where the face contributions of a cell come from: the phase kernels' global arrays
-// (edge fluxes of k_eflux, stored gradients) ...
-template <class R>
+// (edge fluxes from the face records or left by k_tile, stored gradients) ...
+template <class R, bool kTile>
 struct FacesGlobal {
   const Dev& d;
   const Geo<R>& G;
-  const double* __restrict__ hs;
   int c;
-  const double* __restrict__ u_in;  // stage-input velocities (the cell's own, for weslp2 walls)
-  const double* __restrict__ v_in;
   // the faces in the order their terms are added (slots, kinds, references), read
   // from the per-cell arrays kept in that order so that none waits on forder
   __device__ __forceinline__ uint8_t order(int (&fj)[3], int (&fkd)[3], int (&fe)[3]) const {
@@ -1410,19 +1990,26 @@ struct FacesGlobal {
   }
   // flux*length of the interior face in slot j (edge e), and whether the edge produced one
   __device__ __forceinline__ bool iface(int j, int e, R* f) const {
+    if (!kTile) {
+      bool bad = false;  // (k_cell reports it)
+      if (!interior_flux(d, G, e, f, &bad)) return false;
+      const R len = G.elen[e];
+      f[0] = f[0] * len;
+      f[1] = f[1] * len;
+      f[2] = f[2] * len;
+      return true;
+    }
     f[0] = G.efx[e];
     f[1] = G.efx[d.ne + e];
     f[2] = G.efx[2 * d.ne + e];
     return d.eok[e] != 0;
   }
-  // the cell's own reconstructed state at face j (weslp2 walls)
+  // the cell's own reconstructed state at face j (weslp2 walls): its face record, whose
+  // depth is clipped at zero; weslp2 skips any state below h_dry > 0, so the clip never
+  // changes its result
   __device__ __forceinline__ EdgeState own(int j) const {
-    const int q = j * d.T + c;
-    EdgeState s;
-    s.h = recon(hs[c], G.delh_x[c], G.rc_x[q], G.delh_y[c], G.rc_y[q]);
-    s.u = recon(post_fix<R>(d, u_in, d.u_b, c), G.delu_x[c], G.rc_x[q], G.delu_y[c], G.rc_y[q]);
-    s.v = recon(post_fix<R>(d, v_in, d.v_b, c), G.delv_x[c], G.rc_x[q], G.delv_y[c], G.rc_y[q]);
-    return s;
+    const Rec r = ld_rec(d.fs + d.fpos[j * d.T + c]);
+    return EdgeState{r.h, r.u, r.v};
   }
   __device__ __forceinline__ void dh(R* x, R* y) const {
     *x = G.delh_x[c];
@@ -1537,30 +2124,16 @@ __device__ __forceinline__ void assemble_phi(const Dev& d, const Geo<R>& G, cons
     } else if (kind == FACE_WALL) {
       if (dry_c) continue;
       const double nx = d.fnx[q], ny = d.fny[q], len = d.flen[q];
-      if (d.btype == 0) {  // wenslp3_fluxes.f90:34-67
+      double f2 = kZero, f3 = kZero;
+      if (d.btype == 0) {
         double h1, h2;
         fs.hwall(j, fe[t], &h1, &h2);
-        double hedge = qsqrt((h1 * h1 + h1 * h2 + h2 * h2) * kOneThird);
-        if (hedge < kZero) hedge = kZero;
-        if (hedge < d.h_dry) continue;
-        p2 = p2 - kHalf * kG * hedge * hedge * nx * len;
-        p3 = p3 - kHalf * kG * hedge * hedge * ny * len;
-      } else {  // weslp2_fluxes.f90:34-76
-        const EdgeState o = fs.own(j);
-        const double hleft = o.h;
-        if (hleft < d.h_dry) continue;
-        const double uleft = o.u;
-        const double vleft = o.v;
-        const double tx = -ny, ty = nx;  // edges%tang flipped with the normal
-        double uright = uleft * tx + vleft * ty;
-        uright = uright + 2.0 * sqrt(kG * hleft);
-        const double hright = uright * uright / 4.0 / kG;
-        const double f2 = kHalf * kG * hright * hright * nx;
-        const double f3 = kHalf * kG * hright * hright * ny;
-        const double dh = kZero;
-        p2 = p2 - (f2 + dh * nx) * len;
-        p3 = p3 - (f3 + dh * ny) * len;
+        wall_noslip(d, h1, h2, nx, ny, &f2, &f3);
+      } else {
+        wall_slip(d, fs.own(j), nx, ny, &f2, &f3);
       }
+      p2 = p2 - f2 * len;
+      p3 = p3 - f3 * len;
     } else if (kind == FACE_BC) {
       const int e = fe[t];
       p1 = p1 - d.bc_c[e];
@@ -1572,7 +2145,7 @@ __device__ __forceinline__ void assemble_phi(const Dev& d, const Geo<R>& G, cons
     double s2, s3;
     R dhx, dhy;
     fs.dh(&dhx, &dhy);
-    bed_source(d, G, c, h_c, dhx, dhy, &s2, &s3);
+    bed_source(d, c, h_c, dhx, dhy, G.delz_x[c], G.delz_y[c], d.area[c], d.rad[c], G, &s2, &s3);
     p2 = p2 - s2;
     p3 = p3 - s3;
     if (d.wcoef1) {  // wind forcing (solverFVT.f90:218-224)
@@ -1580,55 +2153,36 @@ __device__ __forceinline__ void assemble_phi(const Dev& d, const Geo<R>& G, cons
       p3 = p3 + d.wcoef2[c];
     }
   }
-  if (ord & kOrderHasCulvert) {  // culvert sources and sinks (solverFVT.f90:227-233)
-    int lo = 0, hi = d.ncvc;  // first term of cell c
-    while (lo < hi) {
-      const int mid = (lo + hi) >> 1;
-      if (d.cvc_cell[mid] < c) lo = mid + 1;
-      else hi = mid;
-    }
-    for (int k = lo; k < d.ncvc && d.cvc_cell[k] == c; k++) {
-      const int code = d.cvc_code[k];
-      if (code & 1) p1 = p1 + d.cvsrc[code >> 1];
-      else p1 = p1 - d.cvsrc[code >> 1];
-    }
-  }
+  if (ord & kOrderHasCulvert) p1 = culvert_terms(d, c, p1);
   *p1o = p1;
   *p2o = p2;
   *p3o = p3;
 }
 
-// The RK update of stage s (1-based) for cell c from its phi (solverFVT.f90:259-325).
-__device__ __forceinline__ void rk_update(const Dev& d, int s, int c, double h_c, bool dry_c, double p1, double p2,
-                                          double p3, uint8_t* __restrict__ dry_next, const double* __restrict__ u_in,
-                                          const double* __restrict__ v_in, double* __restrict__ u_out,
-                                          double* __restrict__ v_out) {
-  const int T = d.T;
-  // RK update (solverFVT.f90:259-283)
-  const double u_c = u_in[c], v_c = v_in[c];
-  double delt;
-  if (d.steady) {
-    const double um = (h_c < d.h_dry) ? kZero : qsqrt(u_c * u_c + v_c * v_c);
-    const double wc = dry_c ? kZero : sqrt(kG * h_c);
-    delt = um + wc;
-    if (delt < SMALL_F) delt = 1.044;
-    delt = d.cfl * d.area[c] / (delt * d.perim[c]);
-    Scalars& sc = d.sc[cell_scenario(d, c)];
-    if (s == d.K && c == sc.last_cell) sc.delt_fric = delt;
-  } else {
-    delt = d.sc[cell_scenario(d, c)].delt;
-  }
-  const double dt = delt / d.area[c];
+// What the RK update reads of one cell: levels 0 and s-1 (momentum; level 0's depth too),
+// area and perimeter.
+struct CellIn {
+  double rkh0, rku0, rkv0, rku1, rkv1, area, perim;
+};
+struct CellOut {
+  double h, u, v, ru, rv;
+};
+
+// The RK update of stage s (1-based) of a cell from its phi (solverFVT.f90:259-325).
+__device__ __forceinline__ CellOut rk_combine(const Dev& d, int s, const Rec& own, bool dry_c, const CellIn& in,
+                                              double delt, double p1, double p2, double p3) {
+  const double dt = delt / in.area;
   double rh = kZero, ru = kZero, rv = kZero;
-  for (int j = 0; j <= s - 1; j++) {
-    // a zero coefficient (SSP-RK3 stage 3, level 1) adds a signed zero to a sum that
-    // started at +0, which leaves its bits unchanged: skip the loads
-    if (d.alpha[s][j] == kZero) continue;
-    const int q = j * T + c;
-    rh = rh + d.alpha[s][j] * d.rkh[q];
-    ru = ru + d.alpha[s][j] * d.rku[q];
-    rv = rv + d.alpha[s][j] * d.rkv[q];
+  // a zero coefficient (SSP-RK3 stage 3, level 1) adds a signed zero to a sum that
+  // started at +0, which leaves its bits unchanged; so the levels are 0 and s-1
+  if (s > 1) {
+    rh = rh + d.alpha[s][0] * in.rkh0;
+    ru = ru + d.alpha[s][0] * in.rku0;
+    rv = rv + d.alpha[s][0] * in.rkv0;
   }
+  rh = rh + d.alpha[s][s - 1] * own.h;  // level s-1's depth is the stage input's
+  ru = ru + d.alpha[s][s - 1] * in.rku1;
+  rv = rv + d.alpha[s][s - 1] * in.rkv1;
   rh = rh + d.beta[s] * dt * p1;
   ru = (ru + d.beta[s] * dt * p2);
   rv = (rv + d.beta[s] * dt * p3);
@@ -1641,38 +2195,139 @@ __device__ __forceinline__ void rk_update(const Dev& d, int s, int c, double h_c
     }
   }
   rh = fmax2(rh, kZero);  // :300-325
-  double un, vn;
+  CellOut o;
+  o.h = rh;
   const double h_delta = dry_c ? d.h_wet : d.h_dry;
   if (rh > h_delta) {
-    un = qdiv(ru, rh);
-    vn = qdiv(rv, rh);
+    o.u = qdiv(ru, rh);
+    o.v = qdiv(rv, rh);
+    o.ru = ru;
+    o.rv = rv;
   } else {
-    ru = kZero; rv = kZero; un = kZero; vn = kZero;
+    o.ru = kZero; o.rv = kZero; o.u = kZero; o.v = kZero;
   }
-  const int qs = s * T + c;
-  d.rkh[qs] = rh;
-  d.rku[qs] = ru;
-  d.rkv[qs] = rv;
-  u_out[c] = un;
-  v_out[c] = vn;
-  if (s < d.K) {
-    double um;
-    dry_next[c] = dry_flag(rh, un, vn, d.h_dry, d.h_wet, &um);
-  } else {
-    d.phimax[c] = fmax2(fmax2(fmax2(kZero, fabs(p1)), fabs(p2)), fabs(p3));
-  }
+  return o;
 }
 
-template <class R>
-__device__ __forceinline__ void flux_cell(const Dev& d, const Geo<R>& G, int s, int c, const double* __restrict__ hs,
-                                          const uint8_t* __restrict__ dry, uint8_t* __restrict__ dry_next,
-                                          const double* __restrict__ u_in, const double* __restrict__ v_in,
-                                          double* __restrict__ u_out, double* __restrict__ v_out) {
-  double p1, p2, p3;
-  const double h_c = hs[c];
-  const bool dry_c = dry[c] != 0;
-  assemble_phi<R>(d, G, FacesGlobal<R>{d, G, hs, c, u_in, v_in}, c, h_c, dry_c, &p1, &p2, &p3);
-  rk_update(d, s, c, h_c, dry_c, p1, p2, p3, dry_next, u_in, v_in, u_out, v_out);
+// Its operands from memory.
+__device__ __forceinline__ CellIn cell_in(const Dev& d, int s, int c) {
+  const int T = d.T, q = (s - 1) * T + c;
+  CellIn in;
+  in.rkh0 = s > 1 ? d.rkh[c] : kZero;
+  in.rku0 = s > 1 ? d.rku[c] : kZero;
+  in.rkv0 = s > 1 ? d.rkv[c] : kZero;
+  in.rku1 = d.rku[q];
+  in.rkv1 = d.rkv[q];
+  in.area = d.area[c];
+  in.perim = d.perim[c];
+  return in;
+}
+__device__ __forceinline__ double cell_dt(const Dev& d, int c, const Rec& own, bool dry_c, const CellIn& in) {
+  return d.steady ? local_dt(d, own, dry_c, in.area, in.perim) : d.sc[cell_scenario(d, c)].delt;
+}
+// The stored form of an update: the next stage's input, the level, max |phi| of the last.
+__device__ __forceinline__ void store_update(const Dev& d, int s, int c, const Rec& own, const CellOut& o, double p1,
+                                             double p2, double p3, Rec* __restrict__ qo) {
+  const int qs = s * d.T + c;
+  if (s == d.K - 1) d.rkh[qs] = o.h;  // the output step's depths
+  d.rku[qs] = o.ru;
+  d.rkv[qs] = o.rv;
+  st_rec(qo + c, Rec{o.h, own.z, o.u, o.v});
+  if (s == d.K) d.phimax[c] = fmax2(fmax2(fmax2(kZero, fabs(p1)), fabs(p2)), fabs(p3));
+}
+__device__ __forceinline__ void rk_update(const Dev& d, int s, int c, const Rec& own, bool dry_c, double p1, double p2,
+                                          double p3, Rec* __restrict__ qo) {
+  const CellIn in = cell_in(d, s, c);
+  const double delt = cell_dt(d, c, own, dry_c, in);
+  if (d.steady && s == d.K) {
+    Scalars& sc = d.sc[cell_scenario(d, c)];
+    if (c == sc.last_cell) sc.delt_fric = delt;
+  }
+  store_update(d, s, c, own, rk_combine(d, s, own, dry_c, in, delt, p1, p2, p3), p1, p2, p3, qo);
+}
+
+// The friction step of a cell after the last stage and its terms of the iteration's
+// reductions (solverFVT.f90:335-386, 407-445): find_dry_cells, fric_terms_impl, the
+// numerical valve, the copy to RK level 0.
+struct FricTerms {
+  double st = kZero, sb = kZero, tm = kZero, rm = kZero, dt = kVlarge;
+};
+__device__ __forceinline__ FricTerms fric_cell(const Dev& d, int sid, int c, const CellOut& in, double z, double h0,
+                                               double phimax, double cd, double area, double perim) {
+  const int T = d.T;
+  const double h = in.h;
+  double u = in.u, v = in.v, ru = in.ru, rv = in.rv;
+  double um;
+  const bool dry2 = dry_flag(h, u, v, d.h_dry, d.h_wet, &um);
+  d.dry_out[c] = dry2;
+  double rough = kZero;
+  switch (d.fric) {
+    case 0:
+      if (!dry2) rough = kG * cd * cd / pow(h, kOneThird);
+      break;
+    case 1:
+      rough = (cd < kFmachp) ? kVlarge : kG / (cd * cd);
+      break;
+    case 2:
+      rough = cd;
+      break;
+    case 3:
+      if (!dry2) {
+        double re = qdiv(um * h, d.visc);
+        re = fmax2(re, 1000.0);
+        re = fmin2(re, (double)2.5e7f);
+        rough = cd;
+        if (cd / h > 0.20) rough = 0.20 * h;
+        const double ln = log(1.725 / re + pow(rough / (14.8 * h), (double)1.11f));
+        rough = 0.204 / (ln * ln);
+      }
+      break;
+    default:
+      if (!dry2) {
+        rough = pow(100.0 * cd, 0.16666666666666667) / 51.79;
+        rough = kG * rough * rough / pow(h, kOneThird);
+      }
+      break;
+  }
+  const double dtf = d.steady ? d.sc[sid].delt_fric : d.sc[sid].delt;
+  if (!dry2) rough = h / (h + dtf * rough * um);
+  u = u * rough;
+  v = v * rough;
+  if (!dry2) {
+    ru = h * u;
+    rv = h * v;
+  }
+  // numerical valve at stage-boundary edges (solverFVT.f90:357-370)
+  const uint8_t hm = d.hvalve ? d.hvmask[c] : 0;
+  if (hm) {
+    bool zero = false;
+#pragma unroll
+    for (int j = 0; j < 3; j++)
+      if (hm & (1u << j)) {
+        const int q = j * T + c;
+        const double dot = u * d.fnx[q] + v * d.fny[q];
+        if (dot < 0) zero = true;
+      }
+    if (zero) {
+      u = kZero;
+      v = kZero;
+    }
+  }
+  d.rku[c] = ru;  // rk(:,0) <- rk(:,rkorder) of the next iteration (:138-142)
+  d.rkv[c] = rv;
+  d.rkh[c] = h;
+  st_rec(d.q + c, Rec{h, z, u, v});
+  double um1;
+  const bool dry1 = dry_flag(h, u, v, d.h_dry, d.h_wet, &um1);
+  FricTerms t;
+  t.st = (h - h0) * (h - h0);
+  t.sb = h0 * h0;
+  t.tm = h * area;
+  t.rm = dry2 ? kZero : phimax;
+  const double wc1 = dry1 ? kZero : sqrt(kG * h);
+  t.dt = d.cfl * area / ((um1 + wc1 + SMALL_F) * perim);
+  if (!isfinite(h) || !isfinite(u) || !isfinite(v)) atomicOr(&d.sc[sid].status, 1);
+  return t;
 }
 
 // Residual smoothing (solverFVT.f90:238-256, activateRSAVG): the stage's phi is
@@ -1680,23 +2335,7 @@ __device__ __forceinline__ void flux_cell(const Dev& d, const Geo<R>& G, int s, 
 // cells of one colour of the t2t stencil at a time (cells of a colour share no
 // stencil edge, so each reads its neighbours' latest values exactly as a serial sweep
 // in colour order does), then every cell is updated.
-template <class R>
-__global__ void __launch_bounds__(128) k_flux_phi(Dev d, Geo<R> G, const double* __restrict__ hs,
-                                              const uint8_t* __restrict__ dry, const double* __restrict__ u_in,
-                                              const double* __restrict__ v_in, int bc_cells) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  int c;
-  if (bc_cells) {
-    if (i >= d.nbc_cells) return;
-    c = d.bc_cells[i];
-  } else {
-    if (i >= d.T) return;
-    c = i;
-    if (d.forder[c] & kOrderHasBc) return;
-  }
-  if (!cell_live(d, c)) return;
-  double p1, p2, p3;
-  assemble_phi<R>(d, G, FacesGlobal<R>{d, G, hs, c, u_in, v_in}, c, hs[c], dry[c] != 0, &p1, &p2, &p3);
+__device__ __forceinline__ void store_phi(const Dev& d, int c, double p1, double p2, double p3) {
   const size_t T = d.T;
   d.phi[c] = p1;
   d.phi[T + c] = p2;
@@ -1713,7 +2352,7 @@ __global__ void __launch_bounds__(256) k_rsavg(Dev d, int off, int cnt) {
   const int c = d.rs_cells[off + q];
   if (!cell_live(d, c)) return;
   const size_t T = d.T;
-  const int n = d.nst[c];
+  const int n = d.nst[c] & kNstCount;
   for (int k = 0; k < 3; k++) {
     double p = d.rs_fac1 * d.phi0[k * T + c];
     for (int m = 0; m < n; m++) p = p + d.rs_fac2 * d.phi[k * T + d.st_id[m * T + c]];
@@ -1721,41 +2360,198 @@ __global__ void __launch_bounds__(256) k_rsavg(Dev d, int off, int cnt) {
   }
 }
 
-__global__ void __launch_bounds__(128) k_update(Dev d, int s, const double* __restrict__ hs,
-                                            const uint8_t* __restrict__ dry, uint8_t* __restrict__ dry_next) {
+__global__ void __launch_bounds__(128) k_update(Dev d, int s, const Rec* q, Rec* qo) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= d.T) return;
   if (!cell_live(d, c)) return;
   const size_t T = d.T;
-  rk_update(d, s, c, hs[c], dry[c] != 0, d.phi[c], d.phi[T + c], d.phi[2 * T + c], dry_next, d.u_a, d.v_a, d.u_a,
-            d.v_a);
+  const Rec own = ld_rec(q + c);
+  rk_update(d, s, c, own, rec_dry(d, own), d.phi[c], d.phi[T + c], d.phi[2 * T + c], qo);
 }
 #endif  // !STORM_FVT_F32_TU
 
-// All cells without an open-boundary face (those wait for k_bc in k_flux_bc).
-template <class R>
-__global__ void __launch_bounds__(128, 10) k_flux(Dev d, Geo<R> G, int s, const double* __restrict__ hs,
-                                              const uint8_t* __restrict__ dry, uint8_t* __restrict__ dry_next,
-                                              const double* __restrict__ u_in, const double* __restrict__ v_in,
-                                              double* __restrict__ u_out, double* __restrict__ v_out) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= d.T) return;
-  if (!cell_live(d, c)) return;
-  if (d.forder[c] & kOrderHasBc) return;
-  flux_cell<R>(d, G, s, c, hs, dry, dry_next, u_in, v_in, u_out, v_out);
+// Reduction terms of the i-th cell with an open-boundary face
+__device__ __forceinline__ void store_bc_terms(const Dev& d, int i, const FricTerms& t) {
+  const size_t n = d.nbc_cells;
+  d.bcpart[i] = t.st;
+  d.bcpart[n + i] = t.sb;
+  d.bcpart[2 * n + i] = t.tm;
+  d.bcpart[3 * n + i] = t.rm;
+  d.bcpart[4 * n + i] = t.dt;
 }
 
-// The cells with an open-boundary face, after k_bc.
+// A stage's edge fluxes and cell updates, one block per 256 cell slots: the flux of every
+// edge and wall of the block's cells into shared memory (an edge between two blocks is
+// evaluated by both), then the ordered face sums, sources and the RK update of its
+// cells without an open-boundary face (those wait for k_bc in k_flux_bc); in the last
+// stage of an iteration also the friction step and the block's reductions (CELL_FRIC).
+//
+// Fluxes never pass through memory, and what the cells read -- contiguous pieces of a
+// dozen columns -- comes in by bulk copies issued before the edges are evaluated, so it
+// waits in shared memory when they are done.
+//
+// Two-million-cell meander, FP64 Roe, per stage: 120 us (edges) + 98 us (cells) and 68 us
+// of friction per iteration before; 174 us with the friction step in the third stage.
+// 256 threads, four blocks to an SM (64 registers; 205 us with three and 80 registers,
+// 241 us with two and 112): the kernel waits on long chains of
+// FP64 operations, and more warps beat fewer spills.  Meshes with no more blocks than
+// SMs take 512 threads, which evaluate all of a block's edges (about 410) in one round.
 template <class R>
-__global__ void __launch_bounds__(128) k_flux_bc(Dev d, Geo<R> G, int s, const double* __restrict__ hs,
-                                                 const uint8_t* __restrict__ dry, uint8_t* __restrict__ dry_next,
-                                                 const double* __restrict__ u_in, const double* __restrict__ v_in,
-                                                 double* __restrict__ u_out, double* __restrict__ v_out) {
+struct CellSmem {
+  Rec q[256];
+  double rku1[256], rkv1[256], rkh0[256], rku0[256], rkv0[256], area[256], perim[256], cd[256];
+  R dzx[256], dzy[256], dhx[256], dhy[256];
+  uint32_t desc[256];
+  float rad[256];
+  uint16_t lfe[3][256];
+};
+
+template <class R, int kMode, int kThreads>
+__global__ void __launch_bounds__(kThreads, kThreads == 256 ? 4 : 1) k_cell(const __grid_constant__ Dev d,
+                                                          const __grid_constant__ Geo<R> G, int s) {
+  extern __shared__ __align__(128) unsigned char cell_smem[];
+  __shared__ uint64_t bar;
+  __shared__ double red[5 * (kThreads / 32)];
+  CellSmem<R>& S = *reinterpret_cast<CellSmem<R>*>(cell_smem);
+  double* s_w = reinterpret_cast<double*>(cell_smem + sizeof(CellSmem<R>));  // [3][cnw_max]
+  R* s_f = reinterpret_cast<R*>(s_w + 3 * d.cnw_max);                         // [3][cne_max]
+  const int t = blockIdx.x, tid = threadIdx.x, c0 = t * 256, c = c0 + tid, T = d.T;
+  const int4 i0 = reinterpret_cast<const int4*>(d.ct + t)[0], i1 = reinterpret_cast<const int4*>(d.ct + t)[1];
+  const int sid = d.nscen == 1 ? 0 : d.cell_sid[c0];  // a block never spans two scenarios
+  if (d.sc[sid].converged) return;
+  const bool fric = kMode == CELL_FRIC;
+  if (tid < 32) {  // a column for each lane
+    const CellCol col = d.ccol[((s - 1) * 3 + kMode) * kCellCols + tid];
+    const uint32_t bytes = __reduce_add_sync(0xffffffffu, col.bytes);
+    if (tid == 0) {
+      umma::mbar_init(&bar, 1);
+      umma::fence_async_smem();
+      umma::mbar_expect(&bar, bytes);
+    }
+    __syncwarp();
+    if (col.bytes) umma::bulk_load(cell_smem + col.dst, col.base + (size_t)t * col.bytes, col.bytes, &bar);
+  }
+
+  // edges: the block's range, then the listed ones
+  const int er0 = i0.x, nr = i0.y, boff = i0.z, ne = nr + i0.w, nem = d.cne_max;
+  const auto edge_at = [&](int le) { return le < nr ? er0 + le : le < ne ? d.cbe[boff + le - nr] : 0; };
+  int e_next = edge_at(tid);
+  for (int le = tid; le < ne; le += kThreads) {
+    const int e = e_next;
+    e_next = edge_at(le + kThreads);  // a listed index is there when its turn comes
+    R f[3];
+    bool bad = false;
+    if (interior_flux(d, G, e, f, &bad)) {
+      const R len = G.elen[e];
+      f[0] = f[0] * len;
+      f[1] = f[1] * len;
+      f[2] = f[2] * len;
+    } else {
+      f[0] = f[1] = f[2] = R(0);  // an edge without a flux adds nothing
+    }
+    s_f[le] = f[0];
+    s_f[nem + le] = f[1];
+    s_f[2 * nem + le] = f[2];
+    if (bad) atomicOr(&d.sc[sid].status, 2);
+  }
+  const int w0 = i1.x, nw = i1.y, nwm = d.cnw_max;
+  for (int w = tid; w < nw; w += kThreads) {
+    double f2, f3;
+    wall_flux(d, d.walls[w0 + w], &f2, &f3);
+    s_w[w] = f2;
+    s_w[nwm + w] = f3;
+    s_w[2 * nwm + w] = d.walls[w0 + w].len;
+  }
+  __syncthreads();
+  if (!umma::mbar_wait(&bar, 0)) {  // cannot happen: copies within this GPU
+    if (tid == 0) atomicOr(&d.sc[sid].status, 4);
+    umma::mbar_wait(&bar, 0);
+    return;
+  }
+
+  FricTerms ft;
+  if (kThreads > 256 && tid >= 256) return;
+  const uint32_t desc = S.desc[tid];
+  if ((desc & kDescReal) && !(desc & kOrderHasBc)) {
+    const Rec own = S.q[tid];
+    const bool dry_c = rec_dry(d, own);
+    double p1 = kZero, p2 = kZero, p3 = kZero;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {  // in the order invisc_fluxes.f90 visits the faces
+      const int kind = (desc >> (8 + 3 * k)) & 7, l = S.lfe[k][tid];
+      if (kind == FACE_LEFT) {
+        p1 = p1 - s_f[l];
+        p2 = p2 - s_f[nem + l];
+        p3 = p3 - s_f[2 * nem + l];
+      } else if (kind == FACE_RIGHT) {
+        p1 = p1 + s_f[l];
+        p2 = p2 + s_f[nem + l];
+        p3 = p3 + s_f[2 * nem + l];
+      } else if (kind == FACE_WALL) {
+        p2 = p2 - s_w[l] * s_w[2 * nwm + l];
+        p3 = p3 - s_w[nwm + l] * s_w[2 * nwm + l];
+      }
+    }
+    if (!dry_c) {
+      double s2, s3;
+      bed_source(d, c, own.h, S.dhx[tid], S.dhy[tid], S.dzx[tid], S.dzy[tid], S.area[tid], S.rad[tid], G, &s2, &s3);
+      p2 = p2 - s2;
+      p3 = p3 - s3;
+      if (d.wcoef1) {  // wind forcing (solverFVT.f90:218-224)
+        p2 = p2 + d.wcoef1[c];
+        p3 = p3 + d.wcoef2[c];
+      }
+    }
+    if (desc & kOrderHasCulvert) p1 = culvert_terms(d, c, p1);
+    if (kMode == CELL_PHI) {
+      store_phi(d, c, p1, p2, p3);
+    } else {
+      CellIn in;
+      in.rkh0 = S.rkh0[tid];
+      in.rku0 = S.rku0[tid];
+      in.rkv0 = S.rkv0[tid];
+      in.rku1 = S.rku1[tid];
+      in.rkv1 = S.rkv1[tid];
+      in.area = S.area[tid];
+      const double delt = d.steady ? local_dt(d, own, dry_c, in.area, S.perim[tid]) : d.sc[sid].delt;
+      const CellOut o = rk_combine(d, s, own, dry_c, in, delt, p1, p2, p3);
+      if (fric) {
+        const double pm = fmax2(fmax2(fmax2(kZero, fabs(p1)), fabs(p2)), fabs(p3));
+        ft = fric_cell(d, sid, c, o, own.z, s > 1 ? in.rkh0 : own.h, pm, S.cd[tid], in.area, S.perim[tid]);
+      } else {
+        if (d.steady && s == d.K && c == d.sc[sid].last_cell) d.sc[sid].delt_fric = delt;
+        store_update(d, s, c, own, o, p1, p2, p3, d.q);
+      }
+    }
+  }
+  if (fric) block_reduce5<256>(ft.st, ft.sb, ft.tm, ft.rm, ft.dt, red, d.part + t, d.nblk_red);
+}
+
+// The cells with an open-boundary face, after k_bc: their interior faces' fluxes again
+// from the face records, so that this needs nothing of k_cell and runs beside it
+// (kTile: from the arrays the fused kernel leaves them in).
+template <class R, int kMode, bool kTile>
+__global__ void __launch_bounds__(128) k_flux_bc(Dev d, Geo<R> G, int s, const Rec* q, Rec* qo) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= d.nbc_cells) return;
   const int c = d.bc_cells[i];
   if (!cell_live(d, c)) return;
-  flux_cell<R>(d, G, s, c, hs, dry, dry_next, u_in, v_in, u_out, v_out);
+  const Rec own = ld_rec(q + c);
+  const bool dry_c = rec_dry(d, own);
+  double p1, p2, p3;
+  assemble_phi<R>(d, G, FacesGlobal<R, kTile>{d, G, c}, c, own.h, dry_c, &p1, &p2, &p3);
+  if (kMode == CELL_PHI) {
+    store_phi(d, c, p1, p2, p3);
+  } else if (kMode == CELL_FRIC) {
+    const CellIn in = cell_in(d, s, c);
+    const CellOut o = rk_combine(d, s, own, dry_c, in, cell_dt(d, c, own, dry_c, in), p1, p2, p3);
+    const double pm = fmax2(fmax2(fmax2(kZero, fabs(p1)), fabs(p2)), fabs(p3));
+    const FricTerms t = fric_cell(d, cell_scenario(d, c), c, o, own.z, s > 1 ? in.rkh0 : own.h, pm, d.cd[c], in.area,
+                                  in.perim);
+    store_bc_terms(d, i, t);
+  } else {
+    rk_update(d, s, c, own, dry_c, p1, p2, p3, qo);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -1806,10 +2602,8 @@ __host__ __device__ inline TileSmem tile_smem_layout(int ns, int ng, int ne, int
 
 template <class R>
 __global__ void __launch_bounds__(kTileThreads, 3)
-    k_tile(Dev d, Geo<R> G, TileDev tp, int s, const double* __restrict__ hs, const uint8_t* __restrict__ dry,
-           uint8_t* __restrict__ dry_next, const double* __restrict__ u_in, const double* __restrict__ v_in,
-           double* __restrict__ u_out, double* __restrict__ v_out, double* __restrict__ rku_prev,
-           double* __restrict__ rkv_prev) {
+    k_tile(Dev d, Geo<R> G, TileDev tp, int s, const Rec* __restrict__ q, Rec* __restrict__ qo,
+           double* __restrict__ rku_prev, double* __restrict__ rkv_prev) {
   extern __shared__ __align__(16) unsigned char tsm[];
   // persistent: each CTA takes tiles blockIdx.x, blockIdx.x + gridDim.x, ...
   for (int t = blockIdx.x; t < tp.ntiles; t += gridDim.x) {
@@ -1841,11 +2635,12 @@ __global__ void __launch_bounds__(kTileThreads, 3)
   // A: stage-input state of every local cell
   for (int l = threadIdx.x; l < nS; l += blockDim.x) {
     const int g = l < nown ? c0 + l : tp.halo[hoff + l - nown];
-    s_h[l] = hs[g];
-    s_z[l] = d.z[g];
-    s_u[l] = u_in[g];
-    s_v[l] = v_in[g];
-    s_dry[l] = dry[g];
+    const Rec r = ld_rec(q + g);
+    s_h[l] = r.h;
+    s_z[l] = r.z;
+    s_u[l] = r.u;
+    s_v[l] = r.v;
+    s_dry[l] = rec_dry(d, r);
   }
   __syncthreads();
 
@@ -1966,9 +2761,11 @@ __global__ void __launch_bounds__(kTileThreads, 3)
       const bool dl = s_dry[a], dr = s_dry[b];
       const EdgeState fa{s_fh[ml * ngm + a], s_fu[ml * ngm + a], s_fv[ml * ngm + a]};
       const EdgeState fb{s_fh[mr * ngm + b], s_fu[mr * ngm + b], s_fv[mr * ngm + b]};
+      const bool rus = d.flux == STORM_FLUX_RUSANOV;
+      const auto cel = [&](bool dr_, double h_) { return rus && !dr_ ? sqrt(kG * h_) : kZero; };
       R f[3];
       bool bad = false;
-      ok = edge_flux<R>(d, dl, dr, fa, fb, s_z[a], s_z[b], s_h[a], s_h[b], G.enx[e], G.eny[e],
+      ok = edge_flux<R>(d, dl, dr, fa, fb, s_z[a], s_z[b], cel(dl, s_h[a]), cel(dr, s_h[b]), G.enx[e], G.eny[e],
                         (dl || dr) ? d.ez0[e] : kZero, f, &bad);
       if (ok) {
         const R len = G.elen[e];
@@ -2005,7 +2802,7 @@ __global__ void __launch_bounds__(kTileThreads, 3)
                           d.forder, d.fkind};
     double p1, p2, p3;
     assemble_phi<R>(d, G, fs, c, h_c, dry_c, &p1, &p2, &p3);
-    rk_update(d, s, c, h_c, dry_c, p1, p2, p3, dry_next, u_in, v_in, u_out, v_out);
+    rk_update(d, s, c, Rec{h_c, s_z[l], s_u[l], s_v[l]}, dry_c, p1, p2, p3, qo);
   }
   __syncthreads();  // the next tile reuses the shared memory
   }
@@ -2047,11 +2844,10 @@ void set_tile_smem_limit(int bytes) {
 // After the RK stages: find_dry_cells, fric_terms_impl, hvalve, rk level copy and the
 // block partials of the iteration's reductions (solverFVT.f90:335-386, 407-445).
 // kHalo: the handle links partitions, and halo cells stay out of the partials.
-// u_src/v_src: the velocities of the last stage (the fused path's ping-pong buffer);
-// the friction step writes the next iteration's start into d.u_a/d.v_a.
+// src: the state after the last stage (the fused path's ping-pong buffer, or d.q); the
+// friction step writes the next iteration's start into d.q.
 template <bool kHalo>
-__global__ void __launch_bounds__(kRedThreads) k_fric(Dev d, const double* __restrict__ u_src,
-                                                      const double* __restrict__ v_src) {
+__global__ void __launch_bounds__(kRedThreads) k_fric(Dev d, const Rec* src) {
   __shared__ double sm[5 * (kRedThreads / 32)];
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   const int T = d.T, K = d.K;
@@ -2062,91 +2858,25 @@ __global__ void __launch_bounds__(kRedThreads) k_fric(Dev d, const double* __res
   // a block never spans two scenarios, so this test is uniform over the block
   const int bsid = one ? 0 : d.cell_sid[blockIdx.x * blockDim.x];
   if (d.sc[bsid < 0 ? 0 : bsid].converged) return;
-  double st = kZero, sb = kZero, tm = kZero, rm = kZero, dtc = kVlarge;
+  FricTerms ft;
   if (sid >= 0) {
     const int qk = K * T + c;
-    const double h = d.rkh[qk];
-    double u = u_src[c], v = v_src[c];
-    double ru = d.rku[qk], rv = d.rkv[qk];
-    const double h0 = d.rkh[c];  // rkh(i,0), the iteration's starting depth
-    double um;
-    const bool dry2 = dry_flag(h, u, v, d.h_dry, d.h_wet, &um);
-    d.dry_out[c] = dry2;
-    const double cd = d.cd[c];
-    double rough = kZero;
-    switch (d.fric) {
-      case 0:
-        if (!dry2) rough = kG * cd * cd / pow(h, kOneThird);
-        break;
-      case 1:
-        rough = (cd < kFmachp) ? kVlarge : kG / (cd * cd);
-        break;
-      case 2:
-        rough = cd;
-        break;
-      case 3:
-        if (!dry2) {
-          double re = qdiv(um * h, d.visc);
-          re = fmax2(re, 1000.0);
-          re = fmin2(re, (double)2.5e7f);
-          rough = cd;
-          if (cd / h > 0.20) rough = 0.20 * h;
-          const double ln = log(1.725 / re + pow(rough / (14.8 * h), (double)1.11f));
-          rough = 0.204 / (ln * ln);
-        }
-        break;
-      default:
-        if (!dry2) {
-          rough = pow(100.0 * cd, 0.16666666666666667) / 51.79;
-          rough = kG * rough * rough / pow(h, kOneThird);
-        }
-        break;
-    }
-    const double dtf = d.steady ? d.sc[sid].delt_fric : d.sc[sid].delt;
-    if (!dry2) rough = h / (h + dtf * rough * um);
-    u = u * rough;
-    v = v * rough;
-    if (!dry2) {
-      ru = h * u;
-      rv = h * v;
-    }
-    // numerical valve at stage-boundary edges (solverFVT.f90:357-370)
-    const uint8_t hm = d.hvalve ? d.hvmask[c] : 0;
-    if (hm) {
-      bool zero = false;
-#pragma unroll
-      for (int j = 0; j < 3; j++)
-        if (hm & (1u << j)) {
-          const int q = j * T + c;
-          const double dot = u * d.fnx[q] + v * d.fny[q];
-          if (dot < 0) zero = true;
-        }
-      if (zero) {
-        u = kZero;
-        v = kZero;
+    const Rec in = ld_rec(src + c);
+    ft = fric_cell(d, sid, c, CellOut{in.h, in.u, in.v, d.rku[qk], d.rkv[qk]}, in.z, d.rkh[c], d.phimax[c], d.cd[c],
+                   d.area[c], d.perim[c]);
+    if (kHalo && d.halo_mask[c]) ft = FricTerms();  // a halo copy: its owner counts it
+    if (d.forder[c] & kOrderHasBc) {  // summed by k_final, as when k_flux_bc did the friction step
+      int lo = 0, hi = d.nbc_cells;
+      while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (d.bc_cells[mid] < c) lo = mid + 1;
+        else hi = mid;
       }
-    }
-    d.rku[c] = ru;  // rk(:,0) <- rk(:,rkorder) of the next iteration (:138-142)
-    d.rkv[c] = rv;
-    d.rkh[c] = h;
-    d.u_a[c] = u;
-    d.v_a[c] = v;
-    double um1;
-    const bool dry1 = dry_flag(h, u, v, d.h_dry, d.h_wet, &um1);
-    d.dry_a[c] = dry1;
-    st = (h - h0) * (h - h0);
-    sb = h0 * h0;
-    tm = h * d.area[c];
-    rm = dry2 ? kZero : d.phimax[c];
-    const double wc1 = dry1 ? kZero : sqrt(kG * h);
-    dtc = d.cfl * d.area[c] / ((um1 + wc1 + SMALL_F) * d.perim[c]);
-    if (kHalo && d.halo_mask[c]) {  // a halo copy: its owner counts it
-      st = kZero; sb = kZero; tm = kZero; rm = kZero; dtc = kVlarge;
-    } else if (!isfinite(h) || !isfinite(u) || !isfinite(v)) {
-      atomicOr(&d.sc[sid].status, 1);
+      store_bc_terms(d, lo, ft);
+      ft = FricTerms();
     }
   }
-  block_reduce5<kRedThreads>(st, sb, tm, rm, dtc, sm, d.part + blockIdx.x, d.nblk_red);
+  block_reduce5<kRedThreads>(ft.st, ft.sb, ft.tm, ft.rm, ft.dt, sm, d.part + blockIdx.x, d.nblk_red);
 }
 
 #ifndef STORM_FVT_F32_TU
@@ -2180,6 +2910,16 @@ __global__ void __launch_bounds__(kFinalThreads) k_final(Dev d) {
       a2 = a2 + r[k][2];
       a3 = fmax2(a3, r[k][3]);
       a4 = fmin2(a4, r[k][4]);
+    }
+  }
+  {  // the cells with an open-boundary face are not in the blocks' partials
+    const size_t n = d.nbc_cells;
+    for (int i = sc->bc_off + threadIdx.x; i < sc->bc_off + sc->bc_cnt; i += kFinalThreads) {
+      a0 = a0 + d.bcpart[i];
+      a1 = a1 + d.bcpart[n + i];
+      a2 = a2 + d.bcpart[2 * n + i];
+      a3 = fmax2(a3, d.bcpart[3 * n + i]);
+      a4 = fmin2(a4, d.bcpart[4 * n + i]);
     }
   }
   block_reduce5<kFinalThreads>(a0, a1, a2, a3, a4, sm, red);
@@ -2251,8 +2991,7 @@ __global__ void __launch_bounds__(256) k_out_depth(Dev d, OutputArgs a) {
 }
 #endif  // !STORM_FVT_F32_TU
 
-// to_vertices.f90:44-55 on the solution (and the next stage's dry flag of a cell whose
-// velocity it zeroes), error_est.f90 etype 2
+// to_vertices.f90:44-55 on the solution, error_est.f90 etype 2
 template <class R>
 __global__ void __launch_bounds__(256) k_out_cell(Dev d, Geo<R> G, OutputArgs a) {
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2263,10 +3002,8 @@ __global__ void __launch_bounds__(256) k_out_cell(Dev d, Geo<R> G, OutputArgs a)
   if (!d.dry_out[c]) {
     const bool flag = (a.hv[n1] > d.h_dry) && (a.hv[n2] > d.h_dry) && (a.hv[n3] > d.h_dry);
     if (!flag) {
-      d.u_a[c] = kZero;
-      d.v_a[c] = kZero;
-      double um;
-      d.dry_a[c] = dry_flag(h, kZero, kZero, d.h_dry, d.h_wet, &um);
+      d.q[c].u = kZero;
+      d.q[c].v = kZero;
     }
   }
   if (a.e_est) {
@@ -2299,8 +3036,8 @@ __global__ void __launch_bounds__(256) k_out_vel(Dev d, OutputArgs a) {
   for (int q = b0; q < b1; q++) {
     const int k = d.n2t_cell[q];
     const double w = d.n2t_w[q] / tdist;
-    su = su + w * d.u_a[k];
-    sv = sv + w * d.v_a[k];
+    su = su + w * d.q[k].u;
+    sv = sv + w * d.q[k].v;
     scd = scd + w * d.cd[k];
     if (d.dry_out[k]) dryt = true;
     else wett = true;
@@ -2426,7 +3163,7 @@ __global__ void __launch_bounds__(kRedThreads) k_out_dt(Dev d) {
   if (c < d.T && d.cell_sid[c] >= 0) {
     const double h = d.rkh[c];
     double um1;
-    const bool dry1 = dry_flag(h, d.u_a[c], d.v_a[c], d.h_dry, d.h_wet, &um1);
+    const bool dry1 = dry_flag(h, d.q[c].u, d.q[c].v, d.h_dry, d.h_wet, &um1);
     const double wc1 = dry1 ? kZero : sqrt(kG * h);
     dtc = d.cfl * d.area[c] / ((um1 + wc1 + SMALL_F) * d.perim[c]);
   }
@@ -2465,13 +3202,13 @@ void launch_output(const Dev& d, const Geo<double>& Gd, const Geo<float>& Gf, bo
 // inlet cell's centroid (zeta + (delh + delz) . rcv) minus the invert elevation, and
 // the discharge is interpolated linearly in the culvert's performance curve.
 template <class R>
-__global__ void k_culvert(Dev d, Geo<R> G, const double* __restrict__ hs, const uint8_t* __restrict__ dry) {
+__global__ void k_culvert(Dev d, Geo<R> G, const Rec* __restrict__ rec) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= d.ncv) return;
   double src = kZero;
   const int c = d.cv_in[i];
-  if (!dry[c]) {
-    const double zeta = hs[c] + d.z[c];
+  if (!rec_dry(d, rec[c])) {
+    const double zeta = rec[c].h + d.z[c];
     const double dhx = (double)G.delh_x[c], dhy = (double)G.delh_y[c];
     double head = zeta + (dhx + d.delz_x[c]) * d.cv_rx[i] + (dhy + d.delz_y[c]) * d.cv_ry[i];
     head = head - d.cv_zinv[i];
@@ -2501,20 +3238,19 @@ __global__ void k_culvert(Dev d, Geo<R> G, const double* __restrict__ hs, const 
 // one clock, so the first one's stop flag stands for all.
 
 #ifndef STORM_FVT_F32_TU
-// Every halo cell takes its owner's values of one RK level, the velocities and up to
-// two flag arrays.
-__global__ void __launch_bounds__(256) k_halo(Dev d, int level, uint8_t* f1, uint8_t* f2) {
+// Every halo cell takes its owner's values of one RK level, its state and one flag
+// array (may be null).
+__global__ void __launch_bounds__(256) k_halo(Dev d, int level, uint8_t* f1) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= d.nhalo || d.sc[0].converged) return;
   const int dst = d.halo_dst[i], src = d.halo_src[i];
   const size_t off = (size_t)level * d.T;
-  d.rkh[off + dst] = d.rkh[off + src];
+  if (level == 0 || level == d.K - 1) d.rkh[off + dst] = d.rkh[off + src];
   d.rku[off + dst] = d.rku[off + src];
   d.rkv[off + dst] = d.rkv[off + src];
-  d.u_a[dst] = d.u_a[src];
-  d.v_a[dst] = d.v_a[src];
+  const Rec r = ld_rec(d.q + src);
+  st_rec(d.q + dst, Rec{r.h, d.z[dst], r.u, r.v});
   if (f1) f1[dst] = f1[src];
-  if (f2) f2[dst] = f2[src];
 }
 
 // Unsteady runs: the first dt after a state is set comes from each part's own CFL
@@ -2577,37 +3313,45 @@ __global__ void k_part_scalar(Dev d, int which, double v) {
 
 // out[6][n]: h (= rkh of the level), u, v, rkh, rku, rkv of the listed slots
 __global__ void __launch_bounds__(256) k_pack(Dev d, int level, int n, const int32_t* __restrict__ slots,
-                                              const double* __restrict__ u, const double* __restrict__ v,
-                                              double* __restrict__ out) {
+                                              const Rec* __restrict__ rec, double* __restrict__ out) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   const int c = slots[k];
   const size_t q = (size_t)level * d.T + c;
-  out[k] = d.rkh[q];
-  out[n + k] = u[c];
-  out[2 * (size_t)n + k] = v[c];
-  out[3 * (size_t)n + k] = d.rkh[q];
+  const Rec r = ld_rec(rec + c);
+  out[k] = r.h;
+  out[n + k] = r.u;
+  out[2 * (size_t)n + k] = r.v;
+  out[3 * (size_t)n + k] = r.h;
   out[4 * (size_t)n + k] = d.rku[q];
   out[5 * (size_t)n + k] = d.rkv[q];
 }
 
-// The received values into the listed (halo) slots, and their dry flags as the owner
-// derived them from the same state (find_dry_cells, as rk_update and k_fric do)
+// The received values into the listed (halo) slots (their dry flags follow from the
+// same state as the owner's)
 __global__ void __launch_bounds__(256) k_unpack(Dev d, int level, int n, const int32_t* __restrict__ slots,
-                                                const double* __restrict__ in, double* __restrict__ u,
-                                                double* __restrict__ v, uint8_t* __restrict__ dry) {
+                                                const double* __restrict__ in, Rec* __restrict__ rec) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= n) return;
   const int c = slots[k];
   const size_t q = (size_t)level * d.T + c;
-  const double hh = in[3 * (size_t)n + k], uu = in[n + k], vv = in[2 * (size_t)n + k];
-  d.rkh[q] = hh;
+  const double hh = in[3 * (size_t)n + k];
+  if (level == 0 || level == d.K - 1) d.rkh[q] = hh;
   d.rku[q] = in[4 * (size_t)n + k];
   d.rkv[q] = in[5 * (size_t)n + k];
-  u[c] = uu;
-  v[c] = vv;
-  double um;
-  dry[c] = dry_flag(hh, uu, vv, d.h_dry, d.h_wet, &um);
+  st_rec(rec + c, Rec{hh, d.z[c], in[n + k], in[2 * (size_t)n + k]});
+}
+
+__global__ void __launch_bounds__(256) k_split(Dev d, int c0, int n, int dry) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const Rec r = ld_rec(d.q + c0 + i);
+  if (dry) {
+    reinterpret_cast<uint8_t*>(d.io)[i] = rec_dry(d, r);
+  } else {
+    d.io[i] = r.u;
+    d.io[(size_t)n + i] = r.v;
+  }
 }
 
 // The iteration's residual, mass, max |phi| and stop test from the sums of all parts
@@ -2633,25 +3377,26 @@ __global__ void k_part_finish(Dev d, double top, double bot, double tm, double r
 void launch_part_scalar(const Dev& d, int which, double v, cudaStream_t st) {
   k_part_scalar<<<1, 32, 0, st>>>(d, which, v);
 }
-void launch_pack(const Dev& d, int level, int n, const int32_t* slots, const double* u, const double* v,
-                 double* out, cudaStream_t st) {
-  if (n > 0) k_pack<<<(n + 255) / 256, 256, 0, st>>>(d, level, n, slots, u, v, out);
+void launch_pack(const Dev& d, int level, int n, const int32_t* slots, const Rec* q, double* out, cudaStream_t st) {
+  if (n > 0) k_pack<<<(n + 255) / 256, 256, 0, st>>>(d, level, n, slots, q, out);
 }
-void launch_unpack(const Dev& d, int level, int n, const int32_t* slots, const double* in, double* u, double* v,
-                   uint8_t* dry, cudaStream_t st) {
-  if (n > 0) k_unpack<<<(n + 255) / 256, 256, 0, st>>>(d, level, n, slots, in, u, v, dry);
+void launch_unpack(const Dev& d, int level, int n, const int32_t* slots, const double* in, Rec* q, cudaStream_t st) {
+  if (n > 0) k_unpack<<<(n + 255) / 256, 256, 0, st>>>(d, level, n, slots, in, q);
+}
+void launch_split(const Dev& d, int c0, int n, int dry, cudaStream_t st) {
+  k_split<<<(n + 255) / 256, 256, 0, st>>>(d, c0, n, dry);
 }
 void launch_part_finish(const Dev& d, const double* sums, cudaStream_t st) {
   k_part_finish<<<1, 32, 0, st>>>(d, sums[0], sums[1], sums[2], sums[3]);
 }
 
-void launch_halo(const Dev& d, int level, uint8_t* f1, uint8_t* f2, cudaStream_t st) {
-  k_halo<<<(d.nhalo + 255) / 256, 256, 0, st>>>(d, level, f1, f2);
+void launch_halo(const Dev& d, int level, uint8_t* f1, cudaStream_t st) {
+  k_halo<<<(d.nhalo + 255) / 256, 256, 0, st>>>(d, level, f1);
 }
 void launch_link_fric(const Dev& d, cudaStream_t st) { k_link_fric<<<1, 32, 0, st>>>(d); }
-void launch_fric(const Dev& d, const double* u_src, const double* v_src, cudaStream_t st) {
-  if (d.nhalo > 0) k_fric<true><<<d.nblk_red, kRedThreads, 0, st>>>(d, u_src, v_src);
-  else k_fric<false><<<d.nblk_red, kRedThreads, 0, st>>>(d, u_src, v_src);
+void launch_fric(const Dev& d, const Rec* src, cudaStream_t st) {
+  if (d.nhalo > 0) k_fric<true><<<d.nblk_red, kRedThreads, 0, st>>>(d, src);
+  else k_fric<false><<<d.nblk_red, kRedThreads, 0, st>>>(d, src);
 }
 void launch_link_dt(const Dev& d, cudaStream_t st) { k_link_dt<<<1, 32, 0, st>>>(d); }
 void launch_link(const Dev& d, cudaStream_t st) { k_link<<<1, 32, 0, st>>>(d); }
@@ -2659,41 +3404,50 @@ void launch_link(const Dev& d, cudaStream_t st) { k_link<<<1, 32, 0, st>>>(d); }
 
 // ---------------------------------------------------------------------------
 // Host launchers of the templated stage kernels (api.cu is not templated).
+template <class R, int kThreads>
+static void launch_cell(const StageLaunch& L, const Dev& d, const Geo<R>& G) {
+  if (L.mode == CELL_PHI) k_cell<R, CELL_PHI, kThreads><<<L.grid, kThreads, L.smem, L.stream>>>(d, G, L.s);
+  else if (L.mode == CELL_FRIC) k_cell<R, CELL_FRIC, kThreads><<<L.grid, kThreads, L.smem, L.stream>>>(d, G, L.s);
+  else k_cell<R, CELL_UPDATE, kThreads><<<L.grid, kThreads, L.smem, L.stream>>>(d, G, L.s);
+}
 template <class R>
 static void launch_stage_t(const StageLaunch& L, const Dev& d, const Geo<R>& G) {
   switch (L.which) {
     case STAGE_GRAD:
-      k_grad<R, false><<<L.grid, L.block, 0, L.stream>>>(d, G, L.hs, L.dry, L.rku_prev, L.rkv_prev, L.u_in, L.v_in);
+      k_grad<R, false><<<L.grid, L.block, L.block.x / 32 * sizeof(GradBlock<R>), L.stream>>>(d, G, L.s, L.q, L.rku_prev,
+                                                                                             L.rkv_prev);
+      break;
+    case STAGE_GRAD_GEN:
+      k_grad<R, true><<<L.grid, L.block, L.block.x / 32 * sizeof(GradBlock<R>), L.stream>>>(d, G, L.s, L.q, L.rku_prev,
+                                                                                            L.rkv_prev);
       break;
     case STAGE_GRAD_BC:
-      k_grad<R, true><<<L.grid, L.block, 0, L.stream>>>(d, G, L.hs, L.dry, L.rku_prev, L.rkv_prev, L.u_in, L.v_in);
+      k_grad_bc<R><<<L.grid, L.block, 0, L.stream>>>(d, G, L.q, L.rku_prev, L.rkv_prev);
+      break;
+    case STAGE_PACK:
+      k_pack_geo<R><<<L.grid, L.block, 0, L.stream>>>(d, G);
       break;
     case STAGE_BC:
-      k_bc<R><<<L.grid, L.block, L.smem, L.stream>>>(d, G, L.hs, L.dry, L.u_in, L.v_in);
+      k_bc<R><<<L.grid, L.block, L.smem, L.stream>>>(d, G, L.q);
       break;
-    case STAGE_EFLUX:
-      k_eflux<R><<<L.grid, L.block, 0, L.stream>>>(d, G, L.hs, L.dry, L.u_in, L.v_in);
-      break;
-    case STAGE_FLUX:
-      k_flux<R><<<L.grid, L.block, 0, L.stream>>>(d, G, L.s, L.hs, L.dry, L.dry_next, L.u_in, L.v_in, L.u_out,
-                                                   L.v_out);
+    case STAGE_CELL:
+      if (L.block.x == 256) launch_cell<R, 256>(L, d, G);
+      else launch_cell<R, 512>(L, d, G);
       break;
     case STAGE_FLUX_BC:
-      k_flux_bc<R><<<L.grid, L.block, 0, L.stream>>>(d, G, L.s, L.hs, L.dry, L.dry_next, L.u_in, L.v_in, L.u_out,
-                                                      L.v_out);
+      if (L.mode == CELL_PHI) k_flux_bc<R, CELL_PHI, false><<<L.grid, L.block, 0, L.stream>>>(d, G, L.s, L.q, L.qo);
+      else if (L.mode == CELL_FRIC)
+        k_flux_bc<R, CELL_FRIC, false><<<L.grid, L.block, 0, L.stream>>>(d, G, L.s, L.q, L.qo);
+      else k_flux_bc<R, CELL_UPDATE, false><<<L.grid, L.block, 0, L.stream>>>(d, G, L.s, L.q, L.qo);
       break;
-    case STAGE_PHI:
-      k_flux_phi<R><<<L.grid, L.block, 0, L.stream>>>(d, G, L.hs, L.dry, L.u_in, L.v_in, 0);
-      break;
-    case STAGE_PHI_BC:
-      k_flux_phi<R><<<L.grid, L.block, 0, L.stream>>>(d, G, L.hs, L.dry, L.u_in, L.v_in, 1);
+    case STAGE_FLUX_BC_TILE:
+      k_flux_bc<R, CELL_UPDATE, true><<<L.grid, L.block, 0, L.stream>>>(d, G, L.s, L.q, L.qo);
       break;
     case STAGE_CULVERT:
-      k_culvert<R><<<L.grid, L.block, 0, L.stream>>>(d, G, L.hs, L.dry);
+      k_culvert<R><<<L.grid, L.block, 0, L.stream>>>(d, G, L.q);
       break;
     case STAGE_TILE:
-      k_tile<R><<<L.grid, L.block, L.smem, L.stream>>>(d, G, *L.tiles, L.s, L.hs, L.dry, L.dry_next, L.u_in, L.v_in,
-                                                        L.u_out, L.v_out, L.rku_prev, L.rkv_prev);
+      k_tile<R><<<L.grid, L.block, L.smem, L.stream>>>(d, G, *L.tiles, L.s, L.q, L.qo, L.rku_prev, L.rkv_prev);
       break;
   }
 }
@@ -2701,17 +3455,19 @@ static void launch_stage_t(const StageLaunch& L, const Dev& d, const Geo<R>& G) 
 #ifndef STORM_FVT_F32_TU
 void launch_stage(const StageLaunch& L, const Dev& d, const Geo<double>& Gd, const Geo<float>& Gf, bool mixed) {
   if (L.which == STAGE_UPDATE) {  // not templated: the same kernel on both paths
-    k_update<<<L.grid, L.block, 0, L.stream>>>(d, L.s, L.hs, L.dry, L.dry_next);
+    k_update<<<L.grid, L.block, 0, L.stream>>>(d, L.s, L.q, L.qo);
     return;
   }
   if (mixed) launch_stage_f32(L, d, Gf);
   else launch_stage_t<double>(L, d, Gd);
 }
 
-void launch_node(const Dev& d, const double* hs, const uint8_t* dry, const int32_t* list, int n, int block,
+void launch_node(const Dev& d, const Rec* q, const int32_t* list, int n, bool mark, bool full, int block,
                  cudaStream_t st) {
   const int cnt = list ? n : d.N;
-  if (cnt > 0) k_node<<<(cnt + block - 1) / block, block, 0, st>>>(d, hs, dry, list, n);
+  if (cnt <= 0) return;
+  if (mark) k_node<true><<<(cnt + block - 1) / block, block, 0, st>>>(d, q, list, n, full);
+  else k_node<false><<<(cnt + block - 1) / block, block, 0, st>>>(d, q, list, n, full);
 }
 
 void launch_rsavg(const Dev& d, int off, int cnt, cudaStream_t st) {
@@ -2728,7 +3484,75 @@ void set_bc_smem_limit(int bytes) {
 }
 #endif  // !STORM_FVT_F32_TU
 
+template <class R>
+static size_t cell_smem_t(const Dev& d) {
+  return sizeof(CellSmem<R>) + 24 * (size_t)d.cnw_max + 3 * sizeof(R) * (size_t)d.cne_max;
+}
+template <class R, int kThreads>
+static void set_cell_smem_n(int bytes) {
+  cudaFuncSetAttribute(k_cell<R, CELL_UPDATE, kThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  cudaFuncSetAttribute(k_cell<R, CELL_PHI, kThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  cudaFuncSetAttribute(k_cell<R, CELL_FRIC, kThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+}
+template <class R>
+static void set_cell_smem_t(int bytes) {
+  set_cell_smem_n<R, 256>(bytes);
+  set_cell_smem_n<R, 512>(bytes);
+}
+template <class R>
+static void cell_columns_t(const Dev& d, const Geo<R>& G, int s, int mode, CellCol* out) {
+  int n = 0;
+  for (int i = 0; i < kCellCols; i++) out[i] = CellCol{nullptr, 0, 0};
+  const auto col = [&](size_t dst, const auto* src, bool want = true) {
+    if (want)
+      out[n++] = CellCol{reinterpret_cast<const unsigned char*>(src), (uint32_t)(256 * sizeof(*src)), (uint32_t)dst};
+  };
+  using S = CellSmem<R>;
+  const size_t lv = (size_t)(s - 1) * d.T, T = d.T;
+  const bool upd = mode != CELL_PHI, l0 = upd && s > 1;
+  col(offsetof(S, q), d.q);
+  col(offsetof(S, desc), d.fdesc);
+  for (int k = 0; k < 3; k++) col(offsetof(S, lfe) + 512 * k, d.lfe + k * T);
+  col(offsetof(S, rad), d.rad);
+  col(offsetof(S, area), d.area);
+  col(offsetof(S, dzx), G.delz_x);
+  col(offsetof(S, dzy), G.delz_y);
+  col(offsetof(S, dhx), G.delh_x);
+  col(offsetof(S, dhy), G.delh_y);
+  col(offsetof(S, rku1), d.rku + lv, upd);
+  col(offsetof(S, rkv1), d.rkv + lv, upd);
+  col(offsetof(S, rkh0), d.rkh, l0);
+  col(offsetof(S, rku0), d.rku, l0);
+  col(offsetof(S, rkv0), d.rkv, l0);
+  col(offsetof(S, perim), d.perim, upd && (d.steady || mode == CELL_FRIC));
+  col(offsetof(S, cd), d.cd, mode == CELL_FRIC);
+}
+#ifndef STORM_FVT_F32_TU
+void cell_columns_f32(const Dev& d, const Geo<float>& G, int s, int mode, CellCol* out);
+void cell_columns(const Dev& d, const Geo<double>& Gd, const Geo<float>& Gf, bool mixed, int s, int mode,
+                  CellCol* out) {
+  if (mixed) cell_columns_f32(d, Gf, s, mode, out);
+  else cell_columns_t<double>(d, Gd, s, mode, out);
+}
+size_t cell_smem_f32(const Dev& d);
+void set_cell_smem_f32(int bytes);
+size_t cell_smem_bytes(const Dev& d, bool mixed) { return mixed ? cell_smem_f32(d) : cell_smem_t<double>(d); }
+void set_cell_smem_limit(int bytes) {
+  static int lim[64] = {0};
+  static std::mutex mu;
+  std::lock_guard<std::mutex> lock(mu);
+  const int b = raise_smem_limit(lim, bytes);
+  set_cell_smem_t<double>(b);
+  set_cell_smem_f32(b);
+}
+#endif
+
 #ifdef STORM_FVT_F32_TU
+void cell_columns_f32(const Dev& d, const Geo<float>& G, int s, int mode, CellCol* out) {
+  cell_columns_t<float>(d, G, s, mode, out);
+}
+size_t cell_smem_f32(const Dev& d) { return cell_smem_t<float>(d); }
+void set_cell_smem_f32(int bytes) { set_cell_smem_t<float>(bytes); }
 int tile_blocks_per_sm_f32(size_t smem) {
   int n = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_tile<float>, kTileThreads, smem);

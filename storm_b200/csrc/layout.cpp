@@ -110,6 +110,35 @@ int build_layout(const StormFvtMesh& m, const StormFvtOptions& opt, HostLayout& 
   auto NN = [&](int32_t old1) { return L.node_new[old1 - 1]; };
   L.last_cell_new = L.cell_new[T - 1];
 
+  // ---- face slots ------------------------------------------------------------
+  // A cell whose LSQ stencil is its three face neighbours (every interior cell of a
+  // mesh built by elemnt_db) numbers its faces in stencil order, so that the gradient
+  // kernel's neighbour k is both stencil member k and face neighbour k and is gathered
+  // once.  face_slot(i, j): slot (0-based) of the reference's local edge j of element i.
+  std::vector<uint8_t> slot_of(3 * (size_t)T);
+  L.plain.assign(T, 0);
+  for (int32_t o = 0; o < T; o++) {
+    uint8_t* sl = &slot_of[3 * (size_t)o];
+    for (int j = 0; j < 3; j++) sl[j] = (uint8_t)j;
+    if (m.t2t[o] != 3) continue;
+    int to[3] = {-1, -1, -1};
+    bool ok = true, used[3] = {false, false, false};
+    for (int j = 0; j < 3 && ok; j++) {
+      const int32_t nb = m.t2t3[3 * (size_t)o + j];
+      ok = nb >= 1 && nb <= T;
+      for (int k = 0; k < 3 && ok && to[j] < 0; k++)
+        if (!used[k] && m.t2t[(size_t)(k + 1) * T + o] == nb) {
+          to[j] = k;
+          used[k] = true;
+        }
+      ok = ok && to[j] >= 0;
+    }
+    if (!ok) continue;
+    for (int j = 0; j < 3; j++) sl[j] = (uint8_t)to[j];
+    L.plain[L.cell_new[o]] = 1;
+  }
+  auto face_slot = [&](int32_t i, int j) { return (int)slot_of[3 * (size_t)(i - 1) + (j - 1)]; };
+
   // ---- nodes ---------------------------------------------------------------
   L.zvtx.resize(N);
   L.node_x.resize(N);
@@ -193,7 +222,7 @@ int build_layout(const StormFvtMesh& m, const StormFvtOptions& opt, HostLayout& 
       int32_t pos = (int32_t)L.bce_cell.size();
       bce_of_edge[k] = pos;
       L.bce_cell.push_back(CN(i));
-      L.bce_slot.push_back(mm - 1);
+      L.bce_slot.push_back(face_slot(i, mm));
       L.bce_nx.push_back(nx);
       L.bce_ny.push_back(ny);
       L.bce_tx.push_back(tx);
@@ -292,7 +321,7 @@ int build_layout(const StormFvtMesh& m, const StormFvtOptions& opt, HostLayout& 
       ie_of[k] = e;
       L.eL[e] = CN(e1);
       L.eR[e] = CN(e2);
-      L.eslot[e] = (uint8_t)((m1 - 1) | ((m2 - 1) << 2));
+      L.eslot[e] = (uint8_t)(face_slot(e1, m1) | (face_slot(e2, m2) << 2));
       L.enx[e] = nx;
       L.eny[e] = ny;
       L.elen[e] = m.edge_length[k - 1];
@@ -375,8 +404,9 @@ int build_layout(const StormFvtMesh& m, const StormFvtOptions& opt, HostLayout& 
     // per-slot data
     int64_t key[3];
     for (int j = 1; j <= 3; j++) {
-      size_t q = (size_t)(j - 1) * T + c;
-      L.vert[q] = NN(GV(i1, j));
+      L.vert[(size_t)(j - 1) * T + c] = NN(GV(i1, j));
+      const int sj = face_slot(i1, j);
+      const size_t q = (size_t)sj * T + c;
       int32_t nb = m.t2t3[3 * (size_t)o + (j - 1)];
       L.t2t3[q] = (nb >= 1 && nb <= T) ? CN(nb) : -1;
       L.rc_x[q] = m.rc_x[(size_t)(j - 1) * T + o];
@@ -397,10 +427,10 @@ int build_layout(const StormFvtMesh& m, const StormFvtOptions& opt, HostLayout& 
         if (e1 != i1 && e2 != i1) return set_error(STORM_ERR_MESH, "storm_fvt_create: edge/element tables disagree");
         int mo = local_edge(other, k);
         if (mo < 1) return set_error(STORM_ERR_MESH, "storm_fvt_create: edge not in its element");
-        L.fkind[q] = (uint8_t)((e1 == i1 ? FACE_LEFT : FACE_RIGHT) | ((mo - 1) << 4));
+        L.fkind[q] = (uint8_t)((e1 == i1 ? FACE_LEFT : FACE_RIGHT) | (face_slot(other, mo) << 4));
         L.fref[q] = ie_of[k];  // the interior-edge record holding this face's flux
         L.fz0[q] = kHalf * (m.zvtx[EP(k, 1) - 1] + m.zvtx[EP(k, 2) - 1]);
-        key[j - 1] = (int64_t)k;
+        key[sj] = (int64_t)k;
       } else {
         if (GE(i1, j) < 0) {
           nx = -nx;
@@ -410,16 +440,16 @@ int build_layout(const StormFvtMesh& m, const StormFvtOptions& opt, HostLayout& 
           if (in_elem(k) != i1) return set_error(STORM_ERR_MESH, "storm_fvt_create: wall edge element mismatch");
           L.fkind[q] = FACE_WALL;
           L.fref[q] = wall_pos[k];
-          key[j - 1] = ((int64_t)1 << 40) + k;
+          key[sj] = ((int64_t)1 << 40) + k;
         } else {
           auto it = bce_of_edge.find(k);
           if (it != bce_of_edge.end() && in_elem(k) == i1) {
             L.fkind[q] = FACE_BC;
             L.fref[q] = it->second;
-            key[j - 1] = ((int64_t)2 << 40) + it->second;
+            key[sj] = ((int64_t)2 << 40) + it->second;
           } else {
             L.fkind[q] = FACE_NONE;
-            key[j - 1] = ((int64_t)3 << 40) + j;
+            key[sj] = ((int64_t)3 << 40) + sj;
           }
         }
       }
@@ -515,7 +545,7 @@ int build_layout(const StormFvtMesh& m, const StormFvtOptions& opt, HostLayout& 
     int32_t i = in_elem(k);
     int mm = local_edge(i, k);
     if (i < 1 || mm < 1) return set_error(STORM_ERR_MESH, "storm_fvt_create: stage edge without element");
-    L.hvmask[CN(i)] |= (uint8_t)(1u << (mm - 1));
+    L.hvmask[CN(i)] |= (uint8_t)(1u << face_slot(i, mm));
   }
   (void)opt;
   return 0;
@@ -557,7 +587,7 @@ void merge_layouts(const std::vector<HostLayout>& parts, int block, HostLayout& 
   M.area.assign(T, 1.0); M.perim.assign(T, 1.0); M.xc.assign(T, 0.0); M.yc.assign(T, 0.0);
   M.z.assign(T, 0.0); M.delz_x.assign(T, 0.0); M.delz_y.assign(T, 0.0); M.zmax.assign(T, 0.0);
   M.cd.assign(T, 0.0); M.lsq_a.assign(T, 1.0); M.lsq_b.assign(T, 0.0); M.lsq_c.assign(T, 1.0);
-  M.lsq_det.assign(T, 1.0); M.nst.assign(T, 0); M.forder.assign(T, 0); M.hvmask.assign(T, 0);
+  M.lsq_det.assign(T, 1.0); M.nst.assign(T, 0); M.plain.assign(T, 0); M.forder.assign(T, 0); M.hvmask.assign(T, 0);
   // padding slots are never live, so only the scenarios' own cells decide
   M.lsq_derived = true;
   for (const HostLayout& P : parts) M.lsq_derived = M.lsq_derived && P.lsq_derived;
@@ -582,7 +612,7 @@ void merge_layouts(const std::vector<HostLayout>& parts, int block, HostLayout& 
       M.area[g] = P.area[c]; M.perim[g] = P.perim[c]; M.xc[g] = P.xc[c]; M.yc[g] = P.yc[c];
       M.z[g] = P.z[c]; M.delz_x[g] = P.delz_x[c]; M.delz_y[g] = P.delz_y[c]; M.zmax[g] = P.zmax[c];
       M.cd[g] = P.cd[c]; M.lsq_a[g] = P.lsq_a[c]; M.lsq_b[g] = P.lsq_b[c]; M.lsq_c[g] = P.lsq_c[c];
-      M.lsq_det[g] = P.lsq_det[c]; M.nst[g] = P.nst[c]; M.forder[g] = P.forder[c]; M.hvmask[g] = P.hvmask[c];
+      M.lsq_det[g] = P.lsq_det[c]; M.nst[g] = P.nst[c]; M.plain[g] = P.plain[c]; M.forder[g] = P.forder[c]; M.hvmask[g] = P.hvmask[c];
       if (!P.wcoef1.empty()) { M.wcoef1[g] = P.wcoef1[c]; M.wcoef2[g] = P.wcoef2[c]; }
       for (int j = 0; j < 3; j++) {
         const size_t q = (size_t)j * P.T + c, qg = (size_t)j * T + g;

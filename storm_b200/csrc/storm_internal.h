@@ -32,8 +32,13 @@ enum BcKind : int32_t {
   BC_FREE = 5       // free_flow htype 0
 };
 
+constexpr uint32_t kDescReal = 0x80000000u;  // Dev::fdesc: a cell slot that holds a cell
 constexpr uint8_t kOrderHasBc = 0x40;  // forder flag: the cell has an open-boundary face
 constexpr uint8_t kOrderHasCulvert = 0x80;  // forder flag: a culvert end lies in the cell
+constexpr uint8_t kNstPlain = 0x80;  // flag beside the stencil count on the device: HostLayout::plain
+constexpr uint8_t kNstBc = 0x40;     // the cell has an open-boundary face
+constexpr uint8_t kNstLast = 0x20;   // element n_elems of its scenario (steady friction dt)
+constexpr uint8_t kNstCount = 0x1f;
 constexpr int kMaxStencil = 19;   // elemnt_db.f90:42 maxdim = 20 (count + 19 ids)
 constexpr int kMaxBcEdges = 8192; // edges per open boundary handled by one CTA
 
@@ -55,6 +60,7 @@ struct HostLayout {
   // the stencil values it loads instead of reading four more arrays
   bool lsq_derived = false;
   std::vector<uint8_t> nst, forder, hvmask;
+  std::vector<uint8_t> plain;  // 1: the stencil is the three face neighbours, in slot order
   std::vector<int32_t> bc_cells;  // cells with an open-boundary face, increasing
   std::vector<int32_t> rs_cells, rs_off;  // cells by colour of the t2t stencil (new ids), CSR
   // [3][T]

@@ -246,7 +246,7 @@ class Solver:
         return dict(zip(("node", "grad", "eflux", "flux"), ch.tolist()))
 
     def set_stage_path(self, path: int):
-        """STAGE_PHASES (k_node, k_grad, k_eflux, k_flux: the default) or STAGE_FUSED /
+        """STAGE_PHASES (k_node, k_grad, k_cell: the default) or STAGE_FUSED /
         STAGE_FUSED_NODE_KERNEL (one tile kernel per stage); results are bitwise the
         same in FP64; re-captures the iteration graph."""
         _chk(lib().storm_fvt_set_stage_path(self._h, int(path)))
