@@ -188,10 +188,8 @@ __device__ __forceinline__ void stage_segment(const Seg& s, int row0, uint8_t* d
     }
     return;
   }
-  // aggregation: sum of the three edge rows of each cell, in rounds of eight chunks
-  // per thread (24 loads in flight) for the forward kernel's producers, four otherwise
-  if (nthr <= 224) stage_agg_rounds<8>(s, row0, dst, tid, nthr, cpr, total);
-  else stage_agg_rounds<4>(s, row0, dst, tid, nthr, cpr, total);
+  // aggregation: sum of the three edge rows of each cell, in rounds of four chunks
+  stage_agg_rounds<4>(s, row0, dst, tid, nthr, cpr, total);
 }
 
 // Stage an fp32 [rows][width] tile as bf16 (width 64 or 128).
@@ -254,8 +252,61 @@ __device__ __forceinline__ void stage_matrix(const bf16* src, int nrows, int nco
   }
 }
 
-constexpr int kProducersAsync = 352;
+// 16 bytes, or zeros without touching memory: a predicated load, so that a batch of them
+// is issued together (branches around loads made each wait for the one before).
+__device__ __forceinline__ uint4 ld_if(const void* p, bool want) {
+  uint4 v = make_uint4(0, 0, 0, 0);
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.s32 p, %5, 0;\n\t"
+      "@p ld.global.v4.u32 {%0, %1, %2, %3}, [%4];\n\t}\n"
+      : "+r"(v.x), "+r"(v.y), "+r"(v.z), "+r"(v.w)
+      : "l"(p), "r"(want ? 1 : 0));
+  return v;
+}
 
+// 64 columns (from col0) of a tile of the aggregation segment into one 128 x 64 block,
+// by 128 threads: rows r + k*agg_stride, k = 0, 1, 2, whose nbr entry is >= 0, added in
+// that order in fp32.  Eight chunks of 16 bytes a thread, in two rounds of four (twelve
+// loads in flight).
+__device__ __forceinline__ void stage_agg_block(const Seg& s, int row0, int col0, uint8_t* dst, int tid) {
+#pragma unroll
+  for (int h = 0; h < 8; h += 4) {
+    uint4 w[4][3];
+    bool m[4][3];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const int row = row0 + (tid >> 3) + (h + i) * 16;
+#pragma unroll
+      for (int k = 0; k < 3; k++) m[i][k] = s.nbr[static_cast<size_t>(k) * s.agg_stride + row] >= 0;
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const int row = row0 + (tid >> 3) + (h + i) * 16;
+#pragma unroll
+      for (int k = 0; k < 3; k++)
+        w[i][k] = ld_if(s.src + (static_cast<size_t>(k) * s.agg_stride + row) * s.width + col0 + (tid & 7) * 8, m[i][k]);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      float acc[8];
+#pragma unroll
+      for (int j = 0; j < 8; j++) acc[j] = 0.f;
+#pragma unroll
+      for (int k = 0; k < 3; k++) {
+        if (!m[i][k]) continue;
+        const bf16* b = reinterpret_cast<const bf16*>(&w[i][k]);
+#pragma unroll
+        for (int j = 0; j < 8; j++) acc[j] += __bfloat162float(b[j]);
+      }
+      uint4 v;
+      bf16* o = reinterpret_cast<bf16*>(&v);
+#pragma unroll
+      for (int j = 0; j < 8; j++) o[j] = __float2bfloat16(acc[j]);
+      *reinterpret_cast<uint4*>(dst + umma::sw128_offset((tid >> 3) + (h + i) * 16, (tid & 7) * 8)) = v;
+    }
+  }
+}
 // Asynchronous copy of one 16-byte chunk global -> shared (zero-filled when `valid` is
 // false); the copies of a thread are grouped with commit / wait_group.
 __device__ __forceinline__ void cp_async16(uint8_t* dst, const void* src, bool valid) {
@@ -269,28 +320,15 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// Issue (without waiting) the copies of one gathered, non-aggregated segment tile by
-// the 352 producer threads: every thread resolves the source rows of its (at most 6)
-// chunks first, all index loads in flight together, then issues its copies.
-constexpr int kMaxAsyncChunks = (kRows * 16 + kProducersAsync - 1) / kProducersAsync;  // 128 x 16 chunks
-__device__ __forceinline__ void stage_segment_async(const Seg& s, int row0, uint8_t* dst, int tid) {
-  const int cpr = s.width >> 3;
-  const int total = kRows * cpr;
-  int srow[kMaxAsyncChunks];
-#pragma unroll
-  for (int i = 0; i < kMaxAsyncChunks; i++) {
-    const int q = tid + i * kProducersAsync;
-    const int row = row0 + q / cpr;
-    srow[i] = (q < total) ? (s.idx ? s.idx[row] : row) : -1;
-  }
-#pragma unroll
-  for (int i = 0; i < kMaxAsyncChunks; i++) {
-    const int q = tid + i * kProducersAsync;
-    if (q >= total) continue;
-    const int r = q / cpr, c = q - r * cpr;
-    const bf16* src = s.src + static_cast<size_t>(srow[i] >= 0 ? srow[i] : 0) * s.width + c * 8;
-    cp_async16(dst + (c >> 3) * (kRows * 128) + umma::sw128_offset(r, (c & 7) * 8), src, srow[i] >= 0);
-  }
+// A lane's four of 128 row-map entries, loaded a tile ahead; by a whole warp, the first
+// entry if they are consecutive rows, else -1.
+__device__ __forceinline__ int4 map_entries(const int32_t* idx, int lane) {
+  const int32_t* e = idx + 4 * lane;
+  return make_int4(e[0], e[1], e[2], e[3]);
+}
+__device__ __forceinline__ int consecutive(int4 e, int lane) {
+  const int first = __shfl_sync(0xffffffffu, e.x, 0), want = first + 4 * lane;
+  return __all_sync(0xffffffffu, e.x == want && e.y == want + 1 && e.z == want + 2 && e.w == want + 3) ? first : -1;
 }
 
 __device__ __forceinline__ uint8_t* align1024(uint8_t* p) {
@@ -311,252 +349,403 @@ __device__ __forceinline__ void mma_kmajor(uint32_t tmem_d, uint32_t a, uint32_t
 
 // ---- forward ----------------------------------------------------------------------
 
-// Shared memory: W1 (128 x k_in), W2 (n_out x 128), two A staging buffers (128 x 128),
-// the hidden tile (128 x 128), barriers.
-__host__ __device__ constexpr size_t fwd_smem_bytes(int k_in, int n_out) {
-  return 1024 + static_cast<size_t>(kHid) * k_in * 2 + static_cast<size_t>(n_out) * kHid * 2 +
-         2 * (kRows * 128 * 2) + kRows * kHid * 2 + 256;
+// Shared memory: W1 (128 x k_in), W2 (n_out x 128), the ring of input blocks (128 rows x
+// 64 columns, 16 KB), the hidden tile (128 x 128), half an output tile, biases, barriers.
+constexpr int kBlk = kRows * 128;  // bytes of a block
+constexpr size_t kSmemMax = 227 * 1024;
+__host__ __device__ constexpr size_t fwd_fixed_bytes(int k_in, int n_out) {
+  return 1024 + static_cast<size_t>(kHid) * k_in * 2 + static_cast<size_t>(n_out) * kHid * 2 + kRows * kHid * 2 + kBlk +
+         4 * (kHid + 128) + 512;
 }
+__host__ __device__ constexpr int fwd_stages(int k_in, int n_out) {
+  const int n = static_cast<int>((kSmemMax - fwd_fixed_bytes(k_in, n_out)) / kBlk);
+  return n < 6 ? n : 6;
+}
+__host__ __device__ constexpr size_t fwd_smem_bytes(int k_in, int n_out) {
+  return fwd_fixed_bytes(k_in, n_out) + static_cast<size_t>(fwd_stages(k_in, n_out)) * kBlk;
+}
+static_assert(fwd_stages(384, 128) == 3, "the widest input leaves three ring stages");
 
-// Warp roles of the forward kernel (512 threads, sixteen warps, so up to 128
-// registers each):
-//   warps 0-10  producers: gather each input segment of the CTA's tiles into the
-//               two-buffer staging ring (a buffer is refilled once the MMAs that read
-//               it have completed); the gathers of scattered rows are what bounds the
-//               kernel, so most warps do them;
-//   warps 11-14 epilogue: TMEM -> bias + ReLU -> hidden tile, then TMEM -> bias
-//               (+ residual) -> output; warp w reads TMEM lanes 32(w%4)..32(w%4)+31;
-//   warp 15     one thread issues the MMAs: D1[slot] = A W1^T over the segments, then
-//               D2[slot] = a1 W2^T once the epilogue has written the hidden tile.
-// D1 and D2 are double-buffered in TMEM (slot = tile parity), so the MMAs of tile t+1
-// proceed while the epilogue drains tile t.  Every wait is bounded; a wait that runs
-// out raises the abort flag, which every role polls.
+struct FwdMaps {  // boxes of 64 columns x 128 rows (w2: n_out rows)
+  CUtensorMap seg[kMaxSeg], w1, w2, out, a1;
+};
+constexpr int kAnyRows = 1 << 30;  // rows of a mapped segment's matrix: the caller does not say
+
+// Warp roles of the forward kernel (512 threads):
+//   warp 0      hands out the ring's stages in the order of the blocks, and fills by TMA
+//               (the weights once, then) each 64-column block of the CTA's tiles whose
+//               rows follow one another (unmapped segments, and mapped ones where the map
+//               is a run, as the receiver's is);
+//   warp 1      one thread issues the MMAs: D1[slot] = A W1^T block by block as the ring
+//               fills, D2[slot] = a1 W2^T one tile behind, so the hidden tile's epilogue
+//               is hidden by the next tile's first products;
+//   warps 4-7   epilogue 1: D1 -> bias + ReLU -> hidden tile (stored by TMA in training);
+//   warps 8-11  epilogue 2: D2 -> bias + residual -> output, through half a tile of
+//               shared memory and a TMA store (direct stores, a row to a thread, take the
+//               L1 32 lines an instruction); its residual rows are read while D2 is still
+//               being computed;
+//   warps 12-15 the other blocks: mapped rows by cp.async (a negative entry reads zeros;
+//               TMA's gather4 took about 130 cycles per four half rows, 135 us for the
+//               edge update below), and the aggregation's sums of three edge rows.
+// One warp alone waits on `empty`, for every block in turn: a parity tells a phase only
+// from the one beside it, so a role that waited for its own blocks alone could take a stage
+// two uses early.  Warps 12-15 get theirs from it through `grant`, which holds no phase
+// but their own.
+// D1 and D2 are double-buffered in TMEM (slot = tile parity).  Every wait is bounded; a
+// wait that runs out raises the abort flag, which every role polls.
+//
+// What bounds it: the ring's three stages at k_in = 384, next to 96 KB of W1: a tile takes
+// about 10k cycles, most of it the way of a block from L2 to its stage.  Measured (us;
+// before, with one role a phase and direct stores): edge update with saved hidden rows
+// 90 (141) at 300,000 rows, 29 (43) at 75,000, 14 (19) at 9,000; node update 68 (77) at
+// 100,000 rows, encoder 46 (72) at 300,000, decoder 19 (25) at 100,000.
 constexpr int kFwdThreads = 512;
 __device__ __forceinline__ bool aborted(const int* flag) { return *reinterpret_cast<const volatile int*>(flag) != 0; }
-constexpr int kProducers = 352;
 
-__global__ void __launch_bounds__(kFwdThreads, 1) k_mlp_fwd(MlpFwd p) {
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+
+__global__ void __launch_bounds__(kFwdThreads, 1) k_mlp_fwd(const __grid_constant__ MlpFwd p,
+                                                              const __grid_constant__ FwdMaps maps) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = align1024(smem_raw);
+  const int nst = fwd_stages(p.k_in, p.n_out);
   uint8_t* w1s = base;
   uint8_t* w2s = w1s + kHid * p.k_in * 2;
-  uint8_t* abuf = w2s + p.n_out * kHid * 2;  // 2 x 32 KB
-  uint8_t* a1s = abuf + 2 * (kRows * 128 * 2);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(a1s + kRows * kHid * 2);
-  uint64_t* full = bars;        // [2] staging buffer filled (one arrival per producer)
-  uint64_t* empty = bars + 2;   // [2] MMAs reading the buffer done (commit)
-  uint64_t* d1full = bars + 4;  // [2] D1[slot] complete (commit)
-  uint64_t* a1full = bars + 6;  // hidden tile written (128 epilogue arrivals)
-  uint64_t* d2full = bars + 7;  // [2] D2[slot] complete (commit)
-  uint64_t* tfree = bars + 9;   // [2] epilogue done with D1/D2[slot] (128 arrivals)
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 11);
+  uint8_t* ring = w2s + p.n_out * kHid * 2;
+  uint8_t* a1s = ring + nst * kBlk;
+  uint8_t* ios = a1s + kRows * kHid * 2;
+  float* b1s = reinterpret_cast<float*>(ios + kBlk);
+  float* b2s = b1s + kHid;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(b2s + 128);
+  uint64_t* full = bars;          // [6] ring stage filled
+  uint64_t* empty = bars + 6;     // [6] MMAs reading the stage done (commit)
+  uint64_t* d1full = bars + 12;   // [2] D1[slot] complete (commit)
+  uint64_t* d1free = bars + 14;   // [2] epilogue 1 has read D1[slot]
+  uint64_t* a1full = bars + 16;   // hidden tile written
+  uint64_t* d2full = bars + 17;   // [2] D2[slot] complete, hidden tile read (commit)
+  uint64_t* d2free = bars + 19;   // [2] epilogue 2 has read D2[slot]
+  uint64_t* wfull = bars + 21;    // weights loaded
+  uint64_t* grant = bars + 22;    // [6] ring stage given to warps 12-15
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 28);
   __shared__ int s_abort;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
-    umma::mbar_init(&full[0], kProducers);
-    umma::mbar_init(&full[1], kProducers);
-    umma::mbar_init(&empty[0], 1);
-    umma::mbar_init(&empty[1], 1);
-    umma::mbar_init(&d1full[0], 1);
-    umma::mbar_init(&d1full[1], 1);
+    for (int i = 0; i < nst; i++) {
+      umma::mbar_init(&full[i], 1);
+      umma::mbar_init(&empty[i], 1);
+      umma::mbar_init(&grant[i], 1);
+    }
+    for (int i = 0; i < 2; i++) {
+      umma::mbar_init(&d1full[i], 1);
+      umma::mbar_init(&d1free[i], kRows);
+      umma::mbar_init(&d2full[i], 1);
+      umma::mbar_init(&d2free[i], kRows);
+    }
     umma::mbar_init(a1full, kRows);
-    umma::mbar_init(&d2full[0], 1);
-    umma::mbar_init(&d2full[1], 1);
-    umma::mbar_init(&tfree[0], kRows);
-    umma::mbar_init(&tfree[1], kRows);
+    umma::mbar_init(wfull, 1);
     umma::mbar_fence_init();
+    umma::fence_async_smem();
     s_abort = 0;
   }
-  if (warp == 0) umma::tmem_alloc(tmem_slot, 512);
-  {  // weights, staged by all threads
-    const int cpr1 = p.k_in >> 3, tot1 = kHid * cpr1;
-    for (int q = threadIdx.x; q < tot1; q += kFwdThreads) {
-      const int r = q / cpr1, c = q - r * cpr1;
-      *reinterpret_cast<uint4*>(w1s + (c >> 3) * (kHid * 128) + umma::sw128_offset(r, (c & 7) * 8)) =
-          *reinterpret_cast<const uint4*>(p.w1 + static_cast<size_t>(r) * p.k_in + c * 8);
-    }
-    const int cpr2 = kHid >> 3, tot2 = p.n_out * cpr2;
-    for (int q = threadIdx.x; q < tot2; q += kFwdThreads) {
-      const int r = q / cpr2, c = q - r * cpr2;
-      *reinterpret_cast<uint4*>(w2s + (c >> 3) * (p.n_out * 128) + umma::sw128_offset(r, (c & 7) * 8)) =
-          *reinterpret_cast<const uint4*>(p.w2 + static_cast<size_t>(r) * kHid + c * 8);
-    }
-  }
-  umma::fence_async_smem();
+  if (warp == 1) umma::tmem_alloc(tmem_slot, 512);
+  if (threadIdx.x >= 128 && threadIdx.x < 128 + kHid) b1s[threadIdx.x - 128] = p.b1[threadIdx.x - 128];
+  if (threadIdx.x >= 256 && static_cast<int>(threadIdx.x) < 256 + p.n_out) b2s[threadIdx.x - 256] = p.b2[threadIdx.x - 256];
   umma::fence_before_sync();
   __syncthreads();
   umma::fence_after_sync();
   const uint32_t tmem = *tmem_slot;
   const int ntiles = p.rows / kRows;
 
-  if (warp < 11) {
-    // ---- producers
-    // Gathered segments are copied with cp.async, keeping the copies of two segments
-    // in flight (a segment is announced once the next one has been issued); the
-    // aggregation segment sums three rows in registers.
-    const int tid = threadIdx.x;
+  if (warp == 0) {
+    // ---- TMA
+    if (lane == 0) {
+      umma::mbar_expect(wfull, static_cast<uint32_t>(kHid * p.k_in * 2 + p.n_out * kHid * 2));
+      for (int x = 0; x < p.k_in; x += 64) umma::tma_load(w1s + (x >> 6) * (kHid * 128), &maps.w1, x, 0, wfull);
+      for (int x = 0; x < kHid; x += 64) umma::tma_load(w2s + (x >> 6) * (p.n_out * 128), &maps.w2, x, 0, wfull);
+    }
     uint32_t g = 0;
-    int pending = -1;  // buffer whose cp.async copies are issued but not yet announced
-    for (int tile = blockIdx.x; tile < ntiles && !aborted(&s_abort); tile += gridDim.x) {
-      for (int s = 0; s < p.nseg; s++, g++) {
-        const int b = g & 1;
-        if (g >= 2 && !umma::mbar_wait(&empty[b], ((g >> 1) - 1) & 1)) {
-          s_abort = 1;
-          break;
+    bool ok = true;
+    int4 ent[kMaxSeg];
+#pragma unroll
+    for (int s = 0; s < kMaxSeg; s++)
+      if (s < p.nseg && p.seg[s].idx) ent[s] = map_entries(p.seg[s].idx + blockIdx.x * kRows, lane);
+    for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+      const int row0 = tile * kRows;
+      const int next = tile + gridDim.x < ntiles ? (tile + gridDim.x) * kRows : row0;
+      int run[kMaxSeg];  // first row of a segment whose 128 rows are consecutive, else -1
+#pragma unroll
+      for (int s = 0; s < kMaxSeg; s++) {
+        run[s] = row0;
+        if (s < p.nseg && p.seg[s].idx) {
+          run[s] = consecutive(ent[s], lane);
+          ent[s] = map_entries(p.seg[s].idx + next, lane);
         }
-        uint8_t* dst = abuf + b * (kRows * 128 * 2);
-        if (p.seg[s].agg) {
-          if (pending >= 0) {
-            cp_async_wait<0>();
-            umma::fence_async_smem();
-            umma::mbar_arrive(&full[pending]);
-            pending = -1;
+      }
+#pragma unroll
+      for (int s = 0; s < kMaxSeg; s++) {
+        if (s >= p.nseg) break;
+        const int nb = p.seg[s].width >> 6;
+        for (int b = 0; b < nb && ok; b++, g++) {
+          const int st = g % nst;
+          const uint32_t use = g / nst;
+          if (use > 0 && !umma::warp_wait(&empty[st], (use - 1) & 1)) ok = false;
+          ok = __all_sync(0xffffffffu, ok && !aborted(&s_abort));
+          if (!ok) break;
+          if (lane == 0) {
+            if (p.seg[s].agg || run[s] < 0) {
+              umma::mbar_arrive(&grant[st]);
+            } else {
+              umma::mbar_expect(&full[st], kBlk);
+              umma::tma_load(ring + st * kBlk, &maps.seg[s], b * 64, run[s], &full[st]);
+            }
           }
-          stage_segment(p.seg[s], tile * kRows, dst, tid, kProducers);
-          umma::fence_async_smem();
-          umma::mbar_arrive(&full[b]);
-        } else {
-          stage_segment_async(p.seg[s], tile * kRows, dst, tid);
-          cp_async_commit();
-          if (pending >= 0) {
-            cp_async_wait<1>();
-            umma::fence_async_smem();
-            umma::mbar_arrive(&full[pending]);
-          }
-          pending = b;
         }
       }
     }
-    if (pending >= 0) {
-      cp_async_wait<0>();
-      umma::fence_async_smem();
-      umma::mbar_arrive(&full[pending]);
+    if (!ok) s_abort = 1;
+    // the copies still in flight land before the block's shared memory is given up
+    for (uint32_t k = g > static_cast<uint32_t>(nst) ? g - nst : 0; k < g; k++) umma::warp_wait(&full[k % nst], (k / nst) & 1);
+    umma::warp_wait(wfull, 0);
+  } else if (warp == 1) {
+    // ---- MMA issuer
+    if (lane == 0) {
+      const uint32_t w1a = umma::smem_addr(w1s), w2a = umma::smem_addr(w2s);
+      const uint32_t ra = umma::smem_addr(ring), a1a = umma::smem_addr(a1s);
+      const uint32_t idesc1 = umma::idesc_bf16(kRows, kHid, false, false);
+      const uint32_t idesc2 = umma::idesc_bf16(kRows, p.n_out, false, false);
+      const int nblk = p.k_in >> 6;
+      const int mine = blockIdx.x < ntiles ? (ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
+      uint32_t g = 0;
+      bool ok = umma::mbar_wait(wfull, 0);
+      for (int t = 0; t <= mine && ok; t++) {
+        const int slot = t & 1;
+        if (t < mine) {  // D1 of tile t
+          if (t >= 2 && !umma::mbar_wait(&d1free[slot], ((t >> 1) - 1) & 1)) ok = false;
+          if (ok) umma::fence_after_sync();
+          for (int b = 0; b < nblk && ok; b++, g++) {
+            const int st = g % nst;
+            if (!umma::mbar_wait(&full[st], (g / nst) & 1)) {
+              ok = false;
+              break;
+            }
+            umma::fence_after_sync();
+            mma_kmajor(tmem + slot * 128, ra + st * kBlk, kBlk, w1a + b * (kHid * 128), kHid * 128, 64, idesc1, b > 0);
+            umma::commit(&empty[st]);
+          }
+          if (!ok) break;
+          umma::commit(&d1full[slot]);
+        }
+        if (t > 0) {  // D2 of tile t - 1
+          const int u = t - 1, us = u & 1;
+          if (u >= 2 && !umma::mbar_wait(&d2free[us], ((u >> 1) - 1) & 1)) ok = false;
+          if (!ok || !umma::mbar_wait(a1full, u & 1)) {
+            ok = false;
+            break;
+          }
+          umma::fence_after_sync();
+          mma_kmajor(tmem + 256 + us * 128, a1a, kBlk, w2a, p.n_out * 128, kHid, idesc2, false);
+          umma::commit(&d2full[us]);
+        }
+      }
+      // the last commits, before shared memory and TMEM are given up
+      if (ok)
+        for (uint32_t k = g > static_cast<uint32_t>(nst) ? g - nst : 0; k < g; k++)
+          if (!umma::mbar_wait(&empty[k % nst], (k / nst) & 1)) ok = false;
+      if (ok && mine > 0 && !umma::mbar_wait(&d2full[(mine - 1) & 1], ((mine - 1) >> 1) & 1)) ok = false;
+      if (!ok) s_abort = 1;
     }
-  } else if (warp < 15) {
-    // ---- epilogue
-    const int q = warp & 3;
-    const int r = q * 32 + lane;  // row of the tile = TMEM lane
-    const uint32_t lane_off = static_cast<uint32_t>(q * 32) << 16;
+  } else if (warp >= 4 && warp < 8) {
+    // ---- epilogue 1
+    const int r = (warp & 3) * 32 + lane;  // row of the tile = TMEM lane
+    const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
     uint32_t t = 0;
-    for (int tile = blockIdx.x; tile < ntiles && !aborted(&s_abort); tile += gridDim.x, t++) {
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, t++) {
       const int slot = t & 1;
-      const uint32_t d1 = tmem + slot * 128, d2 = tmem + 256 + slot * 128;
-      const size_t row = static_cast<size_t>(tile) * kRows + r;
-      if (!umma::mbar_wait(&d1full[slot], (t >> 1) & 1)) {
+      // the hidden tile is free once D2 of the tile before, and its copy out, have read it
+      const bool ok = umma::warp_wait(&d1full[slot], (t >> 1) & 1) &&
+                      (t == 0 || umma::warp_wait(&d2full[(t - 1) & 1], ((t - 1) >> 1) & 1)) && !aborted(&s_abort);
+      if (p.a1_save && warp == 4 && lane == 0) umma::tma_store_wait_read();
+      if (!umma::bar_all(1, kRows, ok)) {  // the four warps go on, or stop, together
         s_abort = 1;
         break;
       }
+      __syncwarp();
       umma::fence_after_sync();
+#pragma unroll
       for (int col0 = 0; col0 < kHid; col0 += 32) {
         float v[32];
-        umma::tmem_ld32(d1 + lane_off + col0, v);
-        uint4 pk[4];
-        bf16* o = reinterpret_cast<bf16*>(pk);
-#pragma unroll
-        for (int j = 0; j < 32; j++) o[j] = __float2bfloat16(fmaxf(v[j] + p.b1[col0 + j], 0.f));
+        umma::tmem_ld32(tmem + slot * 128 + lane_off + col0, v);
+        const float4* bp = reinterpret_cast<const float4*>(b1s + col0);
 #pragma unroll
         for (int j = 0; j < 4; j++) {
+          const float4 x = bp[2 * j], y = bp[2 * j + 1];
+          uint4 o;
+          o.x = pack_bf16(fmaxf(v[8 * j] + x.x, 0.f), fmaxf(v[8 * j + 1] + x.y, 0.f));
+          o.y = pack_bf16(fmaxf(v[8 * j + 2] + x.z, 0.f), fmaxf(v[8 * j + 3] + x.w, 0.f));
+          o.z = pack_bf16(fmaxf(v[8 * j + 4] + y.x, 0.f), fmaxf(v[8 * j + 5] + y.y, 0.f));
+          o.w = pack_bf16(fmaxf(v[8 * j + 6] + y.z, 0.f), fmaxf(v[8 * j + 7] + y.w, 0.f));
           const int c = col0 + j * 8;
-          *reinterpret_cast<uint4*>(a1s + (c >> 6) * (kRows * 128) + umma::sw128_offset(r, c & 63)) = pk[j];
-          if (p.a1_save) *reinterpret_cast<uint4*>(p.a1_save + row * kHid + c) = pk[j];
+          *reinterpret_cast<uint4*>(a1s + (c >> 6) * kBlk + umma::sw128_offset(r, c & 63)) = o;
         }
       }
       umma::fence_async_smem();
       umma::fence_before_sync();
+      umma::mbar_arrive(&d1free[slot]);
       umma::mbar_arrive(a1full);
-      if (!umma::mbar_wait(&d2full[slot], (t >> 1) & 1)) {
+      if (p.a1_save) {
+        umma::bar_sync(1, kRows);
+        if (warp == 4 && lane == 0) {
+          umma::tma_store(&maps.a1, 0, tile * kRows, a1s);
+          umma::tma_store(&maps.a1, 64, tile * kRows, a1s + kBlk);
+        }
+      }
+    }
+    if (p.a1_save && warp == 4 && lane == 0) umma::tma_store_wait();
+  } else if (warp >= 8 && warp < 12) {
+    // ---- epilogue 2
+    const int r = (warp & 3) * 32 + lane;
+    const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
+    const bool leader = warp == 8 && lane == 0;
+    uint32_t t = 0;
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, t++) {
+      const int slot = t & 1;
+      const size_t row = static_cast<size_t>(tile) * kRows + r;
+      uint4 res[16];
+#pragma unroll
+      for (int j = 0; j < 16; j++) {
+        res[j] = make_uint4(0, 0, 0, 0);
+        if (p.res && j * 8 < p.n_out) res[j] = reinterpret_cast<const uint4*>(p.res + row * p.n_out)[j];
+      }
+      const bool ok = umma::warp_wait(&d2full[slot], (t >> 1) & 1) && !aborted(&s_abort);
+      if (leader) umma::tma_store_wait_read();  // the half tile before has been read
+      if (!umma::bar_all(2, kRows, ok)) {
         s_abort = 1;
         break;
       }
       umma::fence_after_sync();
-      for (int col0 = 0; col0 < p.n_out; col0 += 32) {
-        float v[32];
-        const size_t o0 = row * p.n_out + col0;
-        if (p.res) {
-          uint4 rr[4];
-          const uint4* rp = reinterpret_cast<const uint4*>(p.res + o0);
 #pragma unroll
-          for (int j = 0; j < 4; j++) rr[j] = rp[j];
-          umma::tmem_ld32(d2 + lane_off + col0, v);
+      for (int half = 0; half < 2; half++) {
+        if (half * 64 >= p.n_out) break;
+        if (half > 0) {
+          if (leader) umma::tma_store_wait_read();
+          umma::bar_sync(2, kRows);
+        }
+#pragma unroll
+        for (int cc = 0; cc < 64; cc += 32) {
+          const int col0 = half * 64 + cc;
+          float v[32];
+          umma::tmem_ld32(tmem + 256 + slot * 128 + lane_off + col0, v);
+          if (p.res) {
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+              const uint4 w = res[(col0 >> 3) + j];
+              const uint32_t x[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+              for (int u = 0; u < 4; u++) {
+                v[8 * j + 2 * u] += __uint_as_float(x[u] << 16);
+                v[8 * j + 2 * u + 1] += __uint_as_float(x[u] & 0xffff0000u);
+              }
+            }
+          }
+          const float4* bp = reinterpret_cast<const float4*>(b2s + col0);
+#pragma unroll
+          for (int j = 0; j < 8; j++) {
+            const float4 x = bp[j];
+            v[4 * j] += x.x;
+            v[4 * j + 1] += x.y;
+            v[4 * j + 2] += x.z;
+            v[4 * j + 3] += x.w;
+          }
 #pragma unroll
           for (int j = 0; j < 4; j++) {
-            const bf16* b = reinterpret_cast<const bf16*>(&rr[j]);
-#pragma unroll
-            for (int u = 0; u < 8; u++) v[j * 8 + u] += __bfloat162float(b[u]);
+            const uint4 o = make_uint4(pack_bf16(v[8 * j], v[8 * j + 1]), pack_bf16(v[8 * j + 2], v[8 * j + 3]),
+                                       pack_bf16(v[8 * j + 4], v[8 * j + 5]), pack_bf16(v[8 * j + 6], v[8 * j + 7]));
+            *reinterpret_cast<uint4*>(ios + umma::sw128_offset(r, cc + j * 8)) = o;
           }
-        } else {
-          umma::tmem_ld32(d2 + lane_off + col0, v);
+          if (p.out_f32) {
+            float4* fp = reinterpret_cast<float4*>(p.out_f32 + row * p.n_out + col0);
+#pragma unroll
+            for (int j = 0; j < 8; j++) fp[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+          }
         }
-#pragma unroll
-        for (int j = 0; j < 32; j++) v[j] += p.b2[col0 + j];
-        uint4 pk[4];
-        bf16* o = reinterpret_cast<bf16*>(pk);
-#pragma unroll
-        for (int j = 0; j < 32; j++) o[j] = __float2bfloat16(v[j]);
-        uint4* op = reinterpret_cast<uint4*>(p.out + o0);
-#pragma unroll
-        for (int j = 0; j < 4; j++) op[j] = pk[j];
-        if (p.out_f32) {
-          float4* fp = reinterpret_cast<float4*>(p.out_f32 + o0);
-#pragma unroll
-          for (int j = 0; j < 8; j++) fp[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-        }
+        umma::fence_async_smem();
+        umma::bar_sync(2, kRows);
+        if (leader) umma::tma_store(&maps.out, half * 64, tile * kRows, ios);
+        __syncwarp();
       }
       umma::fence_before_sync();
-      umma::mbar_arrive(&tfree[slot]);
+      umma::mbar_arrive(&d2free[slot]);
     }
-  } else if (lane == 0) {
-    // ---- MMA issuer
-    const uint32_t w1a = umma::smem_addr(w1s), w2a = umma::smem_addr(w2s);
-    const uint32_t a1a = umma::smem_addr(a1s);
-    const uint32_t idesc1 = umma::idesc_bf16(kRows, kHid, false, false);
-    const uint32_t idesc2 = umma::idesc_bf16(kRows, p.n_out, false, false);
-    uint32_t g = 0, t = 0;
+    if (leader) umma::tma_store_wait();
+  } else if (warp >= 12) {
+    // ---- mapped rows and aggregation
+    const int tid = threadIdx.x - 384;
+    uint32_t g = 0, granted = 0;  // (bit: parity of a stage's next grant)
     bool ok = true;
-    for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, t++) {
-      const int slot = t & 1;
-      const uint32_t d1 = tmem + slot * 128, d2 = tmem + 256 + slot * 128;
-      if (t >= 2 && !umma::mbar_wait(&tfree[slot], ((t >> 1) - 1) & 1)) ok = false;
-      int kcol = 0;
-      for (int s = 0; s < p.nseg && ok; s++, g++) {
-        const int b = g & 1;
-        if (!umma::mbar_wait(&full[b], (g >> 1) & 1)) {
-          ok = false;
-          break;
+    int4 ent[kMaxSeg];
+#pragma unroll
+    for (int s = 0; s < kMaxSeg; s++)
+      if (s < p.nseg && p.seg[s].idx) ent[s] = map_entries(p.seg[s].idx + blockIdx.x * kRows, lane);
+    for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+      const int row0 = tile * kRows;
+      const int next = tile + gridDim.x < ntiles ? (tile + gridDim.x) * kRows : row0;
+#pragma unroll
+      for (int s = 0; s < kMaxSeg; s++) {
+        if (s >= p.nseg || !ok) break;
+        const Seg& sg = p.seg[s];
+        const int nb = sg.width >> 6;
+        bool mine = sg.agg;
+        if (!mine && sg.idx) {
+          mine = consecutive(ent[s], lane) < 0;
+          ent[s] = map_entries(sg.idx + next, lane);
         }
-        umma::fence_after_sync();
-        mma_kmajor(d1, umma::smem_addr(abuf + b * (kRows * 128 * 2)), kRows * 128,
-                   w1a + (kcol >> 6) * (kHid * 128), kHid * 128, p.seg[s].width, idesc1, s > 0);
-        umma::commit(&empty[b]);
-        kcol += p.seg[s].width;
+        if (!mine) {
+          g += nb;
+          continue;
+        }
+        // the segment's one or two blocks in flight together
+        for (int b = 0; b < nb && ok; b++) {
+          const int st = (g + b) % nst;
+          const bool given = umma::warp_wait(&grant[st], (granted >> st) & 1);
+          granted ^= 1u << st;
+          ok = umma::bar_all(4, kRows, given && !aborted(&s_abort));  // the four warps go on, or stop, together
+          if (!ok) break;
+          uint8_t* dst = ring + st * kBlk;
+          if (sg.agg) {
+            stage_agg_block(sg, row0, b * 64, dst, tid);
+          } else {
+            int src[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) src[i] = sg.idx[row0 + (tid >> 3) + i * 16];
+#pragma unroll
+            for (int i = 0; i < 8; i++)
+              cp_async16(dst + umma::sw128_offset((tid >> 3) + i * 16, (tid & 7) * 8),
+                         sg.src + static_cast<size_t>(src[i] >= 0 ? src[i] : 0) * sg.width + b * 64 + (tid & 7) * 8,
+                         src[i] >= 0);
+          }
+          cp_async_commit();
+        }
+        for (int b = 0; b < nb && ok; b++) {
+          if (b + 1 < nb) cp_async_wait<1>();
+          else cp_async_wait<0>();
+          umma::fence_async_smem();
+          umma::bar_sync(3, kRows);
+          if (tid == 0) umma::mbar_arrive(&full[(g + b) % nst]);
+        }
+        g += nb;
       }
-      if (!ok) break;
-      umma::commit(&d1full[slot]);
-      if (!umma::mbar_wait(a1full, t & 1)) {
-        ok = false;
-        break;
-      }
-      umma::fence_after_sync();
-      mma_kmajor(d2, a1a, kRows * 128, w2a, p.n_out * 128, kHid, idesc2, false);
-      umma::commit(&d2full[slot]);
     }
-    // drain: the last arrivals on the staging barriers before shared memory is released
-    if (ok && g > 0) {
-      const uint32_t uses0 = (g + 1) >> 1, uses1 = g >> 1;
-      if (uses0 > 0 && !umma::mbar_wait(&empty[0], (uses0 - 1) & 1)) ok = false;
-      if (uses1 > 0 && !umma::mbar_wait(&empty[1], (uses1 - 1) & 1)) ok = false;
-    }
-    if (t > 0 && ok) {  // the last D2 of each slot (the epilogue waited for them too)
-      const uint32_t last = t - 1;
-      if (!umma::mbar_wait(&d2full[last & 1], (last >> 1) & 1)) ok = false;
-    }
+    cp_async_wait<0>();
     if (!ok) s_abort = 1;
   }
   umma::fence_before_sync();
   __syncthreads();
   if (s_abort && threadIdx.x == 0) set_err(p.err, 1);
-  if (warp == 0) {
+  if (warp == 1) {
     umma::fence_after_sync();
     umma::tmem_dealloc(tmem, 512);
   }
@@ -1040,6 +1229,34 @@ int grid_for(int rows) {
   return tiles < num_sms() ? tiles : num_sms();
 }
 
+// Row-major bf16 [rows][cols] (cols a multiple of 64) in boxes of 64 columns x box_rows,
+// 128-byte swizzle.  cuTensorMapEncodeTiled comes from the runtime's driver entry point,
+// so the library needs no link to libcuda.
+using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                              const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                              CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+int tensor_map(CUtensorMap* m, const void* ptr, int rows, int cols, int box_rows) {
+  static const EncodeFn encode = [] {
+    void* fn = nullptr;
+    cudaDriverEntryPointQueryResult q{};
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+      fn = nullptr;
+    return reinterpret_cast<EncodeFn>(fn);
+  }();
+  if (!encode) return storm::set_error(STORM_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
+  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
+  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(cols) * 2};
+  const cuuint32_t box[2] = {64, static_cast<cuuint32_t>(box_rows)}, es[2] = {1, 1};
+  const CUresult r = encode(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, es,
+                            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                            CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS)
+    return storm::set_error(STORM_ERR_ARG, "matrix rows must start on 16-byte boundaries (tensor map error " +
+                                               std::to_string(static_cast<int>(r)) + ")");
+  return STORM_OK;
+}
+
 }  // namespace
 
 extern "C" {
@@ -1066,9 +1283,19 @@ int storm_gnn_mlp_forward(const StormGnnMlpFwd* a, int32_t* dev_err, void* strea
   p.w2 = static_cast<const bf16*>(a->w2); p.b2 = a->b2;
   p.res = static_cast<const bf16*>(a->res); p.out = static_cast<bf16*>(a->out);
   p.out_f32 = a->out_f32; p.a1_save = static_cast<bf16*>(a->a1_save); p.err = dev_err;
+  FwdMaps maps{};
+  for (int i = 0; i < a->nseg; i++) {
+    const Seg& g = p.seg[i];
+    if (g.agg) continue;
+    if ((rc = tensor_map(&maps.seg[i], g.src, g.idx ? kAnyRows : a->rows, g.width, kRows))) return rc;
+  }
+  if ((rc = tensor_map(&maps.w1, p.w1, kHid, a->k_in, kHid)) || (rc = tensor_map(&maps.w2, p.w2, a->n_out, kHid, a->n_out)) ||
+      (rc = tensor_map(&maps.out, p.out, a->rows, a->n_out, kRows)))
+    return rc;
+  if (p.a1_save && (rc = tensor_map(&maps.a1, p.a1_save, a->rows, kHid, kRows))) return rc;
   const size_t smem = fwd_smem_bytes(a->k_in, a->n_out);
   cudaFuncSetAttribute(k_mlp_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-  k_mlp_fwd<<<grid_for(a->rows), kFwdThreads, smem, static_cast<cudaStream_t>(stream)>>>(p);
+  k_mlp_fwd<<<grid_for(a->rows), kFwdThreads, smem, static_cast<cudaStream_t>(stream)>>>(p, maps);
   g_launches++;
   return cuda_check("k_mlp_fwd");
 }

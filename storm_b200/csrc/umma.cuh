@@ -12,6 +12,7 @@
 
 #include <cstdint>
 
+#include <cuda.h>
 #include <cuda_bf16.h>
 
 namespace storm {
@@ -130,6 +131,51 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
                "l"(src), "r"(bytes), "r"(smem_addr(bar))
                : "memory");
 }
+// ---- TMA (2-D tensor maps, 128-byte swizzle, 64 bf16 columns to a box) -----------
+// A tile {column x, row y} of the box's size.
+__device__ __forceinline__ void tma_load(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
+  asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+                   smem_addr(dst)),
+               "l"(map), "r"(x), "r"(y), "r"(smem_addr(bar))
+               : "memory");
+}
+__device__ __forceinline__ void tma_store(const CUtensorMap* map, int x, int y, const void* src) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(map), "r"(x),
+               "r"(y), "r"(smem_addr(src))
+               : "memory");
+  asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+// The thread's stores have read their shared memory / are complete.
+__device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void tma_store_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+__device__ __forceinline__ void tma_prefetch_map(const CUtensorMap* map) {
+  asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
+}
+// Barrier `id` (1..15) among `n` threads of the block, in whole warps: the warp's threads
+// are brought together first, and the unaligned form asks nothing more of them.
+__device__ __forceinline__ void bar_sync(int id, int n) {
+  __syncwarp();
+  asm volatile("barrier.cta.sync %0, %1;" ::"r"(id), "r"(n) : "memory");
+  __syncwarp();
+}
+
+// The same barrier; whether `ok` holds for all of them (so that they go on, or stop,
+// together).
+__device__ __forceinline__ bool bar_all(int id, int n, bool ok) {
+  int r;
+  __syncwarp();
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.s32 p, %3, 0;\n\t"
+      "barrier.cta.red.and.pred q, %1, %2, p;\n\t"
+      "selp.s32 %0, 1, 0, q;\n\t}\n"
+      : "=r"(r)
+      : "r"(id), "r"(n), "r"(ok ? 1 : 0)
+      : "memory");
+  __syncwarp();
+  return r != 0;
+}
+
 // Bounded wait for the phase with the given parity to complete.  Returns false when
 // the limit runs out (the caller records an error and abandons the tile).
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32_t limit = (1u << 22)) {
@@ -146,6 +192,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
     if (done) return true;
   }
   return false;
+}
+
+// The same by a whole warp, which leaves the wait together (a spin loop may let go of its
+// threads one by one, and TMEM loads, aligned barriers and elected copies need them all).
+__device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity));
 }
 
 }  // namespace umma

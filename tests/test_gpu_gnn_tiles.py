@@ -1,0 +1,95 @@
+"""The forward MLP kernel with several 128-row tiles per CTA: its ring of input blocks is
+filled by two roles (TMA for rows that follow one another, per-row copies for maps and
+aggregation), so the cases mix both from tile to tile, from one tile in all to a ragged
+last wave.
+
+Tolerance: as for single MLPs against the oracle (1e-2 relative L2, bf16 roundings flipped
+by the fp32 summation order), held by every tile by itself and by every row's
+largest error: a quarter of the row's largest value (64 bf16 roundings at its size), where
+a block from another tile is off by its whole size."""
+import numpy as np
+import pytest
+
+from oracle.gnn_oracle import GnnOracle, to_bf16
+from storm_b200 import gnn
+
+pytestmark = pytest.mark.gpu
+
+SMS = 148
+
+
+def _close(got, ref):
+    got, ref = np.asarray(got, np.float64), np.asarray(ref, np.float64)
+    d = (got - ref).reshape(-1, 128 * ref.shape[1])
+    r = ref.reshape(d.shape)
+    assert np.all(np.linalg.norm(d, axis=1) < 1e-2 * np.linalg.norm(r, axis=1))
+    assert np.all(np.abs(got - ref).max(1) < 64 * 2.0 ** -8 * np.abs(ref).max(1))
+
+
+def _map(rng, kind, rows, n):
+    """A row map into n rows: runs of 128, scattered rows with gaps, or both by tile."""
+    tiles = rows // 128
+    start = rng.integers(0, n - 127, size=tiles)
+    run = (start[:, None] + np.arange(128)).ravel()
+    any_ = rng.integers(-1, n, size=rows)
+    near = run.copy()
+    near[127::128] = -1  # a run but for its last row
+    if kind == "run":
+        out = run
+    elif kind == "scatter":
+        out = any_
+    else:
+        pick = np.repeat(rng.integers(0, 3, size=tiles), 128)
+        out = np.choose(pick, [run, any_, near])
+    return out.astype(np.int32)
+
+
+@pytest.mark.parametrize("tiles", [1, SMS - 1, SMS + 1, 3 * SMS + 5])
+@pytest.mark.parametrize("layer,kinds", [("edge0", ("run", "scatter")), ("edge0", ("mixed", "mixed")), ("node0", ()),
+                                         ("enc_edge", ()), ("dec", ())])
+def test_forward_many_tiles(storm_lib, tiles, layer, kinds):
+    import torch
+    net = gnn.WarmStartNet(seed=11)
+    dev = net.device
+    rng = np.random.default_rng(tiles)
+    rows, n = 128 * tiles, 128 * 40
+
+    def mat(r, w):
+        a = to_bf16(rng.normal(size=(r, w)))
+        return a, torch.tensor(a, dtype=torch.bfloat16, device=dev)
+
+    res = res_t = a1 = f32 = None
+    n_out = 64 if layer == "dec" else 128
+    orc = GnnOracle(net.specs, net.params_numpy(), net.n_layers)
+    if layer == "edge0":
+        res, res_t = mat(rows, 128)
+        h, h_t = mat(n, 128)
+        idx = [_map(rng, k, rows, n) for k in kinds]
+        idx_t = [torch.tensor(i, device=dev) for i in idx]
+        segs = [net._seg(res_t)] + [net._seg(h_t, idx=i) for i in idx_t]
+        A = np.concatenate([res] + [GnnOracle.gather(h, i) for i in idx], axis=1)
+        a1 = torch.empty((rows, 128), dtype=torch.bfloat16, device=dev)
+    elif layer == "node0":
+        res, res_t = mat(rows, 128)
+        e, e_t = mat(3 * rows, 128)
+        nbr = rng.integers(-1, 3, size=(3, rows)).astype(np.int32)
+        nbr_t = torch.tensor(nbr, device=dev)
+        segs = [net._seg(res_t), net._seg(e_t, agg=True, stride=rows, nbr=nbr_t)]
+        A = np.concatenate([res, orc.agg(e, nbr, rows)], axis=1)
+    else:
+        A, x_t = mat(rows, 64 if layer == "enc_edge" else 128)
+        segs = [net._seg(x_t, A.shape[1])]
+        if layer == "dec":
+            f32 = torch.empty((rows, 64), dtype=torch.float32, device=dev)
+        else:
+            a1 = torch.empty((rows, 128), dtype=torch.bfloat16, device=dev)
+    out = torch.empty((rows, n_out), dtype=torch.bfloat16, device=dev)
+    net._fwd(layer, rows, segs, out, res=res_t, out_f32=f32, a1_save=a1)
+    torch.cuda.synchronize()
+    net._check_err()
+    _, ref, ref_a1 = orc.mlp(layer, A, res=res)  # (the result before and after its rounding)
+    _close(out.float().cpu().numpy(), ref)
+    if a1 is not None:
+        _close(a1.float().cpu().numpy(), ref_a1)
+    if f32 is not None:
+        _close(f32.cpu().numpy(), ref)
