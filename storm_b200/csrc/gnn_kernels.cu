@@ -753,157 +753,297 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_mlp_fwd(const __grid_constan
 
 // ---- backward: data gradients -------------------------------------------------------
 
-__host__ __device__ constexpr size_t bwd_data_smem_bytes(int k_in, int n_out) {
+// Shared memory: W1 (128 x k_in), W2 (n_out x 128), dy as bf16 (128 x n_out), one or two
+// hidden tiles (a1 in, dz1 out), two output pieces (128 rows x 32 fp32), barriers.
+__host__ __device__ constexpr size_t data_fixed_bytes(int k_in, int n_out) {
   return 1024 + static_cast<size_t>(kHid) * k_in * 2 + static_cast<size_t>(n_out) * kHid * 2 +
-         kRows * 128 * 2 /* dy (up to 128 columns) */ + kRows * kHid * 2 /* dz1 */ + 256;
+         static_cast<size_t>(kRows) * n_out * 2 + 2 * kBlk + 256;
 }
+__host__ __device__ constexpr int data_buffers(int k_in, int n_out) {
+  return data_fixed_bytes(k_in, n_out) + 4 * kBlk + 64 <= kSmemMax ? 2 : 1;
+}
+__host__ __device__ constexpr size_t bwd_data_smem_bytes(int k_in, int n_out) {
+  return data_fixed_bytes(k_in, n_out) + static_cast<size_t>(data_buffers(k_in, n_out)) * 2 * kBlk;
+}
+static_assert(bwd_data_smem_bytes(384, 128) + 64 <= kSmemMax && data_buffers(256, 128) == 2, "shared memory");
 
-__global__ void __launch_bounds__(kThreads, 1) k_mlp_bwd_data(MlpBwdData p) {
+struct DataMaps {  // boxes of 64 bf16 or 32 fp32 columns x 128 rows (w2: n_out rows)
+  CUtensorMap w1, w2, a1, dz, out[kMaxSeg], add[kMaxSeg];
+};
+
+// Warp roles (640 threads), each a tile or more ahead of the next:
+//   warp 0       the weights by TMA;
+//   warp 1       one thread issues the MMAs: da1 = dy W2, then dA = dz1 W1 in chunks of
+//                128 columns, a chunk as soon as the tile before has left its TMEM;
+//   warps 4-7    a1 tile in by TMA, dz1 = da1 where a1 > 0 in its place, out by TMA;
+//   warps 8-15   two warpgroups, each with pieces of 32 columns of a chunk: the addend in
+//                by TMA, the sum in its place, out by TMA (a row to a thread, the direct
+//                loads and stores took the L1 32 lines an instruction);
+//   warps 16-19  dy rows in order, rounded to bf16.
+// da1 takes 128 and dA k_in of the 512 TMEM columns, so neither is doubled.
+// What bounds it: the fp32 rows (edge update: 512 B of dy, 256 of a1 and dz1 each, 1536 of
+// gradients and 512 of addend from L2 a row).  Measured (us; before, one role a phase):
+// edge update 174 (334) at 300,000 rows, 51 (95) at 75,000, 15 (29) at 9,000; node update
+// 60 (112) at 100,000 rows, encoder 58 (125) at 300,000, decoder 27 (62) at 100,000.
+constexpr int kDataThreads = 640;
+__global__ void __launch_bounds__(kDataThreads, 1) k_mlp_bwd_data(const __grid_constant__ MlpBwdData p,
+                                                                    const __grid_constant__ DataMaps maps) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = align1024(smem_raw);
-  uint8_t* w1s = base;                                // [128 hid][k_in] blocks of 64 cols (16 KB)
-  uint8_t* w2s = w1s + kHid * p.k_in * 2;             // [n_out][128]   blocks of 64 cols
-  uint8_t* dys = w2s + p.n_out * kHid * 2;            // [128][n_out]
-  uint8_t* dzs = dys + kRows * 128 * 2;               // [128][128]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(dzs + kRows * kHid * 2);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2);
+  const int ndz = data_buffers(p.k_in, p.n_out);
+  uint8_t* w1s = base;                             // [128 hid][k_in] blocks of 64 cols (16 KB)
+  uint8_t* w2s = w1s + kHid * p.k_in * 2;          // [n_out][128]   blocks of 64 cols
+  uint8_t* dys = w2s + p.n_out * kHid * 2;         // [128][n_out]
+  uint8_t* dzs = dys + kRows * p.n_out * 2;        // [ndz][128][128]
+  uint8_t* piece = dzs + ndz * 2 * kBlk;           // [2][128][32] fp32
+  uint64_t* bars = reinterpret_cast<uint64_t*>(piece + 2 * kBlk);
+  uint64_t* wfull = bars;          // weights loaded
+  uint64_t* dyfull = bars + 1;     // dy tile written
+  uint64_t* d1full = bars + 2;     // da1 complete, dy tile read (commit)
+  uint64_t* d1free = bars + 3;     // da1 read
+  uint64_t* a1full = bars + 4;     // [2] a1 tile loaded
+  uint64_t* dzfull = bars + 6;     // dz1 tile written
+  uint64_t* d2full = bars + 7;     // [3] chunk of dA complete (commit)
+  uint64_t* d2free = bars + 10;    // [3] chunk of dA read
+  uint64_t* addfull = bars + 13;   // [2] addend piece loaded
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
   __shared__ int s_abort;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   bool need_da = false;
   for (int s = 0; s < p.nseg; s++) need_da |= (p.dseg[s].out != nullptr);
   if (threadIdx.x == 0) {
-    umma::mbar_init(&bars[0], 1);
-    umma::mbar_init(&bars[1], 1);
+    umma::mbar_init(wfull, 1);
+    umma::mbar_init(dyfull, kRows);
+    umma::mbar_init(d1full, 1);
+    umma::mbar_init(d1free, kRows);
+    umma::mbar_init(dzfull, kRows);
+    for (int i = 0; i < 2; i++) {
+      umma::mbar_init(&a1full[i], 1);
+      umma::mbar_init(&addfull[i], 1);
+    }
+    for (int i = 0; i < 3; i++) {
+      umma::mbar_init(&d2full[i], 1);
+      umma::mbar_init(&d2free[i], 2 * kRows);
+    }
     umma::mbar_fence_init();
+    umma::fence_async_smem();
     s_abort = 0;
   }
-  if (warp == 0) umma::tmem_alloc(tmem_slot, 512);
-  stage_matrix(p.w1, kHid, p.k_in, w1s);
-  stage_matrix(p.w2, p.n_out, kHid, w2s);
-  umma::fence_async_smem();
+  if (warp == 1) umma::tmem_alloc(tmem_slot, 512);
   umma::fence_before_sync();
   __syncthreads();
   umma::fence_after_sync();
   const uint32_t tmem = *tmem_slot;
   const uint32_t dda1 = tmem, dda = tmem + 128;
-  const uint32_t w1a = umma::smem_addr(w1s), w2a = umma::smem_addr(w2s);
-  const uint32_t dya = umma::smem_addr(dys), dza = umma::smem_addr(dzs);
-  // da1 = dy W2 : A = dy [128 x n_out] K-major, B = W2 viewed [N=128 hid x K=n_out] MN-major
-  const uint32_t idesc_a1 = umma::idesc_bf16(kRows, kHid, false, true);
-  // dA = dz1 W1 : A = dz1 [128 x 128] K-major, B = W1 viewed [N=k_in x K=128] MN-major
-  const int nchunk = p.k_in >= 128 ? 128 : p.k_in;
-  const uint32_t idesc_da = umma::idesc_bf16(kRows, nchunk, false, true);
-
   const int ntiles = p.rows / kRows;
-  const int lane_base = (warp & 3) * 32;
-  const int r = lane_base + lane;
-  const int half = warp >> 2;
-  uint32_t it = 0;
+  const int mine = blockIdx.x < ntiles ? (ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
+  const int nch = (p.k_in + 127) >> 7;
+  const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
+  const int r = (warp & 3) * 32 + lane;  // row of the tile = TMEM lane
 
-  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, it++) {
-    const int row0 = tile * kRows;
-    stage_f32(p.dy, p.n_out, row0, dys);
-    umma::fence_async_smem();
-    umma::fence_before_sync();
-    __syncthreads();
-    if (threadIdx.x == 0) {
+  if (warp == 0) {
+    // ---- weights
+    if (lane == 0) {
+      umma::mbar_expect(wfull, static_cast<uint32_t>((need_da ? kHid * p.k_in * 2 : 0) + p.n_out * kHid * 2));
+      for (int x = 0; x < kHid; x += 64) umma::tma_load(w2s + (x >> 6) * (p.n_out * 128), &maps.w2, x, 0, wfull);
+      if (need_da)
+        for (int x = 0; x < p.k_in; x += 64) umma::tma_load(w1s + (x >> 6) * (kHid * 128), &maps.w1, x, 0, wfull);
+    }
+    umma::warp_wait(wfull, 0);  // landed before the block's shared memory is given up
+  } else if (warp == 1) {
+    // ---- MMA issuer
+    if (lane == 0) {
+      const uint32_t w1a = umma::smem_addr(w1s), w2a = umma::smem_addr(w2s);
+      const uint32_t dya = umma::smem_addr(dys);
+      // da1 = dy W2 : A = dy [128 x n_out] K-major, B = W2 viewed [N=128 hid x K=n_out] MN-major
+      const uint32_t idesc_a1 = umma::idesc_bf16(kRows, kHid, false, true);
+      bool ok = umma::mbar_wait(wfull, 0);
+      for (int t = 0; t < mine && ok; t++) {
+        ok = umma::mbar_wait(dyfull, t & 1) && (t == 0 || umma::mbar_wait(d1free, (t - 1) & 1));
+        if (!ok) break;
+        umma::fence_after_sync();
+        // K = n_out rows of W2; K-step 16 advances dy by 32 bytes (inside a 64-col block)
+        // and the MN-major W2 view by 16 rows (2 KB).
+        for (int k = 0; k < p.n_out; k += 16)
+          umma::mma_bf16(dda1, umma::desc_kmajor(dya + (k >> 6) * kBlk + (k & 63) * 2),
+                         umma::desc_mnmajor(w2a + k * 128, p.n_out * 128), idesc_a1, k > 0 ? 1u : 0u);
+        umma::commit(d1full);
+        if (!need_da) continue;
+        // dA = dz1 W1 : A = dz1 [128 x 128] K-major, B = W1 viewed [N=k_in x K=128] MN-major
+        ok = umma::mbar_wait(dzfull, t & 1);
+        const uint32_t dza = umma::smem_addr(dzs + (t % ndz) * 2 * kBlk);
+        for (int c = 0; c < nch && ok; c++) {
+          if (t > 0) ok = umma::mbar_wait(&d2free[c], (t - 1) & 1);
+          if (!ok) break;
+          umma::fence_after_sync();
+          const uint32_t idesc = umma::idesc_bf16(kRows, p.k_in - c * 128 >= 128 ? 128 : 64, false, true);
+          for (int k = 0; k < kHid; k += 16)
+            // W1 rows k.. (K index = hid), columns 128 c.. (two blocks of 16 KB)
+            umma::mma_bf16(dda + c * 128, umma::desc_kmajor(dza + (k >> 6) * kBlk + (k & 63) * 2),
+                           umma::desc_mnmajor(w1a + c * 2 * (kHid * 128) + k * 128, kHid * 128), idesc, k > 0 ? 1u : 0u);
+          umma::commit(&d2full[c]);
+        }
+      }
+      // the last commits, before shared memory and TMEM are given up
+      if (ok && mine > 0) {
+        ok = umma::mbar_wait(d1full, (mine - 1) & 1);
+        if (need_da) ok = umma::mbar_wait(&d2full[nch - 1], (mine - 1) & 1) && ok;
+      }
+      if (!ok) s_abort = 1;
+    }
+  } else if (warp >= 4 && warp < 8) {
+    // ---- dz1 = da1 * (a1 > 0)
+    const bool leader = warp == 4 && lane == 0;
+    int issued = 0, t = 0;
+    // a1 of the CTA's tile n, once dz1 of the tile before in its buffer has been read
+    auto load_a1 = [&](int n) {
+      uint8_t* dst = dzs + (n % ndz) * 2 * kBlk;
+      if (need_da && n >= ndz && !umma::mbar_wait(&d2full[nch - 1], (n - ndz) & 1)) {
+        s_abort = 1;
+        return;
+      }
+      umma::tma_store_wait_read();
+      umma::mbar_expect(&a1full[n % ndz], 2 * kBlk);
+      umma::tma_load(dst, &maps.a1, 0, (blockIdx.x + n * gridDim.x) * kRows, &a1full[n % ndz]);
+      umma::tma_load(dst + kBlk, &maps.a1, 64, (blockIdx.x + n * gridDim.x) * kRows, &a1full[n % ndz]);
+      issued = n + 1;
+    };
+    if (leader && mine > 0) load_a1(0);
+    for (; t < mine; t++) {
+      uint8_t* dz = dzs + (t % ndz) * 2 * kBlk;
+      if (ndz == 2 && leader && t + 1 < mine) load_a1(t + 1);
+      const bool ok = umma::warp_wait(&a1full[t % ndz], (t / ndz) & 1) && umma::warp_wait(d1full, t & 1) && !aborted(&s_abort);
+      if (!umma::bar_all(1, kRows, ok)) {  // the four warps go on, or stop, together
+        s_abort = 1;
+        break;
+      }
       umma::fence_after_sync();
-      // K = n_out rows of W2; K-step 16 advances dy by 32 bytes (inside a 64-col block)
-      // and the MN-major W2 view by 16 rows (2 KB).
-      for (int k = 0; k < p.n_out; k += 16) {
-        const uint64_t ad = umma::desc_kmajor(dya + (k >> 6) * (kRows * 128) + (k & 63) * 2);
-        const uint64_t bd = umma::desc_mnmajor(w2a + k * 128, p.n_out * 128);
-        umma::mma_bf16(dda1, ad, bd, idesc_a1, k > 0 ? 1u : 0u);
-      }
-      umma::commit(&bars[0]);
-    }
-    if (!umma::mbar_wait(&bars[0], it & 1)) s_abort = 1;
-    __syncthreads();
-    if (s_abort) break;
-    umma::fence_after_sync();
-    // epilogue: dz1 = da1 * (a1 > 0)
-    for (int cc = 0; cc < 64; cc += 32) {
-      const int col0 = half * 64 + cc;
-      float v[32];
-      umma::tmem_ld32(dda1 + (static_cast<uint32_t>(lane_base) << 16) + col0, v);
-      const uint4* ap = reinterpret_cast<const uint4*>(p.a1 + static_cast<size_t>(row0 + r) * kHid + col0);
-      uint4 pk[4];
-      bf16* o = reinterpret_cast<bf16*>(pk);
 #pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const uint4 w = ap[j];
-        const bf16* b = reinterpret_cast<const bf16*>(&w);
+      for (int col0 = 0; col0 < kHid; col0 += 32) {
+        float v[32];
+        umma::tmem_ld32(dda1 + lane_off + col0, v);
 #pragma unroll
-        for (int t = 0; t < 8; t++) o[j * 8 + t] = __float2bfloat16(__bfloat162float(b[t]) > 0.f ? v[j * 8 + t] : 0.f);
-      }
+        for (int j = 0; j < 4; j++) {
+          const int c = col0 + j * 8;
+          uint4* q = reinterpret_cast<uint4*>(dz + (c >> 6) * kBlk + umma::sw128_offset(r, c & 63));
+          const uint4 w = *q;
+          const uint32_t x[4] = {w.x, w.y, w.z, w.w};
+          uint32_t o[4];
 #pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const int c = col0 + j * 8;
-        *reinterpret_cast<uint4*>(dzs + (c >> 6) * (kRows * 128) + umma::sw128_offset(r, c & 63)) = pk[j];
-        if (p.dz1_save)
-          *reinterpret_cast<uint4*>(p.dz1_save + static_cast<size_t>(row0 + r) * kHid + c) = pk[j];
+          for (int u = 0; u < 4; u++)
+            o[u] = pack_bf16(__uint_as_float(x[u] << 16) > 0.f ? v[8 * j + 2 * u] : 0.f,
+                             __uint_as_float(x[u] & 0xffff0000u) > 0.f ? v[8 * j + 2 * u + 1] : 0.f);
+          *q = make_uint4(o[0], o[1], o[2], o[3]);
+        }
       }
-    }
-    if (!need_da) {
+      umma::fence_async_smem();
       umma::fence_before_sync();
-      __syncthreads();
-      continue;
-    }
-    umma::fence_async_smem();
-    umma::fence_before_sync();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      umma::fence_after_sync();
-      for (int n0 = 0; n0 < p.k_in; n0 += nchunk) {
-        for (int k = 0; k < kHid; k += 16) {
-          const uint64_t ad = umma::desc_kmajor(dza + (k >> 6) * (kRows * 128) + (k & 63) * 2);
-          // W1 rows k.. (K index = hid), columns n0.. (block n0/64 of 16 KB)
-          const uint64_t bd = umma::desc_mnmajor(w1a + (n0 >> 6) * (kHid * 128) + k * 128, kHid * 128);
-          umma::mma_bf16(dda + n0, ad, bd, idesc_da, k > 0 ? 1u : 0u);
+      umma::mbar_arrive(d1free);
+      if (need_da) umma::mbar_arrive(dzfull);
+      umma::bar_sync(1, kRows);
+      if (leader) {
+        if (p.dz1_save) {
+          const int row0 = (blockIdx.x + t * gridDim.x) * kRows;
+          umma::tma_store(&maps.dz, 0, row0, dz);
+          umma::tma_store(&maps.dz, 64, row0, dz + kBlk);
         }
+        if (ndz == 1 && t + 1 < mine) load_a1(t + 1);
       }
-      umma::commit(&bars[1]);
     }
-    if (!umma::mbar_wait(&bars[1], it & 1)) s_abort = 1;
-    __syncthreads();
-    if (s_abort) break;
-    umma::fence_after_sync();
-    // epilogue: segment gradients (fp32), plus the residual-path addend
-    {
-      int kcol = 0;
-      for (int s = 0; s < p.nseg; s++) {
-        const int w = p.seg_width[s];
-        const SegGrad g = p.dseg[s];
-        if (g.out) {
-          const int per_half = w / 2;
-          for (int cc = 0; cc < per_half; cc += 32) {
-            const int col0 = half * per_half + cc;
-            float v[32];
-            umma::tmem_ld32(dda + (static_cast<uint32_t>(lane_base) << 16) + kcol + col0, v);
-            const size_t o0 = static_cast<size_t>(row0 + r) * w + col0;
-            if (g.add) {
-              const float4* ap = reinterpret_cast<const float4*>(g.add + o0);
-#pragma unroll
-              for (int j = 0; j < 8; j++) {
-                const float4 a = ap[j];
-                v[4 * j] += a.x; v[4 * j + 1] += a.y; v[4 * j + 2] += a.z; v[4 * j + 3] += a.w;
-              }
+    if (leader) {
+      for (int n = t; n < issued; n++) umma::mbar_wait(&a1full[n % ndz], (n / ndz) & 1);  // (stopped early)
+      umma::tma_store_wait();
+    }
+  } else if (warp >= 8 && warp < 16) {
+    // ---- segment gradients (fp32), plus the residual-path addend
+    const int wg = (warp >> 2) - 2;
+    const bool leader = (warp & 3) == 0 && lane == 0;
+    uint8_t* buf = piece + wg * kBlk;
+    uint32_t nadd = 0;
+    bool ok = true;
+    for (int t = 0; t < mine && ok && need_da; t++) {
+      const int row0 = (blockIdx.x + t * gridDim.x) * kRows;
+      for (int c = 0; c < nch && ok; c++) {
+        const int np = p.k_in - c * 128 >= 128 ? 2 : 1;  // the warpgroup's pieces of the chunk
+        for (int q = 0; q < np; q++) {
+          const int col = c * 128 + (wg * np + q) * 32;
+          int s = 0, first = 0;
+          while (first + p.seg_width[s] <= col) first += p.seg_width[s++];
+          float* out = p.dseg[s].out;
+          const bool add = out && p.dseg[s].add;
+          if (leader && out) {
+            umma::tma_store_wait_read();  // the piece before has been read
+            if (add) {
+              umma::mbar_expect(&addfull[wg], kBlk);
+              umma::tma_load(buf, &maps.add[s], col - first, row0, &addfull[wg]);
             }
-            float4* op = reinterpret_cast<float4*>(g.out + o0);
-#pragma unroll
-            for (int j = 0; j < 8; j++) op[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
           }
+          if (q == 0) ok = umma::warp_wait(&d2full[c], t & 1);
+          if (add) ok = umma::warp_wait(&addfull[wg], nadd++ & 1) && ok;
+          ok = umma::bar_all(2 + wg, kRows, ok && !aborted(&s_abort));
+          if (!ok) break;
+          if (!out) continue;
+          umma::fence_after_sync();
+          float v[32];
+          umma::tmem_ld32(dda + lane_off + col, v);
+#pragma unroll
+          for (int j = 0; j < 8; j++) {
+            float4* o = reinterpret_cast<float4*>(buf + umma::sw128_offset(r, j * 8));
+            float4 a = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+            if (add) {
+              const float4 b = *o;
+              a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
+            }
+            *o = a;
+          }
+          umma::fence_async_smem();
+          umma::bar_sync(2 + wg, kRows);
+          if (leader) umma::tma_store(&maps.out[s], col - first, row0, buf);
         }
-        kcol += w;
+        umma::fence_before_sync();
+        umma::mbar_arrive(&d2free[c]);
       }
     }
-    umma::fence_before_sync();
-    __syncthreads();
+    if (!ok) s_abort = 1;
+    if (leader) umma::tma_store_wait();
+  } else if (warp >= 16) {
+    // ---- dy, rounded to bf16: a float4 a thread, rows in order
+    const int tid = threadIdx.x - 512;
+    const int sh = p.n_out == 128 ? 5 : 4;  // log2 of the float4s of a row
+    const int rounds = p.n_out == 128 ? 2 : 1;
+    constexpr int kIn = 16;                 // loads in flight
+    bool ok = true;
+    for (int t = 0; t < mine && ok; t++) {
+      const float4* src = reinterpret_cast<const float4*>(p.dy + static_cast<size_t>(blockIdx.x + t * gridDim.x) * kRows * p.n_out);
+      for (int h = 0; h < rounds; h++) {
+        float4 v[kIn];
+#pragma unroll
+        for (int i = 0; i < kIn; i++) v[i] = src[(h * kIn + i) * kRows + tid];
+        if (h == 0 && t > 0) ok = umma::warp_wait(d1full, (t - 1) & 1);
+        ok = __all_sync(0xffffffffu, ok && !aborted(&s_abort));
+        if (!ok) break;
+#pragma unroll
+        for (int i = 0; i < kIn; i++) {
+          const int q = (h * kIn + i) * kRows + tid;
+          const int row = q >> sh, c = (q & ((1 << sh) - 1)) * 4;
+          *reinterpret_cast<uint2*>(dys + (c >> 6) * kBlk + umma::sw128_offset(row, c & 56) + (c & 4) * 2) =
+              make_uint2(pack_bf16(v[i].x, v[i].y), pack_bf16(v[i].z, v[i].w));
+        }
+      }
+      if (!ok) break;
+      umma::fence_async_smem();
+      umma::mbar_arrive(dyfull);
+    }
+    if (!ok) s_abort = 1;
   }
-  if (s_abort && threadIdx.x == 0) set_err(p.err, 2);
+  umma::fence_before_sync();
   __syncthreads();
-  if (warp == 0) umma::tmem_dealloc(tmem, 512);
+  if (s_abort && threadIdx.x == 0) set_err(p.err, 2);
+  if (warp == 1) {
+    umma::fence_after_sync();
+    umma::tmem_dealloc(tmem, 512);
+  }
 }
 
 // ---- backward: weight gradients -------------------------------------------------------
@@ -1229,13 +1369,13 @@ int grid_for(int rows) {
   return tiles < num_sms() ? tiles : num_sms();
 }
 
-// Row-major bf16 [rows][cols] (cols a multiple of 64) in boxes of 64 columns x box_rows,
-// 128-byte swizzle.  cuTensorMapEncodeTiled comes from the runtime's driver entry point,
+// Row-major [rows][cols] (cols a multiple of 64) in boxes of 64 bf16 or 32 fp32 columns x
+// box_rows, 128-byte swizzle.  cuTensorMapEncodeTiled comes from the runtime's driver entry point,
 // so the library needs no link to libcuda.
 using EncodeFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                               const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                               CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-int tensor_map(CUtensorMap* m, const void* ptr, int rows, int cols, int box_rows) {
+int tensor_map(CUtensorMap* m, const void* ptr, int rows, int cols, int box_rows, bool f32 = false) {
   static const EncodeFn encode = [] {
     void* fn = nullptr;
     cudaDriverEntryPointQueryResult q{};
@@ -1246,9 +1386,9 @@ int tensor_map(CUtensorMap* m, const void* ptr, int rows, int cols, int box_rows
   }();
   if (!encode) return storm::set_error(STORM_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
   const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
-  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(cols) * 2};
-  const cuuint32_t box[2] = {64, static_cast<cuuint32_t>(box_rows)}, es[2] = {1, 1};
-  const CUresult r = encode(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, es,
+  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(cols) * (f32 ? 4 : 2)};
+  const cuuint32_t box[2] = {f32 ? 32u : 64u, static_cast<cuuint32_t>(box_rows)}, es[2] = {1, 1};
+  const CUresult r = encode(m, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, es,
                             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                             CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS)
@@ -1316,10 +1456,20 @@ int storm_gnn_mlp_backward_data(const StormGnnMlpBwdData* a, int32_t* dev_err, v
   p.dy = a->dy; p.a1 = static_cast<const bf16*>(a->a1);
   p.w1 = static_cast<const bf16*>(a->w1); p.w2 = static_cast<const bf16*>(a->w2);
   p.dz1_save = static_cast<bf16*>(a->dz1_save); p.err = dev_err;
+  DataMaps maps{};
+  if ((rc = tensor_map(&maps.w1, p.w1, kHid, a->k_in, kHid)) || (rc = tensor_map(&maps.w2, p.w2, a->n_out, kHid, a->n_out)) ||
+      (rc = tensor_map(&maps.a1, p.a1, a->rows, kHid, kRows)))
+    return rc;
+  if (p.dz1_save && (rc = tensor_map(&maps.dz, p.dz1_save, a->rows, kHid, kRows))) return rc;
+  for (int s = 0; s < a->nseg; s++) {
+    if (!p.dseg[s].out) continue;
+    if ((rc = tensor_map(&maps.out[s], p.dseg[s].out, a->rows, p.seg_width[s], kRows, true))) return rc;
+    if (p.dseg[s].add && (rc = tensor_map(&maps.add[s], p.dseg[s].add, a->rows, p.seg_width[s], kRows, true))) return rc;
+  }
   size_t smem = bwd_data_smem_bytes(a->k_in, a->n_out);
   if (smem < static_cast<size_t>(kMinBwdSmem)) smem = kMinBwdSmem;
   cudaFuncSetAttribute(k_mlp_bwd_data, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-  k_mlp_bwd_data<<<grid_for(a->rows), kThreads, smem, static_cast<cudaStream_t>(stream)>>>(p);
+  k_mlp_bwd_data<<<grid_for(a->rows), kDataThreads, smem, static_cast<cudaStream_t>(stream)>>>(p, maps);
   g_launches++;
   return cuda_check("k_mlp_bwd_data");
 }

@@ -93,3 +93,35 @@ def test_forward_many_tiles(storm_lib, tiles, layer, kinds):
         _close(a1.float().cpu().numpy(), ref_a1)
     if f32 is not None:
         _close(f32.cpu().numpy(), ref)
+
+
+@pytest.mark.parametrize("tiles", [1, SMS + 1, 3 * SMS + 5])
+@pytest.mark.parametrize("layer,outs", [("edge0", "axx"), ("edge0", "x0a"), ("node0", "ax"), ("node0", "00"),
+                                        ("enc_edge", "0"), ("enc_edge", "a"), ("dec", "x")])
+def test_backward_data_many_tiles(storm_lib, tiles, layer, outs):
+    """`outs`, a letter a segment: no gradient (0), one (x), one with an addend (a)."""
+    import torch
+    net = gnn.WarmStartNet(seed=12)
+    dev = net.device
+    rng = np.random.default_rng(tiles)
+    s = net.by_name[layer]
+    rows, widths = 128 * tiles, [min(s.k_in, 128)] * len(outs)
+    dy = rng.normal(size=(rows, s.n_out)).astype(np.float32)
+    a1 = to_bf16(np.maximum(rng.normal(size=(rows, 128)), 0.0))
+    add = [rng.normal(size=(rows, w)).astype(np.float32) if o == "a" else None for o, w in zip(outs, widths)]
+    dy_t, a1_t = torch.tensor(dy, device=dev), torch.tensor(a1, dtype=torch.bfloat16, device=dev)
+    add_t = [None if a is None else torch.tensor(a, device=dev) for a in add]
+    out_t = [None if o == "0" else torch.empty((rows, w), dtype=torch.float32, device=dev) for o, w in zip(outs, widths)]
+    dz_t = torch.empty((rows, 128), dtype=torch.bfloat16, device=dev)
+    net._bwd_data(layer, rows, widths, dy_t, a1_t, dz_t, out_t, add_t)
+    torch.cuda.synchronize()
+    net._check_err()
+    orc = GnnOracle(net.specs, net.params_numpy(), net.n_layers)
+    _, w1, _, w2, _ = orc.weights(layer)
+    dz = to_bf16((to_bf16(dy) @ w2) * (a1 > 0))
+    _close(dz_t.float().cpu().numpy(), dz)
+    da = np.asarray(dz, np.float64) @ w1
+    for i, (o, a) in enumerate(zip(out_t, add)):
+        if o is not None:
+            ref = da[:, 128 * i:128 * i + widths[i]]
+            _close(o.cpu().numpy(), ref if a is None else ref + a)
