@@ -14,9 +14,9 @@
 // (the message aggregation), so the edge update [e, h_src, h_dst] and the node
 // update [h, sum_k e_k] need no materialised concatenation.
 //
-// One CTA (256 threads) works on tiles of 128 rows.  Forward: D1 = A W1^T over the
-// segments (two staging buffers so a segment's load overlaps the previous segment's
-// MMAs), epilogue bias+ReLU into a shared-memory tile, D2 = a1 W2^T, epilogue
+// One CTA per SM works through tiles of 128 rows (64 in the weight gradients) with its warps
+// in fixed roles: copies, MMA issue, epilogues, rows that TMA cannot fetch.  Forward:
+// D1 = A W1^T over the segments, bias + ReLU into a shared-memory tile, D2 = a1 W2^T,
 // bias (+ residual).  Weights stay resident in shared memory for the CTA's lifetime.
 #include <cstdint>
 #include <cstdio>
@@ -33,7 +33,6 @@ using bf16 = __nv_bfloat16;
 
 constexpr int kRows = 128;     // rows per tile (MMA M)
 constexpr int kHid = 128;      // hidden width
-constexpr int kThreads = 256;  // 8 warps
 constexpr int kMaxSeg = 3;
 
 struct Seg {
@@ -93,165 +92,6 @@ __device__ __forceinline__ void set_err(int32_t* err, int code) {
 
 // ---- shared-memory staging -------------------------------------------------------
 
-// The staging helpers below give every thread up to eight 16-byte chunks of the tile
-// (chunk q = threadIdx.x + i*256) and issue all of a thread's global loads before any
-// of its shared-memory stores, so 32 KB per SM are in flight instead of one load per
-// thread at a time.
-constexpr int kChunksPerThread = 8;  // 128 rows x 16 chunks / 256 threads
-
-__device__ __forceinline__ void store_chunk(uint8_t* dst, int q, int cpr, uint4 v) {
-  const int r = q / cpr, c = q - r * cpr;
-  const int blk = c >> 3;
-  *reinterpret_cast<uint4*>(dst + blk * (kRows * 128) + umma::sw128_offset(r, (c & 7) * 8)) = v;
-}
-
-template <int R>
-__device__ __forceinline__ void stage_agg_rounds(const Seg& s, int row0, uint8_t* dst, int tid, int nthr, int cpr,
-                                                 int total) {
-  for (int h = 0; h * nthr < total; h += R) {
-    uint4 w[R][3];
-    bool m[R][3];
-#pragma unroll
-    for (int i = 0; i < R; i++) {
-      const int q = tid + (h + i) * nthr;
-      const int row = row0 + q / cpr;
-#pragma unroll
-      for (int k = 0; k < 3; k++)
-        m[i][k] = (q < total) && s.nbr[static_cast<size_t>(k) * s.agg_stride + row] >= 0;
-    }
-#pragma unroll
-    for (int i = 0; i < R; i++) {
-      const int q = tid + (h + i) * nthr;
-      const int row = row0 + q / cpr, c = q % cpr;
-#pragma unroll
-      for (int k = 0; k < 3; k++) {
-        w[i][k] = make_uint4(0, 0, 0, 0);
-        if (m[i][k]) {
-          const size_t er = static_cast<size_t>(k) * s.agg_stride + row;
-          w[i][k] = *reinterpret_cast<const uint4*>(s.src + er * s.width + c * 8);
-        }
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < R; i++) {
-      const int q = tid + (h + i) * nthr;
-      if (q >= total) continue;
-      float acc[8];
-#pragma unroll
-      for (int j = 0; j < 8; j++) acc[j] = 0.f;
-#pragma unroll
-      for (int k = 0; k < 3; k++) {
-        if (!m[i][k]) continue;
-        const bf16* b = reinterpret_cast<const bf16*>(&w[i][k]);
-#pragma unroll
-        for (int j = 0; j < 8; j++) acc[j] += __bfloat162float(b[j]);
-      }
-      uint4 v;
-      bf16* o = reinterpret_cast<bf16*>(&v);
-#pragma unroll
-      for (int j = 0; j < 8; j++) o[j] = __float2bfloat16(acc[j]);
-      store_chunk(dst, q, cpr, v);
-    }
-  }
-}
-
-// Stage rows [row0, row0+128) of one segment into `dst` (blocks of 128 x 64, 16 KB
-// each) with `nthr` threads (thread `tid` of them), in rounds of eight chunks per thread.
-__device__ __forceinline__ void stage_segment(const Seg& s, int row0, uint8_t* dst, int tid = -1,
-                                              int nthr = kThreads) {
-  if (tid < 0) tid = threadIdx.x;
-  const int cpr = s.width >> 3;  // 16-byte chunks per row
-  const int total = kRows * cpr;
-  if (!s.agg) {
-    for (int q0 = 0; q0 < total; q0 += kChunksPerThread * nthr) {
-      uint4 v[kChunksPerThread];
-      int srow[kChunksPerThread];
-#pragma unroll
-      for (int i = 0; i < kChunksPerThread; i++) {
-        const int q = q0 + tid + i * nthr;
-        const int row = row0 + q / cpr;
-        srow[i] = (q < total) ? (s.idx ? s.idx[row] : row) : -1;
-      }
-#pragma unroll
-      for (int i = 0; i < kChunksPerThread; i++) {
-        const int q = q0 + tid + i * nthr;
-        const int c = q % cpr;
-        v[i] = make_uint4(0, 0, 0, 0);
-        if (srow[i] >= 0)
-          v[i] = *reinterpret_cast<const uint4*>(s.src + static_cast<size_t>(srow[i]) * s.width + c * 8);
-      }
-#pragma unroll
-      for (int i = 0; i < kChunksPerThread; i++) {
-        const int q = q0 + tid + i * nthr;
-        if (q < total) store_chunk(dst, q, cpr, v[i]);
-      }
-    }
-    return;
-  }
-  // aggregation: sum of the three edge rows of each cell, in rounds of four chunks
-  stage_agg_rounds<4>(s, row0, dst, tid, nthr, cpr, total);
-}
-
-// Stage an fp32 [rows][width] tile as bf16 (width 64 or 128).
-__device__ __forceinline__ void stage_f32(const float* src, int width, int row0, uint8_t* dst) {
-  const int cpr = width >> 3;
-  const int total = kRows * cpr;
-#pragma unroll
-  for (int h = 0; h < kChunksPerThread; h += 4) {
-    float4 a[4], b[4];
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const int q = threadIdx.x + (h + i) * kThreads;
-      a[i] = b[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (q < total) {
-        const int r = q / cpr, c = q - r * cpr;
-        const float4* p = reinterpret_cast<const float4*>(src + static_cast<size_t>(row0 + r) * width + c * 8);
-        a[i] = p[0];
-        b[i] = p[1];
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const int q = threadIdx.x + (h + i) * kThreads;
-      if (q >= total) continue;
-      uint4 v;
-      bf16* o = reinterpret_cast<bf16*>(&v);
-      o[0] = __float2bfloat16(a[i].x); o[1] = __float2bfloat16(a[i].y); o[2] = __float2bfloat16(a[i].z);
-      o[3] = __float2bfloat16(a[i].w); o[4] = __float2bfloat16(b[i].x); o[5] = __float2bfloat16(b[i].y);
-      o[6] = __float2bfloat16(b[i].z); o[7] = __float2bfloat16(b[i].w);
-      store_chunk(dst, q, cpr, v);
-    }
-  }
-}
-
-// Stage a bf16 row-major [nrows][ncols] matrix (ncols multiple of 64) as blocks of
-// nrows x 64 (block stride nrows*128 bytes); loads batched eight per thread.
-__device__ __forceinline__ void stage_matrix(const bf16* src, int nrows, int ncols, uint8_t* dst) {
-  const int cpr = ncols >> 3;
-  const int total = nrows * cpr;
-  for (int q0 = 0; q0 < total; q0 += kChunksPerThread * kThreads) {
-    uint4 v[kChunksPerThread];
-#pragma unroll
-    for (int i = 0; i < kChunksPerThread; i++) {
-      const int q = q0 + threadIdx.x + i * kThreads;
-      v[i] = make_uint4(0, 0, 0, 0);
-      if (q < total) {
-        const int r = q / cpr, c = q - r * cpr;
-        v[i] = *reinterpret_cast<const uint4*>(src + static_cast<size_t>(r) * ncols + c * 8);
-      }
-    }
-#pragma unroll
-    for (int i = 0; i < kChunksPerThread; i++) {
-      const int q = q0 + threadIdx.x + i * kThreads;
-      if (q < total) {
-        const int r = q / cpr, c = q - r * cpr;
-        const int blk = c >> 3;
-        *reinterpret_cast<uint4*>(dst + blk * (nrows * 128) + umma::sw128_offset(r, (c & 7) * 8)) = v[i];
-      }
-    }
-  }
-}
-
 // 16 bytes, or zeros without touching memory: a predicated load, so that a batch of them
 // is issued together (branches around loads made each wait for the one before).
 __device__ __forceinline__ uint4 ld_if(const void* p, bool want) {
@@ -265,13 +105,13 @@ __device__ __forceinline__ uint4 ld_if(const void* p, bool want) {
   return v;
 }
 
-// 64 columns (from col0) of a tile of the aggregation segment into one 128 x 64 block,
-// by 128 threads: rows r + k*agg_stride, k = 0, 1, 2, whose nbr entry is >= 0, added in
-// that order in fp32.  Eight chunks of 16 bytes a thread, in two rounds of four (twelve
-// loads in flight).
+// 64 columns (from col0) of kR rows of the aggregation segment into one kR x 64 block, by
+// 128 threads: rows r + k*agg_stride, k = 0, 1, 2, whose nbr entry is >= 0, added in that
+// order in fp32.  Chunks of 16 bytes, four to a thread and round (twelve loads in flight).
+template <int kR>
 __device__ __forceinline__ void stage_agg_block(const Seg& s, int row0, int col0, uint8_t* dst, int tid) {
 #pragma unroll
-  for (int h = 0; h < 8; h += 4) {
+  for (int h = 0; h < kR / 16; h += 4) {
     uint4 w[4][3];
     bool m[4][3];
 #pragma unroll
@@ -329,6 +169,15 @@ __device__ __forceinline__ int4 map_entries(const int32_t* idx, int lane) {
 __device__ __forceinline__ int consecutive(int4 e, int lane) {
   const int first = __shfl_sync(0xffffffffu, e.x, 0), want = first + 4 * lane;
   return __all_sync(0xffffffffu, e.x == want && e.y == want + 1 && e.z == want + 2 && e.w == want + 3) ? first : -1;
+}
+
+// The same for 64 rows, two entries a lane.
+__device__ __forceinline__ int2 slab_entries(const int32_t* idx, int lane) {
+  return make_int2(idx[2 * lane], idx[2 * lane + 1]);
+}
+__device__ __forceinline__ int consecutive(int2 e, int lane) {
+  const int first = __shfl_sync(0xffffffffu, e.x, 0), want = first + 2 * lane;
+  return __all_sync(0xffffffffu, e.x == want && e.y == want + 1) ? first : -1;
 }
 
 __device__ __forceinline__ uint8_t* align1024(uint8_t* p) {
@@ -716,7 +565,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_mlp_fwd(const __grid_constan
           if (!ok) break;
           uint8_t* dst = ring + st * kBlk;
           if (sg.agg) {
-            stage_agg_block(sg, row0, b * 64, dst, tid);
+            stage_agg_block<kRows>(sg, row0, b * 64, dst, tid);
           } else {
             int src[8];
 #pragma unroll
@@ -1048,135 +897,300 @@ __global__ void __launch_bounds__(kDataThreads, 1) k_mlp_bwd_data(const __grid_c
 
 // ---- backward: weight gradients -------------------------------------------------------
 
-__host__ __device__ constexpr size_t bwd_weight_smem_bytes(int k_in) {
-  return 1024 + static_cast<size_t>(kRows) * k_in * 2 /* A */ + kRows * kHid * 2 /* dz1 */ +
-         kRows * kHid * 2 /* a1 */ + kRows * 128 * 2 /* dy */ + 256;
+// A stage holds 64 rows: A (k_in columns), dz1, a1, dy as bf16, in blocks of 64 columns.
+constexpr int kSlab = 64;
+constexpr int kSlabBlk = kSlab * 128;  // bytes of a block
+__host__ __device__ constexpr int weight_stage_bytes(int k_in, int n_out) {
+  return ((k_in + n_out) / 64 + 4) * kSlabBlk;
 }
+__host__ __device__ constexpr int weight_stages(int k_in, int n_out) {
+  const int n = static_cast<int>((kSmemMax - 1024 - 4096) / weight_stage_bytes(k_in, n_out));
+  return n < 4 ? n : 4;
+}
+__host__ __device__ constexpr size_t bwd_weight_smem_bytes(int k_in, int n_out) {
+  return 1024 + static_cast<size_t>(weight_stages(k_in, n_out)) * weight_stage_bytes(k_in, n_out) + 256;
+}
+static_assert(weight_stages(384, 128) == 2, "the widest input leaves two stages");
 
 __host__ __device__ constexpr int part_stride(int k_in, int n_out) {
   return kHid * k_in + kHid + n_out * kHid + n_out;
 }
 
-__global__ void __launch_bounds__(kThreads, 1) k_mlp_bwd_weight(MlpBwdWeight p) {
+struct WeightMaps {  // boxes of 64 columns x 64 rows
+  CUtensorMap seg[kMaxSeg], a1, dz;
+};
+
+// Warp roles (384 threads) around a ring of 64-row stages:
+//   warp 0      TMA: dz1, a1 and the segments whose rows follow one another;
+//   warp 1      one thread issues the MMAs (K = rows), both gradients staying in TMEM;
+//   warps 2-3   column sums of dz1 (db1), from the stage;
+//   warps 4-7   mapped rows by cp.async, the aggregation's sums of three edge rows;
+//   warps 8-11  dy rounded to bf16, with its column sums (db2, of the fp32 values).
+// Every role takes part in every stage's use, so none can come two uses early.  At the end
+// warps 4-11 write the CTA's partial sums (summed over CTAs, in order, by k_reduce_parts).
+// What bounds it: the rows from HBM (edge update: 256 B each of e, dz1 and a1 and 512 of dy
+// a row, 3.4k cycles a stage), and for few rows the partial sums (262 KB a CTA, 39 MB in
+// all, through L2).  With the reduction, measured (us; before, one stage of 128 rows and
+// db1, db2 summed from global memory): edge update 91 (282) at 300,000 rows, 39 (91) at
+// 75,000, 19 (35) at 9,000; node update 70 (147) at 100,000 rows, encoder 68 (166) at
+// 300,000, decoder 33 (66) at 100,000.
+constexpr int kWeightThreads = 384;
+__global__ void __launch_bounds__(kWeightThreads, 1) k_mlp_bwd_weight(const __grid_constant__ MlpBwdWeight p,
+                                                                        const __grid_constant__ WeightMaps maps) {
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* base = align1024(smem_raw);
-  uint8_t* as = base;                         // [128][k_in] blocks of 64 cols (16 KB each)
-  uint8_t* dzs = as + kRows * p.k_in * 2;     // [128][128]
-  uint8_t* a1s = dzs + kRows * kHid * 2;      // [128][128]
-  uint8_t* dys = a1s + kRows * kHid * 2;      // [128][n_out]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(dys + kRows * 128 * 2);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 1);
+  uint8_t* ring = align1024(smem_raw);
+  const int nst = weight_stages(p.k_in, p.n_out);
+  const int stage_bytes = weight_stage_bytes(p.k_in, p.n_out);
+  const int dz_off = (p.k_in >> 6) * kSlabBlk, a1_off = dz_off + 2 * kSlabBlk, dy_off = a1_off + 2 * kSlabBlk;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(ring + nst * stage_bytes);
+  uint64_t* full = bars;        // [4] stage filled: TMA, 128 gathering and 128 converting threads
+  uint64_t* empty = bars + 4;   // [4] stage read: MMAs (commit) and 64 summing threads
+  uint64_t* done = bars + 8;    // all MMAs complete (commit)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 9);
   __shared__ int s_abort;
-  __shared__ float s_db[2][kHid];
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
-    umma::mbar_init(&bars[0], 1);
+    for (int i = 0; i < nst; i++) {
+      umma::mbar_init(&full[i], 1 + 256);
+      umma::mbar_init(&empty[i], 1 + 64);
+    }
+    umma::mbar_init(done, 1);
     umma::mbar_fence_init();
+    umma::fence_async_smem();
     s_abort = 0;
   }
-  if (warp == 0) umma::tmem_alloc(tmem_slot, 512);
+  if (warp == 1) umma::tmem_alloc(tmem_slot, 512);
   umma::fence_before_sync();
   __syncthreads();
   umma::fence_after_sync();
   const uint32_t tmem = *tmem_slot;
   const uint32_t dw1 = tmem, dw2 = tmem + p.k_in;  // dW1 [128 hid][k_in], dW2^T [128 hid][n_out]
-  const uint32_t aa = umma::smem_addr(as), dza = umma::smem_addr(dzs);
-  const uint32_t a1a = umma::smem_addr(a1s), dya = umma::smem_addr(dys);
-  const int nchunk = p.k_in >= 128 ? 128 : p.k_in;
-  // dW1 = dz1^T A : A-operand dz1^T [M=128 hid, K=rows] MN-major; B = A^T [N=k_in chunk, K=rows] MN-major
-  const uint32_t idesc_w1 = umma::idesc_bf16(kHid, nchunk, true, true);
-  // dW2^T = a1^T dy : A-operand a1^T [M=128, K=rows] MN-major; B = dy^T [N=n_out, K=rows] MN-major
-  const uint32_t idesc_w2 = umma::idesc_bf16(kHid, p.n_out, true, true);
+  const int nslabs = p.rows / kSlab;
+  const int mine = (nslabs - 1 - static_cast<int>(blockIdx.x)) / static_cast<int>(gridDim.x) + 1;  // (grid <= nslabs / 2)
+  auto row_of = [&](int g) { return static_cast<int>(blockIdx.x + g * gridDim.x) * kSlab; };
 
-  float db1 = 0.f, db2 = 0.f;  // thread t < 128: column t of dz1; t >= 128: column t-128 of dy
-  const int ntiles = p.rows / kRows;
-  uint32_t it = 0;
-  bool any = false;
-  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, it++) {
-    const int row0 = tile * kRows;
-    if (it > 0) {
-      if (!umma::mbar_wait(&bars[0], (it - 1) & 1)) s_abort = 1;
-      __syncthreads();
-      if (s_abort) break;
-    }
-    int kcol = 0;
-    for (int s = 0; s < p.nseg; s++) {
-      stage_segment(p.seg[s], row0, as + (kcol >> 6) * (kRows * 128));
-      kcol += p.seg[s].width;
-    }
-    stage_matrix(p.dz1 + static_cast<size_t>(row0) * kHid, kRows, kHid, dzs);
-    stage_matrix(p.a1 + static_cast<size_t>(row0) * kHid, kRows, kHid, a1s);
-    stage_f32(p.dy, p.n_out, row0, dys);
-    // bias gradients from global (fp32 dy, bf16 dz1), fixed row order
-    if (threadIdx.x < kHid) {
-      const int c = threadIdx.x;
-      for (int rr = 0; rr < kRows; rr++) db1 += __bfloat162float(p.dz1[static_cast<size_t>(row0 + rr) * kHid + c]);
-    } else if (threadIdx.x - kHid < p.n_out) {
-      const int c = threadIdx.x - kHid;
-      for (int rr = 0; rr < kRows; rr++) db2 += p.dy[static_cast<size_t>(row0 + rr) * p.n_out + c];
-    }
-    umma::fence_async_smem();
-    umma::fence_before_sync();
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      umma::fence_after_sync();
-      for (int k = 0; k < kRows; k += 16) {  // K = rows of the tile; 16 rows = 2 KB
-        const uint64_t ad = umma::desc_mnmajor(dza + k * 128, kRows * 128);
-        for (int n0 = 0; n0 < p.k_in; n0 += nchunk) {
-          const uint64_t bd = umma::desc_mnmajor(aa + (n0 >> 6) * (kRows * 128) + k * 128, kRows * 128);
-          umma::mma_bf16(dw1 + n0, ad, bd, idesc_w1, (it > 0 || k > 0) ? 1u : 0u);
+  float sum[4] = {0.f, 0.f, 0.f, 0.f};  // warps 2-3: two columns of dz1; 8-11: four of dy
+  bool ok = true;
+  if (warp == 0) {
+    // ---- TMA
+    int2 ent[kMaxSeg];
+#pragma unroll
+    for (int s = 0; s < kMaxSeg; s++)
+      if (s < p.nseg && p.seg[s].idx) ent[s] = slab_entries(p.seg[s].idx + row_of(0), lane);
+    int g = 0;
+    for (; g < mine; g++) {
+      const int st = g % nst, row0 = row_of(g), next = row_of(g + 1 < mine ? g + 1 : g);
+      int run[kMaxSeg];  // first row of a segment whose 64 rows are consecutive, else -1
+      uint32_t bytes = 4 * kSlabBlk;
+#pragma unroll
+      for (int s = 0; s < kMaxSeg; s++) {
+        run[s] = -1;
+        if (s >= p.nseg || p.seg[s].agg) continue;
+        run[s] = row0;
+        if (p.seg[s].idx) {
+          run[s] = consecutive(ent[s], lane);
+          ent[s] = slab_entries(p.seg[s].idx + next, lane);
         }
-        const uint64_t a2 = umma::desc_mnmajor(a1a + k * 128, kRows * 128);
-        const uint64_t b2 = umma::desc_mnmajor(dya + k * 128, kRows * 128);
-        umma::mma_bf16(dw2, a2, b2, idesc_w2, (it > 0 || k > 0) ? 1u : 0u);
+        if (run[s] >= 0) bytes += (p.seg[s].width >> 6) * kSlabBlk;
       }
-      umma::commit(&bars[0]);
+      if (g >= nst) ok = umma::warp_wait(&empty[st], (g / nst - 1) & 1);
+      ok = __all_sync(0xffffffffu, ok && !aborted(&s_abort));
+      if (!ok) break;
+      if (lane == 0) {
+        uint8_t* dst = ring + st * stage_bytes;
+        umma::mbar_expect(&full[st], bytes);
+#pragma unroll
+        for (int s = 0; s < kMaxSeg; s++) {
+          if (s >= p.nseg) break;
+          for (int x = 0; x < p.seg[s].width; x += 64, dst += kSlabBlk)
+            if (run[s] >= 0) umma::tma_load(dst, &maps.seg[s], x, run[s], &full[st]);
+        }
+        for (int x = 0; x < kHid; x += 64) {
+          umma::tma_load(dst + (x >> 6) * kSlabBlk, &maps.dz, x, row0, &full[st]);
+          umma::tma_load(dst + (2 + (x >> 6)) * kSlabBlk, &maps.a1, x, row0, &full[st]);
+        }
+      }
+      __syncwarp();
     }
-    any = true;
+    // the copies still in flight land before the block's shared memory is given up
+    for (int k = g > nst ? g - nst : 0; k < g; k++) umma::warp_wait(&full[k % nst], (k / nst) & 1);
+  } else if (warp == 1) {
+    // ---- MMA issuer
+    if (lane == 0) {
+      // dW1 = dz1^T A : A-operand dz1^T [M=128 hid, K=rows] MN-major; B = A^T [N=k_in chunk, K=rows] MN-major
+      // dW2^T = a1^T dy : A-operand a1^T [M=128, K=rows] MN-major; B = dy^T [N=n_out, K=rows] MN-major
+      const uint32_t idesc_w2 = umma::idesc_bf16(kHid, p.n_out, true, true);
+      for (int g = 0; g < mine; g++) {
+        const int st = g % nst;
+        if (!umma::mbar_wait(&full[st], (g / nst) & 1)) {
+          ok = false;
+          break;
+        }
+        umma::fence_after_sync();
+        const uint32_t a = umma::smem_addr(ring + st * stage_bytes);
+        for (int k = 0; k < kSlab; k += 16) {  // 16 rows = 2 KB
+          const uint64_t ad = umma::desc_mnmajor(a + dz_off + k * 128, kSlabBlk);
+          for (int n0 = 0; n0 < p.k_in; n0 += 128)
+            umma::mma_bf16(dw1 + n0, ad, umma::desc_mnmajor(a + (n0 >> 6) * kSlabBlk + k * 128, kSlabBlk),
+                           umma::idesc_bf16(kHid, p.k_in - n0 >= 128 ? 128 : 64, true, true), (g > 0 || k > 0) ? 1u : 0u);
+          umma::mma_bf16(dw2, umma::desc_mnmajor(a + a1_off + k * 128, kSlabBlk),
+                         umma::desc_mnmajor(a + dy_off + k * 128, kSlabBlk), idesc_w2, (g > 0 || k > 0) ? 1u : 0u);
+        }
+        umma::commit(&empty[st]);
+      }
+      umma::commit(done);
+    }
+  } else if (warp < 4) {
+    // ---- db1: column sums of dz1, rows in order
+    const int c = (threadIdx.x - 64) * 2;
+    for (int g = 0; g < mine; g++) {
+      const int st = g % nst;
+      ok = umma::warp_wait(&full[st], (g / nst) & 1);
+      if (!ok) break;
+      const uint8_t* src = ring + st * stage_bytes + dz_off + (c >> 6) * kSlabBlk;
+#pragma unroll 16
+      for (int r = 0; r < kSlab; r++) {
+        const uint32_t w = *reinterpret_cast<const uint32_t*>(src + umma::sw128_offset(r, c & 63));
+        sum[0] += __uint_as_float(w << 16);
+        sum[1] += __uint_as_float(w & 0xffff0000u);
+      }
+      umma::mbar_arrive(&empty[st]);
+    }
+  } else if (warp < 8) {
+    // ---- mapped rows and aggregation
+    const int tid = threadIdx.x - 128;
+    int2 ent[kMaxSeg];
+#pragma unroll
+    for (int s = 0; s < kMaxSeg; s++)
+      if (s < p.nseg && p.seg[s].idx) ent[s] = slab_entries(p.seg[s].idx + row_of(0), lane);
+    for (int g = 0; g < mine; g++) {
+      const int st = g % nst, row0 = row_of(g), next = row_of(g + 1 < mine ? g + 1 : g);
+      if (g >= nst) ok = umma::warp_wait(&empty[st], (g / nst - 1) & 1);
+      ok = __all_sync(0xffffffffu, ok && !aborted(&s_abort));
+      if (!ok) break;
+      uint8_t* dst = ring + st * stage_bytes;
+#pragma unroll
+      for (int s = 0; s < kMaxSeg; s++) {
+        if (s >= p.nseg) break;
+        const Seg& sg = p.seg[s];
+        const int nb = sg.width >> 6;
+        if (sg.agg) {
+          for (int b = 0; b < nb; b++) stage_agg_block<kSlab>(sg, row0, b * 64, dst + b * kSlabBlk, tid);
+        } else if (sg.idx) {
+          const bool mapped = consecutive(ent[s], lane) < 0;
+          ent[s] = slab_entries(sg.idx + next, lane);
+          if (mapped) {
+            int src[4];
+#pragma unroll
+            for (int i = 0; i < 4; i++) src[i] = sg.idx[row0 + (tid >> 3) + i * 16];
+            for (int b = 0; b < nb; b++)
+#pragma unroll
+              for (int i = 0; i < 4; i++)
+                cp_async16(dst + b * kSlabBlk + umma::sw128_offset((tid >> 3) + i * 16, (tid & 7) * 8),
+                           sg.src + static_cast<size_t>(src[i] >= 0 ? src[i] : 0) * sg.width + b * 64 + (tid & 7) * 8,
+                           src[i] >= 0);
+          }
+        }
+        dst += nb * kSlabBlk;
+      }
+      cp_async_commit();
+      cp_async_wait<0>();
+      umma::fence_async_smem();
+      umma::mbar_arrive(&full[st]);
+    }
+  } else {
+    // ---- dy: rounded to bf16, and its column sums
+    const int tid = threadIdx.x - 256;
+    const int sh = p.n_out == 128 ? 5 : 4;  // log2 of the float4s of a row
+    const int n4 = p.n_out == 128 ? 16 : 8; // float4s of a slab and thread, all of one column group
+    float4 v[16];
+    auto load = [&](int g) {
+      const float4* src = reinterpret_cast<const float4*>(p.dy + static_cast<size_t>(row_of(g)) * p.n_out);
+#pragma unroll
+      for (int i = 0; i < 16; i++)
+        if (i < n4) v[i] = src[i * 128 + tid];
+    };
+    load(0);
+    for (int g = 0; g < mine; g++) {
+      const int st = g % nst;
+      if (g >= nst) ok = umma::warp_wait(&empty[st], (g / nst - 1) & 1);
+      ok = __all_sync(0xffffffffu, ok && !aborted(&s_abort));
+      if (!ok) break;
+      uint8_t* dst = ring + st * stage_bytes + dy_off;
+      const int c = (tid & ((1 << sh) - 1)) * 4;
+#pragma unroll
+      for (int i = 0; i < 16; i++) {
+        if (i >= n4) break;
+        const int row = (i * 128 + tid) >> sh;
+        *reinterpret_cast<uint2*>(dst + (c >> 6) * kSlabBlk + umma::sw128_offset(row, c & 56) + (c & 4) * 2) =
+            make_uint2(pack_bf16(v[i].x, v[i].y), pack_bf16(v[i].z, v[i].w));
+        sum[0] += v[i].x;
+        sum[1] += v[i].y;
+        sum[2] += v[i].z;
+        sum[3] += v[i].w;
+      }
+      umma::fence_async_smem();
+      umma::mbar_arrive(&full[st]);
+      if (g + 1 < mine) load(g + 1);
+    }
   }
-  if (any && !s_abort) {
-    if (!umma::mbar_wait(&bars[0], (it - 1) & 1)) s_abort = 1;
-  }
+  if (!ok) s_abort = 1;
+  __syncthreads();
+  if (!umma::warp_wait(done, 0)) s_abort = 1;
   __syncthreads();
   float* part = p.part + static_cast<size_t>(blockIdx.x) * part_stride(p.k_in, p.n_out);
-  if (threadIdx.x < kHid) s_db[0][threadIdx.x] = db1;
-  else if (threadIdx.x - kHid < p.n_out) s_db[1][threadIdx.x - kHid] = db2;
+  float* pw2 = part + kHid * p.k_in + kHid;  // dW2 [n_out][hid]
+  float* s_db2 = reinterpret_cast<float*>(ring + 8 * 4096);  // [rows in flight][n_out]
+  if (warp >= 8) *reinterpret_cast<float4*>(s_db2 + (threadIdx.x - 256) * 4) = make_float4(sum[0], sum[1], sum[2], sum[3]);
   __syncthreads();
   if (!s_abort) {
     umma::fence_after_sync();
-    const int lane_base = (warp & 3) * 32;
-    const int r = lane_base + lane;  // hidden unit
-    const int half = warp >> 2;
-    // dW1 [hid][k_in]
-    const int per_half = p.k_in / 2;
-    for (int cc = 0; cc < per_half; cc += 32) {
-      const int col0 = half * per_half + cc;
-      float v[32];
-      if (any) umma::tmem_ld32(dw1 + (static_cast<uint32_t>(lane_base) << 16) + col0, v);
-      else for (int j = 0; j < 32; j++) v[j] = 0.f;
-      float4* op = reinterpret_cast<float4*>(part + static_cast<size_t>(r) * p.k_in + col0);
+    if (warp >= 2 && warp < 4) {
+      *reinterpret_cast<float2*>(part + kHid * p.k_in + (threadIdx.x - 64) * 2) = make_float2(sum[0], sum[1]);
+      for (int c = threadIdx.x - 64; c < p.n_out; c += 64) {
+        float s = 0.f;
+        for (int q = c; q < 512; q += p.n_out) s += s_db2[q];
+        pw2[p.n_out * kHid + c] = s;
+      }
+    } else if (warp >= 4) {
+      const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
+      const int hid0 = (warp & 3) * 32, half = (warp >> 2) - 1;
+      uint8_t* tr = ring + (warp - 4) * 4096;
+      // dW1 [hid][k_in]: pieces of 32 x 32, turned in shared memory so that eight lanes
+      // write 128 bytes of a row
+      for (int col0 = half * 32; col0 < p.k_in; col0 += 64) {
+        float v[32];
+        umma::tmem_ld32(dw1 + lane_off + col0, v);
 #pragma unroll
-      for (int j = 0; j < 8; j++) op[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-    }
-    float* pw2 = part + kHid * p.k_in + kHid;  // dW2 [n_out][hid]
-    const int per_half2 = p.n_out / 2;
-    for (int cc = 0; cc < per_half2; cc += 32) {
-      const int col0 = half * per_half2 + cc;
-      float v[32];
-      if (any) umma::tmem_ld32(dw2 + (static_cast<uint32_t>(lane_base) << 16) + col0, v);
-      else for (int j = 0; j < 32; j++) v[j] = 0.f;
+        for (int j = 0; j < 8; j++)
+          *reinterpret_cast<float4*>(tr + umma::sw128_offset(lane, j * 8)) =
+              make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+        __syncwarp();
 #pragma unroll
-      for (int j = 0; j < 32; j++) pw2[static_cast<size_t>(col0 + j) * kHid + r] = v[j];
+        for (int j = 0; j < 8; j++) {
+          const int r = j * 4 + (lane >> 3);
+          *reinterpret_cast<float4*>(part + static_cast<size_t>(hid0 + r) * p.k_in + col0 + (lane & 7) * 4) =
+              *reinterpret_cast<const float4*>(tr + umma::sw128_offset(r, (lane & 7) * 8));
+        }
+        __syncwarp();
+      }
+      for (int col0 = half * 32; col0 < p.n_out; col0 += 64) {
+        float v[32];
+        umma::tmem_ld32(dw2 + lane_off + col0, v);
+#pragma unroll
+        for (int j = 0; j < 32; j++) pw2[static_cast<size_t>(col0 + j) * kHid + hid0 + lane] = v[j];
+      }
     }
-    if (threadIdx.x < kHid) part[kHid * p.k_in + threadIdx.x] = s_db[0][threadIdx.x];
-    if (threadIdx.x < p.n_out) pw2[p.n_out * kHid + threadIdx.x] = s_db[1][threadIdx.x];
   } else if (threadIdx.x == 0) {
     set_err(p.err, 3);
   }
   umma::fence_before_sync();
   __syncthreads();
-  if (warp == 0) umma::tmem_dealloc(tmem, 512);
+  if (warp == 1) {
+    umma::fence_after_sync();
+    umma::tmem_dealloc(tmem, 512);
+  }
 }
 
 // ---- small kernels -------------------------------------------------------------------
@@ -1186,7 +1200,15 @@ __global__ void k_reduce_parts(const float* __restrict__ part, int nparts, int n
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   float s = 0.f;
-  for (int b = 0; b < nparts; b++) s += part[static_cast<size_t>(b) * n + i];
+  int b = 0;
+  for (; b + 16 <= nparts; b += 16) {  // loads ahead of the adds, which keep their order
+    float v[16];
+#pragma unroll
+    for (int j = 0; j < 16; j++) v[j] = part[static_cast<size_t>(b + j) * n + i];
+#pragma unroll
+    for (int j = 0; j < 16; j++) s += v[j];
+  }
+  for (; b < nparts; b++) s += part[static_cast<size_t>(b) * n + i];
   grad[i] = s;
 }
 
@@ -1493,11 +1515,19 @@ int storm_gnn_mlp_backward_weight(const StormGnnMlpBwdWeight* a, float* grad, vo
   for (int s = 0; s < a->nseg; s++) p.seg[s] = to_seg(a->seg[s]);
   p.dy = a->dy; p.a1 = static_cast<const bf16*>(a->a1); p.dz1 = static_cast<const bf16*>(a->dz1);
   p.part = static_cast<float*>(scratch); p.err = dev_err;
-  size_t smem = bwd_weight_smem_bytes(a->k_in);
+  WeightMaps maps{};
+  for (int i = 0; i < a->nseg; i++) {
+    const Seg& g = p.seg[i];
+    if (g.agg) continue;
+    if ((rc = tensor_map(&maps.seg[i], g.src, g.idx ? kAnyRows : a->rows, g.width, kSlab))) return rc;
+  }
+  if ((rc = tensor_map(&maps.a1, p.a1, a->rows, kHid, kSlab)) || (rc = tensor_map(&maps.dz, p.dz1, a->rows, kHid, kSlab)))
+    return rc;
+  size_t smem = bwd_weight_smem_bytes(a->k_in, a->n_out);
   if (smem < static_cast<size_t>(kMinBwdSmem)) smem = kMinBwdSmem;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   cudaFuncSetAttribute(k_mlp_bwd_weight, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-  k_mlp_bwd_weight<<<grid, kThreads, smem, st>>>(p);
+  k_mlp_bwd_weight<<<grid, kWeightThreads, smem, st>>>(p, maps);
   k_reduce_parts<<<(n + 255) / 256, 256, 0, st>>>(p.part, grid, n, grad);
   g_launches += 2;
   return cuda_check("k_mlp_bwd_weight");

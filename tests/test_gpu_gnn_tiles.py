@@ -125,3 +125,54 @@ def test_backward_data_many_tiles(storm_lib, tiles, layer, outs):
         if o is not None:
             ref = da[:, 128 * i:128 * i + widths[i]]
             _close(o.cpu().numpy(), ref if a is None else ref + a)
+
+
+@pytest.mark.parametrize("tiles", [1, SMS + 1, 3 * SMS + 5])
+@pytest.mark.parametrize("layer,kinds", [("edge0", ("run", "scatter")), ("edge0", ("mixed", "mixed")), ("node0", ()),
+                                         ("enc_edge", ()), ("dec", ())])
+def test_backward_weight_many_tiles(storm_lib, tiles, layer, kinds):
+    """Operands are bf16 on both sides, so only the fp32 sums differ: at most 57,000 random
+    terms, about 2^-24 sqrt(n) = 1.4e-5 of a sum; 1e-3 leaves room for the tensor cores'
+    own rounding, while one 64-row stage lost or doubled shifts the sums by 3 % or more."""
+    import torch
+    net = gnn.WarmStartNet(seed=13)
+    dev = net.device
+    rng = np.random.default_rng(tiles)
+    s = net.by_name[layer]
+    rows, n = 128 * tiles, 128 * 40
+
+    def mat(r, w):
+        a = to_bf16(rng.normal(size=(r, w)))
+        return a, torch.tensor(a, dtype=torch.bfloat16, device=dev)
+
+    x, x_t = mat(rows, min(s.k_in, 128))
+    segs, A = [net._seg(x_t, x.shape[1])], [x]
+    h, h_t = mat(n, 128)
+    idx = [_map(rng, k, rows, n) for k in kinds]
+    idx_t = [torch.tensor(i, device=dev) for i in idx]
+    segs += [net._seg(h_t, idx=i) for i in idx_t]
+    A += [GnnOracle.gather(h, i) for i in idx]
+    orc = GnnOracle(net.specs, net.params_numpy(), net.n_layers)
+    if layer == "node0":
+        e, e_t = mat(3 * rows, 128)
+        nbr = rng.integers(-1, 3, size=(3, rows)).astype(np.int32)
+        nbr_t = torch.tensor(nbr, device=dev)
+        segs.append(net._seg(e_t, agg=True, stride=rows, nbr=nbr_t))
+        A.append(orc.agg(e, nbr, rows))
+    A = np.concatenate(A, axis=1)
+    (dz, dz_t), (a1, a1_t) = mat(rows, 128), mat(rows, 128)
+    dy = rng.normal(size=(rows, s.n_out)).astype(np.float32)
+    dy_t = torch.tensor(dy, device=dev)
+    net.grad.zero_()
+    net._bwd_weight(layer, rows, segs, dy_t, a1_t, dz_t)
+    torch.cuda.synchronize()
+    net._check_err()
+    got = net.grad.cpu().numpy()[s.offset:s.offset + s.size]
+    f = np.float64
+    parts = [dz.T.astype(f) @ A.astype(f), dz.sum(0, dtype=f), to_bf16(dy).T.astype(f) @ a1.astype(f), dy.sum(0, dtype=f)]
+    o = 0
+    for ref in parts:
+        g = got[o:o + ref.size].astype(f).reshape(ref.shape)
+        assert np.linalg.norm(g - ref) < 1e-3 * np.linalg.norm(ref)
+        o += ref.size
+    assert o == s.size
