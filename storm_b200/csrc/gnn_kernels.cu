@@ -90,6 +90,11 @@ __device__ __forceinline__ void set_err(int32_t* err, int code) {
   if (err) atomicCAS(err, 0, code);
 }
 
+__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+
 // ---- shared-memory staging -------------------------------------------------------
 
 // 16 bytes, or zeros without touching memory: a predicated load, so that a batch of them
@@ -105,48 +110,55 @@ __device__ __forceinline__ uint4 ld_if(const void* p, bool want) {
   return v;
 }
 
-// 64 columns (from col0) of kR rows of the aggregation segment into one kR x 64 block, by
-// 128 threads: rows r + k*agg_stride, k = 0, 1, 2, whose nbr entry is >= 0, added in that
-// order in fp32.  Chunks of 16 bytes, four to a thread and round (twelve loads in flight).
-template <int kR>
-__device__ __forceinline__ void stage_agg_block(const Seg& s, int row0, int col0, uint8_t* dst, int tid) {
+// The aggregation segment: rows r + k*agg_stride, k = 0, 1, 2, whose nbr entry is >= 0, added
+// in that order in fp32.  Eight threads take a row, kThr / 8 rows at a time, four times over.
+// Which of a thread's twelve rows count (bit 3 i + k), asked for ahead of the rows ...
+template <int kThr>
+__device__ __forceinline__ uint32_t agg_mask(const Seg& s, int row0, int tid) {
+  int32_t e[4][3];
 #pragma unroll
-  for (int h = 0; h < kR / 16; h += 4) {
-    uint4 w[4][3];
-    bool m[4][3];
+  for (int i = 0; i < 4; i++)
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const int row = row0 + (tid >> 3) + (h + i) * 16;
+    for (int k = 0; k < 3; k++)
+      e[i][k] = s.nbr[static_cast<size_t>(k) * s.agg_stride + row0 + (tid >> 3) + i * (kThr / 8)];
+  uint32_t m = 0;
 #pragma unroll
-      for (int k = 0; k < 3; k++) m[i][k] = s.nbr[static_cast<size_t>(k) * s.agg_stride + row] >= 0;
-    }
+  for (int i = 0; i < 4; i++)
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const int row = row0 + (tid >> 3) + (h + i) * 16;
+    for (int k = 0; k < 3; k++) m |= (e[i][k] >= 0 ? 1u : 0u) << (3 * i + k);
+  return m;
+}
+// ... and 64 columns (from col0) of kThr / 2 rows into one block, all loads in flight together.
+template <int kThr>
+__device__ __forceinline__ void stage_agg_block(const Seg& s, uint32_t mask, int row0, int col0, uint8_t* dst, int tid) {
+  uint4 w[4][3];
 #pragma unroll
-      for (int k = 0; k < 3; k++)
-        w[i][k] = ld_if(s.src + (static_cast<size_t>(k) * s.agg_stride + row) * s.width + col0 + (tid & 7) * 8, m[i][k]);
-    }
+  for (int i = 0; i < 4; i++)
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-      float acc[8];
+    for (int k = 0; k < 3; k++)
+      w[i][k] = ld_if(s.src + (static_cast<size_t>(k) * s.agg_stride + row0 + (tid >> 3) + i * (kThr / 8)) * s.width + col0 +
+                          (tid & 7) * 8,
+                      (mask >> (3 * i + k)) & 1);
 #pragma unroll
-      for (int j = 0; j < 8; j++) acc[j] = 0.f;
+  for (int i = 0; i < 4; i++) {
+    float acc[8];
 #pragma unroll
-      for (int k = 0; k < 3; k++) {
-        if (!m[i][k]) continue;
-        const bf16* b = reinterpret_cast<const bf16*>(&w[i][k]);
+    for (int j = 0; j < 8; j++) acc[j] = 0.f;
 #pragma unroll
-        for (int j = 0; j < 8; j++) acc[j] += __bfloat162float(b[j]);
+    for (int k = 0; k < 3; k++) {
+      if (!((mask >> (3 * i + k)) & 1)) continue;
+      const uint32_t x[4] = {w[i][k].x, w[i][k].y, w[i][k].z, w[i][k].w};
+#pragma unroll
+      for (int u = 0; u < 4; u++) {
+        acc[2 * u] += __uint_as_float(x[u] << 16);
+        acc[2 * u + 1] += __uint_as_float(x[u] & 0xffff0000u);
       }
-      uint4 v;
-      bf16* o = reinterpret_cast<bf16*>(&v);
-#pragma unroll
-      for (int j = 0; j < 8; j++) o[j] = __float2bfloat16(acc[j]);
-      *reinterpret_cast<uint4*>(dst + umma::sw128_offset((tid >> 3) + (h + i) * 16, (tid & 7) * 8)) = v;
     }
+    *reinterpret_cast<uint4*>(dst + umma::sw128_offset((tid >> 3) + i * (kThr / 8), (tid & 7) * 8)) =
+        make_uint4(pack_bf16(acc[0], acc[1]), pack_bf16(acc[2], acc[3]), pack_bf16(acc[4], acc[5]), pack_bf16(acc[6], acc[7]));
   }
 }
+
 // Asynchronous copy of one 16-byte chunk global -> shared (zero-filled when `valid` is
 // false); the copies of a thread are grouped with commit / wait_group.
 __device__ __forceinline__ void cp_async16(uint8_t* dst, const void* src, bool valid) {
@@ -184,101 +196,127 @@ __device__ __forceinline__ uint8_t* align1024(uint8_t* p) {
   return reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(p) + 1023) & ~static_cast<uintptr_t>(1023));
 }
 
-// Issue D (+)= A B^T over K (multiple of 16), A and B K-major tiles with blocks of 64
-// columns: a_blk / b_blk are the byte strides between their 64-column blocks.
-__device__ __forceinline__ void mma_kmajor(uint32_t tmem_d, uint32_t a, uint32_t a_blk, uint32_t b,
-                                           uint32_t b_blk, int K, uint32_t idesc, bool accumulate) {
-  for (int k = 0; k < K; k += 16) {
-    const uint32_t off = (k & 63) * 2;
-    const uint64_t ad = umma::desc_kmajor(a + (k >> 6) * a_blk + off);
-    const uint64_t bd = umma::desc_kmajor(b + (k >> 6) * b_blk + off);
-    umma::mma_bf16(tmem_d, ad, bd, idesc, (accumulate || k > 0) ? 1u : 0u);
-  }
+// Issue D (+)= A B^T over K (a multiple of 16), A and B K-major tiles with blocks of 64
+// columns: a_blk / b_blk are the byte strides between their 64-column blocks.  Descriptors
+// count 16 bytes.
+template <int K>
+__device__ __forceinline__ void mma_kmajor(uint32_t tmem_d, uint32_t a, uint32_t b, uint32_t idesc, bool accumulate) {
+  static_assert(K <= 64, "one block of columns");
+  const uint64_t ad = umma::desc_kmajor(a), bd = umma::desc_kmajor(b);
+#pragma unroll
+  for (int k = 0; k < K; k += 16)
+    umma::mma_bf16(tmem_d, ad + k / 8, bd + k / 8, idesc, (accumulate || k > 0) ? 1u : 0u);
 }
 
 // ---- forward ----------------------------------------------------------------------
 
 // Shared memory: W1 (128 x k_in), W2 (n_out x 128), the ring of input blocks (128 rows x
-// 64 columns, 16 KB), the hidden tile (128 x 128), half an output tile, biases, barriers.
+// 64 columns, 16 KB), the output tile, half a hidden tile (training), biases, barriers.
 constexpr int kBlk = kRows * 128;  // bytes of a block
 constexpr size_t kSmemMax = 227 * 1024;
-__host__ __device__ constexpr size_t fwd_fixed_bytes(int k_in, int n_out) {
-  return 1024 + static_cast<size_t>(kHid) * k_in * 2 + static_cast<size_t>(n_out) * kHid * 2 + kRows * kHid * 2 + kBlk +
+constexpr int kMaxStages = 8;
+__host__ __device__ constexpr size_t fwd_fixed_bytes(int k_in, int n_out, bool save) {
+  return 1024 + static_cast<size_t>(kHid) * k_in * 2 + static_cast<size_t>(n_out) * kHid * 2 + (n_out / 64 + save) * kBlk +
          4 * (kHid + 128) + 512;
 }
-__host__ __device__ constexpr int fwd_stages(int k_in, int n_out) {
-  const int n = static_cast<int>((kSmemMax - fwd_fixed_bytes(k_in, n_out)) / kBlk);
-  return n < 6 ? n : 6;
+__host__ __device__ constexpr int fwd_stages(int k_in, int n_out, bool save) {
+  const int n = static_cast<int>((kSmemMax - fwd_fixed_bytes(k_in, n_out, save)) / kBlk);
+  return n < kMaxStages ? n : kMaxStages;
 }
-__host__ __device__ constexpr size_t fwd_smem_bytes(int k_in, int n_out) {
-  return fwd_fixed_bytes(k_in, n_out) + static_cast<size_t>(fwd_stages(k_in, n_out)) * kBlk;
+__host__ __device__ constexpr size_t fwd_smem_bytes(int k_in, int n_out, bool save) {
+  return fwd_fixed_bytes(k_in, n_out, save) + static_cast<size_t>(fwd_stages(k_in, n_out, save)) * kBlk;
 }
-static_assert(fwd_stages(384, 128) == 3, "the widest input leaves three ring stages");
+static_assert(fwd_stages(384, 128, false) == 4 && fwd_stages(384, 128, true) == 3, "ring stages of the widest input");
 
 struct FwdMaps {  // boxes of 64 columns x 128 rows (w2: n_out rows)
-  CUtensorMap seg[kMaxSeg], w1, w2, out, a1;
+  CUtensorMap seg[kMaxSeg], w1, w2, out, a1, res;
 };
 constexpr int kAnyRows = 1 << 30;  // rows of a mapped segment's matrix: the caller does not say
 
-// Warp roles of the forward kernel (512 threads):
-//   warp 0      hands out the ring's stages in the order of the blocks, and fills by TMA
-//               (the weights once, then) each 64-column block of the CTA's tiles whose
-//               rows follow one another (unmapped segments, and mapped ones where the map
-//               is a run, as the receiver's is);
+// A place in a ring of n stages: the stage and the parity of its present use.
+struct RingPos {
+  int st = 0;
+  uint32_t par = 0;
+  __device__ __forceinline__ void next(int n) {
+    if (++st == n) {
+      st = 0;
+      par ^= 1;
+    }
+  }
+};
+
+// Warp roles of the forward kernel (512 or 640 threads):
+//   warp 0      one thread hands out the ring's stages in the order of the blocks, and fills
+//               by TMA (the weights with the first tile's) each 64-column block of the CTA's
+//               tiles whose rows follow one another (unmapped segments, and mapped ones where
+//               the map is a run, as the receiver's is);
 //   warp 1      one thread issues the MMAs: D1[slot] = A W1^T block by block as the ring
 //               fills, D2[slot] = a1 W2^T one tile behind, so the hidden tile's epilogue
 //               is hidden by the next tile's first products;
-//   warps 4-7   epilogue 1: D1 -> bias + ReLU -> hidden tile (stored by TMA in training);
-//   warps 8-11  epilogue 2: D2 -> bias + residual -> output, through half a tile of
-//               shared memory and a TMA store (direct stores, a row to a thread, take the
-//               L1 32 lines an instruction); its residual rows are read while D2 is still
-//               being computed;
-//   warps 12-15 the other blocks: mapped rows by cp.async (a negative entry reads zeros;
+//   warp 2      looks through the row maps, up to two tiles ahead of warps 0 and 12 on;
+//   warps 4-7   epilogue 1: D1 -> bias + ReLU -> hidden tile as bf16 in the first half of D1's
+//               own columns, which D2's MMAs read from TMEM (in training also out by TMA);
+//   warps 8-11  epilogue 2: D2 -> residual + bias -> output; the residual comes into the
+//               output tile's shared memory by TMA while D2 is computed, the sum leaves from
+//               there by TMA (direct loads and stores, a row to a thread, take the L1 32
+//               lines an instruction, and every other wait on that path with them);
+//   the warps from 12 on the other blocks: mapped rows by cp.async (a negative entry reads zeros;
 //               TMA's gather4 took about 130 cycles per four half rows, 135 us for the
 //               edge update below), and the aggregation's sums of three edge rows.
 // One warp alone waits on `empty`, for every block in turn: a parity tells a phase only
 // from the one beside it, so a role that waited for its own blocks alone could take a stage
-// two uses early.  Warps 12-15 get theirs from it through `grant`, which holds no phase
+// two uses early.  The warps from 12 on get theirs from it through `grant`, which holds no phase
 // but their own.
-// D1 and D2 are double-buffered in TMEM (slot = tile parity).  Every wait is bounded; a
-// wait that runs out raises the abort flag, which every role polls.
+// D1 and D2 are double-buffered in TMEM (slot = tile parity); the MMAs of one thread run in
+// order, so D1 of a tile may overwrite the hidden tile that D2 two tiles before has read.
+// Every wait is bounded; a wait that runs out raises the abort flag, which every role polls.
 //
-// What bounds it: the ring's three stages at k_in = 384, next to 96 KB of W1: a tile takes
-// about 10k cycles, most of it the way of a block from L2 to its stage.  Measured (us;
-// before, with one role a phase and direct stores): edge update with saved hidden rows
-// 90 (141) at 300,000 rows, 29 (43) at 75,000, 14 (19) at 9,000; node update 68 (77) at
-// 100,000 rows, encoder 46 (72) at 300,000, decoder 19 (25) at 100,000.
-constexpr int kFwdThreads = 512;
+// What bounds it: the latency of a block's way from L2 or HBM to its stage, with three (in
+// training) or four stages at k_in = 384 next to 96 KB of W1.  Every role's loops stay rolled:
+// unrolled over columns and segments, the roles' code no longer fitted the instruction cache
+// and 6 of 17 stall cycles an instruction went on fetching it (0.7 now).  Measured (us;
+// before, unrolled, the hidden tile in shared memory and the residual read a row to a thread):
+// edge update 58 (90) at 300,000 rows, with saved hidden rows 73 (96), at 75,000 rows 22 (29),
+// at 9,000 12 (14); node update 57 (68) at 100,000 rows, encoder 15 (17) at 75,000.
+//
+// Threads that gather: 128 where rows are only copied (256 took 65 us instead of 58 for the
+// edge update of 300,000 rows), 256 where a segment is summed over three edge rows, so that
+// twelve 16-byte loads a thread cover a block (node update of 100,000 rows: 57 us; 128 threads
+// in two rounds 68 us).
+__host__ __device__ constexpr int fwd_gather(bool agg) { return agg ? 256 : 128; }
+__host__ __device__ constexpr int fwd_threads(bool agg) { return 384 + fwd_gather(agg); }
 __device__ __forceinline__ bool aborted(const int* flag) { return *reinterpret_cast<const volatile int*>(flag) != 0; }
 
-__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
-  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-  return *reinterpret_cast<const uint32_t*>(&v);
-}
-
-__global__ void __launch_bounds__(kFwdThreads, 1) k_mlp_fwd(const __grid_constant__ MlpFwd p,
+template <bool kAgg>
+__global__ void __launch_bounds__(fwd_threads(kAgg), 1) k_mlp_fwd(const __grid_constant__ MlpFwd p,
                                                               const __grid_constant__ FwdMaps maps) {
+  constexpr int kGather = fwd_gather(kAgg), kRowsEach = kRows * 8 / kGather;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = align1024(smem_raw);
-  const int nst = fwd_stages(p.k_in, p.n_out);
+  const bool save = p.a1_save != nullptr;
+  const int nst = fwd_stages(p.k_in, p.n_out, save);
   uint8_t* w1s = base;
   uint8_t* w2s = w1s + kHid * p.k_in * 2;
   uint8_t* ring = w2s + p.n_out * kHid * 2;
-  uint8_t* a1s = ring + nst * kBlk;
-  uint8_t* ios = a1s + kRows * kHid * 2;
-  float* b1s = reinterpret_cast<float*>(ios + kBlk);
+  uint8_t* ios = ring + nst * kBlk;               // [n_out / 64] residual in, output out
+  uint8_t* a1s = ios + (p.n_out >> 6) * kBlk;     // half a hidden tile (training)
+  float* b1s = reinterpret_cast<float*>(a1s + (save ? kBlk : 0));
   float* b2s = b1s + kHid;
   uint64_t* bars = reinterpret_cast<uint64_t*>(b2s + 128);
-  uint64_t* full = bars;          // [6] ring stage filled
-  uint64_t* empty = bars + 6;     // [6] MMAs reading the stage done (commit)
-  uint64_t* d1full = bars + 12;   // [2] D1[slot] complete (commit)
-  uint64_t* d1free = bars + 14;   // [2] epilogue 1 has read D1[slot]
-  uint64_t* a1full = bars + 16;   // hidden tile written
-  uint64_t* d2full = bars + 17;   // [2] D2[slot] complete, hidden tile read (commit)
-  uint64_t* d2free = bars + 19;   // [2] epilogue 2 has read D2[slot]
-  uint64_t* wfull = bars + 21;    // weights loaded
-  uint64_t* grant = bars + 22;    // [6] ring stage given to warps 12-15
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 28);
+  uint64_t* full = bars;          // [8] ring stage filled
+  uint64_t* empty = bars + 8;     // [8] MMAs reading the stage done (commit)
+  uint64_t* grant = bars + 16;    // [8] ring stage given to the warps from 12 on
+  uint64_t* d1full = bars + 24;   // [2] D1[slot] complete (commit)
+  uint64_t* a1full = bars + 26;   // [2] hidden tile written over D1[slot]
+  uint64_t* d2full = bars + 28;   // [2] D2[slot] complete (commit)
+  uint64_t* d2free = bars + 30;   // [2] epilogue 2 has read D2[slot]
+  uint64_t* w1full = bars + 32;   // [6] W1 block loaded
+  uint64_t* w2full = bars + 38;   // W2 loaded
+  uint64_t* resfull = bars + 39;  // residual tile loaded
+  uint64_t* runfull = bars + 40;  // [2] row maps of a tile looked through
+  uint64_t* runfree = bars + 42;  // [2] ... and read by warps 0 and 12 on
+  int* runs = reinterpret_cast<int*>(bars + 44);  // [2][4] first row of a segment whose 128 rows are consecutive, else -1
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 48);
   __shared__ int s_abort;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -290,12 +328,15 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_mlp_fwd(const __grid_constan
     }
     for (int i = 0; i < 2; i++) {
       umma::mbar_init(&d1full[i], 1);
-      umma::mbar_init(&d1free[i], kRows);
+      umma::mbar_init(&a1full[i], kRows);
       umma::mbar_init(&d2full[i], 1);
       umma::mbar_init(&d2free[i], kRows);
+      umma::mbar_init(&runfull[i], 1);
+      umma::mbar_init(&runfree[i], 1 + kGather / 32);
     }
-    umma::mbar_init(a1full, kRows);
-    umma::mbar_init(wfull, 1);
+    for (int i = 0; i < 6; i++) umma::mbar_init(&w1full[i], 1);
+    umma::mbar_init(w2full, 1);
+    umma::mbar_init(resfull, 1);
     umma::mbar_fence_init();
     umma::fence_async_smem();
     s_abort = 0;
@@ -308,285 +349,322 @@ __global__ void __launch_bounds__(kFwdThreads, 1) k_mlp_fwd(const __grid_constan
   umma::fence_after_sync();
   const uint32_t tmem = *tmem_slot;
   const int ntiles = p.rows / kRows;
+  const int mine = blockIdx.x < ntiles ? (ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
+  const int nblk = p.k_in >> 6;
+  auto row_of = [&](int t) { return static_cast<int>(blockIdx.x + t * gridDim.x) * kRows; };
 
   if (warp == 0) {
-    // ---- TMA
-    if (lane == 0) {
-      umma::mbar_expect(wfull, static_cast<uint32_t>(kHid * p.k_in * 2 + p.n_out * kHid * 2));
-      for (int x = 0; x < p.k_in; x += 64) umma::tma_load(w1s + (x >> 6) * (kHid * 128), &maps.w1, x, 0, wfull);
-      for (int x = 0; x < kHid; x += 64) umma::tma_load(w2s + (x >> 6) * (p.n_out * 128), &maps.w2, x, 0, wfull);
-    }
-    uint32_t g = 0;
-    bool ok = true;
-    int4 ent[kMaxSeg];
-#pragma unroll
-    for (int s = 0; s < kMaxSeg; s++)
-      if (s < p.nseg && p.seg[s].idx) ent[s] = map_entries(p.seg[s].idx + blockIdx.x * kRows, lane);
-    for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
-      const int row0 = tile * kRows;
-      const int next = tile + gridDim.x < ntiles ? (tile + gridDim.x) * kRows : row0;
-      int run[kMaxSeg];  // first row of a segment whose 128 rows are consecutive, else -1
-#pragma unroll
-      for (int s = 0; s < kMaxSeg; s++) {
-        run[s] = row0;
-        if (s < p.nseg && p.seg[s].idx) {
-          run[s] = consecutive(ent[s], lane);
-          ent[s] = map_entries(p.seg[s].idx + next, lane);
+    // ---- ring and TMA
+    if (umma::elect_one()) {
+      int nw = 0;  // W1 blocks asked for
+      auto load_w1 = [&]() {
+        umma::mbar_expect(&w1full[nw], kHid * 128);
+        umma::tma_load(w1s + nw * (kHid * 128), &maps.w1, nw * 64, 0, &w1full[nw]);
+        nw++;
+      };
+      RingPos r, last;  // the next block; the oldest whose copy may still be in flight
+      int g = 0;        // blocks handed out
+      bool ok = true;
+      for (int t = 0; t < mine && ok; t++) {
+        if (!umma::mbar_wait(&runfull[t & 1], (t >> 1) & 1)) {
+          ok = false;
+          break;
         }
-      }
-#pragma unroll
-      for (int s = 0; s < kMaxSeg; s++) {
-        if (s >= p.nseg) break;
-        const int nb = p.seg[s].width >> 6;
-        for (int b = 0; b < nb && ok; b++, g++) {
-          const int st = g % nst;
-          const uint32_t use = g / nst;
-          if (use > 0 && !umma::warp_wait(&empty[st], (use - 1) & 1)) ok = false;
-          ok = __all_sync(0xffffffffu, ok && !aborted(&s_abort));
-          if (!ok) break;
-          if (lane == 0) {
-            if (p.seg[s].agg || run[s] < 0) {
-              umma::mbar_arrive(&grant[st]);
+#pragma unroll 1
+        for (int s = 0; s < p.nseg; s++) {
+          const int nb = p.seg[s].width >> 6, run = runs[(t & 1) * 4 + s];
+#pragma unroll 1
+          for (int b = 0; b < nb && ok; b++) {
+            if (g >= nst) {
+              ok = umma::mbar_wait(&empty[r.st], r.par ^ 1) && !aborted(&s_abort);
+              if (!ok) break;
+              last.next(nst);
+            }
+            if (nw < nblk) load_w1();
+            if (run < 0) {
+              umma::mbar_arrive(&grant[r.st]);
             } else {
-              umma::mbar_expect(&full[st], kBlk);
-              umma::tma_load(ring + st * kBlk, &maps.seg[s], b * 64, run[s], &full[st]);
+              umma::mbar_expect(&full[r.st], kBlk);
+              umma::tma_load(ring + r.st * kBlk, &maps.seg[s], b * 64, run, &full[r.st]);
+            }
+            r.next(nst);
+            if (++g == (nst < nblk ? nst : nblk)) {  // the first stages are taken: the other weights
+              while (nw < nblk) load_w1();
+              umma::mbar_expect(w2full, p.n_out * kHid * 2);
+              for (int x = 0; x < kHid; x += 64) umma::tma_load(w2s + (x >> 6) * (p.n_out * 128), &maps.w2, x, 0, w2full);
             }
           }
         }
+        umma::mbar_arrive(&runfree[t & 1]);
       }
+      if (!ok) s_abort = 1;
+      // the copies still in flight land before the block's shared memory is given up
+      for (int k = g < nst ? g : nst; k > 0; k--, last.next(nst)) umma::mbar_wait(&full[last.st], last.par);
+      for (int k = 0; k < nw; k++) umma::mbar_wait(&w1full[k], 0);
+      if (nw == nblk) umma::mbar_wait(w2full, 0);
     }
-    if (!ok) s_abort = 1;
-    // the copies still in flight land before the block's shared memory is given up
-    for (uint32_t k = g > static_cast<uint32_t>(nst) ? g - nst : 0; k < g; k++) umma::warp_wait(&full[k % nst], (k / nst) & 1);
-    umma::warp_wait(wfull, 0);
+    __syncwarp();
   } else if (warp == 1) {
     // ---- MMA issuer
-    if (lane == 0) {
-      const uint32_t w1a = umma::smem_addr(w1s), w2a = umma::smem_addr(w2s);
-      const uint32_t ra = umma::smem_addr(ring), a1a = umma::smem_addr(a1s);
+    if (umma::elect_one()) {
+      const uint32_t w1a = umma::smem_addr(w1s), ra = umma::smem_addr(ring);
+      const uint64_t w2d = umma::desc_kmajor(umma::smem_addr(w2s));
+      const uint32_t w2blk = p.n_out * 128 / 16;
       const uint32_t idesc1 = umma::idesc_bf16(kRows, kHid, false, false);
       const uint32_t idesc2 = umma::idesc_bf16(kRows, p.n_out, false, false);
-      const int nblk = p.k_in >> 6;
-      const int mine = blockIdx.x < ntiles ? (ntiles - 1 - blockIdx.x) / gridDim.x + 1 : 0;
-      uint32_t g = 0;
-      bool ok = umma::mbar_wait(wfull, 0);
+      RingPos r;
+      bool ok = true;
       for (int t = 0; t <= mine && ok; t++) {
         const int slot = t & 1;
         if (t < mine) {  // D1 of tile t
-          if (t >= 2 && !umma::mbar_wait(&d1free[slot], ((t >> 1) - 1) & 1)) ok = false;
-          if (ok) umma::fence_after_sync();
-          for (int b = 0; b < nblk && ok; b++, g++) {
-            const int st = g % nst;
-            if (!umma::mbar_wait(&full[st], (g / nst) & 1)) {
+#pragma unroll 1
+          for (int b = 0; b < nblk; b++) {
+            if ((t == 0 && !umma::mbar_wait(&w1full[b], 0)) || !umma::mbar_wait(&full[r.st], r.par)) {
               ok = false;
               break;
             }
             umma::fence_after_sync();
-            mma_kmajor(tmem + slot * 128, ra + st * kBlk, kBlk, w1a + b * (kHid * 128), kHid * 128, 64, idesc1, b > 0);
-            umma::commit(&empty[st]);
+            mma_kmajor<64>(tmem + slot * 128, ra + r.st * kBlk, w1a + b * (kHid * 128), idesc1, b > 0);
+            umma::commit(&empty[r.st]);
+            r.next(nst);
           }
           if (!ok) break;
           umma::commit(&d1full[slot]);
         }
         if (t > 0) {  // D2 of tile t - 1
           const int u = t - 1, us = u & 1;
-          if (u >= 2 && !umma::mbar_wait(&d2free[us], ((u >> 1) - 1) & 1)) ok = false;
-          if (!ok || !umma::mbar_wait(a1full, u & 1)) {
+          if ((u == 0 && !umma::mbar_wait(w2full, 0)) || (u >= 2 && !umma::mbar_wait(&d2free[us], ((u >> 1) - 1) & 1)) ||
+              !umma::mbar_wait(&a1full[us], (u >> 1) & 1)) {
             ok = false;
             break;
           }
           umma::fence_after_sync();
-          mma_kmajor(tmem + 256 + us * 128, a1a, kBlk, w2a, p.n_out * 128, kHid, idesc2, false);
+#pragma unroll
+          for (int k = 0; k < kHid; k += 16)
+            umma::mma_bf16_ts(tmem + 256 + us * 128, tmem + us * 128 + k / 2, w2d + (k >> 6) * w2blk + (k & 63) / 8, idesc2,
+                              k > 0 ? 1u : 0u);
           umma::commit(&d2full[us]);
         }
       }
-      // the last commits, before shared memory and TMEM are given up
-      if (ok)
-        for (uint32_t k = g > static_cast<uint32_t>(nst) ? g - nst : 0; k < g; k++)
-          if (!umma::mbar_wait(&empty[k % nst], (k / nst) & 1)) ok = false;
-      if (ok && mine > 0 && !umma::mbar_wait(&d2full[(mine - 1) & 1], ((mine - 1) >> 1) & 1)) ok = false;
+      // the last commit (of them all, in order), before shared memory and TMEM are given up
+      if (ok && mine > 0) ok = umma::mbar_wait(&d2full[(mine - 1) & 1], ((mine - 1) >> 1) & 1);
       if (!ok) s_abort = 1;
+    }
+    __syncwarp();
+  } else if (warp == 2) {
+    // ---- row maps
+    for (int t = 0; t < mine; t++) {
+      int4 ent[kMaxSeg];
+      int run[kMaxSeg];
+#pragma unroll
+      for (int s = 0; s < kMaxSeg; s++)
+        if (s < p.nseg && p.seg[s].idx && !p.seg[s].agg) ent[s] = map_entries(p.seg[s].idx + row_of(t), lane);
+#pragma unroll
+      for (int s = 0; s < kMaxSeg; s++) {
+        run[s] = row_of(t);
+        if (s >= p.nseg) continue;
+        if (p.seg[s].agg) run[s] = -1;
+        else if (p.seg[s].idx) run[s] = consecutive(ent[s], lane);
+      }
+      if ((t >= 2 && !umma::warp_wait(&runfree[t & 1], ((t >> 1) - 1) & 1)) || aborted(&s_abort)) {
+        s_abort = 1;
+        break;
+      }
+      if (lane == 0) {
+        int* o = runs + (t & 1) * 4;
+        o[0] = run[0];
+        o[1] = run[1];
+        o[2] = run[2];
+        umma::mbar_arrive(&runfull[t & 1]);
+      }
+      __syncwarp();
     }
   } else if (warp >= 4 && warp < 8) {
     // ---- epilogue 1
     const int r = (warp & 3) * 32 + lane;  // row of the tile = TMEM lane
     const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    uint32_t t = 0;
-    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, t++) {
+    const bool leader = warp == 4 && lane == 0;
+    for (int t = 0; t < mine; t++) {
       const int slot = t & 1;
-      // the hidden tile is free once D2 of the tile before, and its copy out, have read it
-      const bool ok = umma::warp_wait(&d1full[slot], (t >> 1) & 1) &&
-                      (t == 0 || umma::warp_wait(&d2full[(t - 1) & 1], ((t - 1) >> 1) & 1)) && !aborted(&s_abort);
-      if (p.a1_save && warp == 4 && lane == 0) umma::tma_store_wait_read();
+      const uint32_t d1 = tmem + slot * 128 + lane_off;
+      const bool ok = umma::warp_wait(&d1full[slot], (t >> 1) & 1) && !aborted(&s_abort);
+      if (save && leader) umma::tma_store_wait_read();  // the half tile before has been read
       if (!umma::bar_all(1, kRows, ok)) {  // the four warps go on, or stop, together
         s_abort = 1;
         break;
       }
-      __syncwarp();
       umma::fence_after_sync();
-#pragma unroll
-      for (int col0 = 0; col0 < kHid; col0 += 32) {
+#pragma unroll 1
+      for (int q = 0; q < 4; q++) {  // 32 columns into 16, over columns already read
         float v[32];
-        umma::tmem_ld32(tmem + slot * 128 + lane_off + col0, v);
-        const float4* bp = reinterpret_cast<const float4*>(b1s + col0);
+        uint32_t o[16];
+        umma::tmem_ld32(d1 + q * 32, v);
+        const float4* bp = reinterpret_cast<const float4*>(b1s + q * 32);
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-          const float4 x = bp[2 * j], y = bp[2 * j + 1];
-          uint4 o;
-          o.x = pack_bf16(fmaxf(v[8 * j] + x.x, 0.f), fmaxf(v[8 * j + 1] + x.y, 0.f));
-          o.y = pack_bf16(fmaxf(v[8 * j + 2] + x.z, 0.f), fmaxf(v[8 * j + 3] + x.w, 0.f));
-          o.z = pack_bf16(fmaxf(v[8 * j + 4] + y.x, 0.f), fmaxf(v[8 * j + 5] + y.y, 0.f));
-          o.w = pack_bf16(fmaxf(v[8 * j + 6] + y.z, 0.f), fmaxf(v[8 * j + 7] + y.w, 0.f));
-          const int c = col0 + j * 8;
-          *reinterpret_cast<uint4*>(a1s + (c >> 6) * kBlk + umma::sw128_offset(r, c & 63)) = o;
+        for (int j = 0; j < 8; j++) {
+          const float4 x = bp[j];
+          o[2 * j] = pack_bf16(fmaxf(v[4 * j] + x.x, 0.f), fmaxf(v[4 * j + 1] + x.y, 0.f));
+          o[2 * j + 1] = pack_bf16(fmaxf(v[4 * j + 2] + x.z, 0.f), fmaxf(v[4 * j + 3] + x.w, 0.f));
         }
-      }
-      umma::fence_async_smem();
-      umma::fence_before_sync();
-      umma::mbar_arrive(&d1free[slot]);
-      umma::mbar_arrive(a1full);
-      if (p.a1_save) {
-        umma::bar_sync(1, kRows);
-        if (warp == 4 && lane == 0) {
-          umma::tma_store(&maps.a1, 0, tile * kRows, a1s);
-          umma::tma_store(&maps.a1, 64, tile * kRows, a1s + kBlk);
+        umma::tmem_st16(d1 + q * 16, o);
+        if (q == 3) {
+          umma::tmem_st_wait();
+          umma::fence_before_sync();
+          umma::mbar_arrive(&a1full[slot]);
+        }
+        if (!save) continue;
+        if (q == 2) {  // the first half has been read
+          if (leader) umma::tma_store_wait_read();
+          umma::bar_sync(1, kRows);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+          *reinterpret_cast<uint4*>(a1s + umma::sw128_offset(r, (q & 1) * 32 + j * 8)) =
+              make_uint4(o[4 * j], o[4 * j + 1], o[4 * j + 2], o[4 * j + 3]);
+        if (q & 1) {
+          umma::fence_async_smem();
+          umma::bar_sync(1, kRows);
+          if (leader) umma::tma_store(&maps.a1, (q >> 1) * 64, row_of(t), a1s);
+          __syncwarp();
         }
       }
     }
-    if (p.a1_save && warp == 4 && lane == 0) umma::tma_store_wait();
+    if (save && leader) umma::tma_store_wait();
   } else if (warp >= 8 && warp < 12) {
     // ---- epilogue 2
     const int r = (warp & 3) * 32 + lane;
     const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const bool leader = warp == 8 && lane == 0;
-    uint32_t t = 0;
-    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, t++) {
+    for (int t = 0; t < mine; t++) {
       const int slot = t & 1;
-      const size_t row = static_cast<size_t>(tile) * kRows + r;
-      uint4 res[16];
-#pragma unroll
-      for (int j = 0; j < 16; j++) {
-        res[j] = make_uint4(0, 0, 0, 0);
-        if (p.res && j * 8 < p.n_out) res[j] = reinterpret_cast<const uint4*>(p.res + row * p.n_out)[j];
+      const size_t row = static_cast<size_t>(row_of(t)) + r;
+      if (leader) {
+        umma::tma_store_wait_read();  // the tile before has been read
+        if (p.res) {
+          umma::mbar_expect(resfull, p.n_out * 2 * kRows);
+          for (int x = 0; x < p.n_out; x += 64) umma::tma_load(ios + (x >> 6) * kBlk, &maps.res, x, row_of(t), resfull);
+        }
       }
-      const bool ok = umma::warp_wait(&d2full[slot], (t >> 1) & 1) && !aborted(&s_abort);
-      if (leader) umma::tma_store_wait_read();  // the half tile before has been read
-      if (!umma::bar_all(2, kRows, ok)) {
+      __syncwarp();
+      bool ok = umma::warp_wait(&d2full[slot], (t >> 1) & 1);
+      if (p.res) ok = umma::warp_wait(resfull, t & 1) && ok;
+      if (!umma::bar_all(2, kRows, ok && !aborted(&s_abort))) {
         s_abort = 1;
         break;
       }
       umma::fence_after_sync();
-#pragma unroll
-      for (int half = 0; half < 2; half++) {
-        if (half * 64 >= p.n_out) break;
-        if (half > 0) {
-          if (leader) umma::tma_store_wait_read();
-          umma::bar_sync(2, kRows);
-        }
-#pragma unroll
-        for (int cc = 0; cc < 64; cc += 32) {
-          const int col0 = half * 64 + cc;
-          float v[32];
-          umma::tmem_ld32(tmem + 256 + slot * 128 + lane_off + col0, v);
-          if (p.res) {
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-              const uint4 w = res[(col0 >> 3) + j];
-              const uint32_t x[4] = {w.x, w.y, w.z, w.w};
-#pragma unroll
-              for (int u = 0; u < 4; u++) {
-                v[8 * j + 2 * u] += __uint_as_float(x[u] << 16);
-                v[8 * j + 2 * u + 1] += __uint_as_float(x[u] & 0xffff0000u);
-              }
-            }
-          }
-          const float4* bp = reinterpret_cast<const float4*>(b2s + col0);
-#pragma unroll
-          for (int j = 0; j < 8; j++) {
-            const float4 x = bp[j];
-            v[4 * j] += x.x;
-            v[4 * j + 1] += x.y;
-            v[4 * j + 2] += x.z;
-            v[4 * j + 3] += x.w;
-          }
+#pragma unroll 1
+      for (int col0 = 0; col0 < p.n_out; col0 += 32) {
+        uint8_t* io = ios + (col0 >> 6) * kBlk;
+        float v[32];
+        umma::tmem_ld32(tmem + 256 + slot * 128 + lane_off + col0, v);
+        if (p.res) {
 #pragma unroll
           for (int j = 0; j < 4; j++) {
-            const uint4 o = make_uint4(pack_bf16(v[8 * j], v[8 * j + 1]), pack_bf16(v[8 * j + 2], v[8 * j + 3]),
-                                       pack_bf16(v[8 * j + 4], v[8 * j + 5]), pack_bf16(v[8 * j + 6], v[8 * j + 7]));
-            *reinterpret_cast<uint4*>(ios + umma::sw128_offset(r, cc + j * 8)) = o;
-          }
-          if (p.out_f32) {
-            float4* fp = reinterpret_cast<float4*>(p.out_f32 + row * p.n_out + col0);
+            const uint4 w = *reinterpret_cast<const uint4*>(io + umma::sw128_offset(r, (col0 & 32) + j * 8));
+            const uint32_t x[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-            for (int j = 0; j < 8; j++) fp[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+            for (int u = 0; u < 4; u++) {
+              v[8 * j + 2 * u] += __uint_as_float(x[u] << 16);
+              v[8 * j + 2 * u + 1] += __uint_as_float(x[u] & 0xffff0000u);
+            }
           }
+        }
+        const float4* bp = reinterpret_cast<const float4*>(b2s + col0);
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+          const float4 x = bp[j];
+          v[4 * j] += x.x;
+          v[4 * j + 1] += x.y;
+          v[4 * j + 2] += x.z;
+          v[4 * j + 3] += x.w;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+          *reinterpret_cast<uint4*>(io + umma::sw128_offset(r, (col0 & 32) + j * 8)) =
+              make_uint4(pack_bf16(v[8 * j], v[8 * j + 1]), pack_bf16(v[8 * j + 2], v[8 * j + 3]),
+                         pack_bf16(v[8 * j + 4], v[8 * j + 5]), pack_bf16(v[8 * j + 6], v[8 * j + 7]));
+        if (p.out_f32) {
+          float4* fp = reinterpret_cast<float4*>(p.out_f32 + row * p.n_out + col0);
+#pragma unroll
+          for (int j = 0; j < 8; j++) fp[j] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+        }
+        if (!(col0 & 32)) continue;
+        if (col0 + 32 == p.n_out) {
+          umma::fence_before_sync();
+          umma::mbar_arrive(&d2free[slot]);
         }
         umma::fence_async_smem();
         umma::bar_sync(2, kRows);
-        if (leader) umma::tma_store(&maps.out, half * 64, tile * kRows, ios);
+        if (leader) umma::tma_store(&maps.out, col0 - 32, row_of(t), io);
         __syncwarp();
       }
-      umma::fence_before_sync();
-      umma::mbar_arrive(&d2free[slot]);
     }
     if (leader) umma::tma_store_wait();
   } else if (warp >= 12) {
     // ---- mapped rows and aggregation
     const int tid = threadIdx.x - 384;
-    uint32_t g = 0, granted = 0;  // (bit: parity of a stage's next grant)
+    RingPos r;
+    uint32_t granted = 0;  // (bit: parity of a stage's next grant)
     bool ok = true;
-    int4 ent[kMaxSeg];
-#pragma unroll
-    for (int s = 0; s < kMaxSeg; s++)
-      if (s < p.nseg && p.seg[s].idx) ent[s] = map_entries(p.seg[s].idx + blockIdx.x * kRows, lane);
-    for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
-      const int row0 = tile * kRows;
-      const int next = tile + gridDim.x < ntiles ? (tile + gridDim.x) * kRows : row0;
-#pragma unroll
-      for (int s = 0; s < kMaxSeg; s++) {
-        if (s >= p.nseg || !ok) break;
+    for (int t = 0; t < mine && ok; t++) {  // (the gathering warps go on, or stop, together)
+      const int row0 = row_of(t);
+      ok = umma::bar_all(4, kGather, umma::warp_wait(&runfull[t & 1], (t >> 1) & 1) && !aborted(&s_abort));
+#pragma unroll 1
+      for (int s = 0; s < p.nseg && ok; s++) {
         const Seg& sg = p.seg[s];
         const int nb = sg.width >> 6;
-        bool mine = sg.agg;
-        if (!mine && sg.idx) {
-          mine = consecutive(ent[s], lane) < 0;
-          ent[s] = map_entries(sg.idx + next, lane);
-        }
-        if (!mine) {
-          g += nb;
+        if (runs[(t & 1) * 4 + s] >= 0) {
+          r.next(nst);
+          if (nb > 1) r.next(nst);
           continue;
         }
+        // (these loads are on their way while the stage is waited for)
+        const bool agg = kAgg && sg.agg;
+        uint32_t mask = 0;
+        int src[kRowsEach];
+        if constexpr (kAgg) {
+          if (agg) mask = agg_mask<kGather>(sg, row0, tid);
+        }
+        if (!agg) {
+#pragma unroll
+          for (int i = 0; i < kRowsEach; i++) src[i] = sg.idx[row0 + (tid >> 3) + i * (kGather / 8)];
+        }
         // the segment's one or two blocks in flight together
-        for (int b = 0; b < nb && ok; b++) {
-          const int st = (g + b) % nst;
-          const bool given = umma::warp_wait(&grant[st], (granted >> st) & 1);
-          granted ^= 1u << st;
-          ok = umma::bar_all(4, kRows, given && !aborted(&s_abort));  // the four warps go on, or stop, together
+        RingPos w = r;
+#pragma unroll 1
+        for (int b = 0; b < nb; b++) {
+          const bool given = umma::warp_wait(&grant[r.st], (granted >> r.st) & 1);
+          granted ^= 1u << r.st;
+          ok = umma::bar_all(4, kGather, given && !aborted(&s_abort));
           if (!ok) break;
-          uint8_t* dst = ring + st * kBlk;
-          if (sg.agg) {
-            stage_agg_block<kRows>(sg, row0, b * 64, dst, tid);
-          } else {
-            int src[8];
+          uint8_t* dst = ring + r.st * kBlk;
+          if constexpr (kAgg) {
+            if (agg) stage_agg_block<kGather>(sg, mask, row0, b * 64, dst, tid);
+          }
+          if (!agg) {
 #pragma unroll
-            for (int i = 0; i < 8; i++) src[i] = sg.idx[row0 + (tid >> 3) + i * 16];
-#pragma unroll
-            for (int i = 0; i < 8; i++)
-              cp_async16(dst + umma::sw128_offset((tid >> 3) + i * 16, (tid & 7) * 8),
+            for (int i = 0; i < kRowsEach; i++)
+              cp_async16(dst + umma::sw128_offset((tid >> 3) + i * (kGather / 8), (tid & 7) * 8),
                          sg.src + static_cast<size_t>(src[i] >= 0 ? src[i] : 0) * sg.width + b * 64 + (tid & 7) * 8,
                          src[i] >= 0);
           }
           cp_async_commit();
+          r.next(nst);
         }
-        for (int b = 0; b < nb && ok; b++) {
+        if (!ok) break;
+#pragma unroll 1
+        for (int b = 0; b < nb; b++) {
           if (b + 1 < nb) cp_async_wait<1>();
           else cp_async_wait<0>();
           umma::fence_async_smem();
-          umma::bar_sync(3, kRows);
-          if (tid == 0) umma::mbar_arrive(&full[(g + b) % nst]);
+          umma::bar_sync(3, kGather);
+          if (tid == 0) umma::mbar_arrive(&full[w.st]);
+          w.next(nst);
         }
-        g += nb;
       }
+      __syncwarp();
+      if (lane == 0) umma::mbar_arrive(&runfree[t & 1]);
     }
     cp_async_wait<0>();
     if (!ok) s_abort = 1;
@@ -702,9 +780,9 @@ __global__ void __launch_bounds__(kDataThreads, 1) k_mlp_bwd_data(const __grid_c
     umma::warp_wait(wfull, 0);  // landed before the block's shared memory is given up
   } else if (warp == 1) {
     // ---- MMA issuer
-    if (lane == 0) {
+    if (umma::elect_one()) {
       const uint32_t w1a = umma::smem_addr(w1s), w2a = umma::smem_addr(w2s);
-      const uint32_t dya = umma::smem_addr(dys);
+      const uint64_t dyd = umma::desc_kmajor(umma::smem_addr(dys)), w2d = umma::desc_mnmajor(w2a, p.n_out * 128);
       // da1 = dy W2 : A = dy [128 x n_out] K-major, B = W2 viewed [N=128 hid x K=n_out] MN-major
       const uint32_t idesc_a1 = umma::idesc_bf16(kRows, kHid, false, true);
       bool ok = umma::mbar_wait(wfull, 0);
@@ -713,24 +791,26 @@ __global__ void __launch_bounds__(kDataThreads, 1) k_mlp_bwd_data(const __grid_c
         if (!ok) break;
         umma::fence_after_sync();
         // K = n_out rows of W2; K-step 16 advances dy by 32 bytes (inside a 64-col block)
-        // and the MN-major W2 view by 16 rows (2 KB).
-        for (int k = 0; k < p.n_out; k += 16)
-          umma::mma_bf16(dda1, umma::desc_kmajor(dya + (k >> 6) * kBlk + (k & 63) * 2),
-                         umma::desc_mnmajor(w2a + k * 128, p.n_out * 128), idesc_a1, k > 0 ? 1u : 0u);
+        // and the MN-major W2 view by 16 rows (2 KB); descriptors count 16 bytes.
+#pragma unroll
+        for (int k = 0; k < 128; k += 16)
+          if (k < p.n_out)
+            umma::mma_bf16(dda1, dyd + (k >> 6) * (kBlk / 16) + (k & 63) / 8, w2d + k * 8, idesc_a1, k > 0 ? 1u : 0u);
         umma::commit(d1full);
         if (!need_da) continue;
         // dA = dz1 W1 : A = dz1 [128 x 128] K-major, B = W1 viewed [N=k_in x K=128] MN-major
         ok = umma::mbar_wait(dzfull, t & 1);
-        const uint32_t dza = umma::smem_addr(dzs + (t % ndz) * 2 * kBlk);
+        const uint64_t dzd = umma::desc_kmajor(umma::smem_addr(dzs + (t % ndz) * 2 * kBlk));
         for (int c = 0; c < nch && ok; c++) {
           if (t > 0) ok = umma::mbar_wait(&d2free[c], (t - 1) & 1);
           if (!ok) break;
           umma::fence_after_sync();
           const uint32_t idesc = umma::idesc_bf16(kRows, p.k_in - c * 128 >= 128 ? 128 : 64, false, true);
+          // W1 rows k.. (K index = hid), columns 128 c.. (two blocks of 16 KB)
+          const uint64_t w1d = umma::desc_mnmajor(w1a + c * 2 * (kHid * 128), kHid * 128);
+#pragma unroll
           for (int k = 0; k < kHid; k += 16)
-            // W1 rows k.. (K index = hid), columns 128 c.. (two blocks of 16 KB)
-            umma::mma_bf16(dda + c * 128, umma::desc_kmajor(dza + (k >> 6) * kBlk + (k & 63) * 2),
-                           umma::desc_mnmajor(w1a + c * 2 * (kHid * 128) + k * 128, kHid * 128), idesc, k > 0 ? 1u : 0u);
+            umma::mma_bf16(dda + c * 128, dzd + (k >> 6) * (kBlk / 16) + (k & 63) / 8, w1d + k * 8, idesc, k > 0 ? 1u : 0u);
           umma::commit(&d2full[c]);
         }
       }
@@ -1017,7 +1097,7 @@ __global__ void __launch_bounds__(kWeightThreads, 1) k_mlp_bwd_weight(const __gr
     for (int k = g > nst ? g - nst : 0; k < g; k++) umma::warp_wait(&full[k % nst], (k / nst) & 1);
   } else if (warp == 1) {
     // ---- MMA issuer
-    if (lane == 0) {
+    if (umma::elect_one()) {
       // dW1 = dz1^T A : A-operand dz1^T [M=128 hid, K=rows] MN-major; B = A^T [N=k_in chunk, K=rows] MN-major
       // dW2^T = a1^T dy : A-operand a1^T [M=128, K=rows] MN-major; B = dy^T [N=n_out, K=rows] MN-major
       const uint32_t idesc_w2 = umma::idesc_bf16(kHid, p.n_out, true, true);
@@ -1029,13 +1109,17 @@ __global__ void __launch_bounds__(kWeightThreads, 1) k_mlp_bwd_weight(const __gr
         }
         umma::fence_after_sync();
         const uint32_t a = umma::smem_addr(ring + st * stage_bytes);
-        for (int k = 0; k < kSlab; k += 16) {  // 16 rows = 2 KB
-          const uint64_t ad = umma::desc_mnmajor(a + dz_off + k * 128, kSlabBlk);
-          for (int n0 = 0; n0 < p.k_in; n0 += 128)
-            umma::mma_bf16(dw1 + n0, ad, umma::desc_mnmajor(a + (n0 >> 6) * kSlabBlk + k * 128, kSlabBlk),
-                           umma::idesc_bf16(kHid, p.k_in - n0 >= 128 ? 128 : 64, true, true), (g > 0 || k > 0) ? 1u : 0u);
-          umma::mma_bf16(dw2, umma::desc_mnmajor(a + a1_off + k * 128, kSlabBlk),
-                         umma::desc_mnmajor(a + dy_off + k * 128, kSlabBlk), idesc_w2, (g > 0 || k > 0) ? 1u : 0u);
+        const uint64_t dzd = umma::desc_mnmajor(a + dz_off, kSlabBlk), a1d = umma::desc_mnmajor(a + a1_off, kSlabBlk);
+        const uint64_t dyd = umma::desc_mnmajor(a + dy_off, kSlabBlk), ind = umma::desc_mnmajor(a, kSlabBlk);
+#pragma unroll
+        for (int k = 0; k < kSlab; k += 16) {  // 16 rows = 2 KB; descriptors count 16 bytes
+          const uint32_t acc = (g > 0 || k > 0) ? 1u : 0u;
+#pragma unroll
+          for (int n0 = 0; n0 < 384; n0 += 128)
+            if (n0 < p.k_in)
+              umma::mma_bf16(dw1 + n0, dzd + k * 8, ind + (n0 >> 6) * (kSlabBlk / 16) + k * 8,
+                             umma::idesc_bf16(kHid, p.k_in - n0 >= 128 ? 128 : 64, true, true), acc);
+          umma::mma_bf16(dw2, a1d + k * 8, dyd + k * 8, idesc_w2, acc);
         }
         umma::commit(&empty[st]);
       }
@@ -1076,7 +1160,9 @@ __global__ void __launch_bounds__(kWeightThreads, 1) k_mlp_bwd_weight(const __gr
         const Seg& sg = p.seg[s];
         const int nb = sg.width >> 6;
         if (sg.agg) {
-          for (int b = 0; b < nb; b++) stage_agg_block<kSlab>(sg, row0, b * 64, dst + b * kSlabBlk, tid);
+          const uint32_t mask = agg_mask<128>(sg, row0, tid);
+#pragma unroll 1
+          for (int b = 0; b < nb; b++) stage_agg_block<128>(sg, mask, row0, b * 64, dst + b * kSlabBlk, tid);
         } else if (sg.idx) {
           const bool mapped = consecutive(ent[s], lane) < 0;
           ent[s] = slab_entries(sg.idx + next, lane);
@@ -1455,9 +1541,13 @@ int storm_gnn_mlp_forward(const StormGnnMlpFwd* a, int32_t* dev_err, void* strea
       (rc = tensor_map(&maps.out, p.out, a->rows, a->n_out, kRows)))
     return rc;
   if (p.a1_save && (rc = tensor_map(&maps.a1, p.a1_save, a->rows, kHid, kRows))) return rc;
-  const size_t smem = fwd_smem_bytes(a->k_in, a->n_out);
-  cudaFuncSetAttribute(k_mlp_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
-  k_mlp_fwd<<<grid_for(a->rows), kFwdThreads, smem, static_cast<cudaStream_t>(stream)>>>(p, maps);
+  if (p.res && (rc = tensor_map(&maps.res, p.res, a->rows, a->n_out, kRows))) return rc;
+  const size_t smem = fwd_smem_bytes(a->k_in, a->n_out, p.a1_save != nullptr);
+  bool agg = false;
+  for (int i = 0; i < a->nseg; i++) agg |= p.seg[i].agg != 0;
+  auto kernel = agg ? k_mlp_fwd<true> : k_mlp_fwd<false>;
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  kernel<<<grid_for(a->rows), fwd_threads(agg), smem, static_cast<cudaStream_t>(stream)>>>(p, maps);
   g_launches++;
   return cuda_check("k_mlp_fwd");
 }

@@ -96,6 +96,27 @@ def test_forward_many_tiles(storm_lib, tiles, layer, kinds):
 
 
 @pytest.mark.parametrize("tiles", [1, SMS + 1, 3 * SMS + 5])
+@pytest.mark.parametrize("kind", ["run", "scatter", "mixed"])
+def test_forward_does_not_depend_on_saving(storm_lib, tiles, kind):
+    """Saving the hidden rows takes a stage from the ring and changes no bit of the output."""
+    import torch
+    net = gnn.WarmStartNet(seed=14)
+    dev = net.device
+    rng = np.random.default_rng(tiles)
+    rows, n = 128 * tiles, 128 * 40
+    x = torch.randn((rows, 128), device=dev).bfloat16()
+    h = torch.randn((n, 128), device=dev).bfloat16()
+    idx = [torch.tensor(_map(rng, k, rows, n), device=dev) for k in (kind, "run")]
+    segs = [net._seg(x)] + [net._seg(h, idx=i) for i in idx]
+    out = [torch.empty((rows, 128), dtype=torch.bfloat16, device=dev) for _ in range(2)]
+    net._fwd("edge0", rows, segs, out[0], res=x, a1_save=torch.empty_like(out[0]))
+    net._fwd("edge0", rows, segs, out[1], res=x)
+    torch.cuda.synchronize()
+    net._check_err()
+    assert torch.equal(out[0].view(torch.int16), out[1].view(torch.int16))
+
+
+@pytest.mark.parametrize("tiles", [1, SMS + 1, 3 * SMS + 5])
 @pytest.mark.parametrize("layer,outs", [("edge0", "axx"), ("edge0", "x0a"), ("node0", "ax"), ("node0", "00"),
                                         ("enc_edge", "0"), ("enc_edge", "a"), ("dec", "x")])
 def test_backward_data_many_tiles(storm_lib, tiles, layer, outs):
