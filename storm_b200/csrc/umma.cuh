@@ -184,6 +184,12 @@ __device__ __forceinline__ void tma_store_wait() { asm volatile("cp.async.bulk.w
 __device__ __forceinline__ void tma_prefetch_map(const CUtensorMap* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
 }
+// Programmatic dependent launch.  wait: every kernel before this one in the stream has ended
+// and its writes are visible; before it a kernel touches no global memory.  launch: the next
+// kernel's blocks may take what this grid leaves free (they wait as well before they read).
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_launch_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Barrier `id` (1..15) among `n` threads of the block, in whole warps: the warp's threads
 // are brought together first, and the unaligned form asks nothing more of them.
 __device__ __forceinline__ void bar_sync(int id, int n) {
