@@ -1360,25 +1360,35 @@ __global__ void __launch_bounds__(256) k_node_backward(const float* __restrict__
 }
 
 // Masked mean-squared error over the first `nout` columns of y (row stride ld):
-// per-block partial loss and dy = 2 (y - t) w / norm.  A warp takes a row, so that it writes
-// 128 bytes in a row (a row to a thread took 15 us for 25,000 rows).
-constexpr int kMseThreads = 512;
+// per-block partial loss and dy = 2 (y - t) w / norm.  A thread sums the loss of its rows, then
+// the warps write dy of the block's 256 rows, 128 bytes in a row (a row to a thread took 15 us
+// for 25,000 rows).
+constexpr int kMseThreads = 256;
 __global__ void __launch_bounds__(kMseThreads) k_mse(const float* __restrict__ y, int ld, const float* __restrict__ target,
                                                      const float* __restrict__ wmask, int Tp, int nout, float norm,
                                                      float* __restrict__ dy, float* __restrict__ loss_part) {
   __shared__ float red[kMseThreads];
   umma::grid_wait();
   float acc = 0.f;
-  for (int i = blockIdx.x * (kMseThreads / 32) + (threadIdx.x >> 5); i < Tp; i += gridDim.x * (kMseThreads / 32)) {
-    const float w = wmask[i];
-    for (int j = threadIdx.x & 31; j < ld; j += 32) {
-      float g = 0.f;
-      if (j < nout) {
+  for (int r0 = blockIdx.x * kMseThreads; r0 < Tp; r0 += gridDim.x * kMseThreads) {
+    const int i = r0 + threadIdx.x;
+    if (i < Tp) {
+      const float w = wmask[i];
+      for (int j = 0; j < nout; j++) {
         const float d = y[static_cast<size_t>(i) * ld + j] - target[static_cast<size_t>(i) * nout + j];
         acc += w * d * d;
-        g = 2.f * w * d / norm;
       }
-      dy[static_cast<size_t>(i) * ld + j] = g;
+    }
+    for (int r = r0 + (threadIdx.x >> 5); r < min(Tp, r0 + kMseThreads); r += kMseThreads / 32) {
+      const float w = wmask[r];
+      for (int j = threadIdx.x & 31; j < ld; j += 32) {
+        float g = 0.f;
+        if (j < nout) {
+          const float d = y[static_cast<size_t>(r) * ld + j] - target[static_cast<size_t>(r) * nout + j];
+          g = 2.f * w * d / norm;
+        }
+        dy[static_cast<size_t>(r) * ld + j] = g;
+      }
     }
   }
   red[threadIdx.x] = acc;
