@@ -215,6 +215,7 @@ int enqueue_step(StormFvtHandle* h, bool timing, size_t* fev_used, int only = -1
   if (only < 0 && linked && !d.steady && d.dt_op != 0) launch_link_dt(d, h->stream);
   for (int s = 1; s <= K; s++) {
     const int gB = (d.nbc_cells + kFluxThreads - 1) / kFluxThreads;
+    const int gF = (4 * d.nbc_cells + kFluxThreads - 1) / kFluxThreads;  // k_flux_bc off the tiles: four threads a cell
     if (fused) {  // stage s reads one state buffer and writes the other
       q = (s & 1) ? d.q : h->q2;
       qo = (s & 1) ? h->q2 : d.q;
@@ -294,7 +295,7 @@ int enqueue_step(StormFvtHandle* h, bool timing, size_t* fev_used, int only = -1
         // the neighbours' face records (k_grad), the culverts
         CK(cudaEventRecord(h->eflux_ev[s], h->stream));
         CK(cudaStreamWaitEvent(h->side, h->eflux_ev[s], 0));
-        launch(STAGE_FLUX_BC, gB, kFluxThreads, 0, h->side, s);
+        launch(STAGE_FLUX_BC, gF, kFluxThreads, 0, h->side, s);
       }
       if (forked) CK(cudaEventRecord(h->join_ev[s], h->side));
       launch(STAGE_CELL, gC, bC, h->cell_smem, h->stream, s);
@@ -312,7 +313,7 @@ int enqueue_step(StormFvtHandle* h, bool timing, size_t* fev_used, int only = -1
       }
       if (mark(KT_FLUX)) return STORM_ERR_CUDA;
       launch(STAGE_CELL, gC, bC, h->cell_smem, h->stream, s);
-      if (gB > 0) launch(STAGE_FLUX_BC, gB, kFluxThreads, 0, h->stream, s);
+      if (gB > 0) launch(STAGE_FLUX_BC, gF, kFluxThreads, 0, h->stream, s);
       if (done()) return STORM_ERR_CUDA;
     }
     if (rs) {  // solverFVT.f90:238-256, then the update of every cell

@@ -2235,15 +2235,18 @@ __device__ __forceinline__ void store_update(const Dev& d, int s, int c, const R
   st_rec(qo + c, Rec{o.h, own.z, o.u, o.v});
   if (s == d.K) d.phimax[c] = fmax2(fmax2(fmax2(kZero, fabs(p1)), fabs(p2)), fabs(p3));
 }
-__device__ __forceinline__ void rk_update(const Dev& d, int s, int c, const Rec& own, bool dry_c, double p1, double p2,
-                                          double p3, Rec* __restrict__ qo) {
-  const CellIn in = cell_in(d, s, c);
-  const double delt = cell_dt(d, c, own, dry_c, in);
+__device__ __forceinline__ void rk_update(const Dev& d, int s, int c, const Rec& own, bool dry_c, const CellIn& in,
+                                          double delt, double p1, double p2, double p3, Rec* __restrict__ qo) {
   if (d.steady && s == d.K) {
     Scalars& sc = d.sc[cell_scenario(d, c)];
     if (c == sc.last_cell) sc.delt_fric = delt;
   }
   store_update(d, s, c, own, rk_combine(d, s, own, dry_c, in, delt, p1, p2, p3), p1, p2, p3, qo);
+}
+__device__ __forceinline__ void rk_update(const Dev& d, int s, int c, const Rec& own, bool dry_c, double p1, double p2,
+                                          double p3, Rec* __restrict__ qo) {
+  const CellIn in = cell_in(d, s, c);
+  rk_update(d, s, c, own, dry_c, in, cell_dt(d, c, own, dry_c, in), p1, p2, p3, qo);
 }
 
 // The friction step of a cell after the last stage and its terms of the iteration's
@@ -2530,27 +2533,124 @@ __global__ void __launch_bounds__(kThreads, kThreads == 256 ? 4 : 1) k_cell(cons
 // The cells with an open-boundary face, after k_bc: their interior faces' fluxes again
 // from the face records, so that this needs nothing of k_cell and runs beside it
 // (kTile: from the arrays the fused kernel leaves them in).
+// From the face records a cell has four threads: one to a face in the order invisc_fluxes.f90
+// visits them, one for the bed slope; the first adds their terms in that order.  On meshes
+// with fewer blocks of cells than SMs the stage waits for this kernel, and it for one long
+// chain of FP64 operations a cell.  Channel of 8,000 cells 8.19 ms per 100 iterations with a
+// thread to a cell, 7.63 so; 1,200 cells stepped singly 2.22 and 2.09 ms.
+template <class R>
+__device__ __forceinline__ void assemble_phi4(const Dev& d, const Geo<R>& G, int c, int m, bool live, const Rec& own,
+                                              bool dry_c, double* p1o, double* p2o, double* p3o) {
+  const int T = d.T;
+  uint8_t ord = 0;
+  int kind = 0;  // (FACE_NONE: nothing to add)
+  double a0 = kZero, a1 = kZero, a2 = kZero;
+  if (live) {
+    ord = d.forder[c];
+    if (m < 3) {
+      const FacesGlobal<R, false> fs{d, G, c};
+      const int j = (ord >> (2 * m)) & 3, q = j * T + c, e = d.frefo[m * T + c];
+      kind = (d.fko[c] >> (3 * m)) & 7;
+      if (kind == FACE_LEFT || kind == FACE_RIGHT) {
+        R f[3];
+        if (fs.iface(j, e, f)) {
+          a0 = f[0];
+          a1 = f[1];
+          a2 = f[2];
+        } else {
+          kind = FACE_NONE;
+        }
+      } else if (kind == FACE_WALL) {
+        if (dry_c) {
+          kind = FACE_NONE;
+        } else {
+          const double nx = d.fnx[q], ny = d.fny[q];
+          if (d.btype == 0) {
+            double h1, h2;
+            fs.hwall(j, e, &h1, &h2);
+            wall_noslip(d, h1, h2, nx, ny, &a1, &a2);
+          } else {
+            wall_slip(d, fs.own(j), nx, ny, &a1, &a2);
+          }
+          a0 = d.flen[q];
+        }
+      } else if (kind == FACE_BC) {
+        a0 = d.bc_c[e];
+        a1 = d.bc_c[d.nbce + e];
+        a2 = d.bc_c[2 * d.nbce + e];
+      }
+    } else if (!dry_c) {
+      bed_source(d, c, own.h, G.delh_x[c], G.delh_y[c], G.delz_x[c], G.delz_y[c], d.area[c], d.rad[c], G, &a1, &a2);
+    }
+  }
+  double p1 = kZero, p2 = kZero, p3 = kZero;
+#pragma unroll
+  for (int t = 0; t < 3; t++) {
+    const int k = __shfl_sync(0xffffffffu, kind, t, 4);
+    const double f0 = __shfl_sync(0xffffffffu, a0, t, 4), f1 = __shfl_sync(0xffffffffu, a1, t, 4),
+                 f2 = __shfl_sync(0xffffffffu, a2, t, 4);
+    if (k == FACE_LEFT || k == FACE_BC) {
+      p1 = p1 - f0;
+      p2 = p2 - f1;
+      p3 = p3 - f2;
+    } else if (k == FACE_RIGHT) {
+      p1 = p1 + f0;
+      p2 = p2 + f1;
+      p3 = p3 + f2;
+    } else if (k == FACE_WALL) {
+      p2 = p2 - f1 * f0;
+      p3 = p3 - f2 * f0;
+    }
+  }
+  const double s2 = __shfl_sync(0xffffffffu, a1, 3, 4), s3 = __shfl_sync(0xffffffffu, a2, 3, 4);
+  if (live && m == 0) {
+    if (!dry_c) {
+      p2 = p2 - s2;
+      p3 = p3 - s3;
+      if (d.wcoef1) {  // wind forcing (solverFVT.f90:218-224)
+        p2 = p2 + d.wcoef1[c];
+        p3 = p3 + d.wcoef2[c];
+      }
+    }
+    if (ord & kOrderHasCulvert) p1 = culvert_terms(d, c, p1);
+  }
+  *p1o = p1;
+  *p2o = p2;
+  *p3o = p3;
+}
+
 template <class R, int kMode, bool kTile>
 __global__ void __launch_bounds__(128) k_flux_bc(Dev d, Geo<R> G, int s, const Rec* q, Rec* qo) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= d.nbc_cells) return;
-  const int c = d.bc_cells[i];
-  if (!cell_live(d, c)) return;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, i = kTile ? t : t >> 2;
+  bool live = i < d.nbc_cells;
+  const int c = live ? d.bc_cells[i] : 0;
+  live = live && cell_live(d, c);
   const Rec own = ld_rec(q + c);
   const bool dry_c = rec_dry(d, own);
+  CellIn in{};
   double p1, p2, p3;
-  assemble_phi<R>(d, G, FacesGlobal<R, kTile>{d, G, c}, c, own.h, dry_c, &p1, &p2, &p3);
+  if constexpr (kTile) {
+    if (!live) return;
+    assemble_phi<R>(d, G, FacesGlobal<R, true>{d, G, c}, c, own.h, dry_c, &p1, &p2, &p3);
+  } else {
+    if (live && (t & 3) == 0 && kMode != CELL_PHI) in = cell_in(d, s, c);  // on the way meanwhile
+    assemble_phi4<R>(d, G, c, t & 3, live, own, dry_c, &p1, &p2, &p3);
+    if (!live || (t & 3) != 0) return;
+  }
   if (kMode == CELL_PHI) {
     store_phi(d, c, p1, p2, p3);
-  } else if (kMode == CELL_FRIC) {
-    const CellIn in = cell_in(d, s, c);
-    const CellOut o = rk_combine(d, s, own, dry_c, in, cell_dt(d, c, own, dry_c, in), p1, p2, p3);
+    return;
+  }
+  if (kTile) in = cell_in(d, s, c);
+  const double delt = cell_dt(d, c, own, dry_c, in);
+  if (kMode == CELL_FRIC) {
+    const CellOut o = rk_combine(d, s, own, dry_c, in, delt, p1, p2, p3);
     const double pm = fmax2(fmax2(fmax2(kZero, fabs(p1)), fabs(p2)), fabs(p3));
-    const FricTerms t = fric_cell(d, cell_scenario(d, c), c, o, own.z, s > 1 ? in.rkh0 : own.h, pm, d.cd[c], in.area,
-                                  in.perim);
-    store_bc_terms(d, i, t);
+    const FricTerms ft = fric_cell(d, cell_scenario(d, c), c, o, own.z, s > 1 ? in.rkh0 : own.h, pm, d.cd[c], in.area,
+                                   in.perim);
+    store_bc_terms(d, i, ft);
   } else {
-    rk_update(d, s, c, own, dry_c, p1, p2, p3, qo);
+    rk_update(d, s, c, own, dry_c, in, delt, p1, p2, p3, qo);
   }
 }
 

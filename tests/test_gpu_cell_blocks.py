@@ -47,3 +47,12 @@ def test_equal_ratios(limiter, storm_lib, oracle_mod):
     sc.u0 = np.where(rng.random(n) < 0.5, 0.0, 0.0625)
     sc.v0 = np.where(rng.random(n) < 0.5, 0.0, 0.03125)
     _compare(sc, oracle_mod, 20)
+
+
+@pytest.mark.parametrize("ny", [2, 15, 16, 17, 33])
+@pytest.mark.parametrize("flux,btype,steady", [(abi.FLUX_ROE, 0, 1), (abi.FLUX_HLL, 1, 0), (abi.FLUX_RUSANOV, 1, 1)])
+def test_boundary_cells(ny, flux, btype, steady, storm_lib, oracle_mod):
+    """The cells with an open-boundary face (2 ny here, those in the corners with a wall too)
+    around the 32 that a block of k_flux_bc updates."""
+    over = {"steady": steady} if steady else {"steady": 0, "dt_op": 1}
+    _compare(scenarios.channel(nx=9, ny=ny, flux=flux, btype=btype, **over), oracle_mod, 10)
