@@ -34,6 +34,7 @@
 #include <vector>
 
 #include "storm_internal.h"
+#include "umma.cuh"
 
 namespace storm {
 namespace {
@@ -55,11 +56,18 @@ __device__ __forceinline__ double na_min(double a, double b) { return (b < a) ? 
 // The per-cell CFL candidate of k_fric: find_dry_cells (find_dry_cells.f90:25-42),
 // wavec (solverFVT.f90:180-181) and cfl*area/((|u|+c+small)*perim) (deltatFVT.f90:34-37
 // with the cell area and perimeter).
+//
+// Both kernels take microseconds and follow one another, so what bounds a call is the
+// launches: they wait for the kernels before them by themselves (programmatic stream
+// serialization), and the final block is placed while the partials are computed.  300,001
+// cells: 12.1 us a call with plain launches, 10.8 so.
 __global__ void __launch_bounds__(kNaThreads)
     k_cfl_dt_partials(const double* __restrict__ h, const double* __restrict__ u, const double* __restrict__ v,
                       const double* __restrict__ area, const double* __restrict__ perim, int n, double cfl,
                       double h_dry, double h_wet, double* __restrict__ part) {
   __shared__ double sm[kNaThreads / 32];
+  umma::grid_launch_next();
+  umma::grid_wait();
   const int c = blockIdx.x * blockDim.x + threadIdx.x;
   double cand = kVlarge;
   if (c < n) {
@@ -89,7 +97,9 @@ __global__ void __launch_bounds__(kNaThreads)
 __global__ void __launch_bounds__(kNaThreads) k_cfl_dt_final(const double* __restrict__ part, int nblk,
                                                              double* __restrict__ out) {
   __shared__ double sm[kNaThreads / 32];
+  umma::grid_wait();
   double m = kVlarge;
+#pragma unroll 4
   for (int b = threadIdx.x; b < nblk; b += blockDim.x) m = na_min(m, part[b]);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) m = na_min(m, __shfl_xor_sync(0xffffffffu, m, o));
@@ -177,8 +187,18 @@ extern "C" int storm_fvt_cfl_dt_noalloc(const double* d_h, const double* d_u, co
     }
   }
   const int nblk = (n + kNaThreads - 1) / kNaThreads;
-  k_cfl_dt_partials<<<nblk, kNaThreads, 0, s>>>(d_h, d_u, d_v, d_area, d_perim, n, cfl, h_dry, h_wet, part);
-  k_cfl_dt_final<<<1, kNaThreads, 0, s>>>(part, nblk, d_dt);
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(nblk);
+  cfg.blockDim = dim3(kNaThreads);
+  cfg.stream = s;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, k_cfl_dt_partials, d_h, d_u, d_v, d_area, d_perim, static_cast<int>(n), cfl, h_dry, h_wet, part);
+  cfg.gridDim = dim3(1);
+  cudaLaunchKernelEx(&cfg, k_cfl_dt_final, static_cast<const double*>(part), nblk, d_dt);
   e = cudaGetLastError();
   if (e != cudaSuccess)
     return set_error(STORM_ERR_CUDA, std::string("storm_fvt_cfl_dt_noalloc: launch: ") + cudaGetErrorString(e));
