@@ -290,12 +290,15 @@ int enqueue_step(StormFvtHandle* h, bool timing, size_t* fev_used, int only = -1
       }
       const bool forked = gG > 0 || d.nbdr > 0;
       if (d.ncv > 0) launch(STAGE_CULVERT, (d.ncv + 127) / 128, 128, 0, h->stream, s);
-      if (d.nbdr > 0) launch(STAGE_BC, d.nbdr, 128, h->bc_smem, h->side, s);
+      // one launch for both where the stage would wait for two (see k_bc_flux)
+      const bool bc_flux = d.bcf_off && gC <= h->n_sm && h->bc_smem <= 48 * 1024;
+      if (d.nbdr > 0 && !bc_flux) launch(STAGE_BC, d.nbdr, 128, h->bc_smem, h->side, s);
       if (gB > 0) {
         // the neighbours' face records (k_grad), the culverts
         CK(cudaEventRecord(h->eflux_ev[s], h->stream));
         CK(cudaStreamWaitEvent(h->side, h->eflux_ev[s], 0));
-        launch(STAGE_FLUX_BC, gF, kFluxThreads, 0, h->side, s);
+        if (bc_flux) launch(STAGE_BC_FLUX, d.nbdr, 128, h->bc_smem, h->side, s);
+        else launch(STAGE_FLUX_BC, gF, kFluxThreads, 0, h->side, s);
       }
       if (forked) CK(cudaEventRecord(h->join_ev[s], h->side));
       launch(STAGE_CELL, gC, bC, h->cell_smem, h->stream, s);
@@ -619,6 +622,23 @@ int upload(StormFvtHandle* h) {
     if (L.cell_sid[c] >= 0 && !common(c)) gen.push_back(c);
   size_t o_gen = cpy(gen, std::max<size_t>(gen.size(), 1));
   size_t o_bcl = cpy(L.bc_cells, std::max<size_t>(L.bc_cells.size(), 1));
+  // the same by open boundary, if each is on one (and every boundary's cells are among them)
+  std::vector<int32_t> bcf_off(1, 0), bcf_idx;
+  for (size_t b = 0; b < L.bdr_off.size(); b++) {
+    std::vector<int32_t> c(L.bce_cell.begin() + L.bdr_off[b], L.bce_cell.begin() + L.bdr_off[b] + L.bdr_cnt[b]);
+    std::sort(c.begin(), c.end());
+    c.erase(std::unique(c.begin(), c.end()), c.end());
+    for (int32_t x : c) {
+      const auto it = std::lower_bound(L.bc_cells.begin(), L.bc_cells.end(), x);
+      bcf_idx.push_back(it != L.bc_cells.end() && *it == x ? (int32_t)(it - L.bc_cells.begin()) : -1);
+    }
+    bcf_off.push_back((int32_t)bcf_idx.size());
+  }
+  std::vector<int32_t> once = bcf_idx;
+  std::sort(once.begin(), once.end());
+  bool bcf_ok = !once.empty() && once.size() == L.bc_cells.size();
+  for (size_t k = 0; bcf_ok && k < once.size(); k++) bcf_ok = once[k] == (int32_t)k;
+  size_t o_bfo = cpy(bcf_off, bcf_off.size()), o_bfi = cpy(bcf_idx, std::max<size_t>(bcf_idx.size(), 1));
   const bool rsavg = h->opt.rsavg_passes > 0;
   size_t o_rsc = cpy(L.rs_cells, std::max<size_t>(L.rs_cells.size(), 1));
   size_t o_phi = A.take(rsavg ? 8 * 3 * (size_t)T : 8), o_phi0 = A.take(rsavg ? 8 * 3 * (size_t)T : 8);
@@ -800,6 +820,8 @@ int upload(StormFvtHandle* h) {
     }
   }
   d.bc_cells = at<int32_t>(B, o_bcl);
+  d.bcf_off = bcf_ok ? at<int32_t>(B, o_bfo) : nullptr;
+  d.bcf_idx = at<int32_t>(B, o_bfi);
   {
     std::vector<CellCol> cols(9 * kCellCols);
     for (int s = 1; s <= K; s++)

@@ -169,6 +169,8 @@ struct Dev {
   const int32_t* gen_cells;
   int32_t nbc_cells;        // cells with an open-boundary face (finished after k_bc)
   const int32_t* bc_cells;
+  // the entries of bc_cells along each open boundary, where none is on two (k_bc_flux; else null)
+  const int32_t *bcf_off, *bcf_idx;
   int32_t nblk_red;
   Scalars* sc;              // [nscen]
 };
@@ -215,7 +217,7 @@ struct TileDev {
 };
 
 // One launch of a templated stage kernel (see launch_stage in fvt_kernels.cu).
-enum StageKernel { STAGE_GRAD, STAGE_BC, STAGE_CELL, STAGE_FLUX_BC, STAGE_FLUX_BC_TILE,
+enum StageKernel { STAGE_GRAD, STAGE_BC, STAGE_CELL, STAGE_FLUX_BC, STAGE_BC_FLUX, STAGE_FLUX_BC_TILE,
                    STAGE_UPDATE, STAGE_CULVERT, STAGE_GRAD_BC, STAGE_TILE, STAGE_PACK, STAGE_GRAD_GEN };
 // What a cell kernel does with phi: the RK update; phi itself for the residual smoothing;
 // the update and, in the last stage, the friction step and the iteration's reductions.
