@@ -47,10 +47,10 @@ from storm_b200 import scenarios  # noqa: E402
 
 METRIC = "cell-stage updates/s (FVT time step, 2M-triangle meander)"
 # DRAM bytes (read + write) per cell-stage of one iteration's kernels (every stage
-# kernel, k_fric and k_final), from one ncu capture of three whole iterations on the
+# kernel and k_final), from one ncu capture of three whole iterations on the
 # 500k-cell meander (dram__bytes_read.sum + dram__bytes_write.sum); traffic grows in
 # proportion to the cells, so it is scaled to the workload's mesh.
-NCU_DRAM_BYTES_PER_CELL_STAGE = {("meander", "phases"): 648.3}
+NCU_DRAM_BYTES_PER_CELL_STAGE = {("meander", "phases"): 596.0}
 UNIT = "cell-stage updates/s"
 PEAKS_FALLBACK = {"hbm_gbs": 6650.0, "source": "fallback"}
 
@@ -855,7 +855,7 @@ def main():
     roofline = {
         "bound": "hbm", "achieved": achieved, "peak": pk.get("hbm_gbs"), "unit": "GB/s",
         "frac": achieved / pk["hbm_gbs"], "traffic": traffic,
-        "kernel": f"one iteration (CUDA graph: {chain}, k_fric, k_final)",
+        "kernel": f"one iteration (CUDA graph: {chain}, k_final)",
         "algorithmic_bytes_per_launch": B * T * K_rk, "bytes_per_cell_stage": B, "peak_source": pk["source"],
         "traffic_source": "ncu dram__bytes_read+write of three iterations' kernels on the 500k-cell "
                           "meander, per cell-stage, scaled to this mesh" if traffic else None,
