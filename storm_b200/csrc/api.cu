@@ -291,7 +291,7 @@ int enqueue_step(StormFvtHandle* h, bool timing, size_t* fev_used, int only = -1
       const bool forked = gG > 0 || d.nbdr > 0;
       if (d.ncv > 0) launch(STAGE_CULVERT, (d.ncv + 127) / 128, 128, 0, h->stream, s);
       // one launch for both where the stage would wait for two (see k_bc_flux)
-      const bool bc_flux = d.bcf_off && gC <= h->n_sm && h->bc_smem <= 48 * 1024;
+      const bool bc_flux = d.bcf_off && gC <= h->n_sm && h->bc_smem + kBcStatic <= kDefaultSmem;
       if (d.nbdr > 0 && !bc_flux) launch(STAGE_BC, d.nbdr, 128, h->bc_smem, h->side, s);
       if (gB > 0) {
         // the neighbours' face records (k_grad), the culverts
@@ -403,7 +403,7 @@ int configure_tiles(StormFvtHandle* h) {
   t.nodes = h->fuse_nodes ? 1 : 0;
   const size_t smem = tile_smem_bytes(t, h->mixed);
   h->tile_smem = smem;
-  if (smem > 48 * 1024) set_tile_smem_limit((int)smem);
+  if (smem > kDefaultSmem) CK(set_tile_smem_limit((int)smem));
   int nsm = 0;
   CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, h->device));
   const int per_sm = std::max(1, tile_blocks_per_sm(h->mixed, smem));
@@ -757,7 +757,7 @@ int upload(StormFvtHandle* h) {
   d.bcpart = at<double>(B, o_bcp); d.ccol = at<CellCol>(B, o_ccol);
   CK(cudaDeviceGetAttribute(&h->n_sm, cudaDevAttrMultiProcessorCount, h->device));
   h->cell_smem = cell_smem_bytes(d, h->mixed);
-  if (h->cell_smem > 48 * 1024) set_cell_smem_limit((int)h->cell_smem);
+  if (h->cell_smem + kCellStatic > kDefaultSmem) CK(set_cell_smem_limit((int)h->cell_smem));
   d.nbc_cells = (int32_t)L.bc_cells.size();
   d.ngen = (int32_t)gen.size();
   d.gen_cells = at<int32_t>(B, o_gen);
@@ -880,7 +880,7 @@ int upload(StormFvtHandle* h) {
   const size_t cached = (size_t)maxcnt * 6 * sizeof(double) + (((size_t)2 * maxcnt + 7) & ~(size_t)7);
   d.bc_cache = cached <= 200 * 1024;
   h->bc_smem = d.bc_cache ? cached : plain;
-  if (h->bc_smem > 48 * 1024) set_bc_smem_limit((int)h->bc_smem);
+  if (h->bc_smem + kBcStatic > kDefaultSmem) CK(set_bc_smem_limit((int)h->bc_smem));
   return 0;
 }
 

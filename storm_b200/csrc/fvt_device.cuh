@@ -236,15 +236,19 @@ struct StageLaunch {
   Rec* qo;
   const TileDev* tiles;  // STAGE_TILE only
 };
+// A kernel that has not been given a higher limit may take 48 KB of shared memory in a
+// block, its static variables among them (in whole 128 bytes, the alignment of the dynamic
+// part): those of k_cell at most, and of the boundary kernels; k_tile has none.
+constexpr size_t kDefaultSmem = 48 * 1024, kCellStatic = 768, kBcStatic = 128;
 size_t tile_smem_bytes(const TileDev& t, bool mixed);
 int tile_blocks_per_sm(bool mixed, size_t smem);  // resident CTAs of k_tile per SM
-void set_tile_smem_limit(int bytes);
+cudaError_t set_tile_smem_limit(int bytes);
 size_t cell_smem_bytes(const Dev& d, bool mixed);  // k_cell's dynamic shared memory
-void set_cell_smem_limit(int bytes);
+cudaError_t set_cell_smem_limit(int bytes);
 // the columns of stage s in a mode
 void cell_columns(const Dev& d, const Geo<double>& Gd, const Geo<float>& Gf, bool mixed, int s, int mode, CellCol* out);
 void launch_stage(const StageLaunch& L, const Dev& d, const Geo<double>& Gd, const Geo<float>& Gf, bool mixed);
-void set_bc_smem_limit(int bytes);
+cudaError_t set_bc_smem_limit(int bytes);
 // Linked partitions: halo exchange of one level (+ up to two flag arrays), the shared
 // friction dt before k_fric, the shared dt / stop test after k_final.
 void launch_halo(const Dev& d, int level, uint8_t* f1, cudaStream_t st);

@@ -532,8 +532,8 @@ __device__ void time_bcs(const Dev& d, int sid, double time) {
 // the FP64 path keeps every operation rounded as written, the mixed path needs no
 // such order.  These are its entry points.
 int tile_blocks_per_sm_f32(size_t smem);
-void set_tile_smem_attr_f32(int bytes);
-void set_bc_smem_attr_f32(int bytes);
+cudaError_t set_tile_smem_attr_f32(int bytes);
+cudaError_t set_bc_smem_attr_f32(int bytes);
 void launch_stage_f32(const StageLaunch& L, const Dev& d, const Geo<float>& G);
 void launch_out_cell_f32(const Dev& d, const Geo<float>& G, const OutputArgs& a, int grid, cudaStream_t st);
 
@@ -1398,6 +1398,7 @@ __device__ __forceinline__ void boundary_fluxes(const Dev& d, const Geo<R>& G, c
   uint8_t* ok = (uint8_t*)(smb + 2 * cnt);
   __shared__ double s_atotal;
   __shared__ int s_done, s_null;
+  static_assert(sizeof(s_atotal) + sizeof(s_done) + sizeof(s_null) <= kBcStatic, "counted with the dynamic shared memory");
   const double h_dry = d.h_dry;
   // reconstructed edge states (the h/u/v + grad . rc of the boundary element)
   for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
@@ -2419,6 +2420,7 @@ __global__ void __launch_bounds__(kThreads, kThreads == 256 ? 4 : 1) k_cell(cons
   extern __shared__ __align__(128) unsigned char cell_smem[];
   __shared__ uint64_t bar;
   __shared__ double red[5 * (kThreads / 32)];
+  static_assert(sizeof(bar) + sizeof(red) <= kCellStatic, "counted with the dynamic shared memory");
   CellSmem<R>& S = *reinterpret_cast<CellSmem<R>*>(cell_smem);
   double* s_w = reinterpret_cast<double*>(cell_smem + sizeof(CellSmem<R>));  // [3][cnw_max]
   R* s_f = reinterpret_cast<R*>(s_w + 3 * d.cnw_max);                         // [3][cne_max]
@@ -2953,20 +2955,27 @@ int tile_blocks_per_sm(bool mixed, size_t smem) {
 // The dynamic shared-memory limit is a property of the kernel function (per device),
 // shared by every handle: it only ever grows, so a handle that needs less never
 // lowers it under another handle's launches.
-static int raise_smem_limit(int* per_dev, int bytes) {
+struct SmemLimit {
+  std::mutex mu;
+  int lim[64] = {0};
+};
+template <class F>
+static cudaError_t raise_smem_limit(SmemLimit& L, int bytes, F set) {
+  std::lock_guard<std::mutex> lock(L.mu);
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return bytes;
-  if (bytes > per_dev[dev]) per_dev[dev] = bytes;
-  return per_dev[dev];
+  if (cudaError_t e = cudaGetDevice(&dev)) return e;
+  if (dev < 64 && bytes <= L.lim[dev]) return cudaSuccess;
+  const cudaError_t e = set(bytes);
+  if (e == cudaSuccess && dev < 64) L.lim[dev] = bytes;
+  return e;
 }
 
-void set_tile_smem_limit(int bytes) {
-  static int lim[64] = {0};
-  static std::mutex mu;
-  std::lock_guard<std::mutex> lock(mu);
-  const int b = raise_smem_limit(lim, bytes);
-  cudaFuncSetAttribute(k_tile<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-  set_tile_smem_attr_f32(b);
+cudaError_t set_tile_smem_limit(int bytes) {
+  static SmemLimit L;
+  return raise_smem_limit(L, bytes, [](int b) {
+    const cudaError_t e = cudaFuncSetAttribute(k_tile<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+    return e ? e : set_tile_smem_attr_f32(b);
+  });
 }
 #endif  // !STORM_FVT_F32_TU
 
@@ -3609,13 +3618,12 @@ void launch_rsavg(const Dev& d, int off, int cnt, cudaStream_t st) {
   if (cnt > 0) k_rsavg<<<(cnt + 255) / 256, 256, 0, st>>>(d, off, cnt);
 }
 
-void set_bc_smem_limit(int bytes) {
-  static int lim[64] = {0};
-  static std::mutex mu;
-  std::lock_guard<std::mutex> lock(mu);
-  const int b = raise_smem_limit(lim, bytes);
-  cudaFuncSetAttribute(k_bc<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-  set_bc_smem_attr_f32(b);
+cudaError_t set_bc_smem_limit(int bytes) {
+  static SmemLimit L;
+  return raise_smem_limit(L, bytes, [](int b) {
+    const cudaError_t e = cudaFuncSetAttribute(k_bc<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+    return e ? e : set_bc_smem_attr_f32(b);
+  });
 }
 #endif  // !STORM_FVT_F32_TU
 
@@ -3624,15 +3632,18 @@ static size_t cell_smem_t(const Dev& d) {
   return sizeof(CellSmem<R>) + 24 * (size_t)d.cnw_max + 3 * sizeof(R) * (size_t)d.cne_max;
 }
 template <class R, int kThreads>
-static void set_cell_smem_n(int bytes) {
-  cudaFuncSetAttribute(k_cell<R, CELL_UPDATE, kThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  cudaFuncSetAttribute(k_cell<R, CELL_PHI, kThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-  cudaFuncSetAttribute(k_cell<R, CELL_FRIC, kThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+static cudaError_t set_cell_smem_n(int bytes) {
+  const void* kernels[] = {reinterpret_cast<const void*>(k_cell<R, CELL_UPDATE, kThreads>),
+                           reinterpret_cast<const void*>(k_cell<R, CELL_PHI, kThreads>),
+                           reinterpret_cast<const void*>(k_cell<R, CELL_FRIC, kThreads>)};
+  for (const void* k : kernels)
+    if (cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes)) return e;
+  return cudaSuccess;
 }
 template <class R>
-static void set_cell_smem_t(int bytes) {
-  set_cell_smem_n<R, 256>(bytes);
-  set_cell_smem_n<R, 512>(bytes);
+static cudaError_t set_cell_smem_t(int bytes) {
+  const cudaError_t e = set_cell_smem_n<R, 256>(bytes);
+  return e ? e : set_cell_smem_n<R, 512>(bytes);
 }
 template <class R>
 static void cell_columns_t(const Dev& d, const Geo<R>& G, int s, int mode, CellCol* out) {
@@ -3670,15 +3681,14 @@ void cell_columns(const Dev& d, const Geo<double>& Gd, const Geo<float>& Gf, boo
   else cell_columns_t<double>(d, Gd, s, mode, out);
 }
 size_t cell_smem_f32(const Dev& d);
-void set_cell_smem_f32(int bytes);
+cudaError_t set_cell_smem_f32(int bytes);
 size_t cell_smem_bytes(const Dev& d, bool mixed) { return mixed ? cell_smem_f32(d) : cell_smem_t<double>(d); }
-void set_cell_smem_limit(int bytes) {
-  static int lim[64] = {0};
-  static std::mutex mu;
-  std::lock_guard<std::mutex> lock(mu);
-  const int b = raise_smem_limit(lim, bytes);
-  set_cell_smem_t<double>(b);
-  set_cell_smem_f32(b);
+cudaError_t set_cell_smem_limit(int bytes) {
+  static SmemLimit L;
+  return raise_smem_limit(L, bytes, [](int b) {
+    const cudaError_t e = set_cell_smem_t<double>(b);
+    return e ? e : set_cell_smem_f32(b);
+  });
 }
 #endif
 
@@ -3687,17 +3697,17 @@ void cell_columns_f32(const Dev& d, const Geo<float>& G, int s, int mode, CellCo
   cell_columns_t<float>(d, G, s, mode, out);
 }
 size_t cell_smem_f32(const Dev& d) { return cell_smem_t<float>(d); }
-void set_cell_smem_f32(int bytes) { set_cell_smem_t<float>(bytes); }
+cudaError_t set_cell_smem_f32(int bytes) { return set_cell_smem_t<float>(bytes); }
 int tile_blocks_per_sm_f32(size_t smem) {
   int n = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_tile<float>, kTileThreads, smem);
   return n;
 }
-void set_tile_smem_attr_f32(int bytes) {
-  cudaFuncSetAttribute(k_tile<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+cudaError_t set_tile_smem_attr_f32(int bytes) {
+  return cudaFuncSetAttribute(k_tile<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
-void set_bc_smem_attr_f32(int bytes) {
-  cudaFuncSetAttribute(k_bc<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+cudaError_t set_bc_smem_attr_f32(int bytes) {
+  return cudaFuncSetAttribute(k_bc<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
 }
 void launch_stage_f32(const StageLaunch& L, const Dev& d, const Geo<float>& G) { launch_stage_t<float>(L, d, G); }
 void launch_out_cell_f32(const Dev& d, const Geo<float>& G, const OutputArgs& a, int grid, cudaStream_t st) {
