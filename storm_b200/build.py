@@ -18,7 +18,7 @@ CSRC = os.path.join(PKG, "csrc")
 LIB = os.path.join(PKG, "libstorm_fvt.so")
 SOURCES = ["api.cu", "fvt_kernels.cu", "layout.cpp", "tiles.cpp", "mesh_build.cpp", "noalloc.cu", "gnn_kernels.cu"]
 F32_SOURCE = "fvt_kernels_f32.cu"  # includes fvt_kernels.cu
-HEADERS = ["fvt_device.cuh", "storm_internal.h", "umma.cuh", os.path.join("..", "..", "include", "storm_fvt.h"),
+HEADERS = ["fvt_device.cuh", "quotient.cuh", "storm_internal.h", "umma.cuh", os.path.join("..", "..", "include", "storm_fvt.h"),
            os.path.join("..", "..", "include", "storm_gnn.h")]
 
 NVCC_FLAGS = [
