@@ -253,7 +253,10 @@ typedef struct StormFvtStepStats {
   double tmass;        /* SUM(h*area)                                              */
   double cqin3[STORM_MAX_BDR];
   double cqout3[STORM_MAX_BDR];
-  int32_t device_status; /* 0, or the device-side check code                      */
+  int32_t device_status; /* device-side checks since the state was set, 0 or a sum of
+                            1 non-finite depth or velocity, 2 HLL wave speeds out of
+                            order (flux_HLL.f90:88-91, not an error), 4 a kernel's copy
+                            did not arrive; 1 and 4 fail storm_fvt_step              */
   int32_t reserved[7];
 } StormFvtStepStats;
 

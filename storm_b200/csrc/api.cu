@@ -1154,9 +1154,8 @@ int storm_fvt_step(StormFvtHandle* h, int32_t nsteps, StormFvtStepStats* stats) 
   h->last_step_ms = ms;
   if (stats) fill_stats(h, h->sc_host[0], stats);
   for (int sI = 0; sI < h->nscen; sI++)
-    if (h->sc_host[sI].status & 1)
-      return set_error(STORM_ERR_DEVICE, "storm_fvt_step: non-finite depth or velocity in scenario " +
-                                             std::to_string(sI));
+    if (const char* what = status_failure(h->sc_host[sI].status))
+      return set_error(STORM_ERR_DEVICE, std::string("storm_fvt_step: ") + what + " in scenario " + std::to_string(sI));
   return STORM_OK;
 }
 
@@ -1540,9 +1539,12 @@ static int part_handle(StormFvtHandle* h, const char* who) {
   return 0;
 }
 
+// (A part's non-finite values reach the caller in its sums and device_status.)
 static int read_scalars(StormFvtHandle* h) {
   CK(cudaMemcpyAsync(h->sc_host, h->d.sc, sizeof(Scalars), cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
+  if (const int32_t lost = h->sc_host[0].status & DEV_COPY_LOST)
+    return set_error(STORM_ERR_DEVICE, std::string("storm_fvt_iter: ") + status_failure(lost));
   return 0;
 }
 

@@ -47,7 +47,7 @@ struct WallRec {  // a wall edge with a flux, sorted by cell
 struct Scalars {
   int32_t iter;       // iterations completed
   int32_t converged;  // steady: rmax < rstop reached (solverFVT.f90:431)
-  int32_t status;     // bit 0: non-finite state; bit 1: HLL wave-speed inversion
+  int32_t status;     // DevStatus bits since the state was set
   int32_t pad;
   double delt;        // dt of the current iteration (unsteady), or the steady
                       // last-element local dt carried into ttime (solverFVT.f90:155)

@@ -1079,7 +1079,7 @@ __global__ void __launch_bounds__(256, 3) k_grad(const __grid_constant__ Dev d, 
   if (!kGen) {
     __syncwarp();
     if (!umma::mbar_wait(&bars[wp], 0)) {  // cannot happen: a copy within this GPU
-      if (live) atomicOr(&d.sc[cell_scenario(d, c)].status, 4);
+      if (live) atomicOr(&d.sc[cell_scenario(d, c)].status, DEV_COPY_LOST);
       umma::mbar_wait(&bars[wp], 0);
       return;
     }
@@ -2180,7 +2180,7 @@ __device__ __forceinline__ FricTerms fric_cell(const Dev& d, int sid, int c, con
   t.rm = dry2 ? kZero : phimax;
   const double wc1 = dry1 ? kZero : sqrt(kG * h);
   t.dt = d.cfl * area / ((um1 + wc1 + SMALL_F) * perim);
-  if (!isfinite(h) || !isfinite(u) || !isfinite(v)) atomicOr(&d.sc[sid].status, 1);
+  if (!isfinite(h) || !isfinite(u) || !isfinite(v)) atomicOr(&d.sc[sid].status, DEV_NONFINITE);
   return t;
 }
 
@@ -2307,7 +2307,7 @@ __global__ void __launch_bounds__(kThreads, kThreads == 256 ? 4 : 1) k_cell(cons
     s_f[le] = f[0];
     s_f[nem + le] = f[1];
     s_f[2 * nem + le] = f[2];
-    if (bad) atomicOr(&d.sc[sid].status, 2);
+    if (bad) atomicOr(&d.sc[sid].status, DEV_HLL_STOP);
   }
   const int w0 = i1.x, nw = i1.y, nwm = d.cnw_max;
   for (int w = tid; w < nw; w += kThreads) {
@@ -2319,7 +2319,7 @@ __global__ void __launch_bounds__(kThreads, kThreads == 256 ? 4 : 1) k_cell(cons
   }
   __syncthreads();
   if (!umma::mbar_wait(&bar, 0)) {  // cannot happen: copies within this GPU
-    if (tid == 0) atomicOr(&d.sc[sid].status, 4);
+    atomicOr(&d.sc[sid].status, DEV_COPY_LOST);
     umma::mbar_wait(&bar, 0);
     return;
   }
@@ -2762,7 +2762,7 @@ __global__ void __launch_bounds__(kTileThreads, 3)
           G.efx[2 * d.ne + e] = f[2];
         }
       }
-      if (bad) atomicOr(&d.sc[d.edge_sid[e]].status, 2);
+      if (bad) atomicOr(&d.sc[d.edge_sid[e]].status, DEV_HLL_STOP);
     }
     s_eok[le] = ok;
   }

@@ -13,6 +13,19 @@ namespace storm {
 int set_error(int code, const std::string& msg);
 void clear_error();
 
+// ---- device status of a scenario (StormFvtStepStats::device_status) ---------
+enum DevStatus : int32_t {
+  DEV_NONFINITE = 1,  // a depth or velocity is not finite
+  DEV_HLL_STOP = 2,   // wave speeds out of order (flux_HLL.f90:88-91); the run goes on
+  DEV_COPY_LOST = 4   // a kernel gave up waiting for a bulk copy and left cells as they were
+};
+// What makes a state unusable, or nullptr.
+inline const char* status_failure(int32_t status) {
+  if (status & DEV_COPY_LOST) return "a copy to shared memory did not arrive, the state is not valid";
+  if (status & DEV_NONFINITE) return "non-finite depth or velocity";
+  return nullptr;
+}
+
 // ---- face kinds of the per-cell face table ---------------------------------
 enum FaceKind : uint8_t {
   FACE_NONE = 0,   // boundary edge with no flux routine (e.g. between two BC strings)
