@@ -2102,12 +2102,13 @@ __device__ __forceinline__ void rk_update(const Dev& d, int s, int c, const Rec&
 
 // The friction step of a cell after the last stage and its terms of the iteration's
 // reductions (solverFVT.f90:335-386, 407-445): find_dry_cells, fric_terms_impl, the
-// numerical valve, the copy to RK level 0.
+// numerical valve, the copy to RK level 0.  halo: a copy of another part's cell, whose
+// owner counts it and reports its values.
 struct FricTerms {
   double st = kZero, sb = kZero, tm = kZero, rm = kZero, dt = kVlarge;
 };
 __device__ __forceinline__ FricTerms fric_cell(const Dev& d, int sid, int c, const CellOut& in, double z, double h0,
-                                               double phimax, double cd, double area, double perim) {
+                                               double phimax, double cd, double area, double perim, bool halo = false) {
   const int T = d.T;
   const double h = in.h;
   double u = in.u, v = in.v, ru = in.ru, rv = in.rv;
@@ -2174,6 +2175,7 @@ __device__ __forceinline__ FricTerms fric_cell(const Dev& d, int sid, int c, con
   double um1;
   const bool dry1 = dry_flag(h, u, v, d.h_dry, d.h_wet, &um1);
   FricTerms t;
+  if (halo) return t;
   t.st = (h - h0) * (h - h0);
   t.sb = h0 * h0;
   t.tm = h * area;
@@ -2848,8 +2850,7 @@ __global__ void __launch_bounds__(kRedThreads) k_fric(Dev d, const Rec* src) {
     const int qk = K * T + c;
     const Rec in = ld_rec(src + c);
     ft = fric_cell(d, sid, c, CellOut{in.h, in.u, in.v, d.rku[qk], d.rkv[qk]}, in.z, d.rkh[c], d.phimax[c], d.cd[c],
-                   d.area[c], d.perim[c]);
-    if (kHalo && d.halo_mask[c]) ft = FricTerms();  // a halo copy: its owner counts it
+                   d.area[c], d.perim[c], kHalo && d.halo_mask[c]);
     if (d.forder[c] & kOrderHasBc) {  // summed by k_final, as when k_flux_bc did the friction step
       int lo = 0, hi = d.nbc_cells;
       while (lo < hi) {
