@@ -32,7 +32,8 @@ extern "C" {
 /* One 64- or 128-wide segment of an MLP input row. */
 typedef struct StormGnnSeg {
   const void* src;       /* bf16 [*][width]                                         */
-  const int32_t* idx;    /* row map (NULL: identity); a negative entry reads zeros  */
+  const int32_t* idx;    /* row map (NULL: identity); a negative entry reads zeros;
+                            not read with agg                                      */
   int32_t width;         /* 64 or 128                                                */
   int32_t agg;           /* 1: row r is the sum of src rows r + k*agg_stride, k<3,
                             whose nbr entry is >= 0 (message aggregation)           */

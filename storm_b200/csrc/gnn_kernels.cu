@@ -1487,7 +1487,7 @@ int check_shape(int rows, int nseg, int k_in, int n_out, const int* widths) {
 Seg to_seg(const StormGnnSeg& s) {
   Seg o;
   o.src = static_cast<const bf16*>(s.src);
-  o.idx = s.idx;
+  o.idx = s.agg ? nullptr : s.idx;  // an aggregated segment has no row map: the kernels ask for its entries early
   o.width = s.width;
   o.agg = s.agg;
   o.agg_stride = s.agg_stride;
