@@ -474,6 +474,31 @@ int upload_tiles(StormFvtHandle* h) {
   return configure_tiles(h);
 }
 
+// fn(i0, i1) over [0, n) in contiguous chunks on up to 8 host threads (one below
+// 256k items): the state permutations of large meshes are memory-latency bound.
+template <class F>
+void par_chunks(size_t n, F fn) {
+  const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
+  const size_t nt = n < (size_t)1 << 18 ? 1 : std::min<size_t>(std::min(8u, hw), n >> 16);
+  if (nt <= 1) {
+    fn((size_t)0, n);
+    return;
+  }
+  std::vector<std::thread> th;
+  const size_t step = (n + nt - 1) / nt;
+  size_t done = step;  // chunks [step, done) are covered by started threads
+  try {
+    for (size_t t = 1; t < nt; t++) {
+      th.emplace_back(fn, std::min(n, t * step), std::min(n, (t + 1) * step));
+      done = std::min(n, (t + 1) * step);
+    }
+  } catch (const std::system_error&) {  // no more threads: the caller's thread does the rest
+  }
+  fn((size_t)0, std::min(n, step));
+  if (done < n) fn(done, n);
+  for (auto& x : th) x.join();
+}
+
 int upload(StormFvtHandle* h) {
   HostLayout& L = h->L;
   const int T = L.T, N = L.N, K = h->opt.rkorder;
@@ -495,7 +520,7 @@ int upload(StormFvtHandle* h) {
     return o;
   };
   // constant mesh data
-  size_t o_area = cpy(L.area, T), o_perim = cpy(L.perim, T), o_xc = cpy(L.xc, T), o_yc = cpy(L.yc, T);
+  size_t o_area = cpy(L.area, T), o_perim = cpy(L.perim, T);
   size_t o_z = cpy(L.z, T), o_dzx = cpy(L.delz_x, T), o_dzy = cpy(L.delz_y, T), o_zmax = cpy(L.zmax, T);
   size_t o_cd = cpy(L.cd, T), o_la = cpy(L.lsq_a, T), o_lb = cpy(L.lsq_b, T), o_lc = cpy(L.lsq_c, T);
   size_t o_ld = cpy(L.lsq_det, T);
@@ -519,12 +544,14 @@ int upload(StormFvtHandle* h) {
   // face kinds and references in summation order (static; see Dev::fko)
   std::vector<uint16_t> fko(T, 0);
   std::vector<int32_t> frefo(T3, 0);
-  for (size_t c = 0; c < (size_t)T; c++)
-    for (int t = 0; t < 3; t++) {
-      const int j = (L.forder[c] >> (2 * t)) & 3;
-      fko[c] |= (uint16_t)((L.fkind[(size_t)j * T + c] & 7) << (3 * t));
-      frefo[(size_t)t * T + c] = L.fref[(size_t)j * T + c];
-    }
+  par_chunks((size_t)T, [&](size_t c0, size_t c1) {
+    for (size_t c = c0; c < c1; c++)
+      for (int t = 0; t < 3; t++) {
+        const int j = (L.forder[c] >> (2 * t)) & 3;
+        fko[c] |= (uint16_t)((L.fkind[(size_t)j * T + c] & 7) << (3 * t));
+        frefo[(size_t)t * T + c] = L.fref[(size_t)j * T + c];
+      }
+  });
   // stage-boundary slot of a node, -2 for the other ends of wall edges (whose depth the
   // wall fluxes read), -1 for the rest
   std::vector<int16_t> node_code = L.node_hbc;
@@ -533,11 +560,13 @@ int upload(StormFvtHandle* h) {
       if (node_code[n] == -1) node_code[n] = -2;
   // face records (see Dev::fs): interior edges' two sides, and walls where they slip
   std::vector<int32_t> fpos(T3, -1);
-  for (size_t q = 0; q < T3; q++) {
-    const int kind = L.fkind[q] & 7;
-    if (kind == FACE_LEFT || kind == FACE_RIGHT) fpos[q] = 2 * L.fref[q] + (kind == FACE_RIGHT);
-    else if (kind == FACE_WALL && h->opt.btype == 1) fpos[q] = 2 * L.ne + L.fref[q];
-  }
+  par_chunks(T3, [&](size_t q0, size_t q1) {
+    for (size_t q = q0; q < q1; q++) {
+      const int kind = L.fkind[q] & 7;
+      if (kind == FACE_LEFT || kind == FACE_RIGHT) fpos[q] = 2 * L.fref[q] + (kind == FACE_RIGHT);
+      else if (kind == FACE_WALL && h->opt.btype == 1) fpos[q] = 2 * L.ne + L.fref[q];
+    }
+  });
   const size_t nrec = 2 * (size_t)L.ne + (h->opt.btype == 1 ? (size_t)L.nwall : 0);
   // k_cell's work lists (edges are sorted by their smaller slot), and per cell its faces'
   // places in them
@@ -574,29 +603,31 @@ int upload(StormFvtHandle* h) {
   std::vector<uint32_t> fdesc(T, 0);
   std::vector<uint16_t> lfe(T3, 0);
   std::vector<float> rad(T, 0.0f);
-  for (size_t c = 0; c < (size_t)T; c++) {
-    fdesc[c] = L.forder[c] | ((uint32_t)fko[c] << 8) | (L.cell_sid[c] >= 0 ? kDescReal : 0);
-    const CellTile& k = ct[c / kRed];
-    double r = 0.0;
-    for (int t = 0; t < 3; t++) {
-      const size_t q = (size_t)((L.forder[c] >> (2 * t)) & 3) * T + c;
-      const int kind = L.fkind[q] & 7;
-      const int32_t e = L.fref[q];
-      if (kind == FACE_LEFT || kind == FACE_RIGHT) {
-        if (e >= k.er0 && e < k.er0 + k.nr) {
-          lfe[(size_t)t * T + c] = (uint16_t)(e - k.er0);
-        } else {
-          const auto b0 = cbe.begin() + k.boff, b1 = b0 + k.nb;  // increasing
-          lfe[(size_t)t * T + c] = (uint16_t)(k.nr + (std::lower_bound(b0, b1, e) - b0));
+  par_chunks((size_t)T, [&](size_t c0, size_t c1) {
+    for (size_t c = c0; c < c1; c++) {
+      fdesc[c] = L.forder[c] | ((uint32_t)fko[c] << 8) | (L.cell_sid[c] >= 0 ? kDescReal : 0);
+      const CellTile& k = ct[c / kRed];
+      double r = 0.0;
+      for (int t = 0; t < 3; t++) {
+        const size_t q = (size_t)((L.forder[c] >> (2 * t)) & 3) * T + c;
+        const int kind = L.fkind[q] & 7;
+        const int32_t e = L.fref[q];
+        if (kind == FACE_LEFT || kind == FACE_RIGHT) {
+          if (e >= k.er0 && e < k.er0 + k.nr) {
+            lfe[(size_t)t * T + c] = (uint16_t)(e - k.er0);
+          } else {
+            const auto b0 = cbe.begin() + k.boff, b1 = b0 + k.nb;  // increasing
+            lfe[(size_t)t * T + c] = (uint16_t)(k.nr + (std::lower_bound(b0, b1, e) - b0));
+          }
+        } else if (kind == FACE_WALL) {
+          lfe[(size_t)t * T + c] = (uint16_t)wall_at[e];
         }
-      } else if (kind == FACE_WALL) {
-        lfe[(size_t)t * T + c] = (uint16_t)wall_at[e];
+        const int32_t v = L.vert[(size_t)t * T + c];
+        r = std::max({r, std::fabs(L.node_x[v] - L.xc[c]), std::fabs(L.node_y[v] - L.yc[c])});
       }
-      const int32_t v = L.vert[(size_t)t * T + c];
-      r = std::max({r, std::fabs(L.node_x[v] - L.xc[c]), std::fabs(L.node_y[v] - L.yc[c])});
+      rad[c] = std::nextafter((float)r, INFINITY);
     }
-    rad[c] = std::nextafter((float)r, INFINITY);
-  }
+  });
   size_t o_ct = cpy(ct, nct), o_cbe = cpy(cbe, std::max<size_t>(cbe.size(), 1));
   size_t o_walls = cpy(walls, std::max<size_t>(walls.size(), 1)), o_fdesc = cpy(fdesc, T), o_lfe = cpy(lfe, T3);
   size_t o_rad = cpy(rad, T), o_ccol = A.take(9 * kCellCols * sizeof(CellCol)), o_bcp = A.take(8 * 5 * std::max<size_t>(L.bc_cells.size(), 1));
@@ -605,7 +636,7 @@ int upload(StormFvtHandle* h) {
   size_t o_fko = cpy(fko, T), o_frefo = cpy(frefo, T3);
   size_t o_vert = cpy(L.vert, T3), o_t3 = cpy(L.t2t3, T3), o_fref = cpy(L.fref, T3), o_sid = cpy(L.st_id, TK);
   size_t o_rcx = cpy(L.rc_x, T3), o_rcy = cpy(L.rc_y, T3), o_fnx = cpy(L.fnx, T3), o_fny = cpy(L.fny, T3);
-  size_t o_flen = cpy(L.flen, T3), o_fz0 = cpy(L.fz0, T3);
+  size_t o_flen = cpy(L.flen, T3);
   size_t o_sw = cpy(L.st_w, TK), o_sdx = cpy(L.st_dx, TK), o_sdy = cpy(L.st_dy, TK);
   size_t o_wp1 = cpy(L.wall_p1, nwall), o_wp2 = cpy(L.wall_p2, nwall);
   size_t o_zv = cpy(L.zvtx, N), o_nx = cpy(L.node_x, N), o_ny = cpy(L.node_y, N), o_n2w = cpy(L.n2t_w, nnz);
@@ -650,11 +681,13 @@ int upload(StormFvtHandle* h) {
     if ((L.forder[L.eL[e]] & kOrderHasBc) || (L.forder[L.eR[e]] & kOrderHasBc)) eslot[e] |= kEdgeExport;
   // vertex minus centroid of each cell vertex (the differences bed_slope_STD forms)
   std::vector<double> vox(T3), voy(T3);
-  for (size_t q = 0; q < T3; q++) {
-    const int32_t c = (int32_t)(q % (size_t)T), v = L.vert[q];
-    vox[q] = L.node_x[v] - L.xc[c];
-    voy[q] = L.node_y[v] - L.yc[c];
-  }
+  par_chunks(T3, [&](size_t q0, size_t q1) {
+    for (size_t q = q0; q < q1; q++) {
+      const int32_t c = (int32_t)(q % (size_t)T), v = L.vert[q];
+      vox[q] = L.node_x[v] - L.xc[c];
+      voy[q] = L.node_y[v] - L.yc[c];
+    }
+  });
   size_t o_vox = cpy(vox, T3), o_voy = cpy(voy, T3);
   size_t o_eL = cpy(L.eL, ne1), o_eR = cpy(L.eR, ne1), o_es = cpy(eslot, ne1);
   size_t o_enx = cpy(L.enx, ne1), o_eny = cpy(L.eny, ne1), o_el = cpy(L.elen, ne1), o_ez0 = cpy(L.ez0, ne1);
@@ -697,8 +730,8 @@ int upload(StormFvtHandle* h) {
     d.alpha[3][0] = 1.0 / 3.0; d.alpha[3][1] = 0.0; d.alpha[3][2] = 2.0 / 3.0;
     d.beta[1] = 1.0; d.beta[2] = 0.250; d.beta[3] = 2.0 / 3.0;
   }
-  d.area = at<double>(B, o_area); d.perim = at<double>(B, o_perim); d.xc = at<double>(B, o_xc);
-  d.yc = at<double>(B, o_yc); d.z = at<double>(B, o_z); d.delz_x = at<double>(B, o_dzx);
+  d.area = at<double>(B, o_area); d.perim = at<double>(B, o_perim);
+  d.z = at<double>(B, o_z); d.delz_x = at<double>(B, o_dzx);
   d.delz_y = at<double>(B, o_dzy); d.zmax = at<double>(B, o_zmax); d.cd = at<double>(B, o_cd);
   d.lsq_a = at<double>(B, o_la); d.lsq_b = at<double>(B, o_lb); d.lsq_c = at<double>(B, o_lc);
   d.lsq_det = at<double>(B, o_ld);
@@ -715,7 +748,7 @@ int upload(StormFvtHandle* h) {
   d.fko = at<uint16_t>(B, o_fko); d.frefo = at<int32_t>(B, o_frefo);
   d.st_id = at<int32_t>(B, o_sid);
   d.rc_x = at<double>(B, o_rcx); d.rc_y = at<double>(B, o_rcy); d.fnx = at<double>(B, o_fnx);
-  d.fny = at<double>(B, o_fny); d.flen = at<double>(B, o_flen); d.fz0 = at<double>(B, o_fz0);
+  d.fny = at<double>(B, o_fny); d.flen = at<double>(B, o_flen);
   d.st_w = at<double>(B, o_sw); d.st_dx = at<double>(B, o_sdx); d.st_dy = at<double>(B, o_sdy);
   d.wall_p1 = at<int32_t>(B, o_wp1); d.wall_p2 = at<int32_t>(B, o_wp2);
   d.zvtx = at<double>(B, o_zv); d.node_x = at<double>(B, o_nx); d.node_y = at<double>(B, o_ny);
@@ -882,31 +915,6 @@ int upload(StormFvtHandle* h) {
   h->bc_smem = d.bc_cache ? cached : plain;
   if (h->bc_smem + kBcStatic > kDefaultSmem) CK(set_bc_smem_limit((int)h->bc_smem));
   return 0;
-}
-
-// fn(i0, i1) over [0, n) in contiguous chunks on up to 8 host threads (one below
-// 256k items): the state permutations of large meshes are memory-latency bound.
-template <class F>
-void par_chunks(size_t n, F fn) {
-  const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
-  const size_t nt = n < (size_t)1 << 18 ? 1 : std::min<size_t>(std::min(8u, hw), n >> 16);
-  if (nt <= 1) {
-    fn((size_t)0, n);
-    return;
-  }
-  std::vector<std::thread> th;
-  const size_t step = (n + nt - 1) / nt;
-  size_t done = step;  // chunks [step, done) are covered by started threads
-  try {
-    for (size_t t = 1; t < nt; t++) {
-      th.emplace_back(fn, std::min(n, t * step), std::min(n, (t + 1) * step));
-      done = std::min(n, (t + 1) * step);
-    }
-  } catch (const std::system_error&) {  // no more threads: the caller's thread does the rest
-  }
-  fn((size_t)0, std::min(n, step));
-  if (done < n) fn(done, n);
-  for (auto& x : th) x.join();
 }
 
 // Pinned host staging of at least n doubles for the state transfers (page-locked

@@ -80,7 +80,7 @@ struct Dev {
   double h_dry, h_wet, cfl, vceiling, visc, rstop;
   double alpha[4][4], beta[4];
   // cells
-  const double *area, *perim, *xc, *yc, *z, *delz_x, *delz_y, *zmax, *cd;
+  const double *area, *perim, *z, *delz_x, *delz_y, *zmax, *cd;
   const double *vox, *voy;  // [3][T] vertex minus centroid of each cell vertex (bed_slope_STD)
   const double *wcoef1, *wcoef2;  // wind stress terms per cell (null: no wind)
   // linked partitions of one mesh: halo cell slots and their owners' slots, the halo
@@ -101,7 +101,7 @@ struct Dev {
   // each, and references ([3][T]) of the t-th face added
   const uint16_t* fko;
   const int32_t* frefo;
-  const double *rc_x, *rc_y, *fnx, *fny, *flen, *fz0, *st_w, *st_dx, *st_dy;
+  const double *rc_x, *rc_y, *fnx, *fny, *flen, *st_w, *st_dx, *st_dy;
   const int32_t *wall_p1, *wall_p2;
   // interior edges
   int32_t ne;

@@ -7,8 +7,8 @@
 // once before its time loop, with the same expressions:
 //   delz      bed_slope_VTX.f90:22-38 (called at solverFVT.f90:93)
 //   zmax      zvtx(csortedz(i)%p(3)) read by hgradfix2.f90:50
-//   fz0       half*(zvtx(p1)+zvtx(p2)) of invisc_fluxes.f90:89, inflowH.f90:53,
-//             outflowbyH.f90:67
+//   ez0       half*(zvtx(p1)+zvtx(p2)) of invisc_fluxes.f90:89 (bce_zmid: inflowH.f90:53,
+//             outflowbyH.f90:67)
 //   fnx/fny   edges(k)%normal flipped by invert_edge_dirs when grid(i)%edge(m) < 0
 // The per-cell visiting order of faces reproduces the order in which
 // invisc_fluxes.f90 adds edge contributions to phi(i,:) (interior edges in
@@ -338,7 +338,7 @@ int build_layout(const StormFvtMesh& m, const StormFvtOptions& opt, HostLayout& 
   L.vert.resize(3 * (size_t)T); L.t2t3.resize(3 * (size_t)T); L.fref.assign(3 * (size_t)T, 0);
   L.rc_x.resize(3 * (size_t)T); L.rc_y.resize(3 * (size_t)T);
   L.fnx.assign(3 * (size_t)T, 0.0); L.fny.assign(3 * (size_t)T, 0.0);
-  L.flen.assign(3 * (size_t)T, 0.0); L.fz0.assign(3 * (size_t)T, 0.0);
+  L.flen.assign(3 * (size_t)T, 0.0);
   L.fkind.assign(3 * (size_t)T, FACE_NONE);
   int32_t kst = 0;
   for (int32_t i = 0; i < T; i++) kst = std::max(kst, m.t2t[i]);
@@ -429,7 +429,6 @@ int build_layout(const StormFvtMesh& m, const StormFvtOptions& opt, HostLayout& 
         if (mo < 1) return set_error(STORM_ERR_MESH, "storm_fvt_create: edge not in its element");
         L.fkind[q] = (uint8_t)((e1 == i1 ? FACE_LEFT : FACE_RIGHT) | (face_slot(other, mo) << 4));
         L.fref[q] = ie_of[k];  // the interior-edge record holding this face's flux
-        L.fz0[q] = kHalf * (m.zvtx[EP(k, 1) - 1] + m.zvtx[EP(k, 2) - 1]);
         key[sj] = (int64_t)k;
       } else {
         if (GE(i1, j) < 0) {
@@ -593,7 +592,7 @@ void merge_layouts(const std::vector<HostLayout>& parts, int block, HostLayout& 
   for (const HostLayout& P : parts) M.lsq_derived = M.lsq_derived && P.lsq_derived;
   M.vert.assign(T3, 0); M.t2t3.assign(T3, -1); M.fref.assign(T3, 0); M.fkind.assign(T3, FACE_NONE);
   M.rc_x.assign(T3, 0.0); M.rc_y.assign(T3, 0.0); M.fnx.assign(T3, 0.0); M.fny.assign(T3, 0.0);
-  M.flen.assign(T3, 0.0); M.fz0.assign(T3, 0.0);
+  M.flen.assign(T3, 0.0);
   M.st_id.assign((size_t)kst * T, 0); M.st_w.assign((size_t)kst * T, 0.0);
   M.st_dx.assign((size_t)kst * T, 0.0); M.st_dy.assign((size_t)kst * T, 0.0);
   bool any_wind = false;
@@ -626,7 +625,7 @@ void merge_layouts(const std::vector<HostLayout>& parts, int block, HostLayout& 
         M.fref[qg] = r;
         M.fkind[qg] = P.fkind[q];
         M.rc_x[qg] = P.rc_x[q]; M.rc_y[qg] = P.rc_y[q]; M.fnx[qg] = P.fnx[q]; M.fny[qg] = P.fny[q];
-        M.flen[qg] = P.flen[q]; M.fz0[qg] = P.fz0[q];
+        M.flen[qg] = P.flen[q];
       }
       for (int k = 0; k < P.kst; k++) {
         const size_t q = (size_t)k * P.T + c, qg = (size_t)k * T + g;

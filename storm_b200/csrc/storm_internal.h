@@ -78,7 +78,7 @@ struct HostLayout {
   std::vector<int32_t> rs_cells, rs_off;  // cells by colour of the t2t stencil (new ids), CSR
   // [3][T]
   std::vector<int32_t> vert, t2t3, fref;
-  std::vector<double> rc_x, rc_y, fnx, fny, flen, fz0;
+  std::vector<double> rc_x, rc_y, fnx, fny, flen;
   std::vector<uint8_t> fkind;
   // stencil [kst][T]
   std::vector<int32_t> st_id;
