@@ -492,7 +492,7 @@ void par_chunks(size_t n, F fn) {
       th.emplace_back(fn, std::min(n, t * step), std::min(n, (t + 1) * step));
       done = std::min(n, (t + 1) * step);
     }
-  } catch (const std::system_error&) {  // no more threads: the caller's thread does the rest
+  } catch (const std::exception&) {  // no more threads (or memory): the caller's thread does the rest
   }
   fn((size_t)0, std::min(n, step));
   if (done < n) fn(done, n);
@@ -1025,7 +1025,12 @@ int storm_fvt_create_batch(const StormFvtMesh* const* meshes, int32_t n, const S
     release(h);
     return set_error(STORM_ERR_CUDA, std::string("storm_fvt_create: ") + cudaGetErrorString(e));
   }
-  if ((rc = upload(h)) || (rc = capture_graph(h))) {
+  try {  // the device tables are made in host vectors first
+    if (!(rc = upload(h))) rc = capture_graph(h);
+  } catch (const std::bad_alloc&) {
+    rc = set_error(STORM_ERR_NOMEM, "storm_fvt_create: host out of memory");
+  }
+  if (rc) {
     std::string msg = g_err;
     release(h);
     return set_error(rc, msg);
