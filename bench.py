@@ -835,7 +835,7 @@ def main():
     solver.step(kt_steps)
     kt = solver.kernel_times()
     solver.set_kernel_timing(False)
-    stage_ms = sum(kt[k][0] for k in ("node", "grad", "bc", "eflux", "flux", "tile"))
+    stage_ms = sum(kt[k][0] for k in ("node", "grad", "bc", "flux", "tile"))
     B = scenarios.algorithmic_bytes_per_cell_stage(T, E, N)
     pk = peaks()
     # The launch unit is one graph replay = one iteration (K stages of every kernel,

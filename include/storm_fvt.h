@@ -352,8 +352,8 @@ STORM_FVT_API int storm_fvt_kernel_times(const StormFvtHandle* hd, double* ms, i
  * candidate block size of the node and gradient kernels on this handle's meshes
  * (per-kernel CUDA events) and keeps the fastest of each; re-captures the iteration
  * graph and restores the state it started from.  `chosen` (may be NULL) receives four
- * sizes: node, gradient, and twice the cell slots of a block of the cell kernel;
- * storm_fvt_stage_path reports the path. */
+ * sizes: the node and gradient kernels' threads, and twice the 256 cell slots of a block
+ * of the cell kernel (which is not tuned); storm_fvt_stage_path reports the path. */
 STORM_FVT_API int storm_fvt_autotune(StormFvtHandle* hd, int32_t iters, int32_t* chosen);
 
 /* Stage kernels of the captured iteration.  No counterpart in the reference (it

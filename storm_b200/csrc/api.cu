@@ -71,9 +71,8 @@ struct StormFvtHandle {
   std::vector<int> fev_class;    // kernel class of each pair
   double kt_ms[8] = {0};         // per-class totals of the last timed call
   int64_t kt_n[8] = {0};
-  // block sizes of the stage kernels (storm_fvt_autotune picks them)
-  // block sizes of the node, gradient, edge-flux and cell kernels: the autotuner's
-  // choice on the 2M meander (FP64; the mixed path takes 128 for the edge fluxes)
+  // block sizes of k_node and k_grad (storm_fvt_autotune picks them; these are its choice
+  // on the two-million-cell meander)
   int bs_node = 128, bs_grad = 64;
   size_t cell_smem = 0;  // k_cell's dynamic shared memory
   int n_sm = 148;
@@ -155,7 +154,7 @@ T* at(void* base, size_t off) {
 }
 
 // Kernel classes of the per-kernel timing mode.
-enum { KT_NODE = 0, KT_GRAD, KT_BC, KT_FLUX, KT_FRIC, KT_FINAL, KT_EFLUX, KT_TILE, KT_COUNT };
+enum { KT_NODE = 0, KT_GRAD, KT_BC, KT_FLUX, KT_FRIC, KT_FINAL, KT_UNUSED, KT_TILE, KT_COUNT };
 static_assert(KT_COUNT <= 8, "per-class timing arrays hold 8 classes");
 
 constexpr int kTileCellsHost = 256;   // cell slots per tile of k_tile
@@ -1507,7 +1506,7 @@ int storm_fvt_autotune(StormFvtHandle* h, int32_t iters, int32_t* chosen) {
   if (chosen) {
     chosen[0] = h->bs_node;
     chosen[1] = h->bs_grad;
-    chosen[2] = chosen[3] = kRed;  // k_cell: edge fluxes and cell update, one shape
+    chosen[2] = chosen[3] = kRed;  // cell slots of a k_cell block, not tuned
   }
   // re-capture the iteration graph with the chosen shapes
   if (h->exec) cudaGraphExecDestroy(h->exec);

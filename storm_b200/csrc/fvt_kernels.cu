@@ -320,36 +320,6 @@ __device__ __forceinline__ void flux_rusanov(R nx, R ny, R hleft, R uleft, R vle
 
 // Block-level reductions in a fixed order (warp xor-shuffle tree, then warps in order).
 template <int NT>
-__device__ __forceinline__ double block_sum(double x, double* sm) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) x = x + __shfl_xor_sync(0xffffffffu, x, o);
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  __syncthreads();
-  if (l == 0) sm[w] = x;
-  __syncthreads();
-  double r = kZero;
-  if (threadIdx.x == 0) {
-    r = sm[0];
-    for (int i = 1; i < NT / 32; i++) r = r + sm[i];
-  }
-  return r;  // valid on thread 0
-}
-template <int NT>
-__device__ __forceinline__ double block_max(double x, double* sm) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) x = fmax2(x, __shfl_xor_sync(0xffffffffu, x, o));
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  __syncthreads();
-  if (l == 0) sm[w] = x;
-  __syncthreads();
-  double r = kZero;
-  if (threadIdx.x == 0) {
-    r = sm[0];
-    for (int i = 1; i < NT / 32; i++) r = fmax2(r, sm[i]);
-  }
-  return r;
-}
-template <int NT>
 __device__ __forceinline__ double block_min(double x, double* sm) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) x = fmin2(x, __shfl_xor_sync(0xffffffffu, x, o));
@@ -366,8 +336,7 @@ __device__ __forceinline__ double block_min(double x, double* sm) {
 }
 
 // The five iteration reductions in one pass: sums of st, sb, tm, the max of rm and the
-// min of dt, each by the same xor-shuffle tree and the same serial warp order as
-// block_sum / block_max / block_min (so the same bits), with one barrier.
+// min of dt, each by an xor-shuffle tree and a serial pass over the warps, with one barrier.
 template <int NT>
 __device__ __forceinline__ void block_reduce5(double st, double sb, double tm, double rm, double dt, double* sm,
                                               double* out, size_t os = 1) {
@@ -1009,16 +978,16 @@ __device__ __forceinline__ double local_dt(const Dev& d, const Rec& own, bool dr
 // nothing reads (a gradient that hgradfix2 replaces, a dry cell's velocities).  The cells
 // whose stencil is their three face neighbours in slot order (HostLayout::plain) take
 // their constants from one bulk copy per warp.
-// The other cells (along the mesh boundary, with longer stencils) have blocks of their
-// own, the first of the grid: a warp that held one of them would take several times as
-// long as its neighbours.
+// The other cells (along the mesh boundary, with longer stencils) have a launch of their own
+// (kGen, on the side stream beside this one): a warp that held one of them would take
+// several times as long as its neighbours.
 //
-// What bounds it is latency: about 1,100 instructions a warp, a third of them FP64, on
-// data two dependent loads away.  80 registers and 24 warps an SM without spills beat 40
-// warps that spill (the spills were more L2 traffic than the mesh).  Two-million-cell
-// meander, per stage: 156 us with the constants read column by column, the boundary
-// cells among the others and 48 registers; 116 us as it stands (98 us before the
-// boundary cells' launch, which the graph runs beside it).
+// What bounds it is latency: about 950 thread instructions a cell, a third of them FP64, on
+// data two dependent loads away.  80 registers, which allow 24 warps an SM (20 are there on
+// average), without spills beat 40 warps that spill (the spills were more L2 traffic than the
+// mesh).  Two-million-cell meander, by itself per stage: 156 us with the constants read column
+// by column, the boundary cells among the others and 48 registers; 106 us now, and 13 us for
+// the boundary cells' launch beside it.
 // Two passes over the neighbours, the second reading them again from L1: the registers
 // of one pass do not have to live through the other, so nothing is spilled.
 #define PHASE_BARRIER() asm volatile("" ::: "memory")
@@ -2272,7 +2241,7 @@ __global__ void __launch_bounds__(kThreads, kThreads == 256 ? 4 : 1) k_cell(cons
   CellSmem<R>& S = *reinterpret_cast<CellSmem<R>*>(cell_smem);
   double* s_w = reinterpret_cast<double*>(cell_smem + sizeof(CellSmem<R>));  // [3][cnw_max]
   R* s_f = reinterpret_cast<R*>(s_w + 3 * d.cnw_max);                         // [3][cne_max]
-  const int t = blockIdx.x, tid = threadIdx.x, c0 = t * 256, c = c0 + tid, T = d.T;
+  const int t = blockIdx.x, tid = threadIdx.x, c0 = t * 256, c = c0 + tid;
   const int4 i0 = reinterpret_cast<const int4*>(d.ct + t)[0], i1 = reinterpret_cast<const int4*>(d.ct + t)[1];
   const int sid = d.nscen == 1 ? 0 : d.cell_sid[c0];  // a block never spans two scenarios
   if (d.sc[sid].converged) return;
@@ -2544,8 +2513,8 @@ __global__ void __launch_bounds__(kBcThreads) k_bc_flux(Dev d, Geo<R> G, int s, 
 //      (edge_flux); the fluxes the boundary cells' update needs go to global memory;
 //   D  the ordered face gather, sources and SSP-RK update of every owned cell
 //      without an open-boundary face (assemble_phi + rk_update).
-// The boundary cells keep the phase path: their gradients (k_grad over the
-// boundary-cell list) and k_bc run on the side stream beside this kernel, and
+// The boundary cells keep kernels of their own: their gradients (k_grad_bc) and
+// k_bc run on the side stream beside this kernel, and
 // k_flux_bc updates them afterwards.  Velocities ping-pong between two buffers: a
 // tile may still read a neighbour's stage-input velocity while the neighbour's own
 // tile writes its new one.
@@ -2898,7 +2867,10 @@ __global__ void __launch_bounds__(kFinalThreads) k_final(Dev d) {
       a4 = fmin2(a4, r[k][4]);
     }
   }
-  {  // the cells with an open-boundary face are not in the blocks' partials
+  {  // The cells with an open-boundary face, whose friction step runs beside k_cell, are not
+    // in the blocks' partials and come last.  A sum in this order may differ in its last bits
+    // (some 1e-16 of it) from one in cell order, and with it rms and tmass; on a steady run so
+    // may the iteration at which the stop test falls on its very limit.
     const size_t n = d.nbc_cells;
     for (int i = sc->bc_off + threadIdx.x; i < sc->bc_off + sc->bc_cnt; i += kFinalThreads) {
       a0 = a0 + d.bcpart[i];

@@ -181,9 +181,6 @@ __device__ __forceinline__ void tma_store(const CUtensorMap* map, int x, int y, 
 // The thread's stores have read their shared memory / are complete.
 __device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 __device__ __forceinline__ void tma_store_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-__device__ __forceinline__ void tma_prefetch_map(const CUtensorMap* map) {
-  asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
-}
 // Programmatic dependent launch.  wait: every kernel before this one in the stream has ended
 // and its writes are visible; before it a kernel touches no global memory.  launch: the next
 // kernel's blocks may take what this grid leaves free (they wait as well before they read).

@@ -35,6 +35,7 @@ EXPORTS = (
     "storm_fvt_iter_fric", "storm_fvt_iter_finish", "storm_fvt_pack_halo", "storm_fvt_unpack_halo",
 )
 
+# storm_fvt_kernel_times' classes ("eflux": none any more, always zero)
 KERNEL_CLASSES = ("node", "grad", "bc", "flux", "fric", "final", "eflux", "tile")
 STAGE_PHASES, STAGE_FUSED, STAGE_FUSED_NODE_KERNEL = 0, 1, 2
 
@@ -240,7 +241,9 @@ class Solver:
         return {"step_ms": a.value, "flux_ms": b.value, "flux_launches": n.value}
 
     def autotune(self, iters: int = 2) -> dict:
-        """Pick block sizes by timing (state restored afterwards)."""
+        """Pick the stage path and the block sizes of k_node and k_grad by timing (state
+        restored afterwards).  "eflux" and "flux" both give the cell slots of a k_cell
+        block, which is not tuned."""
         ch = np.zeros(4, dtype=np.int32)
         _chk(lib().storm_fvt_autotune(self._h, int(iters), abi.iptr(ch)))
         return dict(zip(("node", "grad", "eflux", "flux"), ch.tolist()))
