@@ -24,6 +24,16 @@ struct alignas(32) Rec {
   double h, z, u, v;
 };
 
+// find_dry_cells.f90:25-42 of a record (h, u, v)
+__host__ __device__ inline bool rec_dry(double h_dry, double h_wet, const Rec& r) {
+  if (r.h < h_dry) return true;
+  if (!(r.h < h_wet)) return false;
+  // equals(sqrt(s), 0): true for a zero, and (its comparison being negated) for an
+  // infinite or NaN speed
+  const double s = r.u * r.u + r.v * r.v;
+  return !(s > 0.0 && s <= 1.7976931348623157e+308);
+}
+
 // k_cell's work list: for every block of 256 cell slots the interior edges whose smaller
 // slot is in it (a contiguous range), those whose larger one is (listed), and its walls.
 struct CellTile {

@@ -79,15 +79,7 @@ __device__ __forceinline__ void st_rec(Rec* p, const Rec& r) {
   *(reinterpret_cast<double2*>(p) + 1) = make_double2(r.u, r.v);
 }
 
-// find_dry_cells.f90:25-42 of a cell's record
-__device__ __forceinline__ bool rec_dry(const Dev& d, const Rec& r) {
-  if (r.h < d.h_dry) return true;
-  if (!(r.h < d.h_wet)) return false;
-  // equals(sqrt(s), 0): true for a zero, and (its comparison being negated) for an
-  // infinite or NaN speed
-  const double s = r.u * r.u + r.v * r.v;
-  return !(s > kZero && s <= kVlarge);
-}
+__device__ __forceinline__ bool rec_dry(const Dev& d, const Rec& r) { return rec_dry(d.h_dry, d.h_wet, r); }
 
 // Whether cell slot c (node n, edge e) belongs to a scenario that is still running.
 // A one-scenario handle answers from the slot number and one flag shared by every
