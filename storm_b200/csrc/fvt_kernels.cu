@@ -1600,10 +1600,11 @@ struct EdgeState {
 
 // invisc_fluxes.f90:39-147 for an interior edge from its two face states: left =
 // e(1), right = e(2), dl/dr their dry flags, zl/zr their bed elevations and cl/cr
-// their cells' celerities (Rusanov; zero when dry); returns false when the edge is
+// their cells' celerities (Rusanov; zero when dry) or, kDepth, the cells' depths, whose
+// celerities are then taken where a flux needs them; returns false when the edge is
 // skipped.  The wet/dry tests and the I1 stage comparison run on the FP64 face
 // states; the flux function in R.
-template <class R>
+template <class R, bool kDepth = false>
 __device__ __forceinline__ bool edge_flux(const Dev& d, bool dl, bool dr, const EdgeState& sl, const EdgeState& sr,
                                           double zl, double zr, double cl, double cr, R nx, R ny, double z0e, R* f,
                                           bool* bad) {
@@ -1633,6 +1634,10 @@ __device__ __forceinline__ bool edge_flux(const Dev& d, bool dl, bool dr, const 
   } else if (d.flux == STORM_FLUX_HLL) {
     flux_hll<R>(nx, ny, (R)hleft, (R)uleft, (R)vleft, (R)hright, (R)uright, (R)vright, (R)d.h_dry, f, bad);
   } else if (d.flux == STORM_FLUX_RUSANOV) {
+    if (kDepth) {  // wavec (solverFVT.f90:180-181)
+      cl = dl ? kZero : sqrt(kG * cl);
+      cr = dr ? kZero : sqrt(kG * cr);
+    }
     flux_rusanov<R>(nx, ny, (R)hleft, (R)uleft, (R)vleft, (R)cl, (R)hright, (R)uright, (R)vright, (R)cr, f);
   } else {
     flux_roe_edge(nx, ny, (R)hleft, (R)uleft, (R)vleft, (R)hright, (R)uright, (R)vright, f);
@@ -2702,11 +2707,9 @@ __global__ void __launch_bounds__(kTileThreads, 3)
       const bool dl = s_dry[a], dr = s_dry[b];
       const EdgeState fa{s_fh[ml * ngm + a], s_fu[ml * ngm + a], s_fv[ml * ngm + a]};
       const EdgeState fb{s_fh[mr * ngm + b], s_fu[mr * ngm + b], s_fv[mr * ngm + b]};
-      const bool rus = d.flux == STORM_FLUX_RUSANOV;
-      const auto cel = [&](bool dr_, double h_) { return rus && !dr_ ? sqrt(kG * h_) : kZero; };
       R f[3];
       bool bad = false;
-      ok = edge_flux<R>(d, dl, dr, fa, fb, s_z[a], s_z[b], cel(dl, s_h[a]), cel(dr, s_h[b]), G.enx[e], G.eny[e],
+      ok = edge_flux<R, true>(d, dl, dr, fa, fb, s_z[a], s_z[b], s_h[a], s_h[b], G.enx[e], G.eny[e],
                         (dl || dr) ? d.ez0[e] : kZero, f, &bad);
       if (ok) {
         const R len = G.elen[e];
