@@ -1,6 +1,7 @@
 """Creating a handle while the host runs out of memory: whichever of its large allocations
 fails, the call returns an error (nothing leaves the C entry), and the next call succeeds."""
 import os
+import shutil
 import subprocess
 import sys
 
@@ -54,6 +55,7 @@ print("refused", k - 1)
 """
 
 
+@pytest.mark.skipif(not shutil.which("g++"), reason="compiles its hook: needs g++")
 @pytest.mark.parametrize("precision", [0, 1])
 def test_every_large_allocation(precision, tmp_path, storm_lib):
     (tmp_path / "hook.cpp").write_text(HOOK)

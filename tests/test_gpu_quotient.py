@@ -4,6 +4,7 @@ ends of the range of exponents, significands of all ones, zeros, infinities and 
 they cannot answer they must say (`bad`), and nothing else."""
 import ctypes
 import os
+import shutil
 import subprocess
 
 import numpy as np
@@ -69,6 +70,8 @@ extern "C" __attribute__((visibility("default"))) int lim(const double* f, int n
 
 @pytest.fixture(scope="module")
 def probe(tmp_path_factory):
+    if not shutil.which(build.nvcc()):
+        pytest.skip("compiles its probe: needs nvcc")
     d = tmp_path_factory.mktemp("quotient")
     (d / "probe.cu").write_text(SRC)
     subprocess.run([build.nvcc(), *build.NVCC_FLAGS, "-I", build.CSRC, "-shared", "-o", str(d / "probe.so"),
